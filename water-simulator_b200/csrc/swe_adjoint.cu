@@ -696,6 +696,7 @@ struct swe_adjoint {
   cudaStream_t st = nullptr;
   std::vector<double*> allocs;
   double *b, *eta0, *nfield = nullptr, *geom;
+  int tame = 0;                                           // swe_split.cuh, tame_ok
   double *A[3], *Bf[3], *X[3];                            // state, stage-1 output, segment state
   double *ckpt, *tape;                                    // checkpoints, one segment's tapes
   double *dts, *obs = nullptr, *J, *eta_series = nullptr;
@@ -749,7 +750,8 @@ StageArgs stage_args(const swe_adjoint* s, double* const* in, double* const* out
   a.m.dyCFL = g + SWE_GEOM_DYCFL * H; a.m.bedPhi = g + SWE_GEOM_BEDPHI * H; a.m.geoCoef = g + SWE_GEOM_GEOCOEF * H;
   a.m.fRow = g + SWE_GEOM_FROW * H; a.m.tanPhi = g + SWE_GEOM_TANPHI * H;
   a.m.rdxRow = g + (SWE_GEOM_NROWS + 0) * H; a.m.rdyRowN = g + (SWE_GEOM_NROWS + 1) * H;
-  a.m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * H; a.m.R = INFINITY;
+  a.m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * H; a.m.rbedPhi = g + (SWE_GEOM_NROWS + 3) * H; a.m.R = INFINITY;
+  a.tame = s->tame;
   a.minDepth = s->o.min_depth; a.eps4 = s->eps4; a.coriolis = s->o.coriolis;
   a.sph = 0; a.order = s->o.order; a.lim = s->o.limiter;
   a.manning = s->o.manning; a.nfield = s->nfield;
@@ -1060,7 +1062,7 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
   };
   bool ok = true;
   auto A = [&](size_t n) { double* p = alloc(n); ok = ok && p; return p; };
-  s->b = A(N); s->eta0 = A(N); s->geom = A((SWE_GEOM_NROWS + 3) * (size_t)s->H);
+  s->b = A(N); s->eta0 = A(N); s->geom = A((SWE_GEOM_NROWS + 4) * (size_t)s->H);
   if (manning_field) s->nfield = A(N);
   for (int q = 0; q < 3; q++) {
     s->A[q] = A(N); s->Bf[q] = A(N); s->X[q] = A(N);
@@ -1100,14 +1102,16 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
     const char* pe = std::getenv("SWE_B200_PDL");
     s->pdl = !(pe && std::strcmp(pe, "0") == 0);
   }
-  std::vector<double> geom((size_t)(SWE_GEOM_NROWS + 3) * s->H), sc(6);
+  std::vector<double> geom((size_t)(SWE_GEOM_NROWS + 4) * s->H), sc(6);
   int rc = swe_compute_geometry(o, geom.data(), sc.data());
   if (rc) return bail(rc);
-  for (int r = 0; r < 3; r++) {
-    const int src = r == 0 ? SWE_GEOM_DXROW : r == 1 ? SWE_GEOM_DYROWN : SWE_GEOM_DYROWS;
+  for (int r = 0; r < 4; r++) {
+    const int src = r == 0 ? SWE_GEOM_DXROW : r == 1 ? SWE_GEOM_DYROWN : r == 2 ? SWE_GEOM_DYROWS : SWE_GEOM_BEDPHI;
     for (int j = 0; j < s->H; j++)
       geom[(size_t)(SWE_GEOM_NROWS + r) * s->H + j] = 1.0 / geom[(size_t)src * s->H + j];
   }
+  s->tame = swe::tame_ok(o->min_depth, geom.data() + (size_t)SWE_GEOM_DXROW * s->H,
+                         geom.data() + (size_t)SWE_GEOM_BEDPHI * s->H, s->H);
   cudaMemcpyAsync(s->geom, geom.data(), sizeof(double) * geom.size(), cudaMemcpyHostToDevice, s->st);
   cudaMemcpyAsync(s->b, b, sizeof(double) * N, cudaMemcpyHostToDevice, s->st);
   cudaMemcpyAsync(s->eta0, eta0, sizeof(double) * N, cudaMemcpyHostToDevice, s->st);

@@ -63,8 +63,9 @@ struct swe_sim {
   int nx, ny, W, H, N;
   double dx, dy, eps4, R, dlam, dphi, totalArea;
   std::vector<double> geom[SWE_GEOM_NROWS];
-  std::vector<double> recip[3];
+  std::vector<double> recip[4];
   int dryfold = 0;                                 // every reciprocal row finite
+  int tame = 0;                                    // swe_split.cuh, tame_ok
   cudaStream_t st = nullptr;
   double* d_b = nullptr;
   double* d_A[3] = {nullptr, nullptr, nullptr};
@@ -258,7 +259,7 @@ swe::Metric metric(const swe_sim* s) {
   m.bedPhi = g + SWE_GEOM_BEDPHI * H; m.geoCoef = g + SWE_GEOM_GEOCOEF * H;
   m.fRow = g + SWE_GEOM_FROW * H; m.tanPhi = g + SWE_GEOM_TANPHI * H;
   m.rdxRow = g + (SWE_GEOM_NROWS + 0) * H; m.rdyRowN = g + (SWE_GEOM_NROWS + 1) * H;
-  m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * H;
+  m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * H; m.rbedPhi = g + (SWE_GEOM_NROWS + 3) * H;
   m.R = s->R;
   return m;
 }
@@ -280,6 +281,7 @@ swe::StageArgs stage_args(const swe_sim* s, double* const* in, double* const* ou
   a.part_max = s->d_part; a.part_fl1 = s->d_part + s->part_cap; a.part_fl2 = s->d_part + 2 * s->part_cap;
   a.nblocks = s->nblocks;
   a.dryfold = s->dryfold;
+  a.tame = s->tame;
   return a;
 }
 
@@ -601,15 +603,16 @@ void view_of(swe_sim* s, int* dims, double* opts, const double** b, const double
 
 namespace {
 
-// Reciprocals of the three flux divisors (rows after the 13 metric rows).
+// Reciprocals of the flux divisors and the bed term's (rows after the 13 metric rows).
 void fill_reciprocals(swe_sim* s) {
-  const int src[3] = {SWE_GEOM_DXROW, SWE_GEOM_DYROWN, SWE_GEOM_DYROWS};
-  for (int q = 0; q < 3; q++) {
+  const int src[4] = {SWE_GEOM_DXROW, SWE_GEOM_DYROWN, SWE_GEOM_DYROWS, SWE_GEOM_BEDPHI};
+  for (int q = 0; q < 4; q++) {
     s->recip[q].resize(s->H);
     for (int j = 0; j < s->H; j++) s->recip[q][j] = 1.0 / s->geom[src[q]][j];
   }
   s->dryfold = 1;
   for (int q = 0; q < 3; q++) s->dryfold &= swe::dry_fold_ok(s->recip[q].data(), s->recip[q].size());
+  s->tame = swe::tame_ok(s->o.min_depth, s->geom[SWE_GEOM_DXROW].data(), s->geom[SWE_GEOM_BEDPHI].data(), s->H);
 }
 
 int upload_geom(swe_sim* s) {
@@ -617,7 +620,7 @@ int upload_geom(swe_sim* s) {
   for (int r = 0; r < SWE_GEOM_NROWS; r++)
     CU(cudaMemcpyAsync(s->d_geom + (size_t)r * s->H, s->geom[r].data(), sizeof(double) * s->H,
                        cudaMemcpyHostToDevice, s->st));
-  for (int q = 0; q < 3; q++)
+  for (int q = 0; q < 4; q++)
     CU(cudaMemcpyAsync(s->d_geom + (size_t)(SWE_GEOM_NROWS + q) * s->H, s->recip[q].data(),
                        sizeof(double) * s->H, cudaMemcpyHostToDevice, s->st));
   return SWE_OK;
@@ -709,7 +712,7 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
   CUB(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
   CUB(cudaMalloc(&s->d_b, nb));
   for (int q = 0; q < 3; q++) { CUB(cudaMalloc(&s->d_A[q], nb)); CUB(cudaMalloc(&s->d_B[q], nb)); }
-  CUB(cudaMalloc(&s->d_geom, sizeof(double) * (SWE_GEOM_NROWS + 3) * s->H));
+  CUB(cudaMalloc(&s->d_geom, sizeof(double) * (SWE_GEOM_NROWS + 4) * s->H));
   CUB(cudaMalloc(&s->d_part, sizeof(double) * (3 * s->part_cap + 3 * swe::CLOSE_BLOCKS)));   // + the close's scratch
   CUB(cudaMalloc(&s->d_rows, sizeof(double) * std::max(1, s->ny)));
   CUB(cudaMalloc(&s->d_ctl, sizeof(swe::Control)));
@@ -865,6 +868,7 @@ int swe_set_geom(swe_sim* s, int row, const double* in) {
   if (rc) return rc;
   CU(cudaStreamSynchronize(s->st));
   s->cfl_valid = false;
+  s->version++;                     // the cached graphs hold dryfold and tame
   return SWE_OK;
 }
 

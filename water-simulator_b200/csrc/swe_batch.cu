@@ -452,11 +452,11 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     if (o.limiter < 0 || o.limiter > 2) return bail(fail(SWE_EINVAL, "unknown limiter; have minmod,mc,central"));
     s->W.push_back(o.nx + 4);
     s->H.push_back(o.ny + 4);
-    geom[q].assign((size_t)(SWE_GEOM_NROWS + 3) * s->H[q], 0.0);
+    geom[q].assign((size_t)(SWE_GEOM_NROWS + 4) * s->H[q], 0.0);
     int rc = swe_compute_geometry(&o, geom[q].data(), scal.data());
     if (rc) return bail(rc);
-    for (int r = 0; r < 3; r++) {            // reciprocal rows after the 13 metric rows
-      const int src = r == 0 ? SWE_GEOM_DXROW : r == 1 ? SWE_GEOM_DYROWN : SWE_GEOM_DYROWS;
+    for (int r = 0; r < 4; r++) {            // reciprocal rows after the 13 metric rows
+      const int src = r == 0 ? SWE_GEOM_DXROW : r == 1 ? SWE_GEOM_DYROWN : r == 2 ? SWE_GEOM_DYROWS : SWE_GEOM_BEDPHI;
       for (int j = 0; j < s->H[q]; j++)
         geom[q][(size_t)(SWE_GEOM_NROWS + r) * s->H[q] + j] = 1.0 / geom[q][(size_t)src * s->H[q] + j];
     }
@@ -464,7 +464,7 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     s->off.push_back(total);
     // b, A (3), B (3), the tiled pair's fields, metric rows, partial slots
     // (3 x one per tile, for the most tiles either kernel uses)
-    total += round_up(N) * (7 + swe::SPLIT_FIELDS) + round_up((size_t)(SWE_GEOM_NROWS + 3) * s->H[q]) +
+    total += round_up(N) * (7 + swe::SPLIT_FIELDS) + round_up((size_t)(SWE_GEOM_NROWS + 4) * s->H[q]) +
              round_up(3 * part_slots(s->W[q], s->H[q])) + round_up((split_tiles(s->W[q], s->H[q]) + 1) / 2);
   }
   int ndev = 0;
@@ -492,7 +492,7 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     double* spl = base + 7 * rN;                // the tiled pair's fields
     double* g = base + (7 + swe::SPLIT_FIELDS) * rN;
     const int Hq = s->H[q];
-    double* parts = g + round_up((size_t)(SWE_GEOM_NROWS + 3) * Hq);
+    double* parts = g + round_up((size_t)(SWE_GEOM_NROWS + 4) * Hq);
     const size_t pcap = part_slots(s->W[q], Hq);
     cudaMemcpyAsync(fb, b[q], sizeof(double) * N, cudaMemcpyHostToDevice, s->st);
     cudaMemcpyAsync(A[0], h[q], sizeof(double) * N, cudaMemcpyHostToDevice, s->st);
@@ -507,7 +507,9 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     a.m.bedPhi = g + SWE_GEOM_BEDPHI * Hq; a.m.geoCoef = g + SWE_GEOM_GEOCOEF * Hq;
     a.m.fRow = g + SWE_GEOM_FROW * Hq; a.m.tanPhi = g + SWE_GEOM_TANPHI * Hq;
     a.m.rdxRow = g + (SWE_GEOM_NROWS + 0) * Hq; a.m.rdyRowN = g + (SWE_GEOM_NROWS + 1) * Hq;
-    a.m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * Hq;
+    a.m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * Hq; a.m.rbedPhi = g + (SWE_GEOM_NROWS + 3) * Hq;
+    a.tame = swe::tame_ok(o.min_depth, geom[q].data() + (size_t)SWE_GEOM_DXROW * Hq,
+                          geom[q].data() + (size_t)SWE_GEOM_BEDPHI * Hq, Hq);
     a.dryfold = swe::dry_fold_ok(geom[q].data() + (size_t)SWE_GEOM_NROWS * Hq, (size_t)3 * Hq);
     double Rv = 0;
     {

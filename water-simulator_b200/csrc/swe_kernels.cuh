@@ -73,6 +73,7 @@ struct Metric {   // per-row divisors (src/geometry.mjs)
   // 1/dxRow, 1/dyRowN, 1/dyRowS, formed on the host with the same IEEE
   // division, so theta/dxRow == rdxRow exactly when theta == 1
   const double* rdxRow; const double* rdyRowN; const double* rdyRowS;
+  const double* rbedPhi;                                     // 1/bedPhi, likewise
   double R;
 };
 
@@ -105,6 +106,9 @@ struct StageArgs {
   // every reciprocal metric row (rdxRow, rdyRowN, rdyRowS) finite, so a
   // face value of +0 times any of them is +0
   int dryfold;
+  // minDepth and the divisors of the source terms in the range of the tame
+  // face arithmetic (swe_math.cuh)
+  int tame;
 };
 
 // ---------------------------------------------------------------------------

@@ -38,6 +38,7 @@
 #pragma once
 
 #include <cuda.h>                 // CUtensorMap
+#include <cmath>
 
 #include "swe_kernels.cuh"
 
@@ -95,6 +96,16 @@ __host__ __forceinline__ SplitBufs split_bufs_at(double* base, size_t stride) {
   return b;
 }
 
+// Whether the tame face arithmetic (swe_math.cuh) covers a grid: its minDepth
+// and, over its interior rows, the divisors dxRow and bedPhi.
+__host__ inline int tame_ok(double min_depth, const double* dx_row, const double* bed_phi, int H) {
+  const double lo = std::ldexp(1.0, -60), hi = std::ldexp(1.0, 60);
+  if (!(min_depth >= lo && min_depth < 1048576.0)) return 0;
+  for (int j = 2; j < H - 2; j++)
+    if (!(dx_row[j] >= lo && dx_row[j] < hi && bed_phi[j] >= lo && bed_phi[j] < hi)) return 0;
+  return 1;
+}
+
 // Whether `n` reciprocal metric values are all finite (StageArgs::dryfold).
 __host__ inline int dry_fold_ok(const double* recip, size_t n) {
   for (size_t q = 0; q < n; q++)
@@ -127,8 +138,11 @@ struct FacesSmem {
   double ys[4][SPY + 1][SPX];                   // y slopes of cols i0 .. i0+SPX-1, rows j0 .. j0+SPY
 };
 
-// One cell of a faces tile: its source terms, its east x face and north y face.
-__device__ __forceinline__ void split_faces_cell(const StageArgs& a, const SplitBufs& s, const FacesSmem& sm,
+// One cell of a faces tile: its source terms, its east x face and north y
+// face.  TAME: every cell of the tile's box is tame; returns whether a face
+// must be formed again without.
+template <bool TAME>
+__device__ __forceinline__ bool split_faces_cell(const StageArgs& a, const SplitBufs& s, const FacesSmem& sm,
                                                  int lx, int ly, int gi, int gj, bool sph, bool bedOn) {
   const int W = a.W, H = a.H;
   const double dry = a.minDepth;
@@ -143,14 +157,28 @@ __device__ __forceinline__ void split_faces_cell(const StageArgs& a, const Split
   if (bedOn && gj >= 2 && gj < H - 2 && gi >= 2 && gi < W - 2) {
     const double eC = bk + hk;
     {
-      const double hP = jmax0(eC + 0.5 * xsE - (bk + 0.5 * xsB));
-      const double hM = jmax0(eC - 0.5 * xsE - (bk - 0.5 * xsB));
-      tb0 = div_unless_zero(-SWE_G * 0.5 * (hP + hM) * xsB, xsB, a.m.dxRow[gj]);
+      double hP, hM;
+      if (TAME) {
+        hP = pos(fma(0.5, xsE, eC) - fma(0.5, xsB, bk));
+        hM = pos(fma(-0.5, xsE, eC) - fma(-0.5, xsB, bk));
+      } else {
+        hP = jmax0(eC + 0.5 * xsE - (bk + 0.5 * xsB));
+        hM = jmax0(eC - 0.5 * xsE - (bk - 0.5 * xsB));
+      }
+      const double n = -SWE_G * 0.5 * (hP + hM) * xsB;
+      tb0 = TAME ? div_tame(n, a.m.dxRow[gj], a.m.rdxRow[gj]) : div_unless_zero(n, xsB, a.m.dxRow[gj]);
     }
     {
-      const double hP = jmax0(eC + 0.5 * nsE - (bk + 0.5 * nsB));
-      const double hM = jmax0(eC - 0.5 * nsE - (bk - 0.5 * nsB));
-      tb1 = div_unless_zero(-SWE_G * 0.5 * (hP + hM) * nsB, nsB, a.m.bedPhi[gj]);
+      double hP, hM;
+      if (TAME) {
+        hP = pos(fma(0.5, nsE, eC) - fma(0.5, nsB, bk));
+        hM = pos(fma(-0.5, nsE, eC) - fma(-0.5, nsB, bk));
+      } else {
+        hP = jmax0(eC + 0.5 * nsE - (bk + 0.5 * nsB));
+        hM = jmax0(eC - 0.5 * nsE - (bk - 0.5 * nsB));
+      }
+      const double n = -SWE_G * 0.5 * (hP + hM) * nsB;
+      tb1 = TAME ? div_tame(n, a.m.bedPhi[gj], a.m.rbedPhi[gj]) : div_unless_zero(n, nsB, a.m.bedPhi[gj]);
       if (sph) tg = a.m.geoCoef[gj] * SWE_G * (hP * hP + hM * hM);
     }
   }
@@ -164,11 +192,15 @@ __device__ __forceinline__ void split_faces_cell(const StageArgs& a, const Split
   }
 
   // The east x face (k|k+1), then the north y face (k|k+W; v normal, u
-  // transverse), through one copy of the face solve: a loop of two passes
-  // that is not unrolled, so that the solve, the bulk of the kernel's code,
-  // sits in the instruction cache once.
+  // transverse).  The solve with the operators is the bulk of that kernel's
+  // code, so it is kept once, in a loop that is not unrolled, for the
+  // instruction cache.  The tame solve is a third of its size and is unrolled:
+  // the selects between the two directions go (all-wet 2048 x 2048, 128 steps:
+  // 117.9 -> 115.8 ms).
   constexpr int XS = SPY * (SPX + 1), YS = (SPY + 1) * SPX;   // strides of xs[q], ys[q]
-#pragma unroll 1
+  bool again = false;
+  constexpr int UNROLL = TAME ? 2 : 1;
+#pragma unroll UNROLL
   for (int d = 0; d < 2; d++) {
     const bool on = d == 0 ? (gj >= 2 && gj < H - 2 && gi >= 1 && gi < W - 2)
                            : (gj >= 1 && gj < H - 2 && gi >= 2 && gi < W - 2);
@@ -176,16 +208,25 @@ __device__ __forceinline__ void split_faces_cell(const StageArgs& a, const Split
     const int fs = d == 0 ? XS : YS, no = d == 0 ? 1 : SPX;       // field stride, the neighbour's offset
     const int qn = d == 0 ? 2 : 3, qt = 5 - qn;                  // normal and transverse velocity slopes
     const int ry = d == 0 ? cy : cy + 1, rx = d == 0 ? cx + 1 : cx;
-    Face f = {0, 0, 0, 0, 0};
+    FaceSums f = {0, 0, 0, 0};
     if (on) {
-      f = face_flux(bk, hk, d == 0 ? Uk : Vk, d == 0 ? Vk : Uk, sp[0], sp[fs], sp[qn * fs], sp[qt * fs],
-                    sm.b[ry][rx], sm.h[ry][rx], d == 0 ? sm.U[ry][rx] : sm.V[ry][rx],
-                    d == 0 ? sm.V[ry][rx] : sm.U[ry][rx],
-                    sp[no], sp[fs + no], sp[qn * fs + no], sp[qt * fs + no], dry);
+      const double nl = d == 0 ? Uk : Vk, tl = d == 0 ? Vk : Uk;
+      const double nr = d == 0 ? sm.U[ry][rx] : sm.V[ry][rx], tr = d == 0 ? sm.V[ry][rx] : sm.U[ry][rx];
+      if (TAME) {
+        bool redo;
+        f = face_flux_tame(bk, hk, nl, tl, sp[0], sp[fs], sp[qn * fs], sp[qt * fs], sm.b[ry][rx], sm.h[ry][rx], nr,
+                           tr, sp[no], sp[fs + no], sp[qn * fs + no], sp[qt * fs + no], dry, redo);
+        again |= redo;
+      } else {
+        const Face g = face_flux(bk, hk, nl, tl, sp[0], sp[fs], sp[qn * fs], sp[qt * fs], sm.b[ry][rx],
+                                 sm.h[ry][rx], nr, tr, sp[no], sp[fs + no], sp[qn * fs + no], sp[qt * fs + no], dry);
+        f = {g.M, g.T, g.N + g.pL, g.N + g.pR};
+      }
     }
     double* const* o = d == 0 ? s.fx : s.fy;
-    o[F_M][k] = f.M; o[F_T][k] = f.T; o[F_NPL][k] = f.N + f.pL; o[F_NPR][k] = f.N + f.pR;
+    o[F_M][k] = f.M; o[F_T][k] = f.T; o[F_NPL][k] = f.NpL; o[F_NPR][k] = f.NpR;
   }
+  return again;
 }
 
 __device__ __forceinline__ void split_faces_finish(const StageArgs& a, const SplitBufs& s, int tx, int ty,
@@ -244,74 +285,39 @@ __device__ __forceinline__ void split_faces_tile(const StageArgs& a, const Split
 // Limited slopes of eta, b, u, v at the state-tile cell (cy, cx) along x
 // (DX = 1) or y (DX = 0), src/swe.mjs:364-411: all four are 0 unless `on`
 // and the cell and both neighbours along the direction are wet.  LIM 0 is
-// the MC limiter inline; LIM -1 the options' limiter chosen at run time.
+// the MC limiter of tame cells inline; LIM -1 the options' limiter chosen at
+// run time.
 // out[q * stride]: the slopes of eta, b, u, v in turn (each stored as soon
 // as it is formed).
 template <int DX, int LIM>
 __device__ __forceinline__ void tile_slopes(const FacesSmem& sm, int lim, double dry, bool on, int cy, int cx,
                                             double* out, int stride) {
   constexpr int DY = 1 - DX;
-  const int l = LIM < 0 ? lim : LIM;
+  const auto limit = [lim](double p, double q) { return LIM == 0 ? limiter_mc_tame(p, q) : limiter(lim, p, q); };
   double sE = 0, sB = 0, sU = 0, sV = 0;
   if (on) {
     const double hk = sm.h[cy][cx], hp = sm.h[cy + DY][cx + DX], hm = sm.h[cy - DY][cx - DX];
     if (!(hk <= dry || hp <= dry || hm <= dry)) {
       const double bk = sm.b[cy][cx], bp = sm.b[cy + DY][cx + DX], bm = sm.b[cy - DY][cx - DX];
-      sE = limiter(l, (bk + hk) - (bm + hm), (bp + hp) - (bk + hk));
-      sB = limiter(l, bk - bm, bp - bk);
+      sE = limit((bk + hk) - (bm + hm), (bp + hp) - (bk + hk));
+      sB = limit(bk - bm, bp - bk);
       const double uk = sm.U[cy][cx];
-      sU = limiter(l, uk - sm.U[cy - DY][cx - DX], sm.U[cy + DY][cx + DX] - uk);
+      sU = limit(uk - sm.U[cy - DY][cx - DX], sm.U[cy + DY][cx + DX] - uk);
       const double vk = sm.V[cy][cx];
-      sV = limiter(l, vk - sm.V[cy - DY][cx - DX], sm.V[cy + DY][cx + DX] - vk);
+      sV = limit(vk - sm.V[cy - DY][cx - DX], sm.V[cy + DY][cx + DX] - vk);
     }
   }
   out[0] = sE; out[stride] = sB; out[2 * stride] = sU; out[3 * stride] = sV;
 }
 
-// The rest of a faces tile once its state tile is in shared memory: the
-// dry test, velocities, slopes and faces.  Every thread of the CTA calls it.
+// Slopes of a faces tile (src/swe.mjs:364-411): each thread its own cell in x
+// and y; the east column's x slopes (the first SPY threads) and the north
+// row's y slopes (the second warp) besides.
 template <int LIM>
-__device__ __forceinline__ void split_faces_finish_l(const StageArgs& a, const SplitBufs& s, int tx, int ty,
-                                                     FacesSmem& sm, int t) {
+__device__ __forceinline__ void split_faces_slopes(const StageArgs& a, FacesSmem& sm, int t, int i0, int j0) {
   const int W = a.W, H = a.H;
-  const int i0 = tx * SPX, j0 = ty * SPY;
-  const double dry = a.minDepth, eps4 = a.eps4;
+  const double dry = a.minDepth;
   const bool order2 = a.order >= 2;
-  const bool sph = a.sph != 0;
-  const bool bedOn = order2 || sph;
-  int dryHere = 1;
-  for (int q = t; q < SSX * SSY; q += SP_THREADS) {
-    const int ly = q / SSX, lx = q - ly * SSX;
-    if (!(sm.h[ly][lx + TCOL] == 0)) dryHere = 0;     // zero outside the grid
-  }
-  const bool allDry = __syncthreads_and(dryHere) && s.dry && !s.sl[0];
-  if (s.dry && t == 0) s.dry[ty * s.ntx + tx] = allDry ? 1 : 0;
-  if (allDry) return;                           // uniform across the CTA
-  // velocities over the whole box; a cell outside the grid has h = hu =
-  // hv = 0 there and gets u = v = +0, as it would have kept
-  // The box has more cells than the CTA has threads: the second pass goes
-  // to the last threads, since the first two warps take the extra slopes.
-  constexpr int VREM = SSXT * SSY - SP_THREADS;
-  static_assert(VREM > 0 && VREM <= SP_THREADS, "one or two box cells per thread");
-  for (int pass = 0; pass < 2; pass++) {
-    if (pass == 1 && t < SP_THREADS - VREM) break;
-    const int q = pass == 0 ? t : t + VREM;
-    const int ly = q / SSXT, c = q - ly * SSXT;
-    const double h = sm.h[ly][c], hu = sm.U[ly][c], hv = sm.V[ly][c];
-    double U, V;
-    if (h == 0) {                  // +-0 / den == +-0 and NaN / den == NaN: no division needed
-      U = vel_num(hu, h); V = vel_num(hv, h);
-    } else {
-      const double den = vel_den(h, eps4);
-      U = qdiv(vel_num(hu, h), den); V = qdiv(vel_num(hv, h), den);
-    }
-    sm.U[ly][c] = U; sm.V[ly][c] = V;
-  }
-  __syncthreads();
-
-  // slopes (src/swe.mjs:364-411): each thread its own cell in x and y; the
-  // east column's x slopes (the first SPY threads) and the north row's y
-  // slopes (the second warp) besides
   const int lx = t % SPX, ly = t / SPX;
   const int gi = i0 + lx, gj = j0 + ly;
   constexpr int XS = SPY * (SPX + 1), YS = (SPY + 1) * SPX;   // strides of xs[q], ys[q]
@@ -330,16 +336,66 @@ __device__ __forceinline__ void split_faces_finish_l(const StageArgs& a, const S
     const bool on = order2 && nj >= 1 && nj < H - 1 && ni >= 1 && ni < W - 1;
     tile_slopes<0, LIM>(sm, a.lim, dry, on, SPY + 1, c + 1 + TCOL, &sm.ys[0][SPY][c], YS);
   }
-  __syncthreads();
-
-  if (gi < W && gj < H) split_faces_cell(a, s, sm, lx, ly, gi, gj, sph, bedOn);
-  __syncthreads();
 }
 
+// The rest of a faces tile once its state tile is in shared memory: the
+// dry test, velocities, slopes and faces.  Every thread of the CTA calls it.
+// Whether the box is tame (swe_math.cuh) is voted at the barrier after the
+// velocities; a tile that is not, or one of whose faces met a divisor the
+// tame solve leaves out, is solved with the operators.
 __device__ __forceinline__ void split_faces_finish(const StageArgs& a, const SplitBufs& s, int tx, int ty,
                                                    FacesSmem& sm, int t) {
-  if (a.lim == 0) split_faces_finish_l<0>(a, s, tx, ty, sm, t);    // mc, the default
-  else split_faces_finish_l<-1>(a, s, tx, ty, sm, t);
+  const int W = a.W, H = a.H;
+  const int i0 = tx * SPX, j0 = ty * SPY;
+  const double eps4 = a.eps4;
+  const bool sph = a.sph != 0;
+  const bool bedOn = a.order >= 2 || sph;
+  int dryHere = 1;
+  for (int q = t; q < SSX * SSY; q += SP_THREADS) {
+    const int ly = q / SSX, lx = q - ly * SSX;
+    if (!(sm.h[ly][lx + TCOL] == 0)) dryHere = 0;     // zero outside the grid
+  }
+  const bool allDry = __syncthreads_and(dryHere) && s.dry && !s.sl[0];
+  if (s.dry && t == 0) s.dry[ty * s.ntx + tx] = allDry ? 1 : 0;
+  if (allDry) return;                           // uniform across the CTA
+  // velocities over the whole box; a cell outside the grid has h = hu =
+  // hv = 0 there and gets u = v = +0, as it would have kept
+  // The box has more cells than the CTA has threads: the second pass goes
+  // to the last threads, since the first two warps take the extra slopes.
+  constexpr int VREM = SSXT * SSY - SP_THREADS;
+  static_assert(VREM > 0 && VREM <= SP_THREADS, "one or two box cells per thread");
+  bool tame = a.tame != 0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    if (pass == 1 && t < SP_THREADS - VREM) break;
+    const int q = pass == 0 ? t : t + VREM;
+    const int ly = q / SSXT, c = q - ly * SSXT;
+    const double h = sm.h[ly][c], hu = sm.U[ly][c], hv = sm.V[ly][c];
+    const bool cell = tame_cell(sm.b[ly][c], h, hu, hv);
+    tame = tame && cell;
+    double U, V;
+    if (h == 0) {                  // +-0 / den == +-0 and NaN / den == NaN: no division needed
+      U = vel_num(hu, h); V = vel_num(hv, h);
+    } else if (!(a.tame && cell && vel_tame(hu, hv, h, eps4, U, V))) {
+      const double den = vel_den(h, eps4);
+      U = qdiv(vel_num(hu, h), den); V = qdiv(vel_num(hv, h), den);
+    }
+    sm.U[ly][c] = U; sm.V[ly][c] = V;
+  }
+  tame = __syncthreads_and(tame);
+
+  if (tame && a.lim == 0) split_faces_slopes<0>(a, sm, t, i0, j0);    // mc, the default
+  else split_faces_slopes<-1>(a, sm, t, i0, j0);
+  __syncthreads();
+
+  const int lx = t % SPX, ly = t / SPX;
+  const int gi = i0 + lx, gj = j0 + ly;
+  bool again = !tame;
+  if (tame && gi < W && gj < H) again = split_faces_cell<true>(a, s, sm, lx, ly, gi, gj, sph, bedOn);
+  if (__syncthreads_or(again)) {
+    if (gi < W && gj < H) split_faces_cell<false>(a, s, sm, lx, ly, gi, gj, sph, bedOn);
+    __syncthreads();
+  }
 }
 
 // ---- the state tile by tensor-map copies (TMA) --------------------------------
@@ -422,19 +478,15 @@ __device__ __forceinline__ void split_faces_tile_tma(const StageArgs& a, const S
   split_faces_finish(a, s, tx, ty, sm, t);
 }
 
-// CTAs per SM of the face kernels.  The tensor-map kernel of the stepping
-// loop at 5 (48 registers, 168 / 216 bytes of spills) measured +1.8% on the
-// beach over 4 (64 registers) and the same all-wet; 6 (40 registers) +1.2%.
-// The per-element kernel, which the adjoint's passes use (they also write
-// the slopes and velocities to the tape), stays at 4: at 5 its gradient cost
-// 2% more against an unchanged forward.
+// CTAs per SM of the face kernels: 4, which caps them at 64 registers.  The
+// tame solve has no calls to keep registers across, but two solves in flight:
+// 5 CTAs (48 registers, 248 bytes of spill stores) measured 119.2 ms and 3
+// (80 registers, none) 120.5 ms against 115.8 (112 bytes) for 128 steps of an
+// all-wet 2048 x 2048 grid, and 28.8 and 29.7 against 28.4 on the beach.
 #ifndef SWE_SPLIT_FACES_MIN_BLOCKS
-#define SWE_SPLIT_FACES_MIN_BLOCKS 5
+#define SWE_SPLIT_FACES_MIN_BLOCKS 4
 #endif
-#ifndef SWE_SPLIT_FACES_PLAIN_MIN_BLOCKS
-#define SWE_SPLIT_FACES_PLAIN_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_PLAIN_MIN_BLOCKS)
+__global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_MIN_BLOCKS)
 k_split_faces(StageArgs a, SplitBufs s, Control* ctl) {
   pdl_enter();
   if (ctl->stop) return;
