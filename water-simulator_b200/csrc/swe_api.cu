@@ -75,7 +75,9 @@ struct swe_sim {
   double* d_nfield = nullptr;
   double* d_geom = nullptr;
   double* d_part = nullptr;
+  double* d_red = nullptr;                         // the reductions' partials, behind d_part's (which the stages keep)
   double* d_rows = nullptr;
+  swe::VolChunk* d_vol = nullptr;                  // volume()'s chunks
   double* d_coef = nullptr;                        // weights of swe_eta_projection (ny)
   int diag_order = SWE_DIAG_REFERENCE;
   double* d_sponge = nullptr;
@@ -537,18 +539,19 @@ int enqueue_step(swe_sim* s, int mode, double dt, double t_end, const double* dt
   return launch_stage<2>(s, a2, pdl, listed);
 }
 
-// Blocks of a grid-stride reduction over `cells` cells: one per 256 cells,
-// at most 2368 (16 per SM of a B200), so that the last block's ticket is
-// shared by a few thousand blocks and each thread strides over several cells.
-int reduction_blocks(const swe_sim* s, int cells) {
-  return std::min(s->part_cap, std::min(16 * 148, std::max(1, (cells + 255) / 256)));
+constexpr int REDUCTION_BLOCKS = 16 * 148;
+// The grid of a full-grid reduction (swe_kernels.cuh, for_cells): a block per
+// row and segment, at most 16 per SM of a B200, so that the last block's ticket
+// is shared by a few thousand blocks.
+dim3 reduction_grid(int rows, int cols) {
+  const int segs = std::min(16, (cols + swe::RED_SEG - 1) / swe::RED_SEG);
+  return dim3(std::min(rows, REDUCTION_BLOCKS / segs), segs);
 }
 
 int ensure_cfl(swe_sim* s) {
   if (s->cfl_valid) return SWE_OK;
   swe::StageArgs a = stage_args(s, s->d_A, nullptr);
-  const int nb = reduction_blocks(s, s->nx * s->ny);
-  swe::k_cfl_rate<<<nb, swe::BX, 0, s->st>>>(a, s->d_ctl, s->d_part);
+  swe::k_cfl_rate<<<reduction_grid(s->ny, s->nx), swe::BX, 0, s->st>>>(a, s->d_ctl, s->d_red);
   CU(cudaGetLastError());
   s->cfl_valid = true;
   return SWE_OK;
@@ -634,6 +637,7 @@ void free_all(swe_sim* s) {
                      &s->d_sponge, &s->d_split};
   for (double** p : ptrs) if (*p) { cudaFree(*p); *p = nullptr; }
   if (s->d_ctl) cudaFree(s->d_ctl);
+  if (s->d_vol) cudaFree(s->d_vol);
   if (s->st) cudaStreamDestroy(s->st);
 }
 
@@ -713,11 +717,14 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
   CUB(cudaMalloc(&s->d_b, nb));
   for (int q = 0; q < 3; q++) { CUB(cudaMalloc(&s->d_A[q], nb)); CUB(cudaMalloc(&s->d_B[q], nb)); }
   CUB(cudaMalloc(&s->d_geom, sizeof(double) * (SWE_GEOM_NROWS + 4) * s->H));
-  CUB(cudaMalloc(&s->d_part, sizeof(double) * (3 * s->part_cap + 3 * swe::CLOSE_BLOCKS)));   // + the close's scratch
+  // the tiles' partials, the close's scratch, the reductions' partials
+  const size_t nparts = 3 * (size_t)s->part_cap + 3 * swe::CLOSE_BLOCKS + REDUCTION_BLOCKS;
+  CUB(cudaMalloc(&s->d_part, sizeof(double) * nparts));
+  s->d_red = s->d_part + (nparts - REDUCTION_BLOCKS);
   CUB(cudaMalloc(&s->d_rows, sizeof(double) * std::max(1, s->ny)));
   CUB(cudaMalloc(&s->d_ctl, sizeof(swe::Control)));
   CUB(cudaMemsetAsync(s->d_ctl, 0, sizeof(swe::Control), s->st));
-  CUB(cudaMemsetAsync(s->d_part, 0, sizeof(double) * (3 * s->part_cap + 3 * swe::CLOSE_BLOCKS), s->st));
+  CUB(cudaMemsetAsync(s->d_part, 0, sizeof(double) * nparts, s->st));
   for (int q = 0; q < 3; q++) {
     CUB(cudaMemsetAsync(s->d_A[q], 0, nb, s->st));
     CUB(cudaMemsetAsync(s->d_B[q], 0, nb, s->st));
@@ -1183,13 +1190,11 @@ static int finish_diag(swe_sim* s, double* out) {
   return SWE_OK;
 }
 
-// Per-row sums (one warp per row) of `what`, then the rows in order.
+// Per-row sums of `what`, then the rows in order.
 static int row_diag(swe_sim* s, int what, int mode, const double* w, double* out) {
   swe::StageArgs a = stage_args(s, s->d_A, nullptr);
-  swe::k_row_sums<<<(s->ny + swe::ROWSUM_WARPS - 1) / swe::ROWSUM_WARPS, 32 * swe::ROWSUM_WARPS, 0, s->st>>>(
-      a, what, s->d_rows);
-  CU(cudaGetLastError());
-  swe::k_finish_sum<<<1, 1, 0, s->st>>>(s->d_rows, s->ny, mode, w, s->dx, s->dy, s->d_ctl);
+  swe::k_row_sums<<<(s->ny + swe::ROWSUM_ROWS - 1) / swe::ROWSUM_ROWS, swe::ROWSUM_THREADS, 0, s->st>>>(
+      a, what, s->d_rows, mode, w, s->dx, s->dy, s->d_ctl);
   CU(cudaGetLastError());
   return finish_diag(s, out);
 }
@@ -1199,7 +1204,14 @@ int swe_volume(swe_sim* s, double* out) {
   if (s->o.sphere) return row_diag(s, 0, 0, s->d_geom + SWE_GEOM_AREA * s->H + 2, out);
   if (s->diag_order == SWE_DIAG_ROWS) return row_diag(s, 0, 1, nullptr, out);
   swe::StageArgs a = stage_args(s, s->d_A, nullptr);
-  swe::k_volume_chain<<<1, swe::CHAIN_THREADS, 0, s->st>>>(a, s->dx, s->dy, s->d_ctl);
+  const int chunks = (int)(((long long)s->nx * s->ny + swe::VOL_CELLS - 1) / swe::VOL_CELLS);
+  if (chunks > 2) {                 // a smaller grid's sum is all in its first powers of two
+    if (!s->d_vol) CU(cudaMalloc(&s->d_vol, sizeof(swe::VolChunk) * chunks));
+    swe::k_volume_sums<<<chunks, swe::CHAIN_THREADS, 0, s->st>>>(a, s->d_vol, chunks, s->d_ctl);
+    swe::k_volume_runs<<<chunks, swe::CHAIN_THREADS, 0, s->st>>>(a, s->d_vol);
+  }
+  swe::k_volume_walk<<<1, swe::CHAIN_THREADS, 0, s->st>>>(a, chunks > 2 ? s->d_vol : nullptr, chunks, s->dx, s->dy,
+                                                          s->d_ctl);
   CU(cudaGetLastError());
   return finish_diag(s, out);
 }
@@ -1227,9 +1239,7 @@ int swe_eta_projection(swe_sim* s, const double* coef, double* out) {
 
 static int max_diag(swe_sim* s, int what, double ref, double* out) {
   swe::StageArgs a = stage_args(s, s->d_A, nullptr);
-  const int total = what == 2 ? s->N : s->nx * s->ny;
-  const int nb = reduction_blocks(s, total);
-  swe::k_max_diag<<<nb, swe::BX, 0, s->st>>>(a, what, ref, s->d_part, s->d_ctl);
+  swe::k_max_diag<<<what == 2 ? reduction_grid(s->H, s->W) : reduction_grid(s->ny, s->nx), swe::BX, 0, s->st>>>(a, what, ref, s->d_red, s->d_ctl);
   CU(cudaGetLastError());
   return finish_diag(s, out);
 }

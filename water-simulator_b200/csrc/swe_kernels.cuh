@@ -723,36 +723,54 @@ __device__ __forceinline__ double combine_parts(const double* part, int n, bool 
   return mm;
 }
 
+// The full-grid reductions walk the grid row by row, block (x, y) taking the
+// segments y, y + gridDim.y, ... of RED_SEG columns of the rows x, x +
+// gridDim.x, ... (a division per cell for its row had taken a third of the
+// work of the cheaper ones).
+constexpr int RED_SEG = 8 * BX;
+template <class F>
+__device__ __forceinline__ void for_cells(int j0, int j1, int i0, int i1, F f) {
+  for (int j = j0 + blockIdx.x; j < j1; j += gridDim.x)
+    for (int s = i0 + blockIdx.y * RED_SEG; s < i1; s += gridDim.y * RED_SEG)
+      for (int i = s + threadIdx.x; i < min(s + RED_SEG, i1); i += BX) f(j, i);
+}
+
+// Both velocities of a cell, branch-free where it is tame.
+__device__ __forceinline__ void cell_vel(const StageArgs& a, double h, double hu, double hv, double& u, double& v) {
+  if (tame_cell(0, h, hu, hv) && vel_tame(hu, hv, h, a.eps4, u, v)) return;
+  const double den = vel_den(h, a.eps4);
+  u = qdiv(vel_num(hu, h), den); v = qdiv(vel_num(hv, h), den);
+}
+
 // CFL rate max over wet interior cells (src/swe.mjs:632-647) -> ctl->next_max.
-__global__ void k_cfl_rate(StageArgs a, Control* ctl, double* part) {
+__global__ void __launch_bounds__(BX) k_cfl_rate(StageArgs a, Control* ctl, double* part) {
   __shared__ double s[BX / 32];
   __shared__ bool s_last;
   double m = 0;
-  const int nx = a.nx, ny = a.ny, W = a.W;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nx * ny; q += gridDim.x * blockDim.x) {
-    const int j = q / nx + 2, i = q % nx + 2, k = j * W + i;
-    const double hk = a.h[k];
-    if (hk <= a.minDepth) continue;
+  for_cells(2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
+    const size_t k = (size_t)j * a.W + i;
+    const double hk = a.h[k], huk = a.hu[k], hvk = a.hv[k];
+    if (hk <= a.minDepth) return;
     const double cc = sqrt(SWE_G * hk);
-    const double den = vel_den(hk, a.eps4);
-    const double u = fabs(qdiv(vel_num(a.hu[k], hk), den)), v = fabs(qdiv(vel_num(a.hv[k], hk), den));
-    const double sr = (u + cc) / a.m.dxRow[j] + (v + cc) / a.m.dyCFL[j];
+    double u, v;
+    cell_vel(a, hk, huk, hvk, u, v);
+    const double sr = (fabs(u) + cc) / a.m.dxRow[j] + (fabs(v) + cc) / a.m.dyCFL[j];
     if (sr > m) m = sr;
-  }
+  });
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = m;
   __syncthreads();
   if (threadIdx.x == 0) {
     double mm = s[0];
     for (int w = 1; w < (int)blockDim.x / 32; w++) mm = fmax(mm, s[w]);
-    part[blockIdx.x] = mm;
+    part[blockIdx.y * gridDim.x + blockIdx.x] = mm;
     __threadfence();
-    s_last = atomicAdd(&ctl->counter, 1u) == gridDim.x - 1;
+    s_last = atomicAdd(&ctl->counter, 1u) == gridDim.x * gridDim.y - 1;
   }
   __syncthreads();
   if (!s_last) return;                            // uniform per block
   __threadfence();
-  const double mm = combine_parts(part, gridDim.x, false, s);
+  const double mm = combine_parts(part, gridDim.x * gridDim.y, false, s);
   if (threadIdx.x == 0) {
     ctl->next_max = mm;
     ctl->counter = 0;
@@ -803,32 +821,259 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_dry_clean(StageArgs a, Contro
 }
 
 // The Cartesian volume() (src/swe.mjs:818-827): one running sum of h over
-// every interior cell in row-major order, then one multiply by dx and dy.
-// The order is the reference's exactly; the chunks of the next iteration are
-// loaded by the whole block while the first thread adds.
-__global__ void __launch_bounds__(CHAIN_THREADS) k_volume_chain(StageArgs a, double dx, double dy, Control* ctl) {
-  __shared__ double buf[2][CHAIN_CELLS];
-  const int n = a.nx * a.ny, t = threadIdx.x;
-  const int chunks = (n + CHAIN_CELLS - 1) / CHAIN_CELLS;
+// every interior cell in row-major order, then one multiply by dx and dy, to
+// the reference's bits.
+//
+// Adding the cells one after the other is a chain of nx * ny dependent
+// additions (11.3 ms for 1536 x 1024 cells, one thread at work).  The chain
+// can be cut because depths are not negative.  While the running sum s stays
+// in one binade it is S ulps, S a whole number, and adding x rounds to
+//   S + floor(x / ulp) + (1 if the rest is over half an ulp, or half and the sum so far odd),
+// which depends on S by its parity alone.  A run of cells is therefore a pair
+// of whole numbers, what it adds to an even S and to an odd one, and two runs
+// compose: VolRun.  k_volume_sums estimates where the sum stands before each
+// chunk of VOL_CELLS cells, k_volume_runs forms the runs of the chunks that
+// stay in one binade by that estimate, and k_volume_walk goes through the
+// chunks in order: a run whose binade is the sum's is applied at once, any
+// other chunk (the sum crosses a power of two some 20 times) is scanned by the
+// block from the exact sum, the 16 cells around a crossing one by one.  What is
+// not a finite depth >= 0 is left to the chain, from its chunk on.
+// 1536 x 1024 cells: 11.3 ms -> 0.11 ms (the sums 14 us, the runs 15, the walk
+// 85, with 35 scans; chunks of 4096 cells gave a walk of 215 us).
+struct VolRun { long long even, odd; };
+__device__ __forceinline__ VolRun vol_then(VolRun a, VolRun b) {        // a, then b
+  constexpr long long CAP = 1ll << 61;            // past a binade's 2^53 the exact count no longer matters
+  return {min(a.even + (a.even & 1 ? b.odd : b.even), CAP), min(a.odd + (a.odd & 1 ? b.even : b.odd), CAP)};
+}
+// One cell x >= 0, scale = 1 / ulp.
+__device__ __forceinline__ VolRun vol_cell(double x, double scale) {
+  const double t = x * scale;                     // exact (a power of two) where it matters
+  if (!(t < 9007199254740992.0)) return {1ll << 53, 1ll << 53};
+  const long long q = (long long)t;
+  const double f = t - (double)q;
+  const long long up = q + (f > 0.5 ? 1 : 0);
+  return {f == 0.5 ? q + (q & 1) : up, f == 0.5 ? q + 1 - (q & 1) : up};
+}
+__device__ __forceinline__ int vol_exp(double s) { return (int)((unsigned long long)__double_as_longlong(s) >> 52); }
+__device__ __forceinline__ double vol_scale(int e) { return __longlong_as_double((long long)(2098 - e) << 52); }
+constexpr int VOL_PER = 4, VOL_CELLS = CHAIN_THREADS * VOL_PER;        // cells per thread and per chunk
+constexpr int VOL_SMEM = VOL_CELLS + VOL_CELLS / VOL_PER;               // a thread's cells, one bank further than its neighbour's
+struct VolChunk { double sum; VolRun run; int exp; int pad; };          // exp: the binade of run; 0: all zero; -1: none
+// f(r, depth) for the cells r * CHAIN_THREADS + threadIdx.x of chunk c (0 past
+// the end), one division for all of a thread's rows.
+template <class F>
+__device__ __forceinline__ void vol_cells(const StageArgs& a, int c, F f) {
+  const long long q = (long long)c * VOL_CELLS + threadIdx.x;
+  int j = (int)(q / a.nx), i = (int)(q - (long long)j * a.nx);
+  const int dj = CHAIN_THREADS / a.nx, di = CHAIN_THREADS - dj * a.nx;
+  double x[VOL_PER];
+  for (int r = 0; r < VOL_PER; r++) {
+    x[r] = j < a.ny ? a.h[(size_t)(j + 2) * a.W + i + 2] : 0.0;
+    j += dj;
+    i += di;
+    if (i >= a.nx) { i -= a.nx; j++; }
+  }
+  for (int r = 0; r < VOL_PER; r++) f(r, x[r]);
+}
+// The cells of chunk c in shared memory, thread by thread in order.
+__device__ __forceinline__ void vol_load(const StageArgs& a, int c, double* buf) {
+  vol_cells(a, c, [&](int r, double x) {
+    const int i = r * CHAIN_THREADS + threadIdx.x;
+    buf[i + i / VOL_PER] = x;
+  });
+  __syncthreads();
+}
+__device__ __forceinline__ VolRun vol_shfl(VolRun r, int from) {
+  return {__shfl_sync(0xffffffffu, r.even, from), __shfl_sync(0xffffffffu, r.odd, from)};
+}
+// The runs of the block's threads up to and including this one.
+__device__ __forceinline__ VolRun vol_scan(VolRun r, VolRun* warps) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int o = 1; o < 32; o <<= 1) {
+    const VolRun p = vol_shfl(r, max(lane - o, 0));
+    if (lane >= o) r = vol_then(p, r);
+  }
+  __syncthreads();                                // the last scan's totals have been read
+  if (lane == 31) warps[w] = r;
+  __syncthreads();
+  VolRun before = {0, 0};
+  for (int q = 0; q < w; q++) before = vol_then(before, warps[q]);
+  return vol_then(before, r);
+}
+
+// Each chunk's sum, and by the last block the estimate of the sum before it.
+__global__ void __launch_bounds__(CHAIN_THREADS) k_volume_sums(StageArgs a, VolChunk* ch, int chunks, Control* ctl) {
+  __shared__ double part[CHAIN_THREADS / 32 + 1];
+  __shared__ bool last;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  double v = 0;
+  vol_cells(a, blockIdx.x, [&](int, double x) { v += x; });
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) part[w] = v;
+  __syncthreads();
+  if (t == 0) {
+    for (int q = 1; q < CHAIN_THREADS / 32; q++) v += part[q];
+    ch[blockIdx.x].run.even = __double_as_longlong(v);      // the chunk's own sum, until its run is formed
+    __threadfence();
+    last = atomicAdd(&ctl->counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double before = 0;                              // CHAIN_THREADS chunks at a time
+  for (int c0 = 0; c0 < chunks; c0 += CHAIN_THREADS) {
+    const int c = c0 + t;
+    const double own = c < chunks ? __longlong_as_double(__ldcg(&ch[c].run.even)) : 0.0;
+    double x = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double p = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += p;
+    }
+    __syncthreads();
+    if (lane == 31) part[w] = x;
+    __syncthreads();
+    double base = before;
+    for (int q = 0; q < CHAIN_THREADS / 32; q++) {
+      if (q < w) base += part[q];
+      before += part[q];
+    }
+    if (c < chunks) ch[c].sum = base + x - own;
+  }
+  if (t == 0) ctl->counter = 0;
+}
+
+// The run of each chunk in the binade that its estimate gives, unless the
+// estimate comes near a power of two.  It is a guess: the walk applies a run
+// only where the exact sum is in its binade.
+__global__ void __launch_bounds__(CHAIN_THREADS) k_volume_runs(StageArgs a, VolChunk* ch) {
+  __shared__ double buf[VOL_SMEM];
+  __shared__ VolRun warps[CHAIN_THREADS / 32];
+  const int t = threadIdx.x, c = blockIdx.x;
+  const double s0 = ch[c].sum, own = __longlong_as_double(ch[c].run.even);
+  vol_load(a, c, buf);
+  const int e = vol_exp(s0 * (1 - 1e-9));
+  const bool sure = own >= 0 && own < INFINITY && e >= 64 && e < 2046 && vol_exp((s0 + own) * (1 + 1e-9)) == e;
+  const double scale = vol_scale(sure ? e : 1023);
+  VolRun r = {0, 0};
+  bool bad = false;
+  for (int k = 0; k < VOL_PER; k++) {
+    const double x = buf[t * (VOL_PER + 1) + k];
+    bad |= !(x >= 0 && x < INFINITY);
+    if (x > 0) r = vol_then(r, vol_cell(x, scale));
+  }
+  r = vol_scan(r, warps);
+  bad = __syncthreads_or(bad);
+  if (t == CHAIN_THREADS - 1) {
+    ch[c].run = r;
+    ch[c].exp = bad ? -1 : own == 0 ? 0 : sure ? e : -1;
+  }
+}
+
+// The chain from cell `first` on: the block stages a chunk while its first
+// thread adds the one before.
+__device__ __forceinline__ double volume_chain(const StageArgs& a, long long first, double v, double (*buf)[CHAIN_CELLS]) {
+  const long long n = (long long)a.nx * a.ny;
+  const int t = threadIdx.x, chunks = (int)((n - first + CHAIN_CELLS - 1) / CHAIN_CELLS);
   auto stage = [&](int c) {
     for (int r = 0; r < 4; r++) {
-      const int q = c * CHAIN_CELLS + r * CHAIN_THREADS + t;
-      buf[c & 1][r * CHAIN_THREADS + t] = q < n ? a.h[chain_cell(a, q)] : 0.0;
+      const long long q = first + (long long)c * CHAIN_CELLS + r * CHAIN_THREADS + t;
+      buf[c & 1][r * CHAIN_THREADS + t] = q < n ? a.h[chain_cell(a, (int)q)] : 0.0;
     }
   };
-  double v = 0;
   if (chunks > 0) stage(0);
   __syncthreads();
   for (int c = 0; c < chunks; c++) {
     if (c + 1 < chunks) stage(c + 1);
     if (t == 0) {
-      const int m = min(CHAIN_CELLS, n - c * CHAIN_CELLS);
+      const int m = (int)min((long long)CHAIN_CELLS, n - first - (long long)c * CHAIN_CELLS);
       const double* b = buf[c & 1];
       for (int q = 0; q < m; q++) v += b[q];
     }
     __syncthreads();
   }
-  if (t == 0) ctl->diag = v * dx * dy;
+  return v;                                       // thread 0's
+}
+
+// The sum s advanced by the threads' runs r, thread `from` the first, as far
+// as it stays in its binade (r.even >= 2^53 leaves it in any case): returns the
+// first thread whose run was not added, CHAIN_THREADS when none is left.
+__device__ __forceinline__ int vol_advance(double& s, VolRun r, VolRun* warps, double* s_sum, int* s_first) {
+  const int t = threadIdx.x;
+  if (t == 0) *s_first = CHAIN_THREADS;
+  const VolRun up = vol_scan(r, warps);           // has barriers
+  const unsigned long long sb = __double_as_longlong(s);
+  const unsigned long long end = sb + (unsigned long long)(sb & 1 ? up.odd : up.even);
+  if ((end >> 52) != (sb >> 52)) atomicMin(s_first, t);
+  if (t == 0) *s_sum = s;
+  __syncthreads();
+  const int f = *s_first;
+  if (f > 0 && t == f - 1) *s_sum = __longlong_as_double(end);
+  __syncthreads();
+  s = *s_sum;
+  __syncthreads();
+  return f;
+}
+
+// The sum through all chunks, by one block; ch null: no run is known.
+__global__ void __launch_bounds__(CHAIN_THREADS) k_volume_walk(StageArgs a, const VolChunk* ch, int chunks, double dx,
+                                                               double dy, Control* ctl) {
+  __shared__ union { double one[VOL_SMEM]; double two[2][CHAIN_CELLS]; } sm;
+  __shared__ VolRun warps[CHAIN_THREADS / 32];
+  __shared__ double s_sum;
+  __shared__ int s_first;
+  const int t = threadIdx.x;
+  constexpr long long OUT = 1ll << 53;
+  double s = 0;                                   // the same in every thread, as is at
+  int at = 0, held = -1;
+  VolChunk rec = {0, {0, 0}, -1, 0};              // thread t's: of chunk held + t
+  while (at < chunks) {
+    if (ch) {                                     // as far as runs go, CHAIN_THREADS chunks at a time
+      if (held < 0 || at >= held + CHAIN_THREADS) {
+        held = at;
+        rec.exp = 0; rec.run = {0, 0};
+        if (held + t < chunks) rec = ch[held + t];
+      }
+      const int e = vol_exp(s);
+      VolRun r = {0, 0};
+      if (held + t >= at && rec.exp != 0) r = rec.exp == e ? rec.run : VolRun{OUT, OUT};
+      const int f = vol_advance(s, r, warps, &s_sum, &s_first);
+      at = held + f;
+      if (f == CHAIN_THREADS || at >= chunks) continue;
+    }
+    // the chunk `at` by the block, from the exact sum before it
+    vol_load(a, at, sm.one);
+    const double* x = sm.one + t * (VOL_PER + 1);
+    bool bad = false, zero = true;
+    for (int k = 0; k < VOL_PER; k++) { bad |= !(x[k] >= 0 && x[k] < INFINITY); zero = zero && x[k] == 0; }
+    if (__syncthreads_or(bad)) {
+      s = volume_chain(a, (long long)at * VOL_CELLS, s, sm.two);
+      break;
+    }
+    int from = 0;                                 // threads before it are in the sum
+    while (from < CHAIN_THREADS && s != INFINITY) {   // at least one thread's cells per pass
+      const int e = vol_exp(s);
+      VolRun r = {0, 0};
+      if (t >= from && !zero) {
+        r = {OUT, OUT};                           // a sum too small or too large to scan, 0 among them
+        if (e >= 64 && e < 2046) {
+          const double scale = vol_scale(e);
+          r = {0, 0};
+          for (int k = 0; k < VOL_PER; k++) r = vol_then(r, vol_cell(x[k], scale));
+        }
+      }
+      const int f = vol_advance(s, r, warps, &s_sum, &s_first);
+      if (t == f) {
+        for (int k = 0; k < VOL_PER; k++) s += x[k];
+        s_sum = s;
+      }
+      __syncthreads();
+      if (f < CHAIN_THREADS) s = s_sum;
+      from = f + 1;
+    }
+    __syncthreads();
+    at++;
+  }
+  if (t == 0) ctl->diag = s * dx * dy;
 }
 
 // applyFriction alone (src/swe.mjs:659-704).
@@ -851,86 +1096,129 @@ __global__ void k_friction(StageArgs a, double dt) {
   }
 }
 
-// Per-row sums in the reference's order (each row left to right from +0),
-// one warp per row: the lanes load 32 consecutive cells of the row at a time
-// (coalesced) and form each cell's term, lane 0 adds the 32 terms in order.
-// what: 0 h (volume, src/swe.mjs:829-834), 1 the energy term
-// (:862-877), 2 b + h (the eta projection of src/globe.mjs:1414-1421).
-// A cell the energy skips (h <= 0) adds +0 here, which leaves a sum that
-// started at +0 unchanged bit for bit (it can never be -0).
-constexpr int ROWSUM_WARPS = 4;
-__global__ void __launch_bounds__(32 * ROWSUM_WARPS) k_row_sums(StageArgs a, int what, double* rows) {
-  __shared__ double buf[ROWSUM_WARPS][32];
+// The sums in the reference's row order: each row left to right from +0,
+// then the rows in order.  what: 0 h (volume, src/swe.mjs:829-834), 1 the
+// energy term (:862-877), 2 b + h (the eta projection of
+// src/globe.mjs:1414-1421).  A cell the energy skips (h <= 0) adds +0 here,
+// which leaves a sum that started at +0 unchanged bit for bit (it can never
+// be -0).  mode: 0 sum rows[j] * w[j] (the sphere's volume and energy with
+// w = area, src/swe.mjs:829-836, 875), 1 (sum rows) * dx * dy (the Cartesian
+// energy, :876; the Cartesian volume in the row order), 2 sum w[j] * rows[j]
+// with the caller's weights (the projection).
+//
+// Bound by the chain of nx additions of a row.  A block takes ROWSUM_ROWS
+// rows: a warp per row forms the terms of ROWSUM_COLS columns into shared
+// memory while one more warp adds the columns before, a lane per row, so that
+// the rows' chains run side by side and beside the loads.  The last block adds
+// the rows, staged by all of its threads.  Energy at 1536 x 1024: 104 us for a
+// warp per row alone and 44 for the rows on one thread -> 72 for both.
+constexpr int ROWSUM_ROWS = 8, ROWSUM_COLS = 128, ROWSUM_THREADS = 32 * (ROWSUM_ROWS + 1);
+__global__ void __launch_bounds__(ROWSUM_THREADS) k_row_sums(StageArgs a, int what, double* rows, int mode,
+                                                             const double* wt, double dx, double dy, Control* ctl) {
+  __shared__ double buf[2][ROWSUM_ROWS][ROWSUM_COLS + 2];   // a lane per row reads without bank conflicts
+  __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int j = blockIdx.x * ROWSUM_WARPS + w;
-  if (j >= a.ny) return;                            // the whole warp
-  const size_t base = (size_t)(j + 2) * a.W + 2;
+  const int j0 = blockIdx.x * ROWSUM_ROWS, tiles = (a.nx + ROWSUM_COLS - 1) / ROWSUM_COLS;
   double row = 0;
-  for (int i0 = 0; i0 < a.nx; i0 += 32) {
-    const int i = i0 + lane;
-    double term = 0;
-    if (i < a.nx) {
-      const size_t k = base + i;
-      const double hk = a.h[k];
-      if (what == 0) term = hk;
-      else if (what == 2) term = a.b[k] + hk;
-      else if (!(hk <= 0)) {
-        const double den = vel_den(hk, a.eps4);
-        const double u = qdiv(vel_num(a.hu[k], hk), den), v = qdiv(vel_num(a.hv[k], hk), den);
-        term = 0.5 * hk * (u * u + v * v) + 0.5 * SWE_G * hk * (hk + 2 * a.b[k]);
+  for (int c = 0; c <= tiles; c++) {
+    if (w < ROWSUM_ROWS) {
+      if (c < tiles && j0 + w < a.ny) {
+        const size_t base = (size_t)(j0 + w + 2) * a.W + 2;
+        double term[ROWSUM_COLS / 32];
+        for (int r = 0; r < ROWSUM_COLS / 32; r++) {
+          const int i = c * ROWSUM_COLS + r * 32 + lane;
+          term[r] = 0;
+          if (i < a.nx) {
+            const size_t k = base + i;
+            const double hk = a.h[k];
+            if (what == 0) term[r] = hk;
+            else if (what == 2) term[r] = a.b[k] + hk;
+            else {
+              const double huk = a.hu[k], hvk = a.hv[k], bk = a.b[k];
+              if (!(hk <= 0)) {
+                double u, v;
+                cell_vel(a, hk, huk, hvk, u, v);
+                term[r] = 0.5 * hk * (u * u + v * v) + 0.5 * SWE_G * hk * (hk + 2 * bk);
+              }
+            }
+          }
+          buf[c & 1][w][r * 32 + lane] = term[r];
+        }
+      }
+    } else if (lane < ROWSUM_ROWS && c > 0) {
+      const int m = min(ROWSUM_COLS, a.nx - (c - 1) * ROWSUM_COLS);
+      const double* b = buf[(c - 1) & 1][lane];
+      if (j0 + lane < a.ny) {
+        if (m == ROWSUM_COLS) {
+#pragma unroll 16
+          for (int q = 0; q < ROWSUM_COLS; q++) row += b[q];
+        } else {
+          for (int q = 0; q < m; q++) row += b[q];
+        }
       }
     }
-    buf[w][lane] = term;
-    __syncwarp();
-    if (lane == 0) {
-      const int m = min(32, a.nx - i0);
-      for (int q = 0; q < m; q++) row += buf[w][q];
+    __syncthreads();
+  }
+  if (w == ROWSUM_ROWS) {
+    if (lane < ROWSUM_ROWS && j0 + lane < a.ny) {
+      rows[j0 + lane] = row;
+      __threadfence();
     }
     __syncwarp();
+    if (lane == 0) last = atomicAdd(&ctl->counter, 1u) == gridDim.x - 1;
   }
-  if (lane == 0) rows[j] = row;
-}
-
-// The rows summed in order: mode 0 sum rows[j] * w[j] (the sphere's volume
-// and energy with w = area, src/swe.mjs:829-836, 875), mode 1 (sum rows) *
-// dx * dy (the Cartesian energy, :876; the Cartesian volume in the row
-// order), mode 2 sum w[j] * rows[j] with the caller's weights (the
-// projection).  One thread: ny terms.
-__global__ void k_finish_sum(const double* rows, int ny, int mode, const double* w, double dx, double dy,
-                             Control* ctl) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  __syncthreads();
+  if (!last) return;                                // uniform per block
+  __threadfence();
+  constexpr int RC = ROWSUM_ROWS * (ROWSUM_COLS + 2) < ROWSUM_THREADS ? ROWSUM_ROWS * (ROWSUM_COLS + 2) : ROWSUM_THREADS;
   double v = 0;
-  for (int j = 0; j < ny; j++) {
-    if (mode == 1) v += rows[j];
-    else v += rows[j] * w[j];
+  for (int c = 0; c * RC < a.ny; c++) {
+    double* b = buf[c & 1][0];
+    const int j = c * RC + threadIdx.x;
+    if (threadIdx.x < RC && j < a.ny) b[threadIdx.x] = mode == 1 ? __ldcg(rows + j) : __ldcg(rows + j) * wt[j];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int m = min(RC, a.ny - c * RC);
+#pragma unroll 8
+      for (int q = 0; q < m; q++) v += b[q];
+    }
   }
-  ctl->diag = mode == 1 ? v * dx * dy : v;
+  if (threadIdx.x == 0) {
+    ctl->diag = mode == 1 ? v * dx * dy : v;
+    ctl->counter = 0;
+  }
 }
 
 // what: 0 maxSurfaceDeviation(ref) (src/swe.mjs:880-892), 1 maxSpeed (:895-907),
 // 2 finite count of non-finite cells over all N (:912-917).
-__global__ void k_max_diag(StageArgs a, int what, double ref, double* part, Control* ctl) {
+__global__ void __launch_bounds__(BX) k_max_diag(StageArgs a, int what, double ref, double* part, Control* ctl) {
   __shared__ double s[BX / 32];
   __shared__ bool s_last;
   double m = 0;
-  const int nx = a.nx, ny = a.ny, W = a.W;
-  const int total = what == 2 ? a.W * a.H : nx * ny;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
-    if (what == 2) {
-      if (!isfinite(a.h[q]) || !isfinite(a.hu[q]) || !isfinite(a.hv[q])) m += 1;
-      continue;
-    }
-    const int k = (q / nx + 2) * W + (q % nx + 2);
-    const double hk = a.h[k];
-    if (hk <= a.minDepth) continue;
-    double d;
-    if (what == 0) d = fabs(a.b[k] + hk - ref);
-    else {
-      const double den = vel_den(hk, a.eps4);
-      d = hypot(qdiv(vel_num(a.hu[k], hk), den), qdiv(vel_num(a.hv[k], hk), den));
-    }
-    if (d > m) m = d;
-  }
+  if (what == 2)
+    for_cells(0, a.H, 0, a.W, [&](int j, int i) {
+      const size_t q = (size_t)j * a.W + i;
+      const double hk = a.h[q], huk = a.hu[q], hvk = a.hv[q];
+      if (!isfinite(hk) || !isfinite(huk) || !isfinite(hvk)) m += 1;
+    });
+  else if (what == 0)
+    for_cells(2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
+      const size_t k = (size_t)j * a.W + i;
+      const double hk = a.h[k], bk = a.b[k];
+      if (hk <= a.minDepth) return;
+      const double d = fabs(bk + hk - ref);
+      if (d > m) m = d;
+    });
+  else
+    for_cells(2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
+      const size_t k = (size_t)j * a.W + i;
+      const double hk = a.h[k], huk = a.hu[k], hvk = a.hv[k];
+      if (hk <= a.minDepth) return;
+      double u, v;
+      cell_vel(a, hk, huk, hvk, u, v);
+      const double d = hypot(u, v);
+      if (d > m) m = d;
+    });
   for (int o = 16; o > 0; o >>= 1) {
     const double x = __shfl_down_sync(0xffffffffu, m, o);
     m = what == 2 ? m + x : fmax(m, x);
@@ -940,14 +1228,14 @@ __global__ void k_max_diag(StageArgs a, int what, double ref, double* part, Cont
   if (threadIdx.x == 0) {
     double mm = s[0];
     for (int w = 1; w < (int)blockDim.x / 32; w++) mm = what == 2 ? mm + s[w] : fmax(mm, s[w]);
-    part[blockIdx.x] = mm;
+    part[blockIdx.y * gridDim.x + blockIdx.x] = mm;
     __threadfence();
-    s_last = atomicAdd(&ctl->counter, 1u) == gridDim.x - 1;
+    s_last = atomicAdd(&ctl->counter, 1u) == gridDim.x * gridDim.y - 1;
   }
   __syncthreads();
   if (!s_last) return;                            // uniform per block
   __threadfence();
-  const double mm = combine_parts(part, gridDim.x, what == 2, s);
+  const double mm = combine_parts(part, gridDim.x * gridDim.y, what == 2, s);
   if (threadIdx.x == 0) {
     ctl->diag = mm;
     ctl->counter = 0;
