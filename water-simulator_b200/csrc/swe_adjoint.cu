@@ -750,7 +750,8 @@ StageArgs stage_args(const swe_adjoint* s, double* const* in, double* const* out
   a.m.dyCFL = g + SWE_GEOM_DYCFL * H; a.m.bedPhi = g + SWE_GEOM_BEDPHI * H; a.m.geoCoef = g + SWE_GEOM_GEOCOEF * H;
   a.m.fRow = g + SWE_GEOM_FROW * H; a.m.tanPhi = g + SWE_GEOM_TANPHI * H;
   a.m.rdxRow = g + (SWE_GEOM_NROWS + 0) * H; a.m.rdyRowN = g + (SWE_GEOM_NROWS + 1) * H;
-  a.m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * H; a.m.rbedPhi = g + (SWE_GEOM_NROWS + 3) * H; a.m.R = INFINITY;
+  a.m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * H; a.m.rbedPhi = g + (SWE_GEOM_NROWS + 3) * H;
+  a.m.rdyCFL = g + (SWE_GEOM_NROWS + 4) * H; a.m.R = INFINITY;
   a.tame = s->tame;
   a.minDepth = s->o.min_depth; a.eps4 = s->eps4; a.coriolis = s->o.coriolis;
   a.sph = 0; a.order = s->o.order; a.lim = s->o.limiter;
@@ -1062,7 +1063,7 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
   };
   bool ok = true;
   auto A = [&](size_t n) { double* p = alloc(n); ok = ok && p; return p; };
-  s->b = A(N); s->eta0 = A(N); s->geom = A((SWE_GEOM_NROWS + 4) * (size_t)s->H);
+  s->b = A(N); s->eta0 = A(N); s->geom = A((SWE_GEOM_NROWS + 5) * (size_t)s->H);
   if (manning_field) s->nfield = A(N);
   for (int q = 0; q < 3; q++) {
     s->A[q] = A(N); s->Bf[q] = A(N); s->X[q] = A(N);
@@ -1093,7 +1094,7 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
   s->part = A(3 * (size_t)s->pcap);
   {
     double* spl = A((size_t)swe::SPLIT_FIELDS * N);
-    if (spl) s->sb = swe::split_bufs_at(spl, N);
+    if (spl) s->sb = swe::split_bufs_at(spl, N, s->W);
   }
   if (!ok || cudaMalloc(&s->ctl, sizeof(Control)) != cudaSuccess || cudaMalloc(&s->gk, sizeof(int) * n_gauges) != cudaSuccess)
     return bail(fail(SWE_ECUDA, "swe_adjoint_create: device allocation failed"));
@@ -1102,16 +1103,17 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
     const char* pe = std::getenv("SWE_B200_PDL");
     s->pdl = !(pe && std::strcmp(pe, "0") == 0);
   }
-  std::vector<double> geom((size_t)(SWE_GEOM_NROWS + 4) * s->H), sc(6);
+  std::vector<double> geom((size_t)(SWE_GEOM_NROWS + 5) * s->H), sc(6);
   int rc = swe_compute_geometry(o, geom.data(), sc.data());
   if (rc) return bail(rc);
-  for (int r = 0; r < 4; r++) {
-    const int src = r == 0 ? SWE_GEOM_DXROW : r == 1 ? SWE_GEOM_DYROWN : r == 2 ? SWE_GEOM_DYROWS : SWE_GEOM_BEDPHI;
+  for (int r = 0; r < 5; r++) {
+    const int src[5] = {SWE_GEOM_DXROW, SWE_GEOM_DYROWN, SWE_GEOM_DYROWS, SWE_GEOM_BEDPHI, SWE_GEOM_DYCFL};
     for (int j = 0; j < s->H; j++)
-      geom[(size_t)(SWE_GEOM_NROWS + r) * s->H + j] = 1.0 / geom[(size_t)src * s->H + j];
+      geom[(size_t)(SWE_GEOM_NROWS + r) * s->H + j] = 1.0 / geom[(size_t)src[r] * s->H + j];
   }
-  s->tame = swe::tame_ok(o->min_depth, geom.data() + (size_t)SWE_GEOM_DXROW * s->H,
-                         geom.data() + (size_t)SWE_GEOM_BEDPHI * s->H, s->H);
+  const double* div[3] = {geom.data() + (size_t)SWE_GEOM_DXROW * s->H, geom.data() + (size_t)SWE_GEOM_BEDPHI * s->H,
+                          geom.data() + (size_t)SWE_GEOM_DYCFL * s->H};
+  s->tame = swe::tame_ok(o->min_depth, div, s->H);
   cudaMemcpyAsync(s->geom, geom.data(), sizeof(double) * geom.size(), cudaMemcpyHostToDevice, s->st);
   cudaMemcpyAsync(s->b, b, sizeof(double) * N, cudaMemcpyHostToDevice, s->st);
   cudaMemcpyAsync(s->eta0, eta0, sizeof(double) * N, cudaMemcpyHostToDevice, s->st);

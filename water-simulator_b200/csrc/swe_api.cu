@@ -63,7 +63,7 @@ struct swe_sim {
   int nx, ny, W, H, N;
   double dx, dy, eps4, R, dlam, dphi, totalArea;
   std::vector<double> geom[SWE_GEOM_NROWS];
-  std::vector<double> recip[4];
+  std::vector<double> recip[5];
   int dryfold = 0;                                 // every reciprocal row finite
   int tame = 0;                                    // swe_split.cuh, tame_ok
   cudaStream_t st = nullptr;
@@ -262,6 +262,7 @@ swe::Metric metric(const swe_sim* s) {
   m.fRow = g + SWE_GEOM_FROW * H; m.tanPhi = g + SWE_GEOM_TANPHI * H;
   m.rdxRow = g + (SWE_GEOM_NROWS + 0) * H; m.rdyRowN = g + (SWE_GEOM_NROWS + 1) * H;
   m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * H; m.rbedPhi = g + (SWE_GEOM_NROWS + 3) * H;
+  m.rdyCFL = g + (SWE_GEOM_NROWS + 4) * H;
   m.R = s->R;
   return m;
 }
@@ -329,8 +330,7 @@ int launch_bc(swe_sim* s, double* const* f, int respect_stop, bool pdl = false) 
 }
 
 // The driver's tensor-map encoder, or null; and whether the tile copies are
-// on for this grid (SWE_B200_TMA=0 turns them off; a row stride that is not
-// a multiple of 16 bytes cannot take them).
+// on (SWE_B200_TMA=0 turns them off).
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
@@ -343,16 +343,16 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   }
   return encode;
 }
-bool tma_wanted(const swe_sim* s) {
+bool tma_wanted() {
   const char* env = std::getenv("SWE_B200_TMA");
-  if (env && std::strcmp(env, "0") == 0) return false;
-  return (sizeof(double) * (size_t)s->W) % 16 == 0;
+  return !(env && std::strcmp(env, "0") == 0);
 }
-// A 2-D map over one W x H field of doubles with the given box.
-bool encode_field(PFN_cuTensorMapEncodeTiled_v12000 encode, const swe_sim* s, CUtensorMap* m, double* base,
+// A 2-D map over one W x H field of doubles, rows of `pitch` (even), with the
+// given box.
+bool encode_field(PFN_cuTensorMapEncodeTiled_v12000 encode, const swe_sim* s, CUtensorMap* m, double* base, int pitch,
                   int bx, int by) {
   const cuuint64_t dims[2] = {(cuuint64_t)s->W, (cuuint64_t)s->H};
-  const cuuint64_t strides[1] = {(cuuint64_t)s->W * sizeof(double)};
+  const cuuint64_t strides[1] = {(cuuint64_t)pitch * sizeof(double)};
   const cuuint32_t box[2] = {(cuuint32_t)bx, (cuuint32_t)by};
   const cuuint32_t estr[2] = {1, 1};
   return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -361,23 +361,26 @@ bool encode_field(PFN_cuTensorMapEncodeTiled_v12000 encode, const swe_sim* s, CU
 }
 
 // The cell kernel's maps: the face fields (one set of buffers for both
-// stages) and the stage input's depth.
+// stages, whose rows are aligned whatever W is) and the stage input's depth
+// (where W is even; else the kernel copies it element by element).
 void make_cell_maps(swe_sim* s) {
   s->cell_tma = 0;
-  if (!s->d_split || !tma_wanted(s)) return;
+  if (!s->d_split || !tma_wanted()) return;
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode) return;
   using swe::SPX;
   using swe::SPY;
+  const int P = s->sb.P;
   for (int st = 0; st < 2; st++) {
     swe::CellMaps& c = s->cmaps[st];
-    bool ok = encode_field(encode, s, &c.m[swe::CM_XM], s->sb.fx[swe::F_M], SPX + 4, SPY + 2) &&
-              encode_field(encode, s, &c.m[swe::CM_YM], s->sb.fy[swe::F_M], SPX + 4, SPY + 3) &&
-              encode_field(encode, s, &c.m[swe::CM_H], st == 0 ? s->d_A[0] : s->d_B[0], SPX + 4, SPY + 2);
+    bool ok = encode_field(encode, s, &c.m[swe::CM_XM], s->sb.fx[swe::F_M], P, SPX + 4, SPY + 2) &&
+              encode_field(encode, s, &c.m[swe::CM_YM], s->sb.fy[swe::F_M], P, SPX + 4, SPY + 3);
+    if (s->W % 2 == 0)
+      ok = ok && encode_field(encode, s, &c.m[swe::CM_H], st == 0 ? s->d_A[0] : s->d_B[0], s->W, SPX + 4, SPY + 2);
     for (int q = 0; q < 3 && ok; q++)
-      ok = encode_field(encode, s, &c.m[swe::CM_XT + q], s->sb.fx[q + 1], SPX + 2, SPY) &&
-           encode_field(encode, s, &c.m[swe::CM_YT + q], s->sb.fy[q + 1], SPX, SPY + 1) &&
-           encode_field(encode, s, &c.m[swe::CM_TB + q], s->sb.tb[q], SPX, SPY);
+      ok = encode_field(encode, s, &c.m[swe::CM_XT + q], s->sb.fx[q + 1], P, SPX + 2, SPY) &&
+           encode_field(encode, s, &c.m[swe::CM_YT + q], s->sb.fy[q + 1], P, SPX, SPY + 1) &&
+           encode_field(encode, s, &c.m[swe::CM_TB + q], s->sb.tb[q], P, SPX, SPY);
     if (!ok) return;
   }
   s->cell_tma = 1;
@@ -390,13 +393,13 @@ void make_cell_maps(swe_sim* s) {
 // SWE_B200_TMA=0 leaves the per-element copies in use (the same bits).
 void make_tile_maps(swe_sim* s) {
   s->tma = 0;
-  if (!tma_wanted(s)) return;
+  if (!tma_wanted() || s->W % 2 != 0) return;
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (!encode) return;
   double* src[2][4] = {{s->d_b, s->d_A[0], s->d_A[1], s->d_A[2]}, {s->d_b, s->d_B[0], s->d_B[1], s->d_B[2]}};
   for (int st = 0; st < 2; st++)
     for (int f = 0; f < 4; f++)
-      if (!encode_field(encode, s, &s->tmaps[st].m[f], src[st][f], swe::SSXT, swe::SSY)) return;
+      if (!encode_field(encode, s, &s->tmaps[st].m[f], src[st][f], s->W, swe::SSXT, swe::SSY)) return;
   s->tma = 1;
 }
 
@@ -404,14 +407,15 @@ void make_tile_maps(swe_sim* s) {
 // Buffers of the tiled stage kernels (faces and source terms).
 int ensure_split(swe_sim* s) {
   if (s->d_split) return SWE_OK;
-  const size_t N = s->N;
+  const int pitch = swe::split_pitch(s->W);
+  const size_t N = (size_t)pitch * s->H;
   const size_t ntiles = (size_t)s->sgrid.x * s->sgrid.y;
   // + three int flags per tile, and the face and cell kernels' tile lists
   // with two counters each
   const size_t doubles = swe::SPLIT_FIELDS * N + 3 * ((ntiles + 1) / 2) + (ntiles + 2);
   CU(cudaMalloc(&s->d_split, sizeof(double) * doubles));
   CU(cudaMemsetAsync(s->d_split, 0, sizeof(double) * doubles, s->st));
-  s->sb = swe::split_bufs_at(s->d_split, N);
+  s->sb = swe::split_bufs_at(s->d_split, N, pitch);
   s->sb.dry = reinterpret_cast<int*>(s->d_split + swe::SPLIT_FIELDS * N);
   s->sb.ntx = (int)s->sgrid.x;
   s->sb.nty = (int)s->sgrid.y;
@@ -422,11 +426,10 @@ int ensure_split(swe_sim* s) {
   s->d_clist = s->d_fcount + 2;
   s->d_ccount = s->d_clist + ntiles;               // [2]
   make_cell_maps(s);
-  // The face kernel led by a tile list (swe_split.cuh, k_face_list), with
-  // the tensor-map copies; SWE_B200_FACE_LIST=0 keeps every CTA testing its
-  // own tile (the same bits).
+  // The face kernel led by a tile list (swe_split.cuh, k_face_list);
+  // SWE_B200_FACE_LIST=0 keeps every CTA testing its own tile (the same bits).
   const char* fl = std::getenv("SWE_B200_FACE_LIST");
-  s->face_list = s->tma && !(fl && std::strcmp(fl, "0") == 0) ? 1 : 0;
+  s->face_list = s->cell_tma && !(fl && std::strcmp(fl, "0") == 0) ? 1 : 0;
   return SWE_OK;
 }
 
@@ -471,8 +474,12 @@ int launch_stage(swe_sim* s, const swe::StageArgs& a, bool pdl = false, bool lis
       if (!list_done)
         CU(launch(pdl, swe::k_face_list, dim3((s->sgrid.x + swe::LX - 1) / swe::LX, (s->sgrid.y + swe::LY - 1) / swe::LY),
                   dim3(swe::LX * swe::LY), s->st, sb, s->d_ctl, tile_lists<MODE>(s, a)));
-      CU(launch(pdl, swe::k_split_faces_tma_list, dim3(ntiles), blk, s->st, a, sb, s->d_ctl,
-                s->tmaps[MODE - 1], (const int*)s->d_flist, (const int*)(s->d_fcount + (MODE - 1))));
+      const int* fl = s->d_flist;
+      const int* fc = s->d_fcount + (MODE - 1);
+      if (s->tma)
+        CU(launch(pdl, swe::k_split_faces_tma_list, dim3(ntiles), blk, s->st, a, sb, s->d_ctl, s->tmaps[MODE - 1], fl, fc));
+      else
+        CU(launch(pdl, swe::k_split_faces_list, dim3(ntiles), blk, s->st, a, sb, s->d_ctl, fl, fc));
     } else if (s->tma) {
       CU(launch(pdl, swe::k_split_faces_tma, s->sgrid, blk, s->st, a, sb, s->d_ctl, s->tmaps[MODE - 1]));
     }
@@ -606,16 +613,17 @@ void view_of(swe_sim* s, int* dims, double* opts, const double** b, const double
 
 namespace {
 
-// Reciprocals of the flux divisors and the bed term's (rows after the 13 metric rows).
+// Reciprocals of the flux, bed term and CFL divisors (rows after the 13 metric rows).
 void fill_reciprocals(swe_sim* s) {
-  const int src[4] = {SWE_GEOM_DXROW, SWE_GEOM_DYROWN, SWE_GEOM_DYROWS, SWE_GEOM_BEDPHI};
-  for (int q = 0; q < 4; q++) {
+  const int src[5] = {SWE_GEOM_DXROW, SWE_GEOM_DYROWN, SWE_GEOM_DYROWS, SWE_GEOM_BEDPHI, SWE_GEOM_DYCFL};
+  for (int q = 0; q < 5; q++) {
     s->recip[q].resize(s->H);
     for (int j = 0; j < s->H; j++) s->recip[q][j] = 1.0 / s->geom[src[q]][j];
   }
   s->dryfold = 1;
   for (int q = 0; q < 3; q++) s->dryfold &= swe::dry_fold_ok(s->recip[q].data(), s->recip[q].size());
-  s->tame = swe::tame_ok(s->o.min_depth, s->geom[SWE_GEOM_DXROW].data(), s->geom[SWE_GEOM_BEDPHI].data(), s->H);
+  const double* div[3] = {s->geom[SWE_GEOM_DXROW].data(), s->geom[SWE_GEOM_BEDPHI].data(), s->geom[SWE_GEOM_DYCFL].data()};
+  s->tame = swe::tame_ok(s->o.min_depth, div, s->H);
 }
 
 int upload_geom(swe_sim* s) {
@@ -623,7 +631,7 @@ int upload_geom(swe_sim* s) {
   for (int r = 0; r < SWE_GEOM_NROWS; r++)
     CU(cudaMemcpyAsync(s->d_geom + (size_t)r * s->H, s->geom[r].data(), sizeof(double) * s->H,
                        cudaMemcpyHostToDevice, s->st));
-  for (int q = 0; q < 4; q++)
+  for (int q = 0; q < 5; q++)
     CU(cudaMemcpyAsync(s->d_geom + (size_t)(SWE_GEOM_NROWS + q) * s->H, s->recip[q].data(),
                        sizeof(double) * s->H, cudaMemcpyHostToDevice, s->st));
   return SWE_OK;
@@ -716,7 +724,7 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
   CUB(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
   CUB(cudaMalloc(&s->d_b, nb));
   for (int q = 0; q < 3; q++) { CUB(cudaMalloc(&s->d_A[q], nb)); CUB(cudaMalloc(&s->d_B[q], nb)); }
-  CUB(cudaMalloc(&s->d_geom, sizeof(double) * (SWE_GEOM_NROWS + 4) * s->H));
+  CUB(cudaMalloc(&s->d_geom, sizeof(double) * (SWE_GEOM_NROWS + 5) * s->H));
   // the tiles' partials, the close's scratch, the reductions' partials
   const size_t nparts = 3 * (size_t)s->part_cap + 3 * swe::CLOSE_BLOCKS + REDUCTION_BLOCKS;
   CUB(cudaMalloc(&s->d_part, sizeof(double) * nparts));

@@ -452,19 +452,19 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     if (o.limiter < 0 || o.limiter > 2) return bail(fail(SWE_EINVAL, "unknown limiter; have minmod,mc,central"));
     s->W.push_back(o.nx + 4);
     s->H.push_back(o.ny + 4);
-    geom[q].assign((size_t)(SWE_GEOM_NROWS + 4) * s->H[q], 0.0);
+    geom[q].assign((size_t)(SWE_GEOM_NROWS + 5) * s->H[q], 0.0);
     int rc = swe_compute_geometry(&o, geom[q].data(), scal.data());
     if (rc) return bail(rc);
-    for (int r = 0; r < 4; r++) {            // reciprocal rows after the 13 metric rows
-      const int src = r == 0 ? SWE_GEOM_DXROW : r == 1 ? SWE_GEOM_DYROWN : r == 2 ? SWE_GEOM_DYROWS : SWE_GEOM_BEDPHI;
+    for (int r = 0; r < 5; r++) {            // reciprocal rows after the 13 metric rows
+      const int src[5] = {SWE_GEOM_DXROW, SWE_GEOM_DYROWN, SWE_GEOM_DYROWS, SWE_GEOM_BEDPHI, SWE_GEOM_DYCFL};
       for (int j = 0; j < s->H[q]; j++)
-        geom[q][(size_t)(SWE_GEOM_NROWS + r) * s->H[q] + j] = 1.0 / geom[q][(size_t)src * s->H[q] + j];
+        geom[q][(size_t)(SWE_GEOM_NROWS + r) * s->H[q] + j] = 1.0 / geom[q][(size_t)src[r] * s->H[q] + j];
     }
     const size_t N = (size_t)s->W[q] * s->H[q];
     s->off.push_back(total);
     // b, A (3), B (3), the tiled pair's fields, metric rows, partial slots
     // (3 x one per tile, for the most tiles either kernel uses)
-    total += round_up(N) * (7 + swe::SPLIT_FIELDS) + round_up((size_t)(SWE_GEOM_NROWS + 4) * s->H[q]) +
+    total += round_up(N) * 7 + round_up((size_t)swe::split_pitch(s->W[q]) * s->H[q]) * swe::SPLIT_FIELDS + round_up((size_t)(SWE_GEOM_NROWS + 5) * s->H[q]) +
              round_up(3 * part_slots(s->W[q], s->H[q])) + round_up((split_tiles(s->W[q], s->H[q]) + 1) / 2);
   }
   int ndev = 0;
@@ -490,9 +490,10 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     double* A[3] = {base + rN, base + 2 * rN, base + 3 * rN};
     double* Bf[3] = {base + 4 * rN, base + 5 * rN, base + 6 * rN};
     double* spl = base + 7 * rN;                // the tiled pair's fields
-    double* g = base + (7 + swe::SPLIT_FIELDS) * rN;
-    const int Hq = s->H[q];
-    double* parts = g + round_up((size_t)(SWE_GEOM_NROWS + 4) * Hq);
+    const int Hq = s->H[q], pitch = swe::split_pitch(s->W[q]);
+    const size_t rP = round_up((size_t)pitch * Hq);
+    double* g = spl + swe::SPLIT_FIELDS * rP;
+    double* parts = g + round_up((size_t)(SWE_GEOM_NROWS + 5) * Hq);
     const size_t pcap = part_slots(s->W[q], Hq);
     cudaMemcpyAsync(fb, b[q], sizeof(double) * N, cudaMemcpyHostToDevice, s->st);
     cudaMemcpyAsync(A[0], h[q], sizeof(double) * N, cudaMemcpyHostToDevice, s->st);
@@ -508,8 +509,11 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     a.m.fRow = g + SWE_GEOM_FROW * Hq; a.m.tanPhi = g + SWE_GEOM_TANPHI * Hq;
     a.m.rdxRow = g + (SWE_GEOM_NROWS + 0) * Hq; a.m.rdyRowN = g + (SWE_GEOM_NROWS + 1) * Hq;
     a.m.rdyRowS = g + (SWE_GEOM_NROWS + 2) * Hq; a.m.rbedPhi = g + (SWE_GEOM_NROWS + 3) * Hq;
-    a.tame = swe::tame_ok(o.min_depth, geom[q].data() + (size_t)SWE_GEOM_DXROW * Hq,
-                          geom[q].data() + (size_t)SWE_GEOM_BEDPHI * Hq, Hq);
+    a.m.rdyCFL = g + (SWE_GEOM_NROWS + 4) * Hq;
+    const double* gq = geom[q].data();
+    const double* div[3] = {gq + (size_t)SWE_GEOM_DXROW * Hq, gq + (size_t)SWE_GEOM_BEDPHI * Hq,
+                            gq + (size_t)SWE_GEOM_DYCFL * Hq};
+    a.tame = swe::tame_ok(o.min_depth, div, Hq);
     a.dryfold = swe::dry_fold_ok(geom[q].data() + (size_t)SWE_GEOM_NROWS * Hq, (size_t)3 * Hq);
     double Rv = 0;
     {
@@ -532,7 +536,7 @@ int swe_batch_create(int n, const swe_options* opts, const double* const* b, con
     B.bcA = bc; B.bcA.h = A[0]; B.bcA.hu = A[1]; B.bcA.hv = A[2];
     B.bcB = bc; B.bcB.h = Bf[0]; B.bcB.hu = Bf[1]; B.bcB.hv = Bf[2];
     B.ctl = s->ctls + q;
-    B.sp = swe::split_bufs_at(spl, rN);
+    B.sp = swe::split_bufs_at(spl, rP, pitch);
     B.sp.dry = reinterpret_cast<int*>(parts + round_up(3 * pcap));   // one flag per 32 x 8 tile
     B.sp.ntx = (s->W[q] + swe::SPX - 1) / swe::SPX;
     B.sp.nty = (Hq + swe::SPY - 1) / swe::SPY;

@@ -73,7 +73,7 @@ struct Metric {   // per-row divisors (src/geometry.mjs)
   // 1/dxRow, 1/dyRowN, 1/dyRowS, formed on the host with the same IEEE
   // division, so theta/dxRow == rdxRow exactly when theta == 1
   const double* rdxRow; const double* rdyRowN; const double* rdyRowS;
-  const double* rbedPhi;                                     // 1/bedPhi, likewise
+  const double* rbedPhi; const double* rdyCFL;              // 1/bedPhi, 1/dyCFL, likewise
   double R;
 };
 

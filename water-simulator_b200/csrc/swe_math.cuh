@@ -257,15 +257,21 @@ __device__ __forceinline__ bool tame_cell(double b, double h, double hu, double 
   return tame_value<-700, 60>(b) && tame_value<-100, 40>(h) && tame_value<-700, 100>(hu) &&
          tame_value<-700, 100>(hv);
 }
-// Both velocities of a tame cell; false when the operators must be used.
-__device__ __forceinline__ bool vel_tame(double hu, double hv, double h, double eps4, double& u, double& v) {
+// The velocities' denominator of a tame cell and its reciprocal; false when
+// the operators must be used.
+__device__ __forceinline__ bool vel_den_tame(double h, double eps4, double& den, double& y) {
   const double h4 = h * h * h * h;
   double hr;
-  const double den = sqrt_tame(h4 + (h4 > eps4 ? h4 : eps4), hr);
-  const double y = rcp_refine(den, rcp_refine(den, 2 * hr));
+  den = sqrt_tame(h4 + (h4 > eps4 ? h4 : eps4), hr);
+  y = rcp_refine(den, rcp_refine(den, 2 * hr));
+  return !ones_lo(den);
+}
+__device__ __forceinline__ bool vel_tame(double hu, double hv, double h, double eps4, double& u, double& v) {
+  double den, y;
+  const bool ok = vel_den_tame(h, eps4, den, y);
   u = div_tame(vel_num(hu, h), den, y);
   v = div_tame(vel_num(hv, h), den, y);
-  return !ones_lo(den);
+  return ok;
 }
 
 // The MC limiter of non-NaN arguments: of one sign, the least in magnitude of

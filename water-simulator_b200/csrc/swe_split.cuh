@@ -56,7 +56,10 @@ constexpr int SSX = SPX + 3, SSY = SPY + 3;     // state tile: cols i0-1 .. i0+S
 enum { F_M = 0, F_T = 1, F_NPL = 2, F_NPR = 3, SPLIT_FACE_FIELDS = 4 };
 constexpr int SPLIT_FIELDS = 2 * SPLIT_FACE_FIELDS + 4;   // faces, 3 source terms, u
 
+// The fields are W x H as the state is, but with a row pitch P of their own,
+// even where it may be, so that every row starts on a 16-byte boundary.
 struct SplitBufs {
+  int P;
   double* fx[SPLIT_FACE_FIELDS];   // x face (k|k+1)
   double* fy[SPLIT_FACE_FIELDS];   // y face (k|k+W)
   double* tb[3];                   // bed term x, bed term y, geometric source
@@ -78,9 +81,12 @@ struct SplitBufs {
   int* odry_out;
 };
 
-// The SPLIT_FIELDS fields of one grid, `stride` doubles apart from `base`.
-__host__ __forceinline__ SplitBufs split_bufs_at(double* base, size_t stride) {
+// The SPLIT_FIELDS fields of one grid, rows of `pitch` doubles, `stride`
+// doubles apart from `base`.
+__host__ __forceinline__ int split_pitch(int W) { return (W + 1) & ~1; }
+__host__ __forceinline__ SplitBufs split_bufs_at(double* base, size_t stride, int pitch) {
   SplitBufs b;
+  b.P = pitch;
   for (int q = 0; q < SPLIT_FACE_FIELDS; q++) {
     b.fx[q] = base + q * stride;
     b.fy[q] = base + (SPLIT_FACE_FIELDS + q) * stride;
@@ -96,13 +102,15 @@ __host__ __forceinline__ SplitBufs split_bufs_at(double* base, size_t stride) {
   return b;
 }
 
-// Whether the tame face arithmetic (swe_math.cuh) covers a grid: its minDepth
-// and, over its interior rows, the divisors dxRow and bedPhi.
-__host__ inline int tame_ok(double min_depth, const double* dx_row, const double* bed_phi, int H) {
+// Whether the tame arithmetic (swe_math.cuh) covers a grid: its minDepth and,
+// over its interior rows, the divisors of the source terms and the CFL rate
+// (rows: dxRow, bedPhi, dyCFL).
+__host__ inline int tame_ok(double min_depth, const double* const* rows, int H) {
   const double lo = std::ldexp(1.0, -60), hi = std::ldexp(1.0, 60);
   if (!(min_depth >= lo && min_depth < 1048576.0)) return 0;
-  for (int j = 2; j < H - 2; j++)
-    if (!(dx_row[j] >= lo && dx_row[j] < hi && bed_phi[j] >= lo && bed_phi[j] < hi)) return 0;
+  for (int q = 0; q < 3; q++)
+    for (int j = 2; j < H - 2; j++)
+      if (!(rows[q][j] >= lo && rows[q][j] < hi)) return 0;
   return 1;
 }
 
@@ -121,6 +129,10 @@ __device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(sdst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // The state tile is stored SSXT = SSX + 1 columns wide starting one column
@@ -136,6 +148,7 @@ struct FacesSmem {
   alignas(128) double V[SSY][SSXT];
   double xs[4][SPY][SPX + 1];                   // x slopes of cols i0 .. i0+SPX, rows j0 .. j0+SPY-1
   double ys[4][SPY + 1][SPX];                   // y slopes of cols i0 .. i0+SPX-1, rows j0 .. j0+SPY
+  int wet, wild;                                // a cell of the tile or its halo has h != 0; one is not tame
 };
 
 // One cell of a faces tile: its source terms, its east x face and north y
@@ -146,7 +159,7 @@ __device__ __forceinline__ bool split_faces_cell(const StageArgs& a, const Split
                                                  int lx, int ly, int gi, int gj, bool sph, bool bedOn) {
   const int W = a.W, H = a.H;
   const double dry = a.minDepth;
-  const int k = gj * W + gi;
+  const size_t k = (size_t)gj * s.P + gi;
   const int cx = lx + 1 + TCOL, cy = ly + 1;
   const double bk = sm.b[cy][cx], hk = sm.h[cy][cx], Uk = sm.U[cy][cx], Vk = sm.V[cy][cx];
   const double xsE = sm.xs[0][ly][lx], xsB = sm.xs[1][ly][lx];
@@ -154,7 +167,8 @@ __device__ __forceinline__ bool split_faces_cell(const StageArgs& a, const Split
 
   // bed term and geometric source of the cell (src/swe.mjs:570-598)
   double tb0 = 0, tb1 = 0, tg = 0;
-  if (bedOn && gj >= 2 && gj < H - 2 && gi >= 2 && gi < W - 2) {
+  const bool interior = gj >= 2 && gj < H - 2 && gi >= 2 && gi < W - 2;
+  if (bedOn && interior) {
     const double eC = bk + hk;
     {
       double hP, hM;
@@ -182,7 +196,8 @@ __device__ __forceinline__ bool split_faces_cell(const StageArgs& a, const Split
       if (sph) tg = a.m.geoCoef[gj] * SWE_G * (hP * hP + hM * hM);
     }
   }
-  s.tb[0][k] = tb0; s.tb[1][k] = tb1; s.tb[2][k] = tg;
+  s.tb[0][k] = tb0; s.tb[1][k] = tb1;
+  if (sph) s.tb[2][k] = tg;                     // read on a sphere only
   if (s.sl[0]) {
     for (int q = 0; q < 4; q++) { s.sl[q][k] = sm.xs[q][ly][lx]; s.sl[4 + q][k] = sm.ys[q][ly][lx]; }
     s.U[k] = Uk;
@@ -202,8 +217,7 @@ __device__ __forceinline__ bool split_faces_cell(const StageArgs& a, const Split
   constexpr int UNROLL = TAME ? 2 : 1;
 #pragma unroll UNROLL
   for (int d = 0; d < 2; d++) {
-    const bool on = d == 0 ? (gj >= 2 && gj < H - 2 && gi >= 1 && gi < W - 2)
-                           : (gj >= 1 && gj < H - 2 && gi >= 2 && gi < W - 2);
+    const bool on = interior || (d == 0 ? gj >= 2 && gj < H - 2 && gi == 1 : gj == 1 && gi >= 2 && gi < W - 2);
     const double* sp = d == 0 ? &sm.xs[0][ly][lx] : &sm.ys[0][ly][lx];
     const int fs = d == 0 ? XS : YS, no = d == 0 ? 1 : SPX;       // field stride, the neighbour's offset
     const int qn = d == 0 ? 2 : 3, qt = 5 - qn;                  // normal and transverse velocity slopes
@@ -252,11 +266,11 @@ __device__ __forceinline__ bool split_faces_settled(const SplitBufs& s, int tx, 
 // Faces and source terms of the tile (tx, ty).  Every thread of the CTA
 // calls it; it returns with the shared memory free for the next tile.
 __device__ __forceinline__ void split_faces_tile(const StageArgs& a, const SplitBufs& s, int tx, int ty,
-                                                 FacesSmem& sm) {
+                                                 FacesSmem& sm, bool check_settled = true) {
   const int W = a.W, H = a.H;
   const int i0 = tx * SPX, j0 = ty * SPY;
   const int t = threadIdx.x;
-  if (split_faces_settled(s, tx, ty, t)) return;
+  if (check_settled && split_faces_settled(s, tx, ty, t)) return;
 
   // state of the tile and its halo (zero outside the grid): b, h, hu, hv
   // copied into b, h, U, V with every copy of the thread in flight at once;
@@ -278,7 +292,9 @@ __device__ __forceinline__ void split_faces_tile(const StageArgs& a, const Split
   if (t < SSY) {                                // column 0 (i0 - 2) is in the box but not needed
     sm.b[t][0] = 0; sm.h[t][0] = 0; sm.U[t][0] = 0; sm.V[t][0] = 0;
   }
+  if (t == 0) sm.wet = sm.wild = 0;
   cp_async_wait_all();
+  __syncthreads();
   split_faces_finish(a, s, tx, ty, sm, t);
 }
 
@@ -338,11 +354,12 @@ __device__ __forceinline__ void split_faces_slopes(const StageArgs& a, FacesSmem
   }
 }
 
-// The rest of a faces tile once its state tile is in shared memory: the
-// dry test, velocities, slopes and faces.  Every thread of the CTA calls it.
-// Whether the box is tame (swe_math.cuh) is voted at the barrier after the
-// velocities; a tile that is not, or one of whose faces met a divisor the
-// tame solve leaves out, is solved with the operators.
+// The rest of a faces tile once its state tile is in shared memory (and wet
+// and wild are 0, both behind a barrier): velocities, the dry test, slopes and
+// faces.  Every thread of the CTA calls it.  Whether the tile is wet and the
+// box tame (swe_math.cuh) is settled at the barrier after the velocities; a
+// tile that is not tame, or one of whose faces met a divisor the tame solve
+// leaves out, is solved with the operators.
 __device__ __forceinline__ void split_faces_finish(const StageArgs& a, const SplitBufs& s, int tx, int ty,
                                                    FacesSmem& sm, int t) {
   const int W = a.W, H = a.H;
@@ -350,21 +367,13 @@ __device__ __forceinline__ void split_faces_finish(const StageArgs& a, const Spl
   const double eps4 = a.eps4;
   const bool sph = a.sph != 0;
   const bool bedOn = a.order >= 2 || sph;
-  int dryHere = 1;
-  for (int q = t; q < SSX * SSY; q += SP_THREADS) {
-    const int ly = q / SSX, lx = q - ly * SSX;
-    if (!(sm.h[ly][lx + TCOL] == 0)) dryHere = 0;     // zero outside the grid
-  }
-  const bool allDry = __syncthreads_and(dryHere) && s.dry && !s.sl[0];
-  if (s.dry && t == 0) s.dry[ty * s.ntx + tx] = allDry ? 1 : 0;
-  if (allDry) return;                           // uniform across the CTA
   // velocities over the whole box; a cell outside the grid has h = hu =
   // hv = 0 there and gets u = v = +0, as it would have kept
   // The box has more cells than the CTA has threads: the second pass goes
   // to the last threads, since the first two warps take the extra slopes.
   constexpr int VREM = SSXT * SSY - SP_THREADS;
   static_assert(VREM > 0 && VREM <= SP_THREADS, "one or two box cells per thread");
-  bool tame = a.tame != 0;
+  bool tame = a.tame != 0, wet = false;
 #pragma unroll 1
   for (int pass = 0; pass < 2; pass++) {
     if (pass == 1 && t < SP_THREADS - VREM) break;
@@ -376,13 +385,25 @@ __device__ __forceinline__ void split_faces_finish(const StageArgs& a, const Spl
     double U, V;
     if (h == 0) {                  // +-0 / den == +-0 and NaN / den == NaN: no division needed
       U = vel_num(hu, h); V = vel_num(hv, h);
-    } else if (!(a.tame && cell && vel_tame(hu, hv, h, eps4, U, V))) {
-      const double den = vel_den(h, eps4);
-      U = qdiv(vel_num(hu, h), den); V = qdiv(vel_num(hv, h), den);
+    } else {
+      wet = wet || c >= TCOL;      // column 0 of the box is not of the halo
+      if (!(a.tame && cell && vel_tame(hu, hv, h, eps4, U, V))) {
+        const double den = vel_den(h, eps4);
+        U = qdiv(vel_num(hu, h), den); V = qdiv(vel_num(hv, h), den);
+      }
     }
     sm.U[ly][c] = U; sm.V[ly][c] = V;
   }
-  tame = __syncthreads_and(tame);
+  if (wet) sm.wet = 1;
+  if (!tame) sm.wild = 1;
+  __syncthreads();
+  tame = !sm.wild;
+  const bool allDry = !sm.wet && s.dry && !s.sl[0];
+  if (s.dry && t == 0) s.dry[ty * s.ntx + tx] = allDry ? 1 : 0;
+  if (allDry) {                                 // uniform across the CTA
+    __syncthreads();                            // the next tile's writes come after these reads
+    return;
+  }
 
   if (tame && a.lim == 0) split_faces_slopes<0>(a, sm, t, i0, j0);    // mc, the default
   else split_faces_slopes<-1>(a, sm, t, i0, j0);
@@ -438,14 +459,30 @@ __device__ __forceinline__ void tma_load_tile(void* dst, const CUtensorMap* map,
       ::"r"(smem_addr(dst)), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(smem_addr(bar))
       : "memory");
 }
-// Every thread: until the phase `parity` of bar completes, at most `tries`
-// polls (each of which may suspend the thread for a while).
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity, int tries) {
-  for (int it = 0; it < tries; it++)
+// Until the phase `parity` of bar completes, at most TMA_WAIT_TRIES polls
+// (each of which may suspend the thread for a while).
+constexpr int TMA_WAIT_TRIES = 1 << 22;
+__device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsigned parity) {
+  for (int it = 0; it < TMA_WAIT_TRIES; it++)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
-constexpr int TMA_WAIT_TRIES = 1 << 22;
+// The same for the whole CTA: thread 0 polls, the others wait at a barrier
+// (every warp polling had taken a sixth of the cell kernel's issue slots).  A
+// copy that does not complete within the bound sets bit 4 of Control::status
+// and false is returned, in every thread, once it has landed or the bound has
+// passed again.
+__device__ __forceinline__ bool tile_wait(unsigned long long* bar, unsigned parity, Control* ctl) {
+  const int t = threadIdx.x;
+  const bool ok = t != 0 || mbar_wait_bounded(bar, parity);
+  if (__syncthreads_and(ok)) return true;
+  if (t == 0) {
+    atomicOr(&ctl->status, 4);
+    mbar_wait_bounded(bar, parity);
+  }
+  __syncthreads();
+  return false;
+}
 
 // split_faces_tile with the state tile fetched by tensor-map copies.  bar
 // is an initialised mbarrier in shared memory and parity its phase, flipped
@@ -458,6 +495,7 @@ __device__ __forceinline__ void split_faces_tile_tma(const StageArgs& a, const S
   const int t = threadIdx.x;
   if (check_settled && split_faces_settled(s, tx, ty, t)) return;
   if (t == 0) {
+    sm.wet = sm.wild = 0;
     // the generic-proxy accesses of a previous tile come before the copy's writes
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     mbar_expect_tx(bar, TILE_TX_BYTES);
@@ -467,14 +505,9 @@ __device__ __forceinline__ void split_faces_tile_tma(const StageArgs& a, const S
     tma_load_tile(&sm.U[0][0], &maps.m[2], x, y, bar);
     tma_load_tile(&sm.V[0][0], &maps.m[3], x, y, bar);
   }
-  const bool ok = mbar_wait_bounded(bar, parity, TMA_WAIT_TRIES);
+  const bool ok = tile_wait(bar, parity, ctl);
   parity ^= 1u;
-  if (!__syncthreads_and(ok)) {                     // uniform: give up on the tile
-    if (t == 0) atomicOr(&ctl->status, 4);
-    mbar_wait_bounded(bar, parity ^ 1u, TMA_WAIT_TRIES);   // let a late copy land first
-    __syncthreads();
-    return;
-  }
+  if (!ok) return;                                  // uniform: give up on the tile
   split_faces_finish(a, s, tx, ty, sm, t);
 }
 
@@ -645,22 +678,22 @@ k_split_faces_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_cons
   unsigned parity = 0;
   split_faces_tile_tma(a, s, tile % s.ntx, tile / s.ntx, sm, maps, &bar, parity, ctl, false);
 }
+__global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_MIN_BLOCKS)
+k_split_faces_list(StageArgs a, SplitBufs s, Control* ctl, const int* list, const int* count) {
+  __shared__ FacesSmem sm;
+  pdl_enter();
+  if ((int)blockIdx.x >= min(*count, s.ntx * s.nty) || ctl->stop) return;
+  const int tile = list[blockIdx.x];
+  split_faces_tile(a, s, tile % s.ntx, tile / s.ntx, sm, false);
+}
 
-struct CellsSmem {
-  double st[6][SP_THREADS];       // each thread's own cell: h, hu, hv, then U0 (stage 2)
-  double th[SPY + 2][SPX + 2];
-  double red[2][SP_THREADS / 32];
-  int dry[3][3];                  // dry flags of the tile's 3 x 3 neighbourhood
-  int prev;                       // the output tile's record as this kernel left it last time
-  bool last;
-};
-
-// The cell kernel's inputs from the face kernel, staged by tensor-map copies
-// for the tile at (i0, j0) (TMA variant): the mass fluxes of every face the
-// limiter ring and the gather touch, the other face values of the gather and
-// the depths of the ring, and the tile's source terms.  x = i0 - 2 (even)
-// for every box but yt's and tb's (x = i0); cells outside the grid read as
-// zeros, which the dry flags replace in any case.
+// The cell kernel's inputs from the face kernel, staged for the tile at
+// (i0, j0): the mass fluxes of every face the limiter ring and the gather
+// touch, the other face values of the gather, the depths of the ring and the
+// tile's source terms (the geometric one, last, on a sphere only).  x = i0 - 2
+// (even, for the tensor-map copies) for every box but yt's and tb's (x = i0).
+// What a dry tile or the outside of the grid owns is +0 here, so nothing that
+// reads the staged values asks for flags.
 struct CellFaceTiles {
   alignas(128) double xm[SPY + 2][SPX + 4];      // fx M, rows j0-1.., columns i0-2..
   alignas(128) double ym[SPY + 3][SPX + 4];      // fy M, rows j0-2.., columns i0-2..
@@ -672,61 +705,94 @@ struct CellFaceTiles {
 enum { CM_XM, CM_YM, CM_H, CM_XT, CM_YT = CM_XT + 3, CM_TB = CM_YT + 3, CM_COUNT = CM_TB + 3 };
 struct CellMaps { CUtensorMap m[CM_COUNT]; };
 constexpr unsigned CELL_TX_BYTES = sizeof(double) * (unsigned)((SPY + 2) * (SPX + 4) + (SPY + 3) * (SPX + 4) +
-                                                               (SPY + 2) * (SPX + 4) + 3 * SPY * (SPX + 2) +
-                                                               3 * (SPY + 1) * SPX + 3 * SPY * SPX);
+                                                               3 * SPY * (SPX + 2) + 3 * (SPY + 1) * SPX + 2 * SPY * SPX);
+constexpr unsigned CELL_HR_BYTES = sizeof(double) * (SPY + 2) * (SPX + 4);
+constexpr unsigned CELL_TG_BYTES = sizeof(double) * SPY * SPX;
+struct CellsSmem {
+  CellFaceTiles ft;
+  double st[6][SP_THREADS];       // each thread's own cell: h, hu, hv, then U0 (stage 2)
+  double th[SPY + 2][SPX + 2];
+  double red[2][SP_THREADS / 32];
+  bool zero[SP_THREADS / 32];     // every cell of the warp was left with h == 0
+  int dry[3][3];                  // dry flags of the tile's 3 x 3 neighbourhood, 2 outside the grid
+  int prev;                       // the output tile's record as this kernel left it last time
+  bool last;
+};
 
-// A face / source-term value owned by cell (gi, gj) of the 3 x 3 tile
-// neighbourhood of the tile at (i0, j0): +0 when its tile was dry.
-__device__ __forceinline__ double split_load(const CellsSmem& sm, int i0, int j0, int gi, int gj,
-                                             const double* arr, int k) {
-  const int c = gi < i0 ? 0 : (gi >= i0 + SPX ? 2 : 1);
-  const int r = gj < j0 ? 0 : (gj >= j0 + SPY ? 2 : 1);
-  return sm.dry[r][c] ? 0.0 : arr[k];
-}
-
-// Positivity limiter of cell (gi, gj) from its four faces' mass fluxes
-// (src/swe.mjs:511-529), with the same conservative pre-test as stage_tile.
-__device__ __forceinline__ double split_theta(const StageArgs& a, const SplitBufs& s, const CellsSmem& sm,
-                                              int i0, int j0, double dt, int gi, int gj) {
-  const int W = a.W, H = a.H;
-  if (!(dt > 0 && gj >= 1 && gj < H - 1 && gi >= 1 && gi < W - 1)) return 1;
-  const int k = gj * W + gi;
-  const double fxE = split_load(sm, i0, j0, gi, gj, s.fx[F_M], k);
-  const double fxW = split_load(sm, i0, j0, gi - 1, gj, s.fx[F_M], k - 1);
-  const double fyN = split_load(sm, i0, j0, gi, gj, s.fy[F_M], k);
-  const double fyS = split_load(sm, i0, j0, gi, gj - 1, s.fy[F_M], k - W);
-  const double avail = a.h[k];
-  const double est = ((fxE > 0 ? fxE : 0) - (fxW < 0 ? fxW : 0)) * a.m.rdxRow[gj]
-                   + (fyN > 0 ? fyN : 0) * a.m.rdyRowN[gj] - (fyS < 0 ? fyS : 0) * a.m.rdyRowS[gj];
-  double th = 1;
-  if (!(est * dt * (1 + 1e-12) < avail)) {
-    double out = 0;
-    if (fxE > 0) out += fxE / a.m.dxRow[gj];
-    if (fxW < 0) out -= fxW / a.m.dxRow[gj];
-    if (fyN > 0) out += fyN / a.m.dyRowN[gj];
-    if (fyS < 0) out -= fyS / a.m.dyRowS[gj];
-    if (out * dt > avail) th = avail > 0 ? avail / (out * dt) : 0;
+// f(smem, field, x0, y0, rows, cols) for every staged array that faces and
+// source terms own (hr, a state field, is the caller's).
+template <class F>
+__device__ __forceinline__ void for_staged(CellFaceTiles& ft, const SplitBufs& s, int i0, int j0, bool sph, F f) {
+  f(&ft.xm[0][0], s.fx[F_M], i0 - 2, j0 - 1, SPY + 2, SPX + 4);
+  f(&ft.ym[0][0], s.fy[F_M], i0 - 2, j0 - 2, SPY + 3, SPX + 4);
+  for (int q = 0; q < 3; q++) {
+    f(&ft.xt[q][0][0], s.fx[q + 1], i0 - 2, j0, SPY, SPX + 2);
+    f(&ft.yt[q][0][0], s.fy[q + 1], i0, j0 - 1, SPY + 1, SPX);
   }
-  return th;
+  for (int q = 0; q < (sph ? 3 : 2); q++) f(&ft.tb[q][0][0], s.tb[q], i0, j0, SPY, SPX);
 }
-
-// split_theta from the staged tiles: the same values, read from shared
-// memory (+0 where split_load gives +0).
-__device__ __forceinline__ bool split_dry_at(const CellsSmem& sm, int i0, int j0, int gi, int gj) {
+// The flag of the tile of the 3 x 3 neighbourhood that owns (gi, gj).
+__device__ __forceinline__ int owner_flag(const CellsSmem& sm, int i0, int j0, int gi, int gj) {
   const int c = gi < i0 ? 0 : (gi >= i0 + SPX ? 2 : 1);
   const int r = gj < j0 ? 0 : (gj >= j0 + SPY ? 2 : 1);
-  return sm.dry[r][c] != 0;
+  return sm.dry[r][c];
 }
-__device__ __forceinline__ double split_theta_st(const StageArgs& a, const CellFaceTiles& ft, const CellsSmem& sm,
-                                                 int i0, int j0, double dt, int gi, int gj) {
-  const int W = a.W, H = a.H;
-  if (!(dt > 0 && gj >= 1 && gj < H - 1 && gi >= 1 && gi < W - 1)) return 1;
-  const int cx = gi - i0 + 2, rx = gj - j0 + 1, ry = gj - j0 + 2;
-  const double fxE = split_dry_at(sm, i0, j0, gi, gj) ? 0.0 : ft.xm[rx][cx];
-  const double fxW = split_dry_at(sm, i0, j0, gi - 1, gj) ? 0.0 : ft.xm[rx][cx - 1];
-  const double fyN = split_dry_at(sm, i0, j0, gi, gj) ? 0.0 : ft.ym[ry][cx];
-  const double fyS = split_dry_at(sm, i0, j0, gi, gj - 1) ? 0.0 : ft.ym[ry - 1][cx];
-  const double avail = ft.hr[rx][cx];
+// hr element by element: the state's rows start on 8-byte boundaries where W
+// is odd.  Complete, as stage_cells, after a cp_async_wait_all and a barrier.
+__device__ __forceinline__ void stage_depths(const StageArgs& a, CellsSmem& sm, int i0, int j0) {
+  double* dst = &sm.ft.hr[0][0];
+  for (int q = threadIdx.x; q < (SPY + 2) * (SPX + 4); q += SP_THREADS) {
+    const int r = q / (SPX + 4), gi = i0 - 2 + q - r * (SPX + 4), gj = j0 - 1 + r;
+    if (gi >= 0 && gi < a.W && gj >= 0 && gj < a.H) cp_async8(dst + q, a.h + (size_t)gj * a.W + gi);
+    else dst[q] = 0;
+  }
+}
+// Staging without tensor maps: pairs of columns where the fields' rows are
+// aligned (x0 and cols are even; a pair is of one tile), else one by one.
+__device__ __forceinline__ void stage_cells(const StageArgs& a, const SplitBufs& s, CellsSmem& sm, int i0, int j0) {
+  const int P = s.P, H = a.H;
+  unsigned long long bits = P & 1 ? 8 : 0;        // P even and every field 16-byte aligned?
+  for_staged(sm.ft, s, i0, j0, a.sph != 0, [&](double*, const double* src, int, int, int, int) {
+    bits |= reinterpret_cast<unsigned long long>(src);
+  });
+  const bool pairs = (bits & 15) == 0;
+  stage_depths(a, sm, i0, j0);
+  for_staged(sm.ft, s, i0, j0, a.sph != 0, [&](double* dst, const double* src, int x0, int y0, int rows, int cols) {
+    if (pairs) {
+      for (int q = threadIdx.x; q < rows * (cols / 2); q += SP_THREADS) {
+        const int r = q / (cols / 2), gi = x0 + 2 * (q - r * (cols / 2)), gj = y0 + r;
+        if (gi >= 0 && gi < P && gj >= 0 && gj < H && !owner_flag(sm, i0, j0, gi, gj))
+          cp_async16(dst + 2 * q, src + (size_t)gj * P + gi);
+        else dst[2 * q] = dst[2 * q + 1] = 0;
+      }
+    } else {
+      for (int q = threadIdx.x; q < rows * cols; q += SP_THREADS) {
+        const int r = q / cols, gi = x0 + q - r * cols, gj = y0 + r;
+        if (gi >= 0 && gi < a.W && gj >= 0 && gj < H && !owner_flag(sm, i0, j0, gi, gj))
+          cp_async8(dst + q, src + (size_t)gj * P + gi);
+        else dst[q] = 0;
+      }
+    }
+  });
+}
+// After the tensor-map copies: +0 for what dry tiles own (their faces were
+// not written).
+__device__ __forceinline__ void zero_dry_staged(const StageArgs& a, const SplitBufs& s, CellsSmem& sm, int i0, int j0) {
+  for_staged(sm.ft, s, i0, j0, a.sph != 0, [&](double* dst, const double*, int x0, int y0, int rows, int cols) {
+    for (int q = threadIdx.x; q < rows * cols; q += SP_THREADS) {
+      const int r = q / cols;
+      if (owner_flag(sm, i0, j0, x0 + q - r * cols, y0 + r) == 1) dst[q] = 0;
+    }
+  });
+}
+
+// Positivity limiter of cell (gi, gj), the staged tiles' (ly, lx) from the
+// ring's corner, from its four faces' mass fluxes (src/swe.mjs:511-529), with
+// the same conservative pre-test as stage_tile.
+__device__ __forceinline__ double split_theta(const StageArgs& a, const CellFaceTiles& ft, double dt, int gj, int ly,
+                                              int lx) {
+  const double fxE = ft.xm[ly][lx + 1], fxW = ft.xm[ly][lx], fyN = ft.ym[ly + 1][lx + 1], fyS = ft.ym[ly][lx + 1];
+  const double avail = ft.hr[ly][lx + 1];
   const double est = ((fxE > 0 ? fxE : 0) - (fxW < 0 ? fxW : 0)) * a.m.rdxRow[gj]
                    + (fyN > 0 ? fyN : 0) * a.m.rdyRowN[gj] - (fyS < 0 ? fyS : 0) * a.m.rdyRowS[gj];
   double th = 1;
@@ -801,78 +867,58 @@ __device__ __forceinline__ void split_close_block(const StageArgs& a, Control* c
 // metrics (StageArgs::dryfold) each face term is then +0 * (finite) = +-0
 // added to or taken from a +0 sum, and the bed terms are +0, so the sums
 // are +0 with or without them: DRY leaves them out and gives the same bits.
-// ST: the face values come from the staged tiles ft.
-template <int MODE, bool DRY, bool ST = false>
+// inner: the tile holds no ghost cell, so every cell has its four faces.
+template <int MODE, bool DRY>
 __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& s, const CellsSmem& sm, int t,
-                                           int lx, int ly, int gi, int gj, double dt, double& locMax,
-                                           double& locFl, double& hout, const CellFaceTiles* ft = nullptr) {
+                                           int lx, int ly, int gi, int gj, bool inner, double dt, double& locMax,
+                                           double& locFl, double& hout) {
   const int W = a.W, H = a.H;
   const double dry = a.minDepth, eps4 = a.eps4;
   const bool sph = a.sph != 0;
   const bool bedOn = a.order >= 2 || sph;
   const bool corOn = sph || (a.coriolis != 0 && a.coriolis == a.coriolis);
   const int k = gj * W + gi;
-  // every load of the cell first, so they are in flight together
-  const bool rowX = gj >= 2 && gj < H - 2, colY = gi >= 2 && gi < W - 2;
-  const bool hasW = rowX && gi - 1 >= 1 && gi - 1 < W - 2, hasE = rowX && gi >= 1 && gi < W - 2;
-  const bool hasS = colY && gj - 1 >= 1 && gj - 1 < H - 2, hasN = colY && gj >= 1 && gj < H - 2;
-  const bool interior = colY && rowX;
-  double wM = 0, wT = 0, wN = 0, eM = 0, eT = 0, eN = 0, sM = 0, sT = 0, sN = 0, nM = 0, nT = 0, nN = 0;
-  const bool dW = sm.dry[1][lx == 0 ? 0 : 1], dS = sm.dry[ly == 0 ? 0 : 1][1], dC = sm.dry[1][1];
-  if (ST) {
-    if (!DRY && hasW && !dW) { wM = ft->xm[ly + 1][lx + 1]; wT = ft->xt[0][ly][lx + 1]; wN = ft->xt[2][ly][lx + 1]; }
-    if (!DRY && hasE && !dC) { eM = ft->xm[ly + 1][lx + 2]; eT = ft->xt[0][ly][lx + 2]; eN = ft->xt[1][ly][lx + 2]; }
-    if (!DRY && hasS && !dS) { sM = ft->ym[ly + 1][lx + 2]; sT = ft->yt[0][ly][lx]; sN = ft->yt[2][ly][lx]; }
-    if (!DRY && hasN && !dC) { nM = ft->ym[ly + 2][lx + 2]; nT = ft->yt[0][ly + 1][lx]; nN = ft->yt[1][ly + 1][lx]; }
-  } else {
-    if (!DRY && hasW && !dW) { wM = s.fx[F_M][k - 1]; wT = s.fx[F_T][k - 1]; wN = s.fx[F_NPR][k - 1]; }
-    if (!DRY && hasE && !dC) { eM = s.fx[F_M][k]; eT = s.fx[F_T][k]; eN = s.fx[F_NPL][k]; }
-    if (!DRY && hasS && !dS) { sM = s.fy[F_M][k - W]; sT = s.fy[F_T][k - W]; sN = s.fy[F_NPR][k - W]; }
-    if (!DRY && hasN && !dC) { nM = s.fy[F_M][k]; nT = s.fy[F_T][k]; nN = s.fy[F_NPL][k]; }
+  const CellFaceTiles& ft = sm.ft;
+  bool hasW = true, hasE = true, hasS = true, hasN = true, interior = true;
+  if (!inner) {
+    const bool rowX = gj >= 2 && gj < H - 2, colY = gi >= 2 && gi < W - 2;
+    hasW = rowX && gi - 1 >= 1 && gi - 1 < W - 2; hasE = rowX && gi >= 1 && gi < W - 2;
+    hasS = colY && gj - 1 >= 1 && gj - 1 < H - 2; hasN = colY && gj >= 1 && gj < H - 2;
+    interior = colY && rowX;
   }
-  cp_async_wait_all();
   const double hin = sm.st[0][t], huin = sm.st[1][t], hvin = sm.st[2][t];
-  double tb0 = 0, tb1 = 0, tg = 0, Uk = 0;
-  if (!DRY && interior && bedOn && !dC) {
-    if (ST) { tb0 = ft->tb[0][ly][lx]; tb1 = ft->tb[1][ly][lx]; if (sph) tg = ft->tb[2][ly][lx]; }
-    else { tb0 = s.tb[0][k]; tb1 = s.tb[1][k]; if (sph) tg = s.tb[2][k]; }
-  }
-  if (interior && sph) {
-    if (!DRY && !dC) Uk = s.U[k];
-    else Uk = vel_num(huin, hin);               // h is 0 here: the face kernel's u
-  }
   double U0h = 0, U0hu = 0, U0hv = 0;
   if (MODE == 2) { U0h = sm.st[3][t]; U0hu = sm.st[4][t]; U0hv = sm.st[5][t]; }
   const double thC = DRY ? 1.0 : sm.th[ly + 1][lx + 1];
   const double rdx = a.m.rdxRow[gj], dxr = a.m.dxRow[gj];
   double ah = 0, ahu = 0, ahv = 0;
-  if (!DRY && hasW) {                                       // west face, cell is its right side
-    const double thf = wM >= 0 ? sm.th[ly + 1][lx] : thC;
-    const double inv = thf == 1 ? rdx : thf / dxr;
-    ah += wM * inv; ahu += wN * inv; ahv += wT * inv;
-  }
-  if (!DRY && hasE) {                                       // east face, cell is its left side
-    const double thf = eM >= 0 ? thC : sm.th[ly + 1][lx + 2];
-    const double inv = thf == 1 ? rdx : thf / dxr;
-    ah -= eM * inv; ahu -= eN * inv; ahv -= eT * inv;
-  }
-  if (!DRY && hasS) {                                       // south face, cell is its upper side
-    const double thf = sM >= 0 ? sm.th[ly][lx + 1] : thC;
-    const double invR = thf == 1 ? a.m.rdyRowS[gj] : thf / a.m.dyRowS[gj];
-    ah += sM * invR; ahv += sN * invR; ahu += sT * invR;
-  }
-  if (!DRY && hasN) {                                       // north face, cell is its lower side
-    const double thf = nM >= 0 ? thC : sm.th[ly + 2][lx + 1];
-    const double invL = thf == 1 ? a.m.rdyRowN[gj] : thf / a.m.dyRowN[gj];
-    ah -= nM * invL; ahv -= nN * invL; ahu -= nT * invL;
+  if (!DRY) {
+    const double wM = ft.xm[ly + 1][lx + 1], eM = ft.xm[ly + 1][lx + 2];
+    const double sM = ft.ym[ly + 1][lx + 2], nM = ft.ym[ly + 2][lx + 2];
+    // each face's limiter is its upwind cell's
+    const double tW = wM >= 0 ? sm.th[ly + 1][lx] : thC, tE = eM >= 0 ? thC : sm.th[ly + 1][lx + 2];
+    const double tS = sM >= 0 ? sm.th[ly][lx + 1] : thC, tN = nM >= 0 ? thC : sm.th[ly + 2][lx + 1];
+    double iW = rdx, iE = rdx, iS = a.m.rdyRowS[gj], iN = a.m.rdyRowN[gj];
+    if (!(tW == 1 && tE == 1 && tS == 1 && tN == 1)) {
+      if (tW != 1) iW = tW / dxr;
+      if (tE != 1) iE = tE / dxr;
+      if (tS != 1) iS = tS / a.m.dyRowS[gj];
+      if (tN != 1) iN = tN / a.m.dyRowN[gj];
+    }
+    if (hasW) { ah += wM * iW; ahu += ft.xt[2][ly][lx + 1] * iW; ahv += ft.xt[0][ly][lx + 1] * iW; }   // its right side
+    if (hasE) { ah -= eM * iE; ahu -= ft.xt[1][ly][lx + 2] * iE; ahv -= ft.xt[0][ly][lx + 2] * iE; }   // its left side
+    if (hasS) { ah += sM * iS; ahv += ft.yt[2][ly][lx] * iS; ahu += ft.yt[0][ly][lx] * iS; }           // its upper side
+    if (hasN) { ah -= nM * iN; ahv -= ft.yt[1][ly + 1][lx] * iN; ahu -= ft.yt[0][ly + 1][lx] * iN; }   // its lower side
   }
   if (interior) {
     if (!DRY && bedOn) {
-      ahu += tb0;
-      ahv += tb1;
-      if (sph) ahv += tg;
+      ahu += ft.tb[0][ly][lx];
+      ahv += ft.tb[1][ly][lx];
+      if (sph) ahv += ft.tb[2][ly][lx];
     }
     if (sph) {
+      // in a dry tile h is 0 and the face kernel's u the numerator
+      const double Uk = DRY || sm.dry[1][1] ? vel_num(huin, hin) : s.U[(size_t)gj * s.P + gi];
       const double fe = a.m.fRow[gj] + Uk * (a.m.tanPhi[gj] / a.m.R);
       ahu += fe * hvin;
       ahv -= fe * huin;
@@ -905,16 +951,37 @@ __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& 
       // friction, src/swe.mjs:659-704
       const double n = a.nfield ? a.nfield[k] : a.manning;
       const bool fricOn = a.nfield ? true : (n != 0 && n == n);
+      // den of the cell's velocities and its reciprocal, for friction and,
+      // while nothing changes the depth, the CFL rate
+      const bool wet = !(nh <= dry);
+      bool tame = a.tame && wet && tame_cell(0, nh, nhu, nhv);
+      double den = 1, yden = 1;
+      if (tame) tame = vel_den_tame(nh, eps4, den, yden);
+      else if (wet) den = vel_den(nh, eps4);
       if (fricOn) {
         if (nh <= dry) { nhu = 0; nhv = 0; }
         else if (n != 0 && n == n) {
-          const double den = vel_den(nh, eps4);
-          const double u = qdiv(vel_num(nhu, nh), den), v = qdiv(vel_num(nhv, nh), den);
+          const double u = tame ? div_tame(vel_num(nhu, nh), den, yden) : qdiv(vel_num(nhu, nh), den);
+          const double v = tame ? div_tame(vel_num(nhv, nh), den, yden) : qdiv(vel_num(nhv, nh), den);
           const double speed = hypot(u, v);
           if (!(speed < 1e-14)) {
-            const double denom = 1 + dt * SWE_G * n * n * speed / pow43(nh);
-            nhu = qdiv(nhu, denom);
-            nhv = qdiv(nhv, denom);
+            const double num = dt * SWE_G * n * n * speed, p43 = pow43(nh);
+            bool quick = tame && tame_value<-700, 200>(num) && !ones_lo(p43);
+            double denom = 1;
+            if (quick) {
+              denom = 1 + div_tame(num, p43, rcp_tame(p43));
+              quick = denom < 0x1p200 && !ones_lo(denom);
+            }
+            if (quick) {
+              const double y = rcp_tame(denom);
+              nhu = div_tame(nhu, denom, y);
+              nhv = div_tame(nhv, denom, y);
+            } else {
+              denom = 1 + num / p43;
+              nhu = qdiv(nhu, denom);
+              nhv = qdiv(nhv, denom);
+            }
+            tame = tame && tame_value<-700, 100>(nhu) && tame_value<-700, 100>(nhv);
           }
         }
       }
@@ -930,15 +997,23 @@ __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& 
           nh = nh + (target - nh) * f;
           nhu = nhu - nhu * f;
           nhv = nhv - nhv * f;
+          tame = false;
         }
       }
       // CFL rate of the final state, src/swe.mjs:632-647
       if (!(nh <= dry)) {
-        const double cc = sqrt(SWE_G * nh);
-        const double den = vel_den(nh, eps4);
-        const double u = fabs(qdiv(vel_num(nhu, nh), den)), v = fabs(qdiv(vel_num(nhv, nh), den));
-        const double sr5 = (u + cc) / dxr + (v + cc) / a.m.dyCFL[gj];
-        if (sr5 > locMax) locMax = sr5;
+        if (tame) {
+          const double cc = sqrt_tame(SWE_G * nh);
+          const double u = fabs(div_tame(vel_num(nhu, nh), den, yden)), v = fabs(div_tame(vel_num(nhv, nh), den, yden));
+          const double sr5 = div_tame(u + cc, dxr, rdx) + div_tame(v + cc, a.m.dyCFL[gj], a.m.rdyCFL[gj]);
+          if (sr5 > locMax) locMax = sr5;
+        } else {
+          const double cc = sqrt(SWE_G * nh);
+          const double den = vel_den(nh, eps4);
+          const double u = fabs(qdiv(vel_num(nhu, nh), den)), v = fabs(qdiv(vel_num(nhv, nh), den));
+          const double sr5 = (u + cc) / dxr + (v + cc) / a.m.dyCFL[gj];
+          if (sr5 > locMax) locMax = sr5;
+        }
       }
     }
     hout = nh;
@@ -952,14 +1027,14 @@ __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& 
 // by k_split_close after the launch.  Every thread of the CTA calls it.
 // SETTLE: tiles may settle (below); without it the function is the plain
 // tile update, which grids with little dry land run faster.
-// TMA: the limiter ring's and the gather's inputs are staged into ft by
-// tensor-map copies (maps, completing on bar) once the tile is known to be
-// computed; a copy that does not complete within the bound sets bit 4 of
-// Control::status and leaves the tile's output unwritten.
+// The limiter ring's and the gather's inputs are staged into sm.ft once the
+// tile is known to be computed; TMA: by tensor-map copies (maps, completing on
+// bar), of which one that does not complete within the bound leaves the tile's
+// output unwritten (tile_wait).
 template <int MODE, bool SETTLE = false, bool TMA = false>
 __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const SplitBufs& s, Control* ctl, int tx,
                                                  int ty, int part, int nparts, CellsSmem& sm, bool ticket,
-                                                 CellFaceTiles* ft = nullptr, const CellMaps* maps = nullptr,
+                                                 const CellMaps* maps = nullptr,
                                                  unsigned long long* bar = nullptr) {
   static_assert(MODE == 1 || MODE == 2, "stages only");
   const int W = a.W, H = a.H;
@@ -968,6 +1043,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
   const double dt = ctl->dt;
   const int lx = t % SPX, ly = t / SPX;
   const int gi = i0 + lx, gj = j0 + ly;
+  const bool inner = i0 >= 2 && i0 + SPX <= W - 2 && j0 >= 2 && j0 + SPY <= H - 2;   // holds no ghost cell
 
   // Whether the tile could settle (below), from what is known without a
   // load.  When a quarter or more of the tiles settled in each stage of the
@@ -976,8 +1052,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
   // a settled tile reads nothing; otherwise every tile copies its state at
   // once, in flight with the flags.
   const bool canSettle = SETTLE && !ticket && s.odry_out && s.dry && a.dryfold && a.minDepth >= 0 && a.sponge_width <= 0 &&
-                         !a.h0c && !a.tape_th && !a.tape_hpre && !a.tape_pre[0] &&
-                         i0 >= 2 && i0 + SPX <= W - 2 && j0 >= 2 && j0 + SPY <= H - 2;
+                         !a.h0c && !a.tape_th && !a.tape_hpre && !a.tape_pre[0] && inner;
   const bool defer = canSettle && 32 * ctl->settled >= nparts;   // uniform across the grid
   if (!defer && gi < W && gj < H) {
     const int k = gj * W + gi;
@@ -994,14 +1069,18 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
     const int r = t / 3, c = t - 3 * r, txn = tx - 1 + c, tyn = ty - 1 + r;
     int f = 0;                                    // no flags: nothing is skipped
     if (s.dry) {
-      f = 1;                                      // outside the grid: no faces there
+      f = 2;                                      // outside the grid: no faces there
       if (txn >= 0 && txn < s.ntx && tyn >= 0 && tyn < s.nty) f = s.dry[tyn * s.ntx + txn];
     }
     sm.dry[r][c] = f;
   }
   __syncthreads();
-  const bool allDry = sm.dry[0][0] & sm.dry[0][1] & sm.dry[0][2] & sm.dry[1][0] & sm.dry[1][1] &
-                      sm.dry[1][2] & sm.dry[2][0] & sm.dry[2][1] & sm.dry[2][2];
+  bool allDry = true, anyDry = false;
+  for (int q = 0; q < 9; q++) {
+    const int f = sm.dry[q / 3][q % 3];
+    allDry = allDry && f != 0;
+    anyDry = anyDry || f == 1;
+  }
   const bool fold = allDry && a.dryfold;          // uniform across the CTA
   // A folded tile settles without its state.  Its input has h = +-0 on the
   // tile (the flags), and so does U0 in stage 2 (the output record, which
@@ -1045,73 +1124,76 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
       cp_async8(&sm.st[5][t], a.ohv + k);
     }
   }
-  if (TMA && !fold) {
-    if (t == 0) {
-      // the generic-proxy accesses of the shared memory come before the copies' writes
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      mbar_expect_tx(bar, CELL_TX_BYTES);
-      const int x = i0 - 2;
-      tma_load_tile(&ft->xm[0][0], &maps->m[CM_XM], x, j0 - 1, bar);
-      tma_load_tile(&ft->ym[0][0], &maps->m[CM_YM], x, j0 - 2, bar);
-      tma_load_tile(&ft->hr[0][0], &maps->m[CM_H], x, j0 - 1, bar);
-      for (int q = 0; q < 3; q++) {
-        tma_load_tile(&ft->xt[q][0][0], &maps->m[CM_XT + q], x, j0, bar);
-        tma_load_tile(&ft->yt[q][0][0], &maps->m[CM_YT + q], i0, j0 - 1, bar);
-        tma_load_tile(&ft->tb[q][0][0], &maps->m[CM_TB + q], i0, j0, bar);
+  if (!fold) {
+    if (TMA) {
+      if (t == 0) {
+        // the generic-proxy accesses of the shared memory come before the copies' writes
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        mbar_expect_tx(bar, CELL_TX_BYTES + (a.sph ? CELL_TG_BYTES : 0) + (a.W & 1 ? 0 : CELL_HR_BYTES));
+        const int x = i0 - 2;
+        CellFaceTiles& ft = sm.ft;
+        tma_load_tile(&ft.xm[0][0], &maps->m[CM_XM], x, j0 - 1, bar);
+        tma_load_tile(&ft.ym[0][0], &maps->m[CM_YM], x, j0 - 2, bar);
+        if (!(a.W & 1)) tma_load_tile(&ft.hr[0][0], &maps->m[CM_H], x, j0 - 1, bar);
+        for (int q = 0; q < 3; q++) {
+          tma_load_tile(&ft.xt[q][0][0], &maps->m[CM_XT + q], x, j0, bar);
+          tma_load_tile(&ft.yt[q][0][0], &maps->m[CM_YT + q], i0, j0 - 1, bar);
+          if (q < 2 || a.sph) tma_load_tile(&ft.tb[q][0][0], &maps->m[CM_TB + q], i0, j0, bar);
+        }
       }
-    }
-    const bool ok = mbar_wait_bounded(bar, 0, TMA_WAIT_TRIES);
-    if (!__syncthreads_and(ok)) {                   // uniform: give up on the tile
-      if (t == 0) atomicOr(&ctl->status, 4);
-      mbar_wait_bounded(bar, 0, TMA_WAIT_TRIES);    // let a late copy land first
+      if (a.W & 1) stage_depths(a, sm, i0, j0);     // no tensor map of the state
+      cp_async_wait_all();
+      if (!tile_wait(bar, 0, ctl)) return;          // uniform: give up on the tile
+      if (anyDry) { zero_dry_staged(a, s, sm, i0, j0); __syncthreads(); }
+    } else {
+      stage_cells(a, s, sm, i0, j0);
       cp_async_wait_all();
       __syncthreads();
-      return;
     }
-  }
-  if (!fold) {
     // the ring's second pass on the last threads, as the velocities'
     constexpr int TREM = (SPX + 2) * (SPY + 2) - SP_THREADS;
     static_assert(TREM > 0 && TREM <= SP_THREADS, "one or two ring cells per thread");
+#pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
       if (pass == 1 && t < SP_THREADS - TREM) break;
       const int q = pass == 0 ? t : t + TREM;
-      const int ly = q / (SPX + 2), lx = q - ly * (SPX + 2);
-      if (TMA) sm.th[ly][lx] = allDry ? 1.0 : split_theta_st(a, *ft, sm, i0, j0, dt, i0 - 1 + lx, j0 - 1 + ly);
-      else sm.th[ly][lx] = allDry ? 1.0 : split_theta(a, s, sm, i0, j0, dt, i0 - 1 + lx, j0 - 1 + ly);
+      const int ry = q / (SPX + 2), rx = q - ry * (SPX + 2), rj = j0 - 1 + ry, ri = i0 - 1 + rx;
+      const bool on = inner || (rj >= 1 && rj < H - 1 && ri >= 1 && ri < W - 1);
+      sm.th[ry][rx] = on && dt > 0 ? split_theta(a, sm.ft, dt, rj, ry, rx) : 1.0;
     }
-    __syncthreads();
   }
+  cp_async_wait_all();
+  __syncthreads();
 
   double locMax = 0, locFl = 0, hout = 0;
   if (gi < W && gj < H) {
-    if (fold) split_cell<MODE, true>(a, s, sm, t, lx, ly, gi, gj, dt, locMax, locFl, hout);
-    else split_cell<MODE, false, TMA>(a, s, sm, t, lx, ly, gi, gj, dt, locMax, locFl, hout, ft);
+    if (fold) split_cell<MODE, true>(a, s, sm, t, lx, ly, gi, gj, inner, dt, locMax, locFl, hout);
+    else split_cell<MODE, false>(a, s, sm, t, lx, ly, gi, gj, inner, dt, locMax, locFl, hout);
   }
-  if (s.odry_out) {                               // the written tile's flag
-    const bool ghostFree = i0 >= 2 && i0 + SPX <= W - 2 && j0 >= 2 && j0 + SPY <= H - 2;
-    const bool own = __syncthreads_and(hout == 0) && ghostFree;
-    if (t == 0) s.odry_out[ty * s.ntx + tx] = own ? 1 : 0;
+  // Per-tile partials: a warp's maximum and sum, then the tile's by one
+  // thread.  The maximum is that of non-negative doubles, so it is the
+  // integers'; a warp that floored nothing sums to +0.  The same barrier
+  // settles the written tile's record.
+  const unsigned all = 0xffffffffu;
+  const bool zeroWarp = __all_sync(all, hout == 0), floorWarp = __any_sync(all, locFl != 0);
+  if (MODE == 2) {
+    const unsigned hi = __double2hiint(locMax), top = __reduce_max_sync(all, hi);
+    const unsigned low = __reduce_max_sync(all, hi == top ? __double2loint(locMax) : 0u);
+    locMax = __hiloint2double(top, low);
   }
-
-  // per-block partials, then the last block of the grid closes the step.
-  // When no cell contributed (both start at +0 and only change to nonzero
-  // values), the reduction would give +0 and 0: those are written directly.
-  const bool any = __syncthreads_or(locMax != 0 || locFl != 0);   // uniform
-  if (any) {
-    for (int o = 16; o > 0; o >>= 1) {
-      locMax = fmax(locMax, __shfl_down_sync(0xffffffffu, locMax, o));
-      locFl += __shfl_down_sync(0xffffffffu, locFl, o);
-    }
-    if ((t & 31) == 0) { sm.red[0][t >> 5] = locMax; sm.red[1][t >> 5] = locFl; }
-    __syncthreads();
-  }
+  if (floorWarp)
+    for (int o = 16; o > 0; o >>= 1) locFl += __shfl_down_sync(all, locFl, o);
+  if ((t & 31) == 0) { sm.red[0][t >> 5] = locMax; sm.red[1][t >> 5] = locFl; sm.zero[t >> 5] = zeroWarp; }
+  __syncthreads();
   if (t == 0) {
-    double m = 0, f = 0;
-    if (any) {
-      m = sm.red[0][0]; f = sm.red[1][0];
-      for (int w = 1; w < SP_THREADS / 32; w++) { m = fmax(m, sm.red[0][w]); f += sm.red[1][w]; }
+    double m = sm.red[0][0], f = sm.red[1][0];
+    bool zero = sm.zero[0];
+    for (int w = 1; w < SP_THREADS / 32; w++) {
+      if (MODE == 2) m = fmax(m, sm.red[0][w]);
+      f += sm.red[1][w];
+      zero = zero && sm.zero[w];
     }
+    if (s.odry_out) s.odry_out[ty * s.ntx + tx] = zero && inner ? 1 : 0;
     if (MODE == 1) a.part_fl1[part] = f;
     else { a.part_max[part] = m; a.part_fl2[part] = f; }
     if (ticket) {
@@ -1220,13 +1302,12 @@ template <int MODE, bool SETTLE = false>
 __global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_CELLS_MIN_BLOCKS)
 k_split_cells_tma(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ CellMaps maps) {
   __shared__ CellsSmem sm;
-  __shared__ CellFaceTiles ft;
   __shared__ alignas(8) unsigned long long bar;
   if (threadIdx.x == 0) mbar_init(&bar, 1);        // before the wait: touches no global memory
   pdl_enter();
   if (ctl->stop) return;
   split_cells_tile<MODE, SETTLE, true>(a, s, ctl, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x,
-                                       gridDim.x * gridDim.y, sm, false, &ft, &maps, &bar);
+                                       gridDim.x * gridDim.y, sm, false, &maps, &bar);
 }
 
 // The cell kernel over its list: CTA b runs the list's entry b; the CTAs
@@ -1236,15 +1317,13 @@ __global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_CELLS_MIN_BLOCKS)
 k_split_cells_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ CellMaps maps,
                        const int* list, const int* count) {
   __shared__ CellsSmem sm;
-  __shared__ CellFaceTiles ft;
   __shared__ alignas(8) unsigned long long bar;
   pdl_enter();
   const int ntiles = s.ntx * s.nty;
   if ((int)blockIdx.x >= min(*count, ntiles) || ctl->stop) return;
   if (threadIdx.x == 0) mbar_init(&bar, 1);
   const int tile = list[blockIdx.x];
-  split_cells_tile<MODE, SETTLE, true>(a, s, ctl, tile % s.ntx, tile / s.ntx, tile, ntiles, sm, false, &ft, &maps,
-                                       &bar);
+  split_cells_tile<MODE, SETTLE, true>(a, s, ctl, tile % s.ntx, tile / s.ntx, tile, ntiles, sm, false, &maps, &bar);
 }
 
 // Closes the stage k_split_cells left open: one block, no atomics (a
