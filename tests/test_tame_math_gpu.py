@@ -91,3 +91,36 @@ def test_tame_tiles_and_the_others_give_the_fused_kernels_bits(swe, monkeypatch,
         assert np.array_equal(np.isnan(x), np.isnan(y))
         fine = ~np.isnan(x)
         assert np.array_equal(x[fine].view(np.uint64), y[fine].view(np.uint64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", [(28, 4), (29, 5), (590, 244), (589, 245), (1000, 1140), (1001, 1200)])
+@pytest.mark.parametrize("sides", ["mixed", "periodic", "tide"])
+def test_every_size_of_step_gives_the_fused_kernels_bits(swe, monkeypatch, nx, ny, sides):
+    """A step's launches depend on the grid's size (ghosts and dt within the
+    face kernel, one wave or several, one block to close or 32, tile lists)
+    and on whether its width is even: all against the fused kernels."""
+    rng = np.random.default_rng(nx)
+    b = rng.uniform(-0.3, 0.3, (ny + 4, nx + 4))
+    b[:, (2 * nx) // 3:] = 3.0                   # dry land, settled tiles on the larger grids
+    eta = np.where(np.arange(nx + 4) < nx // 3, 2.0, 1.2)[None, :].repeat(ny + 4, 0)
+    out = []
+    for impl in ("fused", "split"):
+        monkeypatch.setenv("SWE_B200_STAGE", impl)
+        sim = swe.ShallowWater(nx=nx, ny=ny, dx=2.0, bed=b, eta0=eta, manning=0.0, coriolis=1e-4)
+        if sides == "periodic":
+            sim.boundaries = {s: swe.periodic for s in ("west", "east", "south", "north")}
+        elif sides == "tide":
+            sim.boundaries.west = swe.flather(swe.Tide({"M2": [0.3, 20.0], "S2": [0.1, 5.0]}, msl=2.0).signal())
+        else:
+            sim.boundaries = {"west": swe.flather(lambda t: 2.0, lambda t: 0.1), "east": swe.outflow,
+                              "south": swe.reflect, "north": swe.outflow}
+        sim.step(1e-3)
+        assert sim.run(5) == 5 if sides != "mixed" else sim.run(2) == 2
+        t_end = sim.t + 1.5 * sim.maxDt()
+        sim.run(6, tEnd=t_end)                  # the third step of these is refused
+        out.append([sim.field(f).view(np.uint64).copy() for f in ("h", "hu", "hv", "b")] + [sim.t, sim.maxDt()])
+        sim.close()
+    for x, y in zip(out[0][:4], out[1][:4]):
+        assert np.array_equal(x, y)
+    assert out[0][4:] == out[1][4:]

@@ -814,6 +814,10 @@ swe::PrepArgs prep_of(const swe_adjoint* s, bool auto_dt, int k) {
   return p;
 }
 
+// The face kernel whose stage input's ghosts a launch before it has filled.
+constexpr auto faces_kernel = &swe::k_split_faces<SWE_SPLIT_FACES_MIN_BLOCKS, false>;
+const swe::GhostFill no_fill = {};
+
 // One forward step of state X in place.
 int fwd_step(swe_adjoint* s, double* const* X, bool auto_dt, int step_index) {
   LAUNCH(swe::k_prepare, dim3(1), dim3(32), s->ctl, prep_of(s, auto_dt, step_index));
@@ -822,12 +826,12 @@ int fwd_step(swe_adjoint* s, double* const* X, bool auto_dt, int step_index) {
   const int nparts = (int)(s->sgrid.x * s->sgrid.y);
   LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, X), (const Control*)s->ctl, 0);
   const StageArgs a1 = stage_args(s, X, s->Bf);
-  LAUNCH(swe::k_split_faces, s->sgrid, spb, a1, s->sb, s->ctl);
+  LAUNCH(faces_kernel, s->sgrid, spb, a1, s->sb, s->ctl, no_fill);
   LAUNCH(swe::k_split_cells<1>, s->sgrid, spb, a1, s->sb, s->ctl);
   LAUNCH(swe::k_split_close<1>, dim3(1), spb, a1, s->ctl, nparts);
   LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, s->Bf), (const Control*)s->ctl, 0);
   const StageArgs a2 = stage_args(s, s->Bf, X);
-  LAUNCH(swe::k_split_faces, s->sgrid, spb, a2, s->sb, s->ctl);
+  LAUNCH(faces_kernel, s->sgrid, spb, a2, s->sb, s->ctl, no_fill);
   LAUNCH(swe::k_split_cells<2>, s->sgrid, spb, a2, s->sb, s->ctl);
   LAUNCH(swe::k_split_close<2>, dim3(1), spb, a2, s->ctl, nparts);
   if (auto_dt) LAUNCH(k_record_dt, dim3(1), dim3(32), (const Control*)s->ctl, s->dts, step_index);
@@ -917,7 +921,7 @@ int tape_step(swe_adjoint* s, double* const* X, int k, const Tape& T) {
   StageArgs a1 = stage_args(s, T.W1, T.Bp);
   a1.tape_th = T.th1; a1.tape_hpre = T.hB;
   const swe::SplitBufs b1 = tape_bufs(s, T.it1);
-  LAUNCH(swe::k_split_faces, s->sgrid, spb, a1, b1, s->ctl);
+  LAUNCH(faces_kernel, s->sgrid, spb, a1, b1, s->ctl, no_fill);
   LAUNCH(swe::k_split_cells<1>, s->sgrid, spb, a1, b1, s->ctl);
   LAUNCH(swe::k_split_close<1>, dim3(1), spb, a1, s->ctl, nparts);
   LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, T.Bp), (const Control*)s->ctl, 0);
@@ -925,7 +929,7 @@ int tape_step(swe_adjoint* s, double* const* X, int k, const Tape& T) {
   a2.tape_th = T.th2; a2.tape_hpre = T.hA;
   for (int q = 0; q < 3; q++) a2.tape_pre[q] = T.Bf[q];
   const swe::SplitBufs b2 = tape_bufs(s, T.it2);
-  LAUNCH(swe::k_split_faces, s->sgrid, spb, a2, b2, s->ctl);
+  LAUNCH(faces_kernel, s->sgrid, spb, a2, b2, s->ctl, no_fill);
   LAUNCH(swe::k_split_cells<2>, s->sgrid, spb, a2, b2, s->ctl);
   LAUNCH(swe::k_split_close<2>, dim3(1), spb, a2, s->ctl, nparts);
   LAUNCH(k_copy, dim3(G1(s)), dim3(256), (size_t)s->N, 1, T.hX, (double*)nullptr, (double*)nullptr,

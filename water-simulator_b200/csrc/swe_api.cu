@@ -128,9 +128,10 @@ struct swe_sim {
 };
 
 namespace {
+bool one_wave(const swe_sim* s);
 // The state was written outside a stage: no tile is known dry any more.
 int forget_dry(swe_sim* s) {
-  if (!s->d_odry[0]) return SWE_OK;
+  if (!s->d_odry[0] || one_wave(s)) return SWE_OK;
   const size_t bytes = sizeof(int) * (size_t)s->sgrid.x * s->sgrid.y;
   CU(cudaMemsetAsync(s->d_odry[0], 0, bytes, s->st));
   CU(cudaMemsetAsync(s->d_odry[1], 0, bytes, s->st));
@@ -403,7 +404,6 @@ void make_tile_maps(swe_sim* s) {
   s->tma = 1;
 }
 
-// One SSP-RK2 step on the device; `mode`/`dt`/`t_end` as k_prepare.
 // Buffers of the tiled stage kernels (faces and source terms).
 int ensure_split(swe_sim* s) {
   if (s->d_split) return SWE_OK;
@@ -434,17 +434,25 @@ int ensure_split(swe_sim* s) {
 }
 
 
+int tiles_of(const swe_sim* s) { return (int)(s->sgrid.x * s->sgrid.y); }
+// A grid whose tiles all run at once (4 CTAs per SM of 148) is bound by the
+// latency of a step's kernels, not by their work: it keeps no records of dry
+// tiles and makes no lists, whose flags only delay its tiles.
+bool one_wave(const swe_sim* s) { return tiles_of(s) <= 4 * 148; }
+bool settles(const swe_sim* s) { return s->settle && !one_wave(s); }
+
 // The stage kernels' buffers of stage MODE (stage 1: A -> B, stage 2: B -> A).
 template <int MODE>
 swe::SplitBufs stage_bufs(const swe_sim* s) {
   swe::SplitBufs sb = s->sb;
-  sb.odry_in = s->d_odry[MODE == 1 ? 0 : 1];
+  if (one_wave(s)) return sb;                      // odry_in, odry_out null
+  if (settles(s)) sb.odry_in = s->d_odry[MODE == 1 ? 0 : 1];   // else the records are kept, and not asked
   sb.odry_out = s->d_odry[MODE == 1 ? 1 : 0];
   return sb;
 }
 // The tile lists pay where tiles settle: with the settling cell kernel
 // (which swe_run keeps only where a quarter or more of the tiles settle).
-bool stage_listed(const swe_sim* s) { return s->stage_impl == 1 && s->face_list && s->settle; }
+bool stage_listed(const swe_sim* s) { return s->stage_impl == 1 && s->face_list && settles(s); }
 // Whether the cell kernel takes its list: when tiles may be left out.
 int cell_listed(const swe_sim* s, const swe::StageArgs& a) {
   return stage_listed(s) && s->cell_tma && a.dryfold && a.minDepth >= 0 && a.sponge_width <= 0 && !a.h0c &&
@@ -460,50 +468,80 @@ swe::TileLists tile_lists(const swe_sim* s, const swe::StageArgs& a) {
   return L;
 }
 
-// One stage (MODE 1 or 2) with the selected kernels; list_done: its lists
-// were made with the ghost fill (launch_bc_lists).
+// Stage MODE with the tile lists.  list_done: they were made with the ghost
+// fill (launch_bc_lists).
+template <int MODE>
+int launch_stage_listed(swe_sim* s, const swe::StageArgs& a, bool pdl, bool list_done) {
+  const swe::SplitBufs sb = stage_bufs<MODE>(s);
+  const dim3 blk(swe::SP_THREADS), tiles(tiles_of(s));
+  const swe::CellMaps& cm = s->cmaps[MODE - 1];
+  if (!list_done)
+    CU(launch(pdl, swe::k_face_list, dim3((s->sgrid.x + swe::LX - 1) / swe::LX, (s->sgrid.y + swe::LY - 1) / swe::LY),
+              dim3(swe::LX * swe::LY), s->st, sb, s->d_ctl, tile_lists<MODE>(s, a)));
+  const int* list = s->d_flist;
+  const int* count = s->d_fcount + (MODE - 1);
+  if (s->tma)
+    CU(launch(pdl, swe::k_split_faces_tma_list, tiles, blk, s->st, a, sb, s->d_ctl, s->tmaps[MODE - 1], list, count));
+  else
+    CU(launch(pdl, swe::k_split_faces_list, tiles, blk, s->st, a, sb, s->d_ctl, list, count));
+  if (cell_listed(s, a))                           // only when tiles may be left out
+    CU(launch(pdl, swe::k_split_cells_tma_list<MODE, true>, tiles, blk, s->st, a, sb, s->d_ctl, cm,
+              (const int*)s->d_clist, (const int*)(s->d_ccount + (MODE - 1))));
+  else
+    CU(launch(pdl, swe::k_split_cells_tma<MODE, true>, s->sgrid, blk, s->st, a, sb, s->d_ctl, cm));
+  return SWE_OK;
+}
+
+// Stage MODE over every tile; F: what the face kernel fills and prepares.
+template <int MODE>
+int launch_stage_tiles(swe_sim* s, const swe::StageArgs& a, bool pdl, const swe::GhostFill& F) {
+  const swe::SplitBufs sb = stage_bufs<MODE>(s);
+  const dim3 blk(swe::SP_THREADS), grid = s->sgrid;
+  const swe::CellMaps& cm = s->cmaps[MODE - 1];
+  const swe::TileMaps& tm = s->tmaps[MODE - 1];
+  swe::Control* ctl = s->d_ctl;
+  constexpr int WIDE = SWE_SPLIT_FACES_MIN_BLOCKS, ROOMY = WIDE - 1;
+  const bool roomy = tiles_of(s) <= ROOMY * 148;   // see k_split_faces
+  if (s->tma) {
+    if (!F.on) CU(launch(pdl, swe::k_split_faces_tma<WIDE, false>, grid, blk, s->st, a, sb, ctl, tm, F));
+    else if (roomy) CU(launch(pdl, swe::k_split_faces_tma<ROOMY, true>, grid, blk, s->st, a, sb, ctl, tm, F));
+    else CU(launch(pdl, swe::k_split_faces_tma<WIDE, true>, grid, blk, s->st, a, sb, ctl, tm, F));
+  } else {
+    if (!F.on) CU(launch(pdl, swe::k_split_faces<WIDE, false>, grid, blk, s->st, a, sb, ctl, F));
+    else if (roomy) CU(launch(pdl, swe::k_split_faces<ROOMY, true>, grid, blk, s->st, a, sb, ctl, F));
+    else CU(launch(pdl, swe::k_split_faces<WIDE, true>, grid, blk, s->st, a, sb, ctl, F));
+  }
+  if (s->cell_tma) {
+    if (settles(s)) CU(launch(pdl, swe::k_split_cells_tma<MODE, true>, grid, blk, s->st, a, sb, ctl, cm));
+    else CU(launch(pdl, swe::k_split_cells_tma<MODE, false>, grid, blk, s->st, a, sb, ctl, cm));
+  } else {
+    if (settles(s)) CU(launch(pdl, swe::k_split_cells<MODE, true>, grid, blk, s->st, a, sb, ctl));
+    else CU(launch(pdl, swe::k_split_cells<MODE, false>, grid, blk, s->st, a, sb, ctl));
+  }
+  return SWE_OK;
+}
+
+// The step's close, after stage 2.
+int launch_close(swe_sim* s, const swe::StageArgs& a, bool pdl) {
+  const int n = tiles_of(s);
+  if (n <= swe::CLOSE_TILES)
+    CU(launch(pdl, swe::k_split_close_step, dim3(1), dim3(32 * swe::CLOSE_BLOCKS), s->st, a, s->d_ctl, n));
+  else
+    CU(launch(pdl, swe::k_split_close_multi<2>, dim3(swe::CLOSE_BLOCKS), dim3(swe::SP_THREADS), s->st, a, s->d_ctl, n,
+              s->d_part + 3 * (size_t)s->part_cap));
+  return SWE_OK;
+}
+
+// One stage (MODE 1 or 2) with the selected kernels, its ghosts filled and
+// the step prepared by launches before it; list_done: and its lists made.
 template <int MODE>
 int launch_stage(swe_sim* s, const swe::StageArgs& a, bool pdl = false, bool list_done = false) {
   if (s->stage_impl == 1) {
-    const swe::SplitBufs sb = stage_bufs<MODE>(s);
-    const dim3 blk(swe::SP_THREADS);
-    const bool listed = stage_listed(s);
-    const int cell_list = cell_listed(s, a);
-    if (listed) {
-      const int ntiles = (int)(s->sgrid.x * s->sgrid.y);
-      if (!list_done)
-        CU(launch(pdl, swe::k_face_list, dim3((s->sgrid.x + swe::LX - 1) / swe::LX, (s->sgrid.y + swe::LY - 1) / swe::LY),
-                  dim3(swe::LX * swe::LY), s->st, sb, s->d_ctl, tile_lists<MODE>(s, a)));
-      const int* fl = s->d_flist;
-      const int* fc = s->d_fcount + (MODE - 1);
-      if (s->tma)
-        CU(launch(pdl, swe::k_split_faces_tma_list, dim3(ntiles), blk, s->st, a, sb, s->d_ctl, s->tmaps[MODE - 1], fl, fc));
-      else
-        CU(launch(pdl, swe::k_split_faces_list, dim3(ntiles), blk, s->st, a, sb, s->d_ctl, fl, fc));
-    } else if (s->tma) {
-      CU(launch(pdl, swe::k_split_faces_tma, s->sgrid, blk, s->st, a, sb, s->d_ctl, s->tmaps[MODE - 1]));
-    }
-    else CU(launch(pdl, swe::k_split_faces, s->sgrid, blk, s->st, a, sb, s->d_ctl));
-    if (cell_list) {                               // only when tiles may be left out
-      const swe::CellMaps& cm = s->cmaps[MODE - 1];
-      const int ntiles = (int)(s->sgrid.x * s->sgrid.y);
-      const int* cl = s->d_clist;
-      const int* cc = s->d_ccount + (MODE - 1);
-      if (s->settle) CU(launch(pdl, swe::k_split_cells_tma_list<MODE, true>, dim3(ntiles), blk, s->st, a, sb, s->d_ctl, cm, cl, cc));
-      else CU(launch(pdl, swe::k_split_cells_tma_list<MODE, false>, dim3(ntiles), blk, s->st, a, sb, s->d_ctl, cm, cl, cc));
-    } else if (s->cell_tma) {
-      const swe::CellMaps& cm = s->cmaps[MODE - 1];
-      if (s->settle) CU(launch(pdl, swe::k_split_cells_tma<MODE, true>, s->sgrid, blk, s->st, a, sb, s->d_ctl, cm));
-      else CU(launch(pdl, swe::k_split_cells_tma<MODE, false>, s->sgrid, blk, s->st, a, sb, s->d_ctl, cm));
-    } else if (s->settle) {
-      CU(launch(pdl, swe::k_split_cells<MODE, true>, s->sgrid, blk, s->st, a, sb, s->d_ctl));
-    } else {
-      CU(launch(pdl, swe::k_split_cells<MODE, false>, s->sgrid, blk, s->st, a, sb, s->d_ctl));
-    }
-    // stage 2's close closes the whole step, stage 1's floored mass included
-    if (MODE == 2)
-      CU(launch(pdl, swe::k_split_close_multi<2>, dim3(swe::CLOSE_BLOCKS), blk, s->st, a, s->d_ctl,
-                (int)(s->sgrid.x * s->sgrid.y), s->d_part + 3 * (size_t)s->part_cap));
+    const swe::GhostFill none = {};
+    int rc = stage_listed(s) ? launch_stage_listed<MODE>(s, a, pdl, list_done)
+                             : launch_stage_tiles<MODE>(s, a, pdl, none);
+    if (rc == SWE_OK && MODE == 2) rc = launch_close(s, a, pdl);
+    if (rc) return rc;
   } else {
     swe::k_stage<MODE><<<s->grid, swe::BX, swe::STAGE_SMEM_BYTES, s->st>>>(a, s->d_ctl);
   }
@@ -511,13 +549,9 @@ int launch_stage(swe_sim* s, const swe::StageArgs& a, bool pdl = false, bool lis
   return SWE_OK;
 }
 
-// The ghost fill of f, and with tile lists the lists of stage MODE in the
-// same launch (k_bc_face_list); returns through `listed` whether it made them.
+// The ghost fill of f and the lists of stage MODE in one launch.
 template <int MODE>
-int launch_bc_lists(swe_sim* s, double* const* f, int respect_stop, bool pdl, const swe::StageArgs& a,
-                    bool& listed) {
-  listed = stage_listed(s);
-  if (!listed) return launch_bc(s, f, respect_stop, pdl);
+int launch_bc_lists(swe_sim* s, double* const* f, int respect_stop, bool pdl, const swe::StageArgs& a) {
   const int nbc = bc_blocks(s);
   const int nrx = (s->sgrid.x + swe::LX - 1) / swe::LX, nry = (s->sgrid.y + swe::LY - 1) / swe::LY;
   CU(launch(pdl, swe::k_bc_face_list, dim3(nbc + nrx * nry), dim3(swe::LX * swe::LY), s->st, bc_args(s, f),
@@ -525,25 +559,49 @@ int launch_bc_lists(swe_sim* s, double* const* f, int respect_stop, bool pdl, co
   return SWE_OK;
 }
 
+// Most tiles of a grid whose face kernels fill the ghosts and prepare the step
+// (8 waves).  128 steps with the fill in the face kernel against launches of its
+// own: 400 x 330 5.97 -> 5.42 ms, 512 x 512 9.27 -> 9.00, 1020 x 512 15.05 -> 14.85,
+// the sphere 1440 x 720 with its tides 31.0 -> 30.3, 1024 x 1024 30.62 -> 30.76,
+// 2048 x 2048 104.4 -> 106.1 (the fill costs every tile registers).
+constexpr int FILL_TILES = 8 * 4 * 148;
+
+// One SSP-RK2 step on the device; `mode`/`dt`/`t_end` as k_prepare.  The
+// tiled kernels, the ghost fills and prepare enter through pdl_enter, so each
+// may be scheduled while its predecessor drains.  Host-checked dt (mode 0)
+// never reaches here refused.  In the device loop a refused step (t reached
+// t_end) changes nothing, ghosts included, as the drivers' `while (sim.t < T)`
+// loop stops calling step().
 int enqueue_step(swe_sim* s, int mode, double dt, double t_end, const double* dt_dev = nullptr) {
-  // The tiled kernels, the ghost fills and prepare enter through pdl_enter,
-  // so each may be scheduled while its predecessor drains.
   const bool pdl = s->pdl && s->stage_impl == 1;
-  CU(launch(pdl, swe::k_prepare, dim3(1), dim3(32), s->st, s->d_ctl, prep_args(s, mode, dt, t_end, dt_dev)));
-  // Host-checked dt (mode 0) never reaches here refused.  In the device loop
-  // a refused step (t reached t_end) changes nothing, ghosts included, as the
-  // drivers' `while (sim.t < T)` loop stops calling step().
-  swe::StageArgs a1 = stage_args(s, s->d_A, s->d_B);
-  bool listed = false;
-  int rc = launch_bc_lists<1>(s, s->d_A, mode == 0 ? 0 : 1, pdl, a1, listed);
-  if (rc) return rc;
-  rc = launch_stage<1>(s, a1, pdl, listed);
-  if (rc) return rc;
+  const swe::PrepArgs prep = prep_args(s, mode, dt, t_end, dt_dev);
+  const swe::StageArgs a1 = stage_args(s, s->d_A, s->d_B);
   swe::StageArgs a2 = stage_args(s, s->d_B, s->d_A);
   if (s->keep_h0) { a2.h0c = s->d_h0[0]; a2.hu0c = s->d_h0[1]; a2.hv0c = s->d_h0[2]; }
-  rc = launch_bc_lists<2>(s, s->d_B, 1, pdl, a2, listed);
-  if (rc) return rc;
-  return launch_stage<2>(s, a2, pdl, listed);
+  int rc;
+  if (s->stage_impl == 1 && !settles(s) && tiles_of(s) <= FILL_TILES) {   // five launches
+    swe::GhostFill F = {};
+    F.on = 1;
+    F.prepare = 1;
+    F.prep = prep;
+    F.bc = bc_args(s, s->d_A);
+    rc = launch_stage_tiles<1>(s, a1, pdl, F);
+    if (rc) return rc;
+    F.prepare = 0;
+    F.bc = bc_args(s, s->d_B);
+    rc = launch_stage_tiles<2>(s, a2, pdl, F);
+    if (rc == SWE_OK) rc = launch_close(s, a2, pdl);
+    if (rc) return rc;
+    CU(cudaGetLastError());
+    return SWE_OK;
+  }
+  CU(launch(pdl, swe::k_prepare, dim3(1), dim3(32), s->st, s->d_ctl, prep));
+  const bool listed = stage_listed(s);
+  rc = listed ? launch_bc_lists<1>(s, s->d_A, mode == 0 ? 0 : 1, pdl, a1) : launch_bc(s, s->d_A, mode == 0 ? 0 : 1, pdl);
+  if (rc == SWE_OK) rc = launch_stage<1>(s, a1, pdl, listed);
+  if (rc == SWE_OK) rc = listed ? launch_bc_lists<2>(s, s->d_B, 1, pdl, a2) : launch_bc(s, s->d_B, 1, pdl);
+  if (rc == SWE_OK) rc = launch_stage<2>(s, a2, pdl, listed);
+  return rc;
 }
 
 constexpr int REDUCTION_BLOCKS = 16 * 148;
@@ -1154,7 +1212,7 @@ int swe_run(swe_sim* s, int n, double dt_fixed, double t_end, int* done) {
   int left = n;
   cudaGraphExec_t exec = nullptr;
   s->settle = s->settle_pref;
-  if (s->stage_impl == 1 && s->d_odry[0] && n >= 4 * chunk) {
+  if (s->stage_impl == 1 && !one_wave(s) && n >= 4 * chunk) {
     // the first chunk settles what it can; the settled-tile count of its
     // last step decides whether the rest (and later short runs) do
     s->settle = 1;

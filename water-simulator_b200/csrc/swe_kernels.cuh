@@ -122,32 +122,40 @@ struct PrepArgs {
   double fl_eta[4], fl_u[4];
 };
 
-__device__ __forceinline__ void prepare_one(Control* ctl, const PrepArgs& a) {
-  double dt;
-  if (a.mode == 0) dt = a.dt_host;
-  else if (a.mode == 2) dt = jmin(a.dt_host, a.t_end - ctl->t);
-  else if (a.mode == 4) dt = *a.dt_dev;
-  else {
-    const double inv = ctl->next_max;
-    double md = inv > 0 ? a.cfl / inv : INFINITY;
-    dt = (a.mode == 3) ? jmin(md, a.t_end - ctl->t) : md;
+__device__ __forceinline__ double prep_dt(const Control* ctl, const PrepArgs& a) {
+  if (a.mode == 0) return a.dt_host;
+  if (a.mode == 2) return jmin(a.dt_host, a.t_end - ctl->t);
+  if (a.mode == 4) return *a.dt_dev;
+  const double inv = ctl->next_max;
+  const double md = inv > 0 ? a.cfl / inv : INFINITY;
+  return (a.mode == 3) ? jmin(md, a.t_end - ctl->t) : md;
+}
+__device__ __forceinline__ bool prep_refused(double dt) { return !(dt > 0) || !isfinite(dt); }
+// The exterior surface and normal velocity of a Flather side.
+__device__ __forceinline__ void prep_flather(const Control* ctl, const PrepArgs& a, int s, double& eta, double& u) {
+  if (a.fl_kind[s] == 1) {
+    const double t = ctl->t;
+    double e = ctl->tide_msl[s];
+    for (int q = 0; q < ctl->tide_n[s]; q++)
+      e += ctl->tide_amp[s][q] * cos(ctl->tide_omega[s][q] * t - ctl->tide_phase[s][q] * 3.141592653589793 / 180);
+    eta = e;
+    u = ctl->tide_ucoef[s] * e;
+  } else {
+    eta = a.fl_eta[s];
+    u = a.fl_u[s];
   }
+}
+__device__ __forceinline__ void prepare_one(Control* ctl, const PrepArgs& a) {
+  const double dt = prep_dt(ctl, a);
   ctl->dt = dt;
-  ctl->stop = (!(dt > 0) || !isfinite(dt)) ? 1 : 0;
+  ctl->stop = prep_refused(dt) ? 1 : 0;
   ctl->settled = ctl->settled_next;
   ctl->settled_next = 0;
-  const double t = ctl->t;
   for (int s = 0; s < 4; s++) {
-    if (a.fl_kind[s] == 1) {
-      double e = ctl->tide_msl[s];
-      for (int q = 0; q < ctl->tide_n[s]; q++)
-        e += ctl->tide_amp[s][q] * cos(ctl->tide_omega[s][q] * t - ctl->tide_phase[s][q] * 3.141592653589793 / 180);
-      ctl->fl_eta[s] = e;
-      ctl->fl_u[s] = ctl->tide_ucoef[s] * e;
-    } else {
-      ctl->fl_eta[s] = a.fl_eta[s];
-      ctl->fl_u[s] = a.fl_u[s];
-    }
+    double e, u;
+    prep_flather(ctl, a, s, e, u);
+    ctl->fl_eta[s] = e;
+    ctl->fl_u[s] = u;
   }
 }
 
@@ -206,13 +214,14 @@ __device__ __forceinline__ Cell load_cell(const BCArgs& a, int i, int j) {
   return c;
 }
 
-// src/swe.mjs:1085-1115: ghost (i,j) on `side` from interior source s.
-__device__ __forceinline__ Cell flather_cell(const BCArgs& a, const Control* ctl, int side, Cell s) {
+// src/swe.mjs:1085-1115: ghost (i,j) on `side` from interior source s, with
+// the exterior surface fl_eta and normal velocity fl_u of every side.
+__device__ __forceinline__ Cell flather_cell(const BCArgs& a, const double* fl_eta, const double* fl_u, int side, Cell s) {
   Cell g;
   g.b = s.b;
   const double bed = g.b;
   const double hInt = s.h;
-  const double e0 = ctl->fl_eta[side], u0 = ctl->fl_u[side];
+  const double e0 = fl_eta[side], u0 = fl_u[side];
   if (hInt <= a.minDepth) { g.h = jmax0(e0 - bed); g.hu = 0; g.hv = 0; return g; }
   const double etaInt = bed + hInt;
   const double r = sqrt(SWE_G / hInt);
@@ -268,11 +277,11 @@ __host__ __device__ __forceinline__ int ghost_source(const int* kind, int nx, in
 }
 
 // Final value of the ghost (i, j).
-__device__ __forceinline__ Cell ghost_cell(const BCArgs& a, const Control* ctl, int i, int j) {
+__device__ __forceinline__ Cell ghost_cell(const BCArgs& a, const double* fl_eta, const double* fl_u, int i, int j) {
   int si, sj;
   const int tr = ghost_source(a.kind, a.nx, a.ny, i, j, si, sj);
   Cell c = load_cell(a, si, sj);
-  if (tr >= GT_FLATHER) return flather_cell(a, ctl, tr - GT_FLATHER, c);
+  if (tr >= GT_FLATHER) return flather_cell(a, fl_eta, fl_u, tr - GT_FLATHER, c);
   if (tr == GT_FLIPU) c.hu = -c.hu;
   else if (tr == GT_FLIPV) c.hv = -c.hv;
   return c;
@@ -295,7 +304,7 @@ __device__ __forceinline__ void apply_bc_range(const BCArgs& a, const Control* c
       const int r = p % 4;
       j = r < 2 ? -1 - r : a.ny + (r - 2);
     }
-    c = ghost_cell(a, ctl, i, j);
+    c = ghost_cell(a, ctl->fl_eta, ctl->fl_u, i, j);
     const int k = (j + 2) * a.W + (i + 2);
     a.b[k] = c.b; a.h[k] = c.h; a.hu[k] = c.hu; a.hv[k] = c.hv;
   }

@@ -149,6 +149,7 @@ struct FacesSmem {
   double xs[4][SPY][SPX + 1];                   // x slopes of cols i0 .. i0+SPX, rows j0 .. j0+SPY-1
   double ys[4][SPY + 1][SPX];                   // y slopes of cols i0 .. i0+SPX-1, rows j0 .. j0+SPY
   int wet, wild;                                // a cell of the tile or its halo has h != 0; one is not tame
+  double fl[2][4];                              // the Flather sides' exterior surface and velocity
 };
 
 // One cell of a faces tile: its source terms, its east x face and north y
@@ -263,41 +264,6 @@ __device__ __forceinline__ bool split_faces_settled(const SplitBufs& s, int tx, 
   return false;
 }
 
-// Faces and source terms of the tile (tx, ty).  Every thread of the CTA
-// calls it; it returns with the shared memory free for the next tile.
-__device__ __forceinline__ void split_faces_tile(const StageArgs& a, const SplitBufs& s, int tx, int ty,
-                                                 FacesSmem& sm, bool check_settled = true) {
-  const int W = a.W, H = a.H;
-  const int i0 = tx * SPX, j0 = ty * SPY;
-  const int t = threadIdx.x;
-  if (check_settled && split_faces_settled(s, tx, ty, t)) return;
-
-  // state of the tile and its halo (zero outside the grid): b, h, hu, hv
-  // copied into b, h, U, V with every copy of the thread in flight at once;
-  // once the tile is known to be wet, each thread turns the hu, hv it
-  // copied into velocities in place
-  for (int q = t; q < SSX * SSY; q += SP_THREADS) {
-    const int ly = q / SSX, lx = q - ly * SSX;
-    const int gi = i0 - 1 + lx, gj = j0 - 1 + ly;
-    if (gi >= 0 && gi < W && gj >= 0 && gj < H) {
-      const int k = gj * W + gi;
-      cp_async8(&sm.b[ly][lx + TCOL], a.b + k);
-      cp_async8(&sm.h[ly][lx + TCOL], a.h + k);
-      cp_async8(&sm.U[ly][lx + TCOL], a.hu + k);
-      cp_async8(&sm.V[ly][lx + TCOL], a.hv + k);
-    } else {
-      sm.b[ly][lx + TCOL] = 0; sm.h[ly][lx + TCOL] = 0; sm.U[ly][lx + TCOL] = 0; sm.V[ly][lx + TCOL] = 0;
-    }
-  }
-  if (t < SSY) {                                // column 0 (i0 - 2) is in the box but not needed
-    sm.b[t][0] = 0; sm.h[t][0] = 0; sm.U[t][0] = 0; sm.V[t][0] = 0;
-  }
-  if (t == 0) sm.wet = sm.wild = 0;
-  cp_async_wait_all();
-  __syncthreads();
-  split_faces_finish(a, s, tx, ty, sm, t);
-}
-
 // Limited slopes of eta, b, u, v at the state-tile cell (cy, cx) along x
 // (DX = 1) or y (DX = 0), src/swe.mjs:364-411: all four are 0 unless `on`
 // and the cell and both neighbours along the direction are wet.  LIM 0 is
@@ -324,6 +290,59 @@ __device__ __forceinline__ void tile_slopes(const FacesSmem& sm, int lim, double
     }
   }
   out[0] = sE; out[stride] = sB; out[2 * stride] = sU; out[3 * stride] = sV;
+}
+
+// ---- the ghost fill and the step's prepare within the face kernel ---------------
+// Every ghost value is a function of one interior cell, which no face kernel
+// writes, so a tile can form the ghosts of its box itself: those it owns go to
+// the state as well, as k_apply_bc would have left them.  And dt, the refusal
+// and the Flather values follow from the control block of the step before, so
+// every CTA of stage 1's face kernel forms what it needs of them, and the first
+// writes them down for the kernels after it.  That saves three of a step's eight
+// launches, each a few microseconds during which little else runs.
+struct GhostFill {
+  int on;                          // fill the ghosts of the stage's input
+  int prepare;                     // the step's first kernel: prepare it too
+  BCArgs bc;
+  PrepArgs prep;
+};
+// Whether the step goes on; the whole CTA calls it before anything else.
+__device__ __forceinline__ bool fill_enter(const GhostFill& F, Control* ctl) {
+  if (!F.prepare) return !ctl->stop;
+  const bool refused = prep_refused(prep_dt(ctl, F.prep));
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) prepare_one(ctl, F.prep);
+  return !refused;
+}
+__device__ __forceinline__ bool fill_touches(const GhostFill& F, int i0, int j0) {
+  return F.on && (i0 < 4 || i0 + SPX + 1 >= F.bc.W - 2 || j0 < 3 || j0 + SPY + 1 >= F.bc.H - 2);
+}
+// Before the barrier that ends the load of the box, and after it.
+__device__ __forceinline__ void fill_sides(const GhostFill& F, const Control* ctl, FacesSmem& sm, int i0, int j0) {
+  const int side = (int)threadIdx.x - 32;
+  if (!fill_touches(F, i0, j0) || side < 0 || side >= 4) return;
+  if (F.prepare) {
+    double e, u;
+    prep_flather(ctl, F.prep, side, e, u);
+    sm.fl[0][side] = e; sm.fl[1][side] = u;
+  } else {
+    sm.fl[0][side] = ctl->fl_eta[side]; sm.fl[1][side] = ctl->fl_u[side];
+  }
+}
+__device__ __forceinline__ void fill_tile(const GhostFill& F, FacesSmem& sm, int i0, int j0) {
+  if (!fill_touches(F, i0, j0)) return;            // uniform
+  const BCArgs& a = F.bc;
+  for (int q = threadIdx.x; q < SSXT * SSY; q += SP_THREADS) {
+    const int ly = q / SSXT, c = q - ly * SSXT, gi = i0 - 2 + c, gj = j0 - 1 + ly;
+    if (gi < 0 || gi >= a.W || gj < 0 || gj >= a.H) continue;
+    if (gi >= 2 && gi < a.W - 2 && gj >= 2 && gj < a.H - 2) continue;
+    const Cell g = ghost_cell(a, sm.fl[0], sm.fl[1], gi - 2, gj - 2);
+    sm.b[ly][c] = g.b; sm.h[ly][c] = g.h; sm.U[ly][c] = g.hu; sm.V[ly][c] = g.hv;
+    if (gi >= i0 && gi < i0 + SPX && gj >= j0 && gj < j0 + SPY) {
+      const size_t k = (size_t)gj * a.W + gi;
+      a.b[k] = g.b; a.h[k] = g.h; a.hu[k] = g.hu; a.hv[k] = g.hv;
+    }
+  }
+  __syncthreads();
 }
 
 // Slopes of a faces tile (src/swe.mjs:364-411): each thread its own cell in x
@@ -419,6 +438,44 @@ __device__ __forceinline__ void split_faces_finish(const StageArgs& a, const Spl
   }
 }
 
+// Faces and source terms of the tile (tx, ty).  Every thread of the CTA
+// calls it; it returns with the shared memory free for the next tile.
+__device__ __forceinline__ void split_faces_tile(const StageArgs& a, const SplitBufs& s, int tx, int ty,
+                                                 FacesSmem& sm, bool check_settled = true,
+                                                 const GhostFill* F = nullptr, const Control* ctl = nullptr) {
+  const int W = a.W, H = a.H;
+  const int i0 = tx * SPX, j0 = ty * SPY;
+  const int t = threadIdx.x;
+  if (check_settled && split_faces_settled(s, tx, ty, t)) return;
+
+  // state of the tile and its halo (zero outside the grid): b, h, hu, hv
+  // copied into b, h, U, V with every copy of the thread in flight at once;
+  // once the tile is known to be wet, each thread turns the hu, hv it
+  // copied into velocities in place
+  for (int q = t; q < SSX * SSY; q += SP_THREADS) {
+    const int ly = q / SSX, lx = q - ly * SSX;
+    const int gi = i0 - 1 + lx, gj = j0 - 1 + ly;
+    if (gi >= 0 && gi < W && gj >= 0 && gj < H) {
+      const int k = gj * W + gi;
+      cp_async8(&sm.b[ly][lx + TCOL], a.b + k);
+      cp_async8(&sm.h[ly][lx + TCOL], a.h + k);
+      cp_async8(&sm.U[ly][lx + TCOL], a.hu + k);
+      cp_async8(&sm.V[ly][lx + TCOL], a.hv + k);
+    } else {
+      sm.b[ly][lx + TCOL] = 0; sm.h[ly][lx + TCOL] = 0; sm.U[ly][lx + TCOL] = 0; sm.V[ly][lx + TCOL] = 0;
+    }
+  }
+  if (t < SSY) {                                // column 0 (i0 - 2) is in the box but not needed
+    sm.b[t][0] = 0; sm.h[t][0] = 0; sm.U[t][0] = 0; sm.V[t][0] = 0;
+  }
+  if (t == 0) sm.wet = sm.wild = 0;
+  if (F) fill_sides(*F, ctl, sm, i0, j0);
+  cp_async_wait_all();
+  __syncthreads();
+  if (F) fill_tile(*F, sm, i0, j0);
+  split_faces_finish(a, s, tx, ty, sm, t);
+}
+
 // ---- the state tile by tensor-map copies (TMA) --------------------------------
 // One thread issues four 2-D bulk tensor copies (b, h, hu, hv of the stage
 // input) of the box SSXT x SSY at column i0 - 2 (even, so its first element
@@ -459,6 +516,9 @@ __device__ __forceinline__ void tma_load_tile(void* dst, const CUtensorMap* map,
       ::"r"(smem_addr(dst)), "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(smem_addr(bar))
       : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
+}
 // Until the phase `parity` of bar completes, at most TMA_WAIT_TRIES polls
 // (each of which may suspend the thread for a while).
 constexpr int TMA_WAIT_TRIES = 1 << 22;
@@ -484,31 +544,32 @@ __device__ __forceinline__ bool tile_wait(unsigned long long* bar, unsigned pari
   return false;
 }
 
-// split_faces_tile with the state tile fetched by tensor-map copies.  bar
-// is an initialised mbarrier in shared memory and parity its phase, flipped
-// here for the next tile.  A copy that does not complete within the bound
-// sets bit 4 of Control::status and leaves the tile's faces unwritten.
-__device__ __forceinline__ void split_faces_tile_tma(const StageArgs& a, const SplitBufs& s, int tx, int ty,
-                                                     FacesSmem& sm, const TileMaps& maps,
-                                                     unsigned long long* bar, unsigned& parity, Control* ctl,
-                                                     bool check_settled = true) {
-  const int t = threadIdx.x;
-  if (check_settled && split_faces_settled(s, tx, ty, t)) return;
-  if (t == 0) {
-    sm.wet = sm.wild = 0;
-    // the generic-proxy accesses of a previous tile come before the copy's writes
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    mbar_expect_tx(bar, TILE_TX_BYTES);
-    const int x = tx * SPX - 2, y = ty * SPY - 1;
-    tma_load_tile(&sm.b[0][0], &maps.m[0], x, y, bar);
-    tma_load_tile(&sm.h[0][0], &maps.m[1], x, y, bar);
-    tma_load_tile(&sm.U[0][0], &maps.m[2], x, y, bar);
-    tma_load_tile(&sm.V[0][0], &maps.m[3], x, y, bar);
-  }
+// split_faces_tile with the state tile fetched by tensor-map copies, in two
+// parts: start_box, in which thread 0 starts them, and the rest.  bar is an
+// initialised mbarrier in shared memory and parity its phase, flipped here for
+// the next tile.  A copy that does not complete within the bound sets bit 4 of
+// Control::status and leaves the tile's faces unwritten.
+__device__ __forceinline__ void start_box(FacesSmem& sm, int tx, int ty, const TileMaps& maps, unsigned long long* bar) {
+  if (threadIdx.x != 0) return;
+  sm.wet = sm.wild = 0;
+  // the generic-proxy accesses of a previous tile come before the copy's writes
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  mbar_expect_tx(bar, TILE_TX_BYTES);
+  const int x = tx * SPX - 2, y = ty * SPY - 1;
+  tma_load_tile(&sm.b[0][0], &maps.m[0], x, y, bar);
+  tma_load_tile(&sm.h[0][0], &maps.m[1], x, y, bar);
+  tma_load_tile(&sm.U[0][0], &maps.m[2], x, y, bar);
+  tma_load_tile(&sm.V[0][0], &maps.m[3], x, y, bar);
+}
+__device__ __forceinline__ void split_faces_started(const StageArgs& a, const SplitBufs& s, int tx, int ty,
+                                                    FacesSmem& sm, unsigned long long* bar, unsigned& parity,
+                                                    Control* ctl, const GhostFill* F = nullptr) {
+  if (F) fill_sides(*F, ctl, sm, tx * SPX, ty * SPY);
   const bool ok = tile_wait(bar, parity, ctl);
   parity ^= 1u;
   if (!ok) return;                                  // uniform: give up on the tile
-  split_faces_finish(a, s, tx, ty, sm, t);
+  if (F) fill_tile(*F, sm, tx * SPX, ty * SPY);
+  split_faces_finish(a, s, tx, ty, sm, threadIdx.x);
 }
 
 // CTAs per SM of the face kernels: 4, which caps them at 64 registers.  The
@@ -519,25 +580,45 @@ __device__ __forceinline__ void split_faces_tile_tma(const StageArgs& a, const S
 #ifndef SWE_SPLIT_FACES_MIN_BLOCKS
 #define SWE_SPLIT_FACES_MIN_BLOCKS 4
 #endif
-__global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_MIN_BLOCKS)
-k_split_faces(StageArgs a, SplitBufs s, Control* ctl) {
+// A grid of at most 3 CTAs per SM has no use for a fourth's place and takes the
+// kernel with 80 registers, which spills nothing: 100 steps of 256 x 256 3.89 ->
+// 3.49 ms.
+template <int MIN_BLOCKS, bool FILL>
+__global__ void __launch_bounds__(SP_THREADS, MIN_BLOCKS)
+k_split_faces(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ GhostFill F) {
   pdl_enter();
-  if (ctl->stop) return;
+  if (FILL ? !fill_enter(F, ctl) : ctl->stop) return;
   __shared__ FacesSmem sm;
-  split_faces_tile(a, s, blockIdx.x, blockIdx.y, sm);
+  split_faces_tile(a, s, blockIdx.x, blockIdx.y, sm, true, FILL ? &F : nullptr, ctl);
 }
 
 // The face kernel with its state tile fetched by tensor-map copies.
-__global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_MIN_BLOCKS)
-k_split_faces_tma(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ TileMaps maps) {
+template <int MIN_BLOCKS, bool FILL>
+__global__ void __launch_bounds__(SP_THREADS, MIN_BLOCKS)
+k_split_faces_tma(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ TileMaps maps,
+                  const __grid_constant__ GhostFill F) {
   __shared__ FacesSmem sm;
   __shared__ alignas(8) unsigned long long bar;
-  if (threadIdx.x == 0) mbar_init(&bar, 1);        // before the wait: touches no global memory
-  pdl_enter();
-  if (ctl->stop) return;
-  __syncthreads();
+  if (threadIdx.x == 0) {                          // before the wait: touches no global memory
+    mbar_init(&bar, 1);
+    for (int q = 0; q < 4; q++) tma_prefetch_map(&maps.m[q]);
+  }
+  const int tx = blockIdx.x, ty = blockIdx.y;
   unsigned parity = 0;
-  split_faces_tile_tma(a, s, blockIdx.x, blockIdx.y, sm, maps, &bar, parity, ctl);
+  pdl_enter();
+  // without records the copies come first: whether the step goes on is known a
+  // memory latency later
+  const bool first = !s.odry_in;
+  if (first) start_box(sm, tx, ty, maps, &bar);
+  if (FILL ? !fill_enter(F, ctl) : ctl->stop) {
+    if (first) tile_wait(&bar, parity, ctl);
+    return;
+  }
+  if (!first) {
+    if (split_faces_settled(s, tx, ty, threadIdx.x)) return;
+    start_box(sm, tx, ty, maps, &bar);
+  }
+  split_faces_started(a, s, tx, ty, sm, &bar, parity, ctl, FILL ? &F : nullptr);
 }
 
 // ---- the face kernel over a list of the tiles it must compute ----------------
@@ -676,7 +757,8 @@ k_split_faces_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_cons
   __syncthreads();
   const int tile = list[blockIdx.x];
   unsigned parity = 0;
-  split_faces_tile_tma(a, s, tile % s.ntx, tile / s.ntx, sm, maps, &bar, parity, ctl, false);
+  start_box(sm, tile % s.ntx, tile / s.ntx, maps, &bar);
+  split_faces_started(a, s, tile % s.ntx, tile / s.ntx, sm, &bar, parity, ctl);
 }
 __global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_MIN_BLOCKS)
 k_split_faces_list(StageArgs a, SplitBufs s, Control* ctl, const int* list, const int* count) {
@@ -775,6 +857,24 @@ __device__ __forceinline__ void stage_cells(const StageArgs& a, const SplitBufs&
     }
   });
 }
+// Staging by tensor maps: thread 0 starts the copies, bar counts their bytes.
+__device__ __forceinline__ void stage_cells_tma(const StageArgs& a, CellsSmem& sm, int i0, int j0, const CellMaps& maps,
+                                                unsigned long long* bar) {
+  if (threadIdx.x != 0) return;
+  // the generic-proxy accesses of the shared memory come before the copies' writes
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  mbar_expect_tx(bar, CELL_TX_BYTES + (a.sph ? CELL_TG_BYTES : 0) + (a.W & 1 ? 0 : CELL_HR_BYTES));
+  const int x = i0 - 2;
+  CellFaceTiles& ft = sm.ft;
+  tma_load_tile(&ft.xm[0][0], &maps.m[CM_XM], x, j0 - 1, bar);
+  tma_load_tile(&ft.ym[0][0], &maps.m[CM_YM], x, j0 - 2, bar);
+  if (!(a.W & 1)) tma_load_tile(&ft.hr[0][0], &maps.m[CM_H], x, j0 - 1, bar);
+  for (int q = 0; q < 3; q++) {
+    tma_load_tile(&ft.xt[q][0][0], &maps.m[CM_XT + q], x, j0, bar);
+    tma_load_tile(&ft.yt[q][0][0], &maps.m[CM_YT + q], i0, j0 - 1, bar);
+    if (q < 2 || a.sph) tma_load_tile(&ft.tb[q][0][0], &maps.m[CM_TB + q], i0, j0, bar);
+  }
+}
 // After the tensor-map copies: +0 for what dry tiles own (their faces were
 // not written).
 __device__ __forceinline__ void zero_dry_staged(const StageArgs& a, const SplitBufs& s, CellsSmem& sm, int i0, int j0) {
@@ -807,6 +907,7 @@ __device__ __forceinline__ double split_theta(const StageArgs& a, const CellFace
   return th;
 }
 
+constexpr int CLOSE_BLOCKS = 32;
 // The close of a stage by one block: the partials of its `nparts` tiles
 // reduced in a fixed order (strided per thread, then a fixed tree), so the
 // sums are the same in every run.
@@ -1023,8 +1124,10 @@ __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& 
 
 // Limiter, gather, update and epilogue of the tile (tx, ty), which holds
 // partial slot `part` of the `nparts` of its grid.  With `ticket`, the last
-// tile of the grid to finish closes the step; without, the step is closed
-// by k_split_close after the launch.  Every thread of the CTA calls it.
+// tile of the grid to finish closes the stage; without, a kernel after the launch
+// closes the step (in the step of one grid that is faster at every size: the
+// ticket's fence is in every tile's way; 256 x 256, 100 steps: 3.84 against
+// 3.75 ms).  Every thread of the CTA calls it.
 // SETTLE: tiles may settle (below); without it the function is the plain
 // tile update, which grids with little dry land run faster.
 // The limiter ring's and the gather's inputs are staged into sm.ft once the
@@ -1040,6 +1143,8 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
   const int W = a.W, H = a.H;
   const int i0 = tx * SPX, j0 = ty * SPY;
   const int t = threadIdx.x;
+  constexpr bool EARLY = TMA && !SETTLE;          // no tile is left out, few are folded: copy before the flags are known
+  if (EARLY) stage_cells_tma(a, sm, i0, j0, *maps, bar);
   const double dt = ctl->dt;
   const int lx = t % SPX, ly = t / SPX;
   const int gi = i0 + lx, gj = j0 + ly;
@@ -1082,6 +1187,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
     anyDry = anyDry || f == 1;
   }
   const bool fold = allDry && a.dryfold;          // uniform across the CTA
+  if (EARLY && fold && !tile_wait(bar, 0, ctl)) return;   // nothing of the copies is used, but they must have landed
   // A folded tile settles without its state.  Its input has h = +-0 on the
   // tile (the flags), and so does U0 in stage 2 (the output record, which
   // describes U0 as this kernel wrote it in the previous step).  Every face
@@ -1126,21 +1232,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
   }
   if (!fold) {
     if (TMA) {
-      if (t == 0) {
-        // the generic-proxy accesses of the shared memory come before the copies' writes
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        mbar_expect_tx(bar, CELL_TX_BYTES + (a.sph ? CELL_TG_BYTES : 0) + (a.W & 1 ? 0 : CELL_HR_BYTES));
-        const int x = i0 - 2;
-        CellFaceTiles& ft = sm.ft;
-        tma_load_tile(&ft.xm[0][0], &maps->m[CM_XM], x, j0 - 1, bar);
-        tma_load_tile(&ft.ym[0][0], &maps->m[CM_YM], x, j0 - 2, bar);
-        if (!(a.W & 1)) tma_load_tile(&ft.hr[0][0], &maps->m[CM_H], x, j0 - 1, bar);
-        for (int q = 0; q < 3; q++) {
-          tma_load_tile(&ft.xt[q][0][0], &maps->m[CM_XT + q], x, j0, bar);
-          tma_load_tile(&ft.yt[q][0][0], &maps->m[CM_YT + q], i0, j0 - 1, bar);
-          if (q < 2 || a.sph) tma_load_tile(&ft.tb[q][0][0], &maps->m[CM_TB + q], i0, j0, bar);
-        }
-      }
+      if (!EARLY) stage_cells_tma(a, sm, i0, j0, *maps, bar);
       if (a.W & 1) stage_depths(a, sm, i0, j0);     // no tensor map of the state
       cp_async_wait_all();
       if (!tile_wait(bar, 0, ctl)) return;          // uniform: give up on the tile
@@ -1233,7 +1325,6 @@ k_split_cells(StageArgs a, SplitBufs s, Control* ctl) {
 // only there, so it is summed here too (the same order as MODE 1 sums it)
 // and stage 1 needs no close of its own.  scratch holds 3 * CLOSE_BLOCKS
 // doubles.
-constexpr int CLOSE_BLOCKS = 32;
 template <int MODE>
 __global__ void __launch_bounds__(SP_THREADS) k_split_close_multi(StageArgs a, Control* ctl, int nparts,
                                                                     double* scratch) {
@@ -1296,6 +1387,46 @@ __global__ void __launch_bounds__(SP_THREADS) k_split_close_multi(StageArgs a, C
   }
 }
 
+// The same by one block of a warp per run, for grids of at most 64 slots a run:
+// no ticket and no second reading.
+constexpr int CLOSE_TILES = 64 * CLOSE_BLOCKS;
+__global__ void __launch_bounds__(32 * CLOSE_BLOCKS) k_split_close_step(StageArgs a, Control* ctl, int nparts) {
+  __shared__ double part[3][CLOSE_BLOCKS];
+  pdl_enter();
+  if (ctl->stop) return;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int chunk = (nparts + CLOSE_BLOCKS - 1) / CLOSE_BLOCKS, q0 = w * chunk, q1 = min(nparts, q0 + chunk);
+  double m = 0, v[2][2];                         // [stage][half of the run]
+  for (int r = 0; r < 2; r++) {
+    const int q = q0 + r * 32 + lane;
+    v[0][r] = q < q1 ? a.part_fl1[q] : 0;
+    v[1][r] = q < q1 ? a.part_fl2[q] : 0;
+    if (q < q1) m = fmax(m, a.part_max[q]);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+    for (int r = 0; r < 2; r++)
+      for (int g = 0; g < 2; g++) v[g][r] += __shfl_down_sync(0xffffffffu, v[g][r], o);
+  }
+  if (lane == 0) { part[0][w] = m; part[1][w] = v[0][0] + v[0][1]; part[2][w] = v[1][0] + v[1][1]; }
+  __syncthreads();
+  if (w) return;
+  m = part[0][t];
+  double f1 = part[1][t], f = part[2][t];
+  for (int o = 16; o > 0; o >>= 1) {
+    m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+    f += __shfl_down_sync(0xffffffffu, f, o);
+    f1 += __shfl_down_sync(0xffffffffu, f1, o);
+  }
+  if (t == 0) {
+    ctl->floored1 = f1;
+    ctl->next_max = m;
+    ctl->mass_floored = f1 + f;
+    ctl->t = ctl->t + ctl->dt;
+    ctl->steps = ctl->steps + 1;
+  }
+}
+
 // The cell kernel with its face and depth inputs staged by tensor-map copies
 // (maps over this simulation's own buffers only, no multicast).
 template <int MODE, bool SETTLE = false>
@@ -1303,7 +1434,10 @@ __global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_CELLS_MIN_BLOCKS)
 k_split_cells_tma(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ CellMaps maps) {
   __shared__ CellsSmem sm;
   __shared__ alignas(8) unsigned long long bar;
-  if (threadIdx.x == 0) mbar_init(&bar, 1);        // before the wait: touches no global memory
+  if (threadIdx.x == 0) {                          // before the wait: touches no global memory
+    mbar_init(&bar, 1);
+    for (int q = 0; q < CM_COUNT; q++) if (q != CM_H || !(a.W & 1)) tma_prefetch_map(&maps.m[q]);
+  }
   pdl_enter();
   if (ctl->stop) return;
   split_cells_tile<MODE, SETTLE, true>(a, s, ctl, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x,
