@@ -81,6 +81,8 @@ struct swe_sim {
   double* d_coef = nullptr;                        // weights of swe_eta_projection (ny)
   int diag_order = SWE_DIAG_REFERENCE;
   double* d_sponge = nullptr;
+  void* d_frame = nullptr;                         // swe_host::frame_of
+  size_t frame_bytes = 0;
   swe::Control* d_ctl = nullptr;
   int bc[4];
   int fl_kind[4] = {0, 0, 0, 0};
@@ -667,6 +669,18 @@ void view_of(swe_sim* s, int* dims, double* opts, const double** b, const double
   *h = field_ptr(s, SWE_FIELD_H);
   *st = s->st;
 }
+// A device buffer of at least `bytes` that the handle keeps for the frames
+// drawn from it (one at a time: the calls on a handle come from one thread, and
+// a frame's call ends when the frame is complete).
+int frame_of(swe_sim* s, size_t bytes, unsigned char** out) {
+  if (s->frame_bytes < bytes) {
+    if (s->d_frame) { CU(cudaFree(s->d_frame)); s->d_frame = nullptr; s->frame_bytes = 0; }
+    CU(cudaMalloc(&s->d_frame, bytes));
+    s->frame_bytes = bytes;
+  }
+  *out = static_cast<unsigned char*>(s->d_frame);
+  return SWE_OK;
+}
 }  // namespace swe_host
 
 namespace {
@@ -704,6 +718,7 @@ void free_all(swe_sim* s) {
   for (double** p : ptrs) if (*p) { cudaFree(*p); *p = nullptr; }
   if (s->d_ctl) cudaFree(s->d_ctl);
   if (s->d_vol) cudaFree(s->d_vol);
+  if (s->d_frame) cudaFree(s->d_frame);
   if (s->st) cudaStreamDestroy(s->st);
 }
 

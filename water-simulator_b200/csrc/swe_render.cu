@@ -21,12 +21,14 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <algorithm>
 #include <string>
 #include <vector>
 
 namespace swe_host {
 void set_error(const std::string& msg);
 void view_of(swe_sim* s, int* dims, double* opts, const double** b, const double** h, cudaStream_t* st);
+int frame_of(swe_sim* s, size_t bytes, unsigned char** out);
 }  // namespace swe_host
 
 struct swe_globe_lut {
@@ -58,8 +60,10 @@ constexpr int RAMP_N = 1025;                    // odd: entry (N-1)/2 is mean se
 constexpr int RAMP_MID = (RAMP_N - 1) >> 1;
 constexpr double PI_D = 3.141592653589793;
 
-__constant__ double c_ramp[3 * RAMP_N];         // src/render.mjs RAMP (unclamped sRGB)
-__constant__ unsigned char c_cbytes[3 * RAMP_N]; // src/globe.mjs CBYTES
+// The tables lie in global memory, not in constant memory, which serves one
+// address at a time: a warp's pixels look up different colours.
+__device__ double g_ramp[3 * RAMP_N];           // src/render.mjs RAMP (unclamped sRGB)
+__device__ __align__(4) unsigned char g_cbytes[4 * RAMP_N];   // src/globe.mjs CBYTES, RGBA
 
 // ---- the colour tables (host) ------------------------------------------------
 // CIE L*a*b* (D65) -> sRGB, unclamped (src/render.mjs:98-110).
@@ -130,6 +134,8 @@ void build_tables(Tables* t) {
   }
 }
 
+bool aligned4(const void* p) { return (reinterpret_cast<size_t>(p) & 3) == 0; }
+
 int ensure_tables() {
   static int done = -1;                        // per process; the constant banks are per device
   static int done_dev = -1;
@@ -138,8 +144,13 @@ int ensure_tables() {
   if (done == 1 && done_dev == dev) return SWE_OK;
   static Tables t;
   build_tables(&t);
-  RCU(cudaMemcpyToSymbol(c_ramp, t.ramp, sizeof t.ramp));
-  RCU(cudaMemcpyToSymbol(c_cbytes, t.cbytes, sizeof t.cbytes));
+  static unsigned char rgba[4 * RAMP_N];
+  for (int i = 0; i < RAMP_N; i++) {
+    for (int c = 0; c < 3; c++) rgba[4 * i + c] = t.cbytes[3 * i + c];
+    rgba[4 * i + 3] = 255;
+  }
+  RCU(cudaMemcpyToSymbol(g_ramp, t.ramp, sizeof t.ramp));
+  RCU(cudaMemcpyToSymbol(g_cbytes, rgba, sizeof rgba));
   done = 1;
   done_dev = dev;
   return SWE_OK;
@@ -147,114 +158,140 @@ int ensure_tables() {
 
 // ---- WaterView map panel -------------------------------------------------------
 // surfaceColour (src/render.mjs:142-153): the RAMP entry for elevation v.
-__device__ __forceinline__ int ramp_offset(double v, double scale) {
+__device__ __forceinline__ int ramp_index(double v, double scale) {
   const double t = js_max(-1, js_min(1, v / scale));
   if (t != t) return -1;                       // NaN: the reference reads undefined -> 0
-  const double q = js_round(fabs(t) * RAMP_MID);
-  return 3 * (t >= 0 ? RAMP_MID + (int)q : RAMP_MID - (int)q);
+  const int q = (int)js_round(fabs(t) * RAMP_MID);
+  return t >= 0 ? RAMP_MID + q : RAMP_MID - q;
 }
 
-__global__ void k_render_map(int nx, int ny, int W, const double* __restrict__ b, const double* __restrict__ h,
-                             double minDepth, double msl, double scale, int showBed,
-                             unsigned char* __restrict__ out) {
-  const long long n = (long long)nx * ny;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(p / nx), i = (int)(p - (long long)j * nx);
-    const long long k = (long long)(j + 2) * W + (i + 2);
-    const long long o = 4 * ((long long)(ny - 1 - j) * nx + i);     // +y up on screen
-    const double depth = h[k], bk = b[k];
-    double c0, c1, c2;
-    if (depth <= minDepth) {                    // landColour, src/render.mjs:193-196
-      const double t = js_max(0, js_min(1, bk / 6));
-      c0 = 96 + 70 * t; c1 = 88 + 62 * t; c2 = 74 + 52 * t;
-    } else {
-      const int ro = ramp_offset(bk + depth - msl, scale);
-      if (ro < 0) { c0 = c1 = c2 = NAN; }
-      else { c0 = c_ramp[ro]; c1 = c_ramp[ro + 1]; c2 = c_ramp[ro + 2]; }
-      if (showBed) {                            // STILL depth shading, src/render.mjs:238-245
-        const double still = js_max(0, msl - bk);
-        const double shade = 0.55 + 0.45 * exp(-still / 12);
-        c0 = c0 * shade; c1 = c1 * shade; c2 = c2 * shade;
+__device__ __forceinline__ unsigned pixel(unsigned char r, unsigned char g, unsigned char b) {
+  return 0xff000000u | (unsigned)b << 16 | (unsigned)g << 8 | r;
+}
+// Pixel p of a frame: one store where the frame lies on a 4-byte boundary (the
+// caller's device buffer may not).
+__device__ __forceinline__ void put_pixel(unsigned char* out, long long p, unsigned rgba, bool aligned) {
+  if (aligned) reinterpret_cast<unsigned*>(out)[p] = rgba;
+  else
+    for (int c = 0; c < 4; c++) out[4 * p + c] = (unsigned char)(rgba >> (8 * c));
+}
+
+// A block per row, or as many as there are.
+constexpr int FRAME_THREADS = 256;
+__global__ void __launch_bounds__(FRAME_THREADS)
+k_render_map(int nx, int ny, int W, const double* __restrict__ b, const double* __restrict__ h,
+             double minDepth, double msl, double scale, int showBed, unsigned char* __restrict__ out, bool aligned) {
+  for (int j = blockIdx.x; j < ny; j += gridDim.x) {
+    const size_t row = (size_t)(j + 2) * W + 2;
+    for (int i = threadIdx.x; i < nx; i += FRAME_THREADS) {
+      const double depth = h[row + i], bk = b[row + i];
+      double c0, c1, c2;
+      if (depth <= minDepth) {                    // landColour, src/render.mjs:193-196
+        const double t = js_max(0, js_min(1, bk / 6));
+        c0 = 96 + 70 * t; c1 = 88 + 62 * t; c2 = 74 + 52 * t;
+      } else {
+        const int ro = ramp_index(bk + depth - msl, scale);
+        if (ro < 0) { c0 = c1 = c2 = NAN; }
+        else { c0 = __ldg(g_ramp + 3 * ro); c1 = __ldg(g_ramp + 3 * ro + 1); c2 = __ldg(g_ramp + 3 * ro + 2); }
+        if (showBed) {                            // STILL depth shading, src/render.mjs:238-245
+          const double still = js_max(0, msl - bk);
+          const double shade = 0.55 + 0.45 * exp(-still / 12);
+          c0 = c0 * shade; c1 = c1 * shade; c2 = c2 * shade;
+        }
       }
+      put_pixel(out, (long long)(ny - 1 - j) * nx + i, pixel(clamp_u8(c0), clamp_u8(c1), clamp_u8(c2)), aligned);  // +y up
     }
-    out[o] = clamp_u8(c0); out[o + 1] = clamp_u8(c1); out[o + 2] = clamp_u8(c2); out[o + 3] = 255;
   }
 }
 
 // ---- renderGlobe ------------------------------------------------------------------
-constexpr int FRAME_THREADS = 256;
 constexpr double LAND_SAT = 2500;               // src/globe.mjs:680-682
 __constant__ double c_land_lo[3] = {92, 84, 70};
 __constant__ double c_land_hi[3] = {188, 172, 144};
 
 // colOfLon (src/globe.mjs:547-550), with the rotation applied as frameLon()'s
 // addition (src/globe.mjs:741).
-__device__ __forceinline__ long long col_of_lon(double lonDeg, int nx) {
+__device__ __forceinline__ int col_of_lon(double lonDeg, int nx) {
   const double i = floor((lonDeg + 180) * nx / 360);
+  if (i >= 0 && i < nx) return (int)i;
+  if (i >= nx && i < 2.0 * nx) return (int)(i - nx);
   const long long ii = (long long)i;
-  return ((ii % nx) + nx) % nx;
+  return (int)(((ii % nx) + nx) % nx);
 }
 
-__global__ void k_render_globe(int count, const int* __restrict__ px, const double* __restrict__ lon,
-                               const int* __restrict__ rowbase, const float* __restrict__ lit, int nx,
-                               const double* __restrict__ b, const double* __restrict__ h, double minDepth,
-                               double rot, double scale, double msl, int landLight, unsigned char* __restrict__ out,
-                               double* __restrict__ part, unsigned int* ticket, double* __restrict__ stats) {
-  __shared__ double s_lo[FRAME_THREADS], s_hi[FRAME_THREADS];
-  __shared__ unsigned int s_wet[FRAME_THREADS], s_dry[FRAME_THREADS], s_sat[FRAME_THREADS];
-  __shared__ bool s_last;
-  double lo = INFINITY, hi = -INFINITY;
-  unsigned int wet = 0, dry = 0, sat = 0;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
-    const long long k = rowbase[p] + col_of_lon(lon[p] + rot, nx);
-    const int o = px[p];
-    const double hk = h[k];
-    if (hk <= minDepth) {
-      dry++;
-      const double t = js_max(0, js_min(1, b[k] / LAND_SAT));
-      const double s = landLight ? 0.30 + 0.70 * (double)lit[p] : 1;
-      for (int c = 0; c < 3; c++) out[o + c] = clamp_u8((c_land_lo[c] + (c_land_hi[c] - c_land_lo[c]) * t) * s);
-      out[o + 3] = 255;
-    } else {
-      wet++;
-      const double e = b[k] + hk - msl;
-      if (e < lo) lo = e;
-      if (e > hi) hi = e;
-      if (e >= scale || e <= -scale) sat++;
-      const int co = ramp_offset(e, scale);     // colourOffset, src/globe.mjs:665-669
-      for (int c = 0; c < 3; c++) out[o + c] = co < 0 ? 0 : c_cbytes[co + c];
-      out[o + 3] = 255;
-    }
+// A frame's statistics: the least and largest elevation and three counts.
+struct FrameStats { double lo, hi; unsigned int wet, dry, sat; };
+__device__ __forceinline__ FrameStats both(FrameStats a, const FrameStats& b) {
+  return {fmin(a.lo, b.lo), fmax(a.hi, b.hi), a.wet + b.wet, a.dry + b.dry, a.sat + b.sat};
+}
+// Over the block, in thread 0.
+__device__ __forceinline__ FrameStats block_stats(FrameStats v, FrameStats* warps) {
+  const unsigned all = 0xffffffffu;
+  for (int o = 16; o > 0; o >>= 1) {
+    FrameStats u = {__shfl_down_sync(all, v.lo, o), __shfl_down_sync(all, v.hi, o), __shfl_down_sync(all, v.wet, o),
+                    __shfl_down_sync(all, v.dry, o), __shfl_down_sync(all, v.sat, o)};
+    v = both(v, u);
   }
-  s_lo[threadIdx.x] = lo; s_hi[threadIdx.x] = hi;
-  s_wet[threadIdx.x] = wet; s_dry[threadIdx.x] = dry; s_sat[threadIdx.x] = sat;
+  if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int w = FRAME_THREADS / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      s_lo[threadIdx.x] = fmin(s_lo[threadIdx.x], s_lo[threadIdx.x + w]);
-      s_hi[threadIdx.x] = fmax(s_hi[threadIdx.x], s_hi[threadIdx.x + w]);
-      s_wet[threadIdx.x] += s_wet[threadIdx.x + w];
-      s_dry[threadIdx.x] += s_dry[threadIdx.x + w];
-      s_sat[threadIdx.x] += s_sat[threadIdx.x + w];
+  if (threadIdx.x == 0)
+    for (int w = 1; w < FRAME_THREADS / 32; w++) v = both(v, warps[w]);
+  return v;
+}
+
+// Bound by the gather of the pixels' cells and, at a million pixels, by the
+// frame's way to the host.  The last block combines the blocks' statistics
+// with all of its threads: one thread reading them in turn took most of the
+// launch (900 x 900 pixels: 140 -> 18 us).
+__global__ void __launch_bounds__(FRAME_THREADS)
+k_render_globe(int count, const int* __restrict__ px, const double* __restrict__ lon,
+               const int* __restrict__ rowbase, const float* __restrict__ lit, int nx,
+               const double* __restrict__ b, const double* __restrict__ h, double minDepth,
+               double rot, double scale, double msl, int landLight, unsigned char* __restrict__ out, bool aligned,
+               FrameStats* __restrict__ part, unsigned int* ticket, double* __restrict__ stats) {
+  __shared__ FrameStats warps[FRAME_THREADS / 32];
+  __shared__ bool s_last;
+  FrameStats v = {INFINITY, -INFINITY, 0, 0, 0};
+  for (int p = blockIdx.x * FRAME_THREADS + threadIdx.x; p < count; p += gridDim.x * FRAME_THREADS) {
+    const long long k = rowbase[p] + col_of_lon(lon[p] + rot, nx);
+    const double hk = h[k], bk = b[k];
+    unsigned rgba;
+    if (hk <= minDepth) {
+      v.dry++;
+      const double t = js_max(0, js_min(1, bk / LAND_SAT));
+      const double s = landLight ? 0.30 + 0.70 * (double)lit[p] : 1;
+      unsigned char c[3];
+      for (int q = 0; q < 3; q++) c[q] = clamp_u8((c_land_lo[q] + (c_land_hi[q] - c_land_lo[q]) * t) * s);
+      rgba = pixel(c[0], c[1], c[2]);
+    } else {
+      v.wet++;
+      const double e = bk + hk - msl;
+      if (e < v.lo) v.lo = e;
+      if (e > v.hi) v.hi = e;
+      if (e >= scale || e <= -scale) v.sat++;
+      const int co = ramp_index(e, scale);      // colourOffset, src/globe.mjs:665-669
+      rgba = co < 0 ? pixel(0, 0, 0) : __ldg(reinterpret_cast<const unsigned*>(g_cbytes) + co);
     }
-    __syncthreads();
+    put_pixel(out, px[p] / 4, rgba, aligned);
   }
+  v = block_stats(v, warps);
   if (threadIdx.x == 0) {
-    double* q = part + 5 * blockIdx.x;
-    q[0] = s_lo[0]; q[1] = s_hi[0]; q[2] = s_wet[0]; q[3] = s_dry[0]; q[4] = s_sat[0];
+    part[blockIdx.x] = v;
     __threadfence();
     s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (s_last && threadIdx.x == 0) {             // the last block closes the frame (no waiting)
-    __threadfence();
-    double L = INFINITY, Hh = -INFINITY, Wt = 0, D = 0, S = 0;
-    for (unsigned int g = 0; g < gridDim.x; g++) {
-      const volatile double* q = part + 5 * g;
-      L = fmin(L, q[0]); Hh = fmax(Hh, q[1]); Wt += q[2]; D += q[3]; S += q[4];
-    }
-    stats[0] = Wt; stats[1] = D; stats[4] = L; stats[5] = Hh; stats[6] = S;
-    stats[7] = Wt > 0 ? S / Wt : 0;
+  if (!s_last) return;                          // the last block closes the frame (no waiting)
+  __threadfence();
+  v = {INFINITY, -INFINITY, 0, 0, 0};
+  for (unsigned int g = threadIdx.x; g < gridDim.x; g += FRAME_THREADS) {
+    const FrameStats* q = part + g;
+    v = both(v, {__ldcg(&q->lo), __ldcg(&q->hi), __ldcg(&q->wet), __ldcg(&q->dry), __ldcg(&q->sat)});
+  }
+  v = block_stats(v, warps);
+  if (threadIdx.x == 0) {
+    stats[0] = v.wet; stats[1] = v.dry; stats[4] = v.lo; stats[5] = v.hi; stats[6] = v.sat;
+    stats[7] = v.wet > 0 ? (double)v.sat / (double)v.wet : 0;
     *ticket = 0;
   }
 }
@@ -303,14 +340,11 @@ int swe_render_map(swe_sim* s, double msl, double scale, int show_bed, unsigned 
   if (rc) return rc;
   const size_t bytes = (size_t)4 * nx * ny;
   unsigned char* out = static_cast<unsigned char*>(rgba_device);
-  bool own = false;
-  if (!out) { RCU(cudaMallocAsync(reinterpret_cast<void**>(&out), bytes, st)); own = true; }
-  long long blocks = ((long long)nx * ny + 255) / 256;
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  k_render_map<<<(int)blocks, 256, 0, st>>>(nx, ny, W, b, h, opts[0], msl, scale, show_bed ? 1 : 0, out);
+  if (!out) { rc = swe_host::frame_of(s, bytes, &out); if (rc) return rc; }
+  k_render_map<<<std::min(ny, 148 * 32), FRAME_THREADS, 0, st>>>(nx, ny, W, b, h, opts[0], msl, scale, show_bed ? 1 : 0,
+                                                                out, aligned4(out));
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && rgba_host) e = cudaMemcpyAsync(rgba_host, out, bytes, cudaMemcpyDeviceToHost, st);
-  if (own) cudaFreeAsync(out, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(SWE_ECUDA, std::string("swe_render_map: ") + cudaGetErrorString(e));
   return SWE_OK;
@@ -388,7 +422,7 @@ int swe_globe_lut_create(swe_sim* s, int size, double tilt_deg, double margin, c
   M(reinterpret_cast<void**>(&L->d_rowbase), sizeof(int) * n);
   M(reinterpret_cast<void**>(&L->d_lit), sizeof(float) * n);
   M(reinterpret_cast<void**>(&L->d_bg), 4 * NP);
-  M(reinterpret_cast<void**>(&L->d_stats), sizeof(double) * (5 * L->nblocks + 8));
+  M(reinterpret_cast<void**>(&L->d_stats), sizeof(double) * 8 + sizeof(FrameStats) * L->nblocks);
   M(reinterpret_cast<void**>(&L->d_ticket), sizeof(unsigned int));
   if (e == cudaSuccess && L->count) {
     e = cudaMemcpy(L->d_px, px.data(), sizeof(int) * L->count, cudaMemcpyHostToDevice);
@@ -447,20 +481,18 @@ int swe_render_globe(swe_sim* s, swe_globe_lut* L, double rot_deg, double scale,
   if (rc) return rc;
   const size_t bytes = (size_t)4 * L->size * L->size;
   unsigned char* out = static_cast<unsigned char*>(rgba_device);
-  bool own = false;
-  if (!out) { RCU(cudaMallocAsync(reinterpret_cast<void**>(&out), bytes, st)); own = true; }
+  if (!out) { rc = swe_host::frame_of(s, bytes, &out); if (rc) return rc; }
   cudaError_t e = cudaMemcpyAsync(out, L->d_bg, bytes, cudaMemcpyDeviceToDevice, st);   // out.set(lut.bg)
-  double* part = L->d_stats + 8;
+  FrameStats* part = reinterpret_cast<FrameStats*>(L->d_stats + 8);
   if (e == cudaSuccess && L->count > 0) {
     k_render_globe<<<L->nblocks, FRAME_THREADS, 0, st>>>(L->count, L->d_px, L->d_lon, L->d_rowbase, L->d_lit,
                                                         dims[0], b, h, opts[0], rot_deg, scale, msl,
-                                                        land_light ? 1 : 0, out, part, L->d_ticket, L->d_stats);
+                                                        land_light ? 1 : 0, out, aligned4(out), part, L->d_ticket, L->d_stats);
     e = cudaGetLastError();
   }
   double st8[8] = {0, 0, 0, 0, INFINITY, -INFINITY, 0, 0};
   if (e == cudaSuccess && L->count > 0) e = cudaMemcpyAsync(st8, L->d_stats, sizeof st8, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess && rgba_host) e = cudaMemcpyAsync(rgba_host, out, bytes, cudaMemcpyDeviceToHost, st);
-  if (own) cudaFreeAsync(out, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(SWE_ECUDA, std::string("swe_render_globe: ") + cudaGetErrorString(e));
   st8[2] = L->capped; st8[3] = L->inside;
