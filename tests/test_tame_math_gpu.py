@@ -124,3 +124,22 @@ def test_every_size_of_step_gives_the_fused_kernels_bits(swe, monkeypatch, nx, n
     for x, y in zip(out[0][:4], out[1][:4]):
         assert np.array_equal(x, y)
     assert out[0][4:] == out[1][4:]
+
+
+@pytest.mark.gpu
+def test_a_flather_side_that_is_set_again_or_changed(swe, monkeypatch):
+    """A driver sets its Flather sides before every run: the same values leave
+    the captured steps alone, others take effect at once."""
+    def tide(a):
+        return swe.flather(swe.Tide({"M2": [a, 30.0]}, msl=2.0).signal())
+    out = []
+    for impl in ("fused", "split"):
+        monkeypatch.setenv("SWE_B200_STAGE", impl)
+        sim = swe.ShallowWater(nx=90, ny=40, dx=5.0, bed=0.0, eta0=2.0, manning=0.0)
+        for west in (tide(0.5), tide(0.5), tide(0.25), swe.reflect, tide(0.25), tide(0.5)):
+            sim.boundaries.west = west
+            sim.run(64)
+        out.append([sim.field(f).copy() for f in ("h", "hu", "hv")] + [sim.t])
+        sim.close()
+    assert all(np.array_equal(x, y) for x, y in zip(out[0][:3], out[1][:3])) and out[0][3] == out[1][3]
+    assert np.max(np.abs(out[0][1])) > 0

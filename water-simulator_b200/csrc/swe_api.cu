@@ -64,9 +64,11 @@ struct swe_sim {
   double dx, dy, eps4, R, dlam, dphi, totalArea;
   std::vector<double> geom[SWE_GEOM_NROWS];
   std::vector<double> recip[5];
+  std::vector<double> geom_rows;                   // both, as d_geom holds them
   int dryfold = 0;                                 // every reciprocal row finite
   int tame = 0;                                    // swe_split.cuh, tame_ok
   cudaStream_t st = nullptr;
+  double* d_all = nullptr;                         // the allocation that holds the fixed buffers below
   double* d_b = nullptr;
   double* d_A[3] = {nullptr, nullptr, nullptr};
   double* d_B[3] = {nullptr, nullptr, nullptr};
@@ -87,6 +89,7 @@ struct swe_sim {
   int bc[4];
   int fl_kind[4] = {0, 0, 0, 0};
   double fl_eta[4] = {0, 0, 0, 0}, fl_u[4] = {0, 0, 0, 0};
+  std::vector<double> tide[4];                     // the device's tide tables: msl, u_coef, then each constituent's three values
   int sponge_side = 1, sponge_width = 0;
   double sponge_ref = 0;
   bool keep_h0 = false;
@@ -700,23 +703,19 @@ void fill_reciprocals(swe_sim* s) {
 
 int upload_geom(swe_sim* s) {
   fill_reciprocals(s);
-  for (int r = 0; r < SWE_GEOM_NROWS; r++)
-    CU(cudaMemcpyAsync(s->d_geom + (size_t)r * s->H, s->geom[r].data(), sizeof(double) * s->H,
-                       cudaMemcpyHostToDevice, s->st));
-  for (int q = 0; q < 5; q++)
-    CU(cudaMemcpyAsync(s->d_geom + (size_t)(SWE_GEOM_NROWS + q) * s->H, s->recip[q].data(),
-                       sizeof(double) * s->H, cudaMemcpyHostToDevice, s->st));
+  std::vector<double>& rows = s->geom_rows;          // kept: the copy may still read it
+  rows.clear();
+  for (int r = 0; r < SWE_GEOM_NROWS; r++) rows.insert(rows.end(), s->geom[r].begin(), s->geom[r].end());
+  for (int q = 0; q < 5; q++) rows.insert(rows.end(), s->recip[q].begin(), s->recip[q].end());
+  CU(cudaMemcpyAsync(s->d_geom, rows.data(), sizeof(double) * rows.size(), cudaMemcpyHostToDevice, s->st));
   return SWE_OK;
 }
 
 void free_all(swe_sim* s) {
   for (auto& g : s->graphs) if (g.exec) cudaGraphExecDestroy(g.exec);
-  double** ptrs[] = {&s->d_b, &s->d_A[0], &s->d_A[1], &s->d_A[2], &s->d_B[0], &s->d_B[1], &s->d_B[2],
-                     &s->d_h0[0], &s->d_h0[1], &s->d_h0[2], &s->d_res[0], &s->d_res[1], &s->d_res[2],
-                     &s->d_res[3], &s->d_nfield, &s->d_geom, &s->d_part, &s->d_rows, &s->d_coef,
-                     &s->d_sponge, &s->d_split};
+  double** ptrs[] = {&s->d_all, &s->d_h0[0], &s->d_h0[1], &s->d_h0[2], &s->d_res[0], &s->d_res[1], &s->d_res[2],
+                     &s->d_res[3], &s->d_nfield, &s->d_coef, &s->d_sponge, &s->d_split};
   for (double** p : ptrs) if (*p) { cudaFree(*p); *p = nullptr; }
-  if (s->d_ctl) cudaFree(s->d_ctl);
   if (s->d_vol) cudaFree(s->d_vol);
   if (s->d_frame) cudaFree(s->d_frame);
   if (s->st) cudaStreamDestroy(s->st);
@@ -795,15 +794,25 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
   CUB(cudaFuncSetAttribute(swe::k_stage<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, swe::STAGE_SMEM_BYTES));
   CUB(cudaFuncSetAttribute(swe::k_stage<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, swe::STAGE_SMEM_BYTES));
   CUB(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
-  CUB(cudaMalloc(&s->d_b, nb));
-  for (int q = 0; q < 3; q++) { CUB(cudaMalloc(&s->d_A[q], nb)); CUB(cudaMalloc(&s->d_B[q], nb)); }
-  CUB(cudaMalloc(&s->d_geom, sizeof(double) * (SWE_GEOM_NROWS + 5) * s->H));
-  // the tiles' partials, the close's scratch, the reductions' partials
+  // The handle's fixed buffers in one allocation, 256 bytes aligned each (a
+  // cudaMalloc and cudaFree for every one took longer than the rest of a small
+  // handle's creation); the partials are the tiles', the close's scratch and the
+  // reductions'.
   const size_t nparts = 3 * (size_t)s->part_cap + 3 * swe::CLOSE_BLOCKS + REDUCTION_BLOCKS;
-  CUB(cudaMalloc(&s->d_part, sizeof(double) * nparts));
+  const size_t N = s->N, sizes[11] = {N, N, N, N, N, N, N, (size_t)(SWE_GEOM_NROWS + 5) * s->H, nparts,
+                                      (size_t)std::max(1, s->ny), (sizeof(swe::Control) + 7) / 8};
+  double** const ptrs[10] = {&s->d_b, &s->d_A[0], &s->d_A[1], &s->d_A[2], &s->d_B[0], &s->d_B[1], &s->d_B[2],
+                             &s->d_geom, &s->d_part, &s->d_rows};
+  size_t total = 0;
+  for (size_t n : sizes) total += (n + 31) & ~size_t(31);
+  CUB(cudaMalloc(&s->d_all, sizeof(double) * total));
+  double* at = s->d_all;
+  for (int q = 0; q < 11; q++) {
+    if (q < 10) *ptrs[q] = at;
+    else s->d_ctl = reinterpret_cast<swe::Control*>(at);
+    at += (sizes[q] + 31) & ~size_t(31);
+  }
   s->d_red = s->d_part + (nparts - REDUCTION_BLOCKS);
-  CUB(cudaMalloc(&s->d_rows, sizeof(double) * std::max(1, s->ny)));
-  CUB(cudaMalloc(&s->d_ctl, sizeof(swe::Control)));
   CUB(cudaMemsetAsync(s->d_ctl, 0, sizeof(swe::Control), s->st));
   CUB(cudaMemsetAsync(s->d_part, 0, sizeof(double) * nparts, s->st));
   for (int q = 0; q < 3; q++) {
@@ -1006,6 +1015,9 @@ int swe_set_boundary(swe_sim* s, int side, int kind) {
 int swe_set_flather_values(swe_sim* s, int side, double eta_ext, double u_ext) {
   if (!s) return fail(SWE_EINVAL, "null argument");
   if (side < 0 || side > 3) return fail(SWE_EINVAL, "side must be 0..3");
+  if (s->bc[side] == SWE_BC_FLATHER && s->fl_kind[side] == 0 && std::memcmp(&s->fl_eta[side], &eta_ext, sizeof eta_ext) == 0 &&
+      std::memcmp(&s->fl_u[side], &u_ext, sizeof u_ext) == 0)
+    return SWE_OK;                  // the graphs hold these values
   s->bc[side] = SWE_BC_FLATHER;
   s->fl_kind[side] = 0;
   s->fl_eta[side] = eta_ext; s->fl_u[side] = u_ext;
@@ -1019,6 +1031,13 @@ int swe_set_flather_tide(swe_sim* s, int side, double msl, int n, const double* 
   if (side < 0 || side > 3) return fail(SWE_EINVAL, "side must be 0..3");
   if (n < 0 || n > swe::MAX_TIDE) return fail(SWE_EINVAL, "tide tables hold at most 16 constituents");
   if (n > 0 && (!amp || !omega || !phase_deg)) return fail(SWE_EINVAL, "null tide table");
+  std::vector<double> table = {msl, u_coef};
+  for (int q = 0; q < n; q++) table.insert(table.end(), {amp[q], omega[q], phase_deg[q]});
+  // the table that is there already (a driver sets it before every run) leaves
+  // the device and the graphs captured with it alone
+  if (s->bc[side] == SWE_BC_FLATHER && s->fl_kind[side] == 1 && table.size() == s->tide[side].size() &&
+      std::memcmp(table.data(), s->tide[side].data(), sizeof(double) * table.size()) == 0)
+    return SWE_OK;
   swe::Control c;
   int rc = read_ctl(s, &c);
   if (rc) return rc;
@@ -1030,6 +1049,7 @@ int swe_set_flather_tide(swe_sim* s, int side, double msl, int n, const double* 
   CU(cudaStreamSynchronize(s->st));
   s->bc[side] = SWE_BC_FLATHER;
   s->fl_kind[side] = 1;
+  s->tide[side] = table;
   s->version++;
   return SWE_OK;
 }

@@ -12,6 +12,7 @@
 #include "../../include/swe_b200.h"
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <string>
@@ -164,13 +165,31 @@ struct DevBuf {
     if (e_ != cudaSuccess) return fail(SWE_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-// Decode `len` characters of base64 into `out` (device, >= 4n bytes), which
-// must come to exactly 4n bytes.
-int decode_layer(const char* b64, size_t len, long long n, float* out, cudaStream_t st, const char* name) {
-  if (!b64) return fail(SWE_EINVAL, std::string("gridlands: layer ") + name + " is missing");
+// One device allocation, taken apart by offsets that stay 256-byte aligned.
+struct Arena {
+  DevBuf buf;
+  size_t used = 0;
+  size_t add(size_t bytes) { const size_t at = used; used += (bytes + 255) & ~size_t(255); return at; }
+  cudaError_t get() { return cudaMalloc(&buf.p, used > 0 ? used : 1); }
+  template <class T>
+  T* at(size_t off) const { return reinterpret_cast<T*>(static_cast<char*>(buf.p) + off); }
+};
+// A layer's text on the device, and the flag and position of a bad character.
+struct TextArea { unsigned char* txt; long long* flag; };
+
+size_t text_length(const char* b64, size_t len) {     // without the padding
   size_t L = len;
   int pad = 0;
   while (L > 0 && b64[L - 1] == '=' && pad < 2) { L--; pad++; }
+  return L;
+}
+
+// Decode `len` characters of base64 into `out` (device, >= 4n bytes), which
+// must come to exactly 4n bytes; w.txt holds `len` characters.
+int decode_layer(const char* b64, size_t len, long long n, float* out, const TextArea& w, cudaStream_t st,
+                 const char* name) {
+  if (!b64) return fail(SWE_EINVAL, std::string("gridlands: layer ") + name + " is missing");
+  const size_t L = text_length(b64, len);
   long long nbytes = (long long)(L / 4) * 3;
   const int rem = (int)(L % 4);
   if (rem == 1) nbytes = -1;
@@ -184,21 +203,16 @@ int decode_layer(const char* b64, size_t len, long long n, float* out, cudaStrea
                   name, nbytes < 0 ? 0LL : nbytes, 4 * n, n);
     return fail(SWE_EINVAL, buf);
   }
-  DevBuf txt, flag;
-  GL_CU(cudaMalloc(&txt.p, L > 0 ? L : 1));
-  GL_CU(cudaMalloc(&flag.p, 16));
-  GL_CU(cudaMemsetAsync(flag.p, 0, 8, st));
-  GL_CU(cudaMemsetAsync(static_cast<char*>(flag.p) + 8, 0xff, 8, st));
-  if (L > 0) GL_CU(cudaMemcpyAsync(txt.p, b64, L, cudaMemcpyHostToDevice, st));
+  GL_CU(cudaMemsetAsync(w.flag, 0, 8, st));
+  GL_CU(cudaMemsetAsync(w.flag + 1, 0xff, 8, st));
+  if (L > 0) GL_CU(cudaMemcpyAsync(w.txt, b64, L, cudaMemcpyHostToDevice, st));
   const long long nq = (long long)(L + 3) / 4;
   if (nq > 0)
-    k_b64_decode<<<grid_blocks(nq), 256, 0, st>>>(static_cast<const unsigned char*>(txt.p), (long long)L, nbytes,
-                                                  reinterpret_cast<unsigned char*>(out),
-                                                  static_cast<int*>(flag.p),
-                                                  reinterpret_cast<long long*>(static_cast<char*>(flag.p) + 8));
+    k_b64_decode<<<grid_blocks(nq), 256, 0, st>>>(w.txt, (long long)L, nbytes, reinterpret_cast<unsigned char*>(out),
+                                                  reinterpret_cast<int*>(w.flag), w.flag + 1);
   GL_CU(cudaGetLastError());
   long long hflag[2];
-  GL_CU(cudaMemcpyAsync(hflag, flag.p, 16, cudaMemcpyDeviceToHost, st));
+  GL_CU(cudaMemcpyAsync(hflag, w.flag, 16, cudaMemcpyDeviceToHost, st));
   GL_CU(cudaStreamSynchronize(st));
   if (hflag[0] & 0xffffffffLL) {
     char buf[200];
@@ -278,13 +292,13 @@ __global__ void k_ccl_flatten(long long n, const int* __restrict__ parent, int* 
   }
 }
 
-int load_layer(const char* b64, size_t len, const float* host, long long n, float* out, cudaStream_t st,
-               const char* name) {
+int load_layer(const char* b64, size_t len, const float* host, long long n, float* out, const TextArea& w,
+               cudaStream_t st, const char* name) {
   if (host) {
     GL_CU(cudaMemcpyAsync(out, host, sizeof(float) * n, cudaMemcpyHostToDevice, st));
     return SWE_OK;
   }
-  return decode_layer(b64, len, n, out, st, name);
+  return decode_layer(b64, len, n, out, w, st, name);
 }
 
 }  // namespace
@@ -295,16 +309,16 @@ int swe_gridlands_decode(const char* b64, size_t len, int n, float* out) {
   if (!out || n < 0) return fail(SWE_EINVAL, "swe_gridlands_decode: null output or negative n");
   cudaStream_t st;
   GL_CU(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  DevBuf d;
-  int rc = SWE_OK;
-  if (cudaMalloc(&d.p, sizeof(float) * (size_t)(n > 0 ? n : 1)) != cudaSuccess) rc = fail(SWE_ECUDA, "cudaMalloc");
-  if (rc == SWE_OK) rc = decode_layer(b64, len, n, static_cast<float*>(d.p), st, "data");
+  struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamDestroy(s); } } sg{st};
+  Arena m;
+  const size_t o_out = m.add(sizeof(float) * (size_t)n), o_txt = m.add(b64 ? len : 0), o_flag = m.add(16);
+  if (m.get() != cudaSuccess) return fail(SWE_ECUDA, "cudaMalloc");
+  int rc = decode_layer(b64, len, n, m.at<float>(o_out), {m.at<unsigned char>(o_txt), m.at<long long>(o_flag)}, st, "data");
   if (rc == SWE_OK && n > 0) {
-    if (cudaMemcpyAsync(out, d.p, sizeof(float) * n, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    if (cudaMemcpyAsync(out, m.at<float>(o_out), sizeof(float) * n, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       rc = fail(SWE_ECUDA, "swe_gridlands_decode: copy back failed");
   }
-  cudaStreamDestroy(st);
   return rc;
 }
 
@@ -358,34 +372,40 @@ int swe_gridlands_create(const swe_options* o, const swe_gridlands* g, swe_sim**
     return fail(SWE_EINVAL, "gridlands: layer manningN is missing");
   cudaStream_t st;
   GL_CU(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamSynchronize(s); cudaStreamDestroy(s); } } sg{st};
-  DevBuf layers, fields, flags;
-  GL_CU(cudaMalloc(&layers.p, sizeof(float) * n * 3));
-  float* bedM = static_cast<float*>(layers.p);
-  float* surfM = bedM + n;
-  float* nM = surfM + n;
-  int rc = load_layer(g->bed_b64, g->bed_len, g->bed_f32, n, bedM, st, "bedM");
-  if (rc == SWE_OK) rc = load_layer(g->surface_b64, g->surface_len, g->surface_f32, n, surfM, st, "surfaceM");
-  if (rc == SWE_OK && want_n) rc = load_layer(g->manning_b64, g->manning_len, g->manning_f32, n, nM, st, "manningN");
-  if (rc != SWE_OK) return rc;
-
+  struct StreamEnd { cudaStream_t s; ~StreamEnd() { cudaStreamDestroy(s); } } se{st};
   const int W = o->nx + 4, H = o->ny + 4;
   const long long N = (long long)W * H;
-  GL_CU(cudaMalloc(&fields.p, sizeof(double) * N * 3));
-  GL_CU(cudaMalloc(&flags.p, 16));
-  GL_CU(cudaMemsetAsync(flags.p, 0, 8, st));
-  GL_CU(cudaMemsetAsync(static_cast<char*>(flags.p) + 8, 0xff, 8, st));
+  // everything in one allocation: the layers, the longest text, the sampled fields
+  Arena m;
+  const size_t o_lay = m.add(sizeof(float) * n * 3), o_fld = m.add(sizeof(double) * N * 3), o_flag = m.add(16);
+  size_t longest = 0;
+  if (!g->bed_f32 && g->bed_b64) longest = std::max(longest, g->bed_len);
+  if (!g->surface_f32 && g->surface_b64) longest = std::max(longest, g->surface_len);
+  if (want_n && !g->manning_f32 && g->manning_b64) longest = std::max(longest, g->manning_len);
+  const size_t o_txt = m.add(longest);
+  GL_CU(m.get());
+  struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamSynchronize(s); } } sg{st};   // before m is freed
+  const TextArea w = {m.at<unsigned char>(o_txt), m.at<long long>(o_flag)};
+  float* bedM = m.at<float>(o_lay);
+  float* surfM = bedM + n;
+  float* nM = surfM + n;
+  int rc = load_layer(g->bed_b64, g->bed_len, g->bed_f32, n, bedM, w, st, "bedM");
+  if (rc == SWE_OK) rc = load_layer(g->surface_b64, g->surface_len, g->surface_f32, n, surfM, w, st, "surfaceM");
+  if (rc == SWE_OK && want_n) rc = load_layer(g->manning_b64, g->manning_len, g->manning_f32, n, nM, w, st, "manningN");
+  if (rc != SWE_OK) return rc;
+  GL_CU(cudaMemsetAsync(w.flag, 0, 8, st));
+  GL_CU(cudaMemsetAsync(w.flag + 1, 0xff, 8, st));
   SampleArgs a;
   a.bedM = bedM; a.surfM = surfM; a.nM = want_n ? nM : nullptr;
   a.Wg = g->width; a.Hg = g->height; a.C = g->cell_m; a.flip = g->flip_rows ? 1 : 0;
   a.W = W; a.H = H; a.dx = o->dx; a.dy = o->dy;
-  a.b = static_cast<double*>(fields.p); a.h = a.b + N; a.n = a.h + N;
-  a.bad_n = static_cast<int*>(flags.p);
-  a.bad_k = reinterpret_cast<long long*>(static_cast<char*>(flags.p) + 8);
+  a.b = m.at<double>(o_fld); a.h = a.b + N; a.n = a.h + N;
+  a.bad_n = reinterpret_cast<int*>(w.flag);
+  a.bad_k = w.flag + 1;
   k_gridlands_sample<<<grid_blocks(N), 256, 0, st>>>(a);
   GL_CU(cudaGetLastError());
   long long hflag[2];
-  GL_CU(cudaMemcpyAsync(hflag, flags.p, 16, cudaMemcpyDeviceToHost, st));
+  GL_CU(cudaMemcpyAsync(hflag, w.flag, 16, cudaMemcpyDeviceToHost, st));
   GL_CU(cudaStreamSynchronize(st));
   if (want_n && (hflag[0] & 0xffffffffLL)) {
     const long long k = hflag[1];

@@ -41,6 +41,8 @@ struct swe_globe_lut {
   int* d_rowbase = nullptr;      // padded index of the row's first interior cell
   float* d_lit = nullptr;        // cos(incidence) of the viewer-fixed light
   unsigned char* d_bg = nullptr; // everything that is not modelled ocean or land
+  unsigned char* d_out = nullptr; // a frame drawn for the host
+  void* d_all = nullptr;         // the allocation that holds them
   double* d_stats = nullptr;     // frame reduction scratch
   unsigned int* d_ticket = nullptr;
   int nblocks = 0;
@@ -415,15 +417,23 @@ int swe_globe_lut_create(swe_sim* s, int size, double tilt_deg, double margin, c
   L->tilt = tilt_deg; L->margin = margin; L->nx = nx; L->ny = ny; L->lat0 = lat0; L->lat1 = lat1;
   const int n = std::max(1, L->count);
   L->nblocks = std::max(1, std::min(148 * 8, (L->count + FRAME_THREADS - 1) / FRAME_THREADS));
-  cudaError_t e = cudaSuccess;
-  auto M = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
-  M(reinterpret_cast<void**>(&L->d_px), sizeof(int) * n);
-  M(reinterpret_cast<void**>(&L->d_lon), sizeof(double) * n);
-  M(reinterpret_cast<void**>(&L->d_rowbase), sizeof(int) * n);
-  M(reinterpret_cast<void**>(&L->d_lit), sizeof(float) * n);
-  M(reinterpret_cast<void**>(&L->d_bg), 4 * NP);
-  M(reinterpret_cast<void**>(&L->d_stats), sizeof(double) * 8 + sizeof(FrameStats) * L->nblocks);
-  M(reinterpret_cast<void**>(&L->d_ticket), sizeof(unsigned int));
+  const size_t sizes[8] = {sizeof(double) * n, sizeof(int) * n, sizeof(int) * n, sizeof(float) * n, 4 * NP, 4 * NP,
+                           sizeof(double) * 8 + sizeof(FrameStats) * L->nblocks, sizeof(unsigned int)};
+  size_t total = 0;
+  for (size_t b : sizes) total += (b + 255) & ~size_t(255);
+  cudaError_t e = cudaMalloc(&L->d_all, total);
+  char* at = static_cast<char*>(L->d_all);
+  auto take = [&](int q) { char* p = at; at += (sizes[q] + 255) & ~size_t(255); return p; };
+  if (e == cudaSuccess) {
+    L->d_lon = reinterpret_cast<double*>(take(0));
+    L->d_px = reinterpret_cast<int*>(take(1));
+    L->d_rowbase = reinterpret_cast<int*>(take(2));
+    L->d_lit = reinterpret_cast<float*>(take(3));
+    L->d_bg = reinterpret_cast<unsigned char*>(take(4));
+    L->d_out = reinterpret_cast<unsigned char*>(take(5));
+    L->d_stats = reinterpret_cast<double*>(take(6));
+    L->d_ticket = reinterpret_cast<unsigned int*>(take(7));
+  }
   if (e == cudaSuccess && L->count) {
     e = cudaMemcpy(L->d_px, px.data(), sizeof(int) * L->count, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(L->d_lon, lon.data(), sizeof(double) * L->count, cudaMemcpyHostToDevice);
@@ -442,8 +452,7 @@ int swe_globe_lut_create(swe_sim* s, int size, double tilt_deg, double margin, c
 
 int swe_globe_lut_destroy(swe_globe_lut* L) {
   if (!L) return SWE_OK;
-  cudaFree(L->d_px); cudaFree(L->d_lon); cudaFree(L->d_rowbase); cudaFree(L->d_lit);
-  cudaFree(L->d_bg); cudaFree(L->d_stats); cudaFree(L->d_ticket);
+  cudaFree(L->d_all);
   delete L;
   return SWE_OK;
 }
@@ -481,7 +490,7 @@ int swe_render_globe(swe_sim* s, swe_globe_lut* L, double rot_deg, double scale,
   if (rc) return rc;
   const size_t bytes = (size_t)4 * L->size * L->size;
   unsigned char* out = static_cast<unsigned char*>(rgba_device);
-  if (!out) { rc = swe_host::frame_of(s, bytes, &out); if (rc) return rc; }
+  if (!out) out = L->d_out;
   cudaError_t e = cudaMemcpyAsync(out, L->d_bg, bytes, cudaMemcpyDeviceToDevice, st);   // out.set(lut.bg)
   FrameStats* part = reinterpret_cast<FrameStats*>(L->d_stats + 8);
   if (e == cudaSuccess && L->count > 0) {

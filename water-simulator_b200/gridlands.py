@@ -190,7 +190,8 @@ def gridlandsTerrain(doc, flipRows=True, settle=False):
     def colOf(x):
         return min(W - 1, max(0, x / C - 0.5))
 
-    bl, sl = bedM.tolist(), surfaceM.tolist()
+    # snapshots that index to Python floats, without making one per cell up front
+    bl, sl = memoryview(bedM.copy()), memoryview(surfaceM.copy())
 
     def bed(x, y):
         fc, fr = colOf(x), rowOf(y)
