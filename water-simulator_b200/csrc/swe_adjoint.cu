@@ -22,6 +22,7 @@
 #include "../../include/swe_b200.h"
 #include "swe_kernels.cuh"
 #include "swe_split.cuh"
+#include "swe_maps.cuh"
 #include "swe_adjoint_math.cuh"
 
 #include <cuda_runtime.h>
@@ -607,9 +608,8 @@ __global__ void k_adj_tail1(int W, int H, double minDepth, double dt, const doub
 // J += sum over gauges, in gauge order, of (b + h - obs)^2; eta at the gauges.
 // The loads run in parallel; one thread adds the squares in order.
 constexpr int MISFIT_THREADS = 256;
-__global__ void k_misfit(const double* b, const double* h, const int* gk, const double* obs, int ng,
-                         double* J, double* eta_out) {
-  pdl_enter();
+__device__ __forceinline__ void misfit(const double* b, const double* h, const int* gk, const double* obs, int ng,
+                                       double* J, double* eta_out) {
   __shared__ double r2[MISFIT_THREADS];
   double s = 0;
   if (threadIdx.x == 0) s = *J;
@@ -646,22 +646,22 @@ __global__ void k_adj_misfit(const double* b, const double* h, const int* gcell,
     lb[k] = ab;
   }
 }
-// After a step's prepare: t and the Flather exterior state into rec (STEP_REC doubles).
-__global__ void k_record_step(const Control* ctl, double* rec) {
+// The forward's record of a step, before its close: t at its start and the
+// Flather exterior state (rec, STEP_REC doubles), its dt (where dts is given)
+// and the misfit of the state it left.
+__global__ void k_record_step(const Control* ctl, double* rec, double* dts, const double* b, const double* h,
+                              const int* gk, const double* obs, int ng, double* J, double* eta_out) {
   pdl_enter();
-  if (threadIdx.x == 0) {
-    rec[0] = ctl->t;
-    for (int q = 0; q < 4; q++) { rec[1 + q] = ctl->fl_eta[q]; rec[5 + q] = ctl->fl_u[q]; }
-  }
+  const int t = threadIdx.x;
+  if (t < 4) { rec[1 + t] = ctl->fl_eta[t]; rec[5 + t] = ctl->fl_u[t]; }
+  if (t == 4) rec[0] = ctl->t;
+  if (t == 5 && dts) *dts = ctl->dt;
+  misfit(b, h, gk, obs, ng, J, eta_out);
 }
 // The time of the step a segment's tape pass starts with.
 __global__ void k_set_t(Control* ctl, const double* rec) {
   pdl_enter();
   if (threadIdx.x == 0) ctl->t = rec[0];
-}
-__global__ void k_record_dt(const Control* ctl, double* dts, int s) {
-  pdl_enter();
-  if (threadIdx.x == 0) dts[s] = ctl->dt;
 }
 // dst[q] = src[q] for q < nf (checkpoints and the segment tape's copies of
 // the state, as a kernel so that the stepping chain stays one of kernels).
@@ -712,6 +712,10 @@ struct swe_adjoint {
   dim3 grid;
   swe::SplitBufs sb;               // the tiled stage kernels' fields
   dim3 sgrid;
+  swe::TileMaps tmaps[2];          // tensor maps of the forward's stages (A -> Bf, Bf -> A)
+  swe::CellMaps cmaps[2];
+  bool tma = false, cell_tma = false;
+  bool ghost_gauges = false;       // a gauge lies in a ghost cell
   int pcap = 0;                    // partial slots per kind (the most tiles either kernel uses)
   bool forward_done = false;
   bool pdl = true;                 // programmatic dependent launch between the stepping kernels
@@ -814,30 +818,42 @@ swe::PrepArgs prep_of(const swe_adjoint* s, bool auto_dt, int k) {
   return p;
 }
 
-// The face kernel whose stage input's ghosts a launch before it has filled.
-constexpr auto faces_kernel = &swe::k_split_faces<SWE_SPLIT_FACES_MIN_BLOCKS, false>;
-const swe::GhostFill no_fill = {};
-
-// One forward step of state X in place.
-int fwd_step(swe_adjoint* s, double* const* X, bool auto_dt, int step_index) {
-  LAUNCH(swe::k_prepare, dim3(1), dim3(32), s->ctl, prep_of(s, auto_dt, step_index));
-  LAUNCH(k_record_step, dim3(1), dim3(32), (const Control*)s->ctl, s->rec + (size_t)STEP_REC * step_index);
-  const dim3 spb(swe::SP_THREADS);
-  const int nparts = (int)(s->sgrid.x * s->sgrid.y);
-  LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, X), (const Control*)s->ctl, 0);
-  const StageArgs a1 = stage_args(s, X, s->Bf);
-  LAUNCH(faces_kernel, s->sgrid, spb, a1, s->sb, s->ctl, no_fill);
-  LAUNCH(swe::k_split_cells<1>, s->sgrid, spb, a1, s->sb, s->ctl);
-  LAUNCH(swe::k_split_close<1>, dim3(1), spb, a1, s->ctl, nparts);
-  LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, s->Bf), (const Control*)s->ctl, 0);
-  const StageArgs a2 = stage_args(s, s->Bf, X);
-  LAUNCH(faces_kernel, s->sgrid, spb, a2, s->sb, s->ctl, no_fill);
-  LAUNCH(swe::k_split_cells<2>, s->sgrid, spb, a2, s->sb, s->ctl);
-  LAUNCH(swe::k_split_close<2>, dim3(1), spb, a2, s->ctl, nparts);
-  if (auto_dt) LAUNCH(k_record_dt, dim3(1), dim3(32), (const Control*)s->ctl, s->dts, step_index);
+// A stage whose face kernel fills its input's ghosts and, with prep, prepares
+// the step (swe_split.cuh, GhostFill).  maps: the tensor maps of the forward's
+// own buffers, or null for the tape's, whose tiles are copied by the threads.
+template <int MODE>
+int stage(swe_adjoint* s, const StageArgs& a, const swe::SplitBufs& sb, double* const* in, const swe::PrepArgs* prep,
+          bool maps) {
+  swe::GhostFill F = {};
+  F.on = 1;
+  F.bc = bc_args(s, in);
+  if (prep) { F.prepare = 1; F.prep = *prep; }
+  const dim3 blk(swe::SP_THREADS);
+  constexpr int WIDE = SWE_SPLIT_FACES_MIN_BLOCKS;
+  if (maps && s->tma) LAUNCH((swe::k_split_faces_tma<WIDE, true>), s->sgrid, blk, a, sb, s->ctl, s->tmaps[MODE - 1], F);
+  else LAUNCH((swe::k_split_faces<WIDE, true>), s->sgrid, blk, a, sb, s->ctl, F);
+  if (maps && s->cell_tma) LAUNCH((swe::k_split_cells_tma<MODE, false>), s->sgrid, blk, a, sb, s->ctl, s->cmaps[MODE - 1]);
+  else LAUNCH((swe::k_split_cells<MODE, false>), s->sgrid, blk, a, sb, s->ctl);
   return SWE_OK;
 }
 
+// Step k of the forward, on A in place, with its record and misfit.
+int fwd_step(swe_adjoint* s, int k) {
+  const swe::PrepArgs prep = prep_of(s, !s->fixed_dt, k);
+  const StageArgs a1 = stage_args(s, s->A, s->Bf), a2 = stage_args(s, s->Bf, s->A);
+  int rc = stage<1>(s, a1, s->sb, s->A, &prep, true);
+  if (rc == SWE_OK) rc = stage<2>(s, a2, s->sb, s->Bf, nullptr, true);
+  if (rc) return rc;
+  LAUNCH(k_record_step, dim3(1), dim3(MISFIT_THREADS), (const Control*)s->ctl, s->rec + (size_t)STEP_REC * k,
+         s->fixed_dt ? (double*)nullptr : s->dts + k, (const double*)s->b, (const double*)s->A[0], (const int*)s->gk,
+         (const double*)(s->obs + (size_t)k * s->ng), s->ng, s->J, s->eta_series + (size_t)k * s->ng);
+  const int n = (int)(s->sgrid.x * s->sgrid.y);
+  if (n <= swe::CLOSE_TILES) LAUNCH(swe::k_split_close_step, dim3(1), dim3(32 * swe::CLOSE_BLOCKS), a2, s->ctl, n);
+  else
+    LAUNCH(swe::k_split_close_multi<2>, dim3(swe::CLOSE_BLOCKS), dim3(swe::SP_THREADS), a2, s->ctl, n,
+           s->part + 3 * (size_t)s->pcap);
+  return SWE_OK;
+}
 
 // R^T: given ab.lR (adjoint of rh, rhu, rhv over all cells) at state X (ghosts
 // filled), add into lX (h, hu, hv) and lb.
@@ -900,6 +916,7 @@ Tape tape_at(const swe_adjoint* s, int t) {
 // go to the tape (the source terms stay in the handle's scratch).
 swe::SplitBufs tape_bufs(const swe_adjoint* s, const Inter& it) {
   swe::SplitBufs b = s->sb;
+  b.P = s->W;
   for (int q = 0; q < swe::SPLIT_FACE_FIELDS; q++) { b.fx[q] = it.fx[q]; b.fy[q] = it.fy[q]; }
   for (int q = 0; q < 8; q++) b.sl[q] = it.s[q];
   b.U = it.U;
@@ -907,33 +924,27 @@ swe::SplitBufs tape_bufs(const swe_adjoint* s, const Inter& it) {
   return b;
 }
 
-// Step k forward from X (in place) and record its tape: the tiled stage
-// kernels write the limiter, the depth before dryClean and friction's input
-// as they go.
-int tape_step(swe_adjoint* s, double* const* X, int k, const Tape& T) {
-  const dim3 spb(swe::SP_THREADS);
-  const int nparts = (int)(s->sgrid.x * s->sgrid.y);
-  if (k % s->every == 0) LAUNCH(k_set_t, dim3(1), dim3(32), s->ctl, (const double*)(s->rec + (size_t)STEP_REC * k));
-  LAUNCH(swe::k_prepare, dim3(1), dim3(32), s->ctl, prep_of(s, false, k));
-  // the step input with its ghosts, in X (U0 of the in-place stage 2) and on the tape
-  LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, X), (const Control*)s->ctl, 0);
-  if (int rc = copy3(s, T.W1, X)) return rc;
+// Step k forward from its tape's W1 into `out` (the next step's W1, or X after
+// the segment's last) and record its tape: the tiled stage kernels write the
+// limiter, the depth before dryClean and friction's input as they go.  Nothing
+// closes the step: its dt and the Flather sides' t are recorded.
+int tape_step(swe_adjoint* s, double* const* out, int k, const Tape& T) {
+  bool tide = false;
+  for (int q = 0; q < 4; q++) tide |= s->fl_kind[q] == 1;
+  if (tide) LAUNCH(k_set_t, dim3(1), dim3(32), s->ctl, (const double*)(s->rec + (size_t)STEP_REC * k));
+  const swe::PrepArgs prep = prep_of(s, false, k);
   StageArgs a1 = stage_args(s, T.W1, T.Bp);
   a1.tape_th = T.th1; a1.tape_hpre = T.hB;
-  const swe::SplitBufs b1 = tape_bufs(s, T.it1);
-  LAUNCH(faces_kernel, s->sgrid, spb, a1, b1, s->ctl, no_fill);
-  LAUNCH(swe::k_split_cells<1>, s->sgrid, spb, a1, b1, s->ctl);
-  LAUNCH(swe::k_split_close<1>, dim3(1), spb, a1, s->ctl, nparts);
-  LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, T.Bp), (const Control*)s->ctl, 0);
-  StageArgs a2 = stage_args(s, T.Bp, X);
+  int rc = stage<1>(s, a1, tape_bufs(s, T.it1), T.W1, &prep, false);
+  if (rc) return rc;
+  StageArgs a2 = stage_args(s, T.Bp, out);
   a2.tape_th = T.th2; a2.tape_hpre = T.hA;
-  for (int q = 0; q < 3; q++) a2.tape_pre[q] = T.Bf[q];
-  const swe::SplitBufs b2 = tape_bufs(s, T.it2);
-  LAUNCH(faces_kernel, s->sgrid, spb, a2, b2, s->ctl, no_fill);
-  LAUNCH(swe::k_split_cells<2>, s->sgrid, spb, a2, b2, s->ctl);
-  LAUNCH(swe::k_split_close<2>, dim3(1), spb, a2, s->ctl, nparts);
-  LAUNCH(k_copy, dim3(G1(s)), dim3(256), (size_t)s->N, 1, T.hX, (double*)nullptr, (double*)nullptr,
-         (const double*)X[0], (const double*)nullptr, (const double*)nullptr);
+  for (int q = 0; q < 3; q++) { a2.tape_pre[q] = T.Bf[q]; a2.u0[q] = T.W1[q]; }
+  rc = stage<2>(s, a2, tape_bufs(s, T.it2), T.Bp, nullptr, false);
+  if (rc) return rc;
+  if (s->ghost_gauges)                             // before the next step fills them
+    LAUNCH(k_copy, dim3(G1(s)), dim3(256), (size_t)s->N, 1, T.hX, (double*)nullptr, (double*)nullptr,
+           (const double*)out[0], (const double*)nullptr, (const double*)nullptr);
   return SWE_OK;
 }
 
@@ -1053,8 +1064,11 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
   s->steps = steps; s->every = checkpoint_every; s->nseg = (steps + checkpoint_every - 1) / checkpoint_every;
   s->ng = n_gauges;
   s->eps4 = std::pow(swe::jmax(o->min_depth, 1e-12), 4.0);
-  for (int q = 0; q < n_gauges; q++)
+  for (int q = 0; q < n_gauges; q++) {
     if (gauge_cells[q] < 0 || gauge_cells[q] >= s->N) return bail(fail(SWE_EINVAL, "gauge cell out of range"));
+    const int i = gauge_cells[q] % s->W, j = gauge_cells[q] / s->W;
+    s->ghost_gauges |= i < 2 || i >= s->W - 2 || j < 2 || j >= s->H - 2;
+  }
   const size_t N = s->N;
   if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(SWE_ECUDA, "swe_adjoint_create: stream"));
@@ -1095,14 +1109,20 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
   s->nblocks = gx * gy;
   s->sgrid = dim3((s->W + swe::SPX - 1) / swe::SPX, (s->H + swe::SPY - 1) / swe::SPY);
   s->pcap = std::max(std::max(s->nblocks, (int)(s->sgrid.x * s->sgrid.y)), 1024);
-  s->part = A(3 * (size_t)s->pcap);
+  s->part = A(3 * (size_t)s->pcap + 3 * swe::CLOSE_BLOCKS);      // + the close's scratch
   {
-    double* spl = A((size_t)swe::SPLIT_FIELDS * N);
-    if (spl) s->sb = swe::split_bufs_at(spl, N, s->W);
+    const int pitch = swe::split_pitch(s->W);
+    const size_t PN = (size_t)pitch * s->H;
+    double* spl = A((size_t)swe::SPLIT_FIELDS * PN);
+    if (spl) s->sb = swe::split_bufs_at(spl, PN, pitch);
   }
   if (!ok || cudaMalloc(&s->ctl, sizeof(Control)) != cudaSuccess || cudaMalloc(&s->gk, sizeof(int) * n_gauges) != cudaSuccess)
     return bail(fail(SWE_ECUDA, "swe_adjoint_create: device allocation failed"));
   cudaMemsetAsync(s->ctl, 0, sizeof(Control), s->st);
+  s->cell_tma = swe::make_cell_maps(s->cmaps[0], s->sb, s->A[0], s->W, s->H) &&
+                swe::make_cell_maps(s->cmaps[1], s->sb, s->Bf[0], s->W, s->H);
+  s->tma = swe::make_tile_maps(s->tmaps[0], s->b, s->A, s->W, s->H) &&
+           swe::make_tile_maps(s->tmaps[1], s->b, s->Bf, s->W, s->H);
   {
     const char* pe = std::getenv("SWE_B200_PDL");
     s->pdl = !(pe && std::strcmp(pe, "0") == 0);
@@ -1188,11 +1208,7 @@ int swe_adjoint_forward(swe_adjoint* s, double* J, double* gauge_eta) {
                         s->ckpt + ((size_t)(k / s->every) * 3 + 2) * s->N};
       if (int rc = copy3(s, dst, s->A)) return rc;
     }
-    int rc = fwd_step(s, s->A, !s->fixed_dt, k);
-    if (rc) return rc;
-    LAUNCH(k_misfit, dim3(1), dim3(MISFIT_THREADS), (const double*)s->b, (const double*)s->A[0],
-           (const int*)s->gk, (const double*)(s->obs + (size_t)k * s->ng), s->ng, s->J,
-           s->eta_series + (size_t)k * s->ng);
+    if (int rc = fwd_step(s, k)) return rc;
   }
   CU(cudaGetLastError());
   if (J) CU(cudaMemcpyAsync(J, s->J, sizeof(double), cudaMemcpyDeviceToHost, s->st));
@@ -1230,13 +1246,15 @@ int swe_adjoint_backward(swe_adjoint* s, double* grad_b, double* grad_n) {
     // the segment forward from its checkpoint, recording each step's tape
     double* src[3] = {s->ckpt + (size_t)sg * 3 * N, s->ckpt + ((size_t)sg * 3 + 1) * N, s->ckpt + ((size_t)sg * 3 + 2) * N};
     // the first kernel after the memsets and the tape allocation waits for them in stream order
-    if (int rc = copy3(s, s->X, src, sg != s->nseg - 1)) return rc;
+    if (int rc = copy3(s, tape_at(s, 0).W1, src, sg != s->nseg - 1)) return rc;
     for (int k = k0; k < k1; k++) {
-      int rc = tape_step(s, s->X, k, tape_at(s, k - k0));
+      const Tape next = tape_at(s, k + 1 < k1 ? k + 1 - k0 : 0);
+      int rc = tape_step(s, k + 1 < k1 ? next.W1 : s->X, k, tape_at(s, k - k0));
       if (rc) return rc;
     }
     for (int k = k1 - 1; k >= k0; k--) {
-      const Tape T = tape_at(s, k - k0);
+      Tape T = tape_at(s, k - k0);
+      if (!s->ghost_gauges) T.hX = k + 1 < k1 ? tape_at(s, k + 1 - k0).W1[0] : s->X[0];
       LAUNCH(k_adj_misfit, dim3((s->ngroups + 127) / 128), dim3(128), (const double*)s->b, (const double*)T.hX,
              (const int*)s->gmeta, (const int*)(s->gmeta + s->ngroups), (const int*)(s->gmeta + 2 * s->ngroups + 1),
              s->ngroups, (const double*)(s->obs + (size_t)k * s->ng), s->lb, s->lA[0]);

@@ -6,9 +6,9 @@
 #include "../../include/swe_b200.h"
 #include "swe_kernels.cuh"
 #include "swe_split.cuh"
+#include "swe_maps.cuh"
 
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>        // PFN_cuTensorMapEncodeTiled (fetched through the runtime, no -lcuda)
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -335,78 +335,14 @@ int launch_bc(swe_sim* s, double* const* f, int respect_stop, bool pdl = false) 
   return SWE_OK;
 }
 
-// The driver's tensor-map encoder, or null; and whether the tile copies are
-// on (SWE_B200_TMA=0 turns them off).
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  if (!encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn)
-      return nullptr;
-    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  }
-  return encode;
-}
-bool tma_wanted() {
-  const char* env = std::getenv("SWE_B200_TMA");
-  return !(env && std::strcmp(env, "0") == 0);
-}
-// A 2-D map over one W x H field of doubles, rows of `pitch` (even), with the
-// given box.
-bool encode_field(PFN_cuTensorMapEncodeTiled_v12000 encode, const swe_sim* s, CUtensorMap* m, double* base, int pitch,
-                  int bx, int by) {
-  const cuuint64_t dims[2] = {(cuuint64_t)s->W, (cuuint64_t)s->H};
-  const cuuint64_t strides[1] = {(cuuint64_t)pitch * sizeof(double)};
-  const cuuint32_t box[2] = {(cuuint32_t)bx, (cuuint32_t)by};
-  const cuuint32_t estr[2] = {1, 1};
-  return encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// The cell kernel's maps: the face fields (one set of buffers for both
-// stages, whose rows are aligned whatever W is) and the stage input's depth
-// (where W is even; else the kernel copies it element by element).
+// The stage kernels' tensor maps (swe_maps.cuh).
 void make_cell_maps(swe_sim* s) {
-  s->cell_tma = 0;
-  if (!s->d_split || !tma_wanted()) return;
-  PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-  if (!encode) return;
-  using swe::SPX;
-  using swe::SPY;
-  const int P = s->sb.P;
-  for (int st = 0; st < 2; st++) {
-    swe::CellMaps& c = s->cmaps[st];
-    bool ok = encode_field(encode, s, &c.m[swe::CM_XM], s->sb.fx[swe::F_M], P, SPX + 4, SPY + 2) &&
-              encode_field(encode, s, &c.m[swe::CM_YM], s->sb.fy[swe::F_M], P, SPX + 4, SPY + 3);
-    if (s->W % 2 == 0)
-      ok = ok && encode_field(encode, s, &c.m[swe::CM_H], st == 0 ? s->d_A[0] : s->d_B[0], s->W, SPX + 4, SPY + 2);
-    for (int q = 0; q < 3 && ok; q++)
-      ok = encode_field(encode, s, &c.m[swe::CM_XT + q], s->sb.fx[q + 1], P, SPX + 2, SPY) &&
-           encode_field(encode, s, &c.m[swe::CM_YT + q], s->sb.fy[q + 1], P, SPX, SPY + 1) &&
-           encode_field(encode, s, &c.m[swe::CM_TB + q], s->sb.tb[q], P, SPX, SPY);
-    if (!ok) return;
-  }
-  s->cell_tma = 1;
+  s->cell_tma = s->d_split && swe::make_cell_maps(s->cmaps[0], s->sb, s->d_A[0], s->W, s->H) &&
+                swe::make_cell_maps(s->cmaps[1], s->sb, s->d_B[0], s->W, s->H);
 }
-
-// Tensor maps of the face kernel's state tile (swe_split.cuh, TileMaps):
-// b, h, hu, hv of A (stage 1's input) and of B (stage 2's), each a 2-D
-// W x H array of doubles, box SSXT x SSY, zeros outside.  A row stride that
-// is not a multiple of 16 bytes (odd W), a driver without the encoder, or
-// SWE_B200_TMA=0 leaves the per-element copies in use (the same bits).
 void make_tile_maps(swe_sim* s) {
-  s->tma = 0;
-  if (!tma_wanted() || s->W % 2 != 0) return;
-  PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-  if (!encode) return;
-  double* src[2][4] = {{s->d_b, s->d_A[0], s->d_A[1], s->d_A[2]}, {s->d_b, s->d_B[0], s->d_B[1], s->d_B[2]}};
-  for (int st = 0; st < 2; st++)
-    for (int f = 0; f < 4; f++)
-      if (!encode_field(encode, s, &s->tmaps[st].m[f], src[st][f], s->W, swe::SSXT, swe::SSY)) return;
-  s->tma = 1;
+  s->tma = swe::make_tile_maps(s->tmaps[0], s->d_b, s->d_A, s->W, s->H) &&
+           swe::make_tile_maps(s->tmaps[1], s->d_b, s->d_B, s->W, s->H);
 }
 
 // Buffers of the tiled stage kernels (faces and source terms).

@@ -103,6 +103,8 @@ struct StageArgs {
   // the cell's positivity limiter, its depth before dryClean and (stage 2)
   // the state after dryClean that friction takes
   double* tape_th; double* tape_hpre; double* tape_pre[3];
+  // U0 of the tiled stage 2 where it is not the output's own (null: in place)
+  const double* u0[3];
   // every reciprocal metric row (rdxRow, rdyRowN, rdyRowS) finite, so a
   // face value of +0 times any of them is +0
   int dryfold;

@@ -1165,9 +1165,9 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
     cp_async8(&sm.st[1][t], a.hu + k);
     cp_async8(&sm.st[2][t], a.hv + k);
     if (MODE == 2) {
-      cp_async8(&sm.st[3][t], a.oh + k);
-      cp_async8(&sm.st[4][t], a.ohu + k);
-      cp_async8(&sm.st[5][t], a.ohv + k);
+      cp_async8(&sm.st[3][t], (a.u0[0] ? a.u0[0] : a.oh) + k);
+      cp_async8(&sm.st[4][t], (a.u0[0] ? a.u0[1] : a.ohu) + k);
+      cp_async8(&sm.st[5][t], (a.u0[0] ? a.u0[2] : a.ohv) + k);
     }
   }
   if (t < 9) {
@@ -1225,9 +1225,9 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
     cp_async8(&sm.st[1][t], a.hu + k);
     cp_async8(&sm.st[2][t], a.hv + k);
     if (MODE == 2) {
-      cp_async8(&sm.st[3][t], a.oh + k);
-      cp_async8(&sm.st[4][t], a.ohu + k);
-      cp_async8(&sm.st[5][t], a.ohv + k);
+      cp_async8(&sm.st[3][t], (a.u0[0] ? a.u0[0] : a.oh) + k);
+      cp_async8(&sm.st[4][t], (a.u0[0] ? a.u0[1] : a.ohu) + k);
+      cp_async8(&sm.st[5][t], (a.u0[0] ? a.u0[2] : a.ohv) + k);
     }
   }
   if (!fold) {
