@@ -153,6 +153,9 @@ int ensure_tables() {
   }
   RCU(cudaMemcpyToSymbol(g_ramp, t.ramp, sizeof t.ramp));
   RCU(cudaMemcpyToSymbol(g_cbytes, rgba, sizeof rgba));
+  // a copy from pageable memory may return before it has reached the device,
+  // and the handles' streams do not wait for the default stream
+  RCU(cudaStreamSynchronize(0));
   done = 1;
   done_dev = dev;
   return SWE_OK;
@@ -434,14 +437,17 @@ int swe_globe_lut_create(swe_sim* s, int size, double tilt_deg, double margin, c
     L->d_stats = reinterpret_cast<double*>(take(6));
     L->d_ticket = reinterpret_cast<unsigned int*>(take(7));
   }
-  if (e == cudaSuccess && L->count) {
-    e = cudaMemcpy(L->d_px, px.data(), sizeof(int) * L->count, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(L->d_lon, lon.data(), sizeof(double) * L->count, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(L->d_rowbase, rowbase.data(), sizeof(int) * L->count, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(L->d_lit, lit.data(), sizeof(float) * L->count, cudaMemcpyHostToDevice);
-  }
-  if (e == cudaSuccess) e = cudaMemcpy(L->d_bg, bgb.data(), 4 * NP, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(L->d_ticket, 0, sizeof(unsigned int));
+  // on the handle's stream, and complete before any other stream may read them
+  auto up = [&](void* dst, const void* src, size_t bytes) {
+    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+  };
+  up(L->d_px, px.data(), sizeof(int) * L->count);
+  up(L->d_lon, lon.data(), sizeof(double) * L->count);
+  up(L->d_rowbase, rowbase.data(), sizeof(int) * L->count);
+  up(L->d_lit, lit.data(), sizeof(float) * L->count);
+  up(L->d_bg, bgb.data(), 4 * NP);
+  if (e == cudaSuccess) e = cudaMemsetAsync(L->d_ticket, 0, sizeof(unsigned int), st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     swe_globe_lut_destroy(L);
     return fail(SWE_ECUDA, std::string("swe_globe_lut_create: ") + cudaGetErrorString(e));
