@@ -1133,12 +1133,13 @@ __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& 
 // The limiter ring's and the gather's inputs are staged into sm.ft once the
 // tile is known to be computed; TMA: by tensor-map copies (maps, completing on
 // bar), of which one that does not complete within the bound leaves the tile's
-// output unwritten (tile_wait).
+// output unwritten (tile_wait); parity is bar's phase, which without SETTLE
+// every tile completes once.
 template <int MODE, bool SETTLE = false, bool TMA = false>
 __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const SplitBufs& s, Control* ctl, int tx,
                                                  int ty, int part, int nparts, CellsSmem& sm, bool ticket,
                                                  const CellMaps* maps = nullptr,
-                                                 unsigned long long* bar = nullptr) {
+                                                 unsigned long long* bar = nullptr, unsigned parity = 0) {
   static_assert(MODE == 1 || MODE == 2, "stages only");
   const int W = a.W, H = a.H;
   const int i0 = tx * SPX, j0 = ty * SPY;
@@ -1187,7 +1188,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
     anyDry = anyDry || f == 1;
   }
   const bool fold = allDry && a.dryfold;          // uniform across the CTA
-  if (EARLY && fold && !tile_wait(bar, 0, ctl)) return;   // nothing of the copies is used, but they must have landed
+  if (EARLY && fold && !tile_wait(bar, parity, ctl)) return;   // nothing of the copies is used, but they must have landed
   // A folded tile settles without its state.  Its input has h = +-0 on the
   // tile (the flags), and so does U0 in stage 2 (the output record, which
   // describes U0 as this kernel wrote it in the previous step).  Every face
@@ -1235,7 +1236,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
       if (!EARLY) stage_cells_tma(a, sm, i0, j0, *maps, bar);
       if (a.W & 1) stage_depths(a, sm, i0, j0);     // no tensor map of the state
       cp_async_wait_all();
-      if (!tile_wait(bar, 0, ctl)) return;          // uniform: give up on the tile
+      if (!tile_wait(bar, parity, ctl)) return;          // uniform: give up on the tile
       if (anyDry) { zero_dry_staged(a, s, sm, i0, j0); __syncthreads(); }
     } else {
       stage_cells(a, s, sm, i0, j0);
