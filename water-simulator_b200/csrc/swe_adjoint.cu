@@ -1072,51 +1072,60 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
   const size_t N = s->N;
   if (cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(SWE_ECUDA, "swe_adjoint_create: stream"));
-  auto alloc = [&](size_t n) -> double* {
-    double* p = nullptr;
-    if (cudaMalloc(&p, sizeof(double) * std::max<size_t>(n, 1)) != cudaSuccess) return nullptr;
-    cudaMemsetAsync(p, 0, sizeof(double) * std::max<size_t>(n, 1), s->st);
-    s->allocs.push_back(p);
+  // every buffer in one allocation, 256 bytes aligned, by two passes over the
+  // same list: sizes, then places (a cudaMalloc for each of the sixty took most
+  // of the handle's creation)
+  double* base = nullptr;
+  size_t used = 0;
+  auto A = [&](size_t n) {
+    double* p = base + used;
+    used += (std::max<size_t>(n, 1) + 31) & ~size_t(31);
     return p;
   };
-  bool ok = true;
-  auto A = [&](size_t n) { double* p = alloc(n); ok = ok && p; return p; };
-  s->b = A(N); s->eta0 = A(N); s->geom = A((SWE_GEOM_NROWS + 5) * (size_t)s->H);
-  if (manning_field) s->nfield = A(N);
-  for (int q = 0; q < 3; q++) {
-    s->A[q] = A(N); s->Bf[q] = A(N); s->X[q] = A(N);
-    s->lA[q] = A(N); s->lB[q] = A(N);
-  }
-  s->ckpt = A(3 * N * (size_t)s->nseg);
-  s->tape = nullptr;               // allocated by the first backward pass
-  s->dts = A(steps);
-  s->rec = A((size_t)STEP_REC * steps);
-  s->obs = A((size_t)steps * n_gauges);
-  s->eta_series = A((size_t)steps * n_gauges);
-  s->J = A(1);
-  s->lb = A(N); s->ln = A(N);
-  for (int q = 0; q < 3; q++) s->ab.lR[q] = A(N);
-  {
-    const int ntx = (s->W + AT_X - 1) / AT_X, nty = (s->H + AT_Y - 1) / AT_Y;
-    s->fs.ntx = ntx;
-    for (int q = 0; q < 8; q++) {
-      s->fs.sx[q] = A(N); s->fs.sy[q] = A(N);
-      s->fs.ex[q] = A((size_t)ntx * s->H); s->fs.ey[q] = A((size_t)nty * s->W);
+  auto layout = [&]() {
+    used = 0;
+    s->b = A(N); s->eta0 = A(N); s->geom = A((SWE_GEOM_NROWS + 5) * (size_t)s->H);
+    if (manning_field) s->nfield = A(N);
+    for (int q = 0; q < 3; q++) {
+      s->A[q] = A(N); s->Bf[q] = A(N); s->X[q] = A(N);
+      s->lA[q] = A(N); s->lB[q] = A(N);
     }
-  }
-  const int gx = (s->W + swe::SX - 1) / swe::SX, gy = (s->H + 31) / 32;
-  s->grid = dim3(gx, gy);
-  s->nblocks = gx * gy;
-  s->sgrid = dim3((s->W + swe::SPX - 1) / swe::SPX, (s->H + swe::SPY - 1) / swe::SPY);
-  s->pcap = std::max(std::max(s->nblocks, (int)(s->sgrid.x * s->sgrid.y)), 1024);
-  s->part = A(3 * (size_t)s->pcap + 3 * swe::CLOSE_BLOCKS);      // + the close's scratch
-  {
-    const int pitch = swe::split_pitch(s->W);
-    const size_t PN = (size_t)pitch * s->H;
-    double* spl = A((size_t)swe::SPLIT_FIELDS * PN);
-    if (spl) s->sb = swe::split_bufs_at(spl, PN, pitch);
-  }
-  if (!ok || cudaMalloc(&s->ctl, sizeof(Control)) != cudaSuccess || cudaMalloc(&s->gk, sizeof(int) * n_gauges) != cudaSuccess)
+    s->ckpt = A(3 * N * (size_t)s->nseg);
+    s->tape = nullptr;               // allocated by the first backward pass
+    s->dts = A(steps);
+    s->rec = A((size_t)STEP_REC * steps);
+    s->obs = A((size_t)steps * n_gauges);
+    s->eta_series = A((size_t)steps * n_gauges);
+    s->J = A(1);
+    s->lb = A(N); s->ln = A(N);
+    for (int q = 0; q < 3; q++) s->ab.lR[q] = A(N);
+    {
+      const int ntx = (s->W + AT_X - 1) / AT_X, nty = (s->H + AT_Y - 1) / AT_Y;
+      s->fs.ntx = ntx;
+      for (int q = 0; q < 8; q++) {
+        s->fs.sx[q] = A(N); s->fs.sy[q] = A(N);
+        s->fs.ex[q] = A((size_t)ntx * s->H); s->fs.ey[q] = A((size_t)nty * s->W);
+      }
+    }
+    const int gx = (s->W + swe::SX - 1) / swe::SX, gy = (s->H + 31) / 32;
+    s->grid = dim3(gx, gy);
+    s->nblocks = gx * gy;
+    s->sgrid = dim3((s->W + swe::SPX - 1) / swe::SPX, (s->H + swe::SPY - 1) / swe::SPY);
+    s->pcap = std::max(std::max(s->nblocks, (int)(s->sgrid.x * s->sgrid.y)), 1024);
+    s->part = A(3 * (size_t)s->pcap + 3 * swe::CLOSE_BLOCKS);      // + the close's scratch
+    {
+      const int pitch = swe::split_pitch(s->W);
+      const size_t PN = (size_t)pitch * s->H;
+      double* spl = A((size_t)swe::SPLIT_FIELDS * PN);
+      s->sb = swe::split_bufs_at(spl, PN, pitch);
+    }
+  };
+  layout();
+  if (cudaMalloc(&base, sizeof(double) * used) != cudaSuccess) return bail(fail(SWE_ECUDA, "swe_adjoint_create: device allocation failed"));
+  s->allocs.push_back(base);
+  cudaMemsetAsync(base, 0, sizeof(double) * used, s->st);
+  layout();
+  if (cudaMalloc(&s->ctl, sizeof(Control)) != cudaSuccess || cudaMalloc(&s->gk, sizeof(int) * n_gauges) != cudaSuccess)
     return bail(fail(SWE_ECUDA, "swe_adjoint_create: device allocation failed"));
   cudaMemsetAsync(s->ctl, 0, sizeof(Control), s->st);
   s->cell_tma = swe::make_cell_maps(s->cmaps[0], s->sb, s->A[0], s->W, s->H) &&

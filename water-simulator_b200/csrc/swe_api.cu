@@ -104,6 +104,7 @@ struct swe_sim {
   int stage_impl = 0;
   int pdl = 1;                                     // programmatic dependent launch in the stepping loop
   double* d_split = nullptr;
+  double* d_split_own = nullptr;                   // d_split, when the handle's allocation does not hold it
   int* d_odry[2] = {nullptr, nullptr};             // per tile of A / B: all h == 0 (swe_split.cuh)
   swe::TileMaps tmaps[2];                          // the face kernel's tensor maps over A and B
   int tma = 0;                                     // 1: they are in use
@@ -346,15 +347,22 @@ void make_tile_maps(swe_sim* s) {
 }
 
 // Buffers of the tiled stage kernels (faces and source terms).
-int ensure_split(swe_sim* s) {
+// The hand-off fields, three int flags per tile, and the face and cell
+// kernels' tile lists with two counters each.
+size_t split_doubles(const swe_sim* s) {
+  const size_t N = (size_t)swe::split_pitch(s->W) * s->H, ntiles = (size_t)s->sgrid.x * s->sgrid.y;
+  return swe::SPLIT_FIELDS * N + 3 * ((ntiles + 1) / 2) + (ntiles + 2);
+}
+// mem: split_doubles() of the handle's own allocation, or null for one of its own.
+int ensure_split(swe_sim* s, double* mem = nullptr) {
   if (s->d_split) return SWE_OK;
   const int pitch = swe::split_pitch(s->W);
-  const size_t N = (size_t)pitch * s->H;
-  const size_t ntiles = (size_t)s->sgrid.x * s->sgrid.y;
-  // + three int flags per tile, and the face and cell kernels' tile lists
-  // with two counters each
-  const size_t doubles = swe::SPLIT_FIELDS * N + 3 * ((ntiles + 1) / 2) + (ntiles + 2);
-  CU(cudaMalloc(&s->d_split, sizeof(double) * doubles));
+  const size_t N = (size_t)pitch * s->H, ntiles = (size_t)s->sgrid.x * s->sgrid.y, doubles = split_doubles(s);
+  if (!mem) {
+    CU(cudaMalloc(&s->d_split_own, sizeof(double) * doubles));
+    mem = s->d_split_own;
+  }
+  s->d_split = mem;
   CU(cudaMemsetAsync(s->d_split, 0, sizeof(double) * doubles, s->st));
   s->sb = swe::split_bufs_at(s->d_split, N, pitch);
   s->sb.dry = reinterpret_cast<int*>(s->d_split + swe::SPLIT_FIELDS * N);
@@ -650,7 +658,7 @@ int upload_geom(swe_sim* s) {
 void free_all(swe_sim* s) {
   for (auto& g : s->graphs) if (g.exec) cudaGraphExecDestroy(g.exec);
   double** ptrs[] = {&s->d_all, &s->d_h0[0], &s->d_h0[1], &s->d_h0[2], &s->d_res[0], &s->d_res[1], &s->d_res[2],
-                     &s->d_res[3], &s->d_nfield, &s->d_coef, &s->d_sponge, &s->d_split};
+                     &s->d_res[3], &s->d_nfield, &s->d_coef, &s->d_sponge, &s->d_split_own};
   for (double** p : ptrs) if (*p) { cudaFree(*p); *p = nullptr; }
   if (s->d_vol) cudaFree(s->d_vol);
   if (s->d_frame) cudaFree(s->d_frame);
@@ -730,13 +738,19 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
   CUB(cudaFuncSetAttribute(swe::k_stage<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, swe::STAGE_SMEM_BYTES));
   CUB(cudaFuncSetAttribute(swe::k_stage<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, swe::STAGE_SMEM_BYTES));
   CUB(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
-  // The handle's fixed buffers in one allocation, 256 bytes aligned each (a
-  // cudaMalloc and cudaFree for every one took longer than the rest of a small
-  // handle's creation); the partials are the tiles', the close's scratch and the
-  // reductions'.
+  {
+    const char* env = std::getenv("SWE_B200_STAGE");
+    s->stage_impl = (env && std::strcmp(env, "fused") == 0) ? 0 : (env && std::strcmp(env, "split") == 0) ? 1
+                                                                  : SWE_DEFAULT_STAGE;
+  }
+  // The handle's buffers in one allocation, 256 bytes aligned each (a cudaMalloc
+  // and cudaFree for every one took longer than the rest of a small handle's
+  // creation: each new 2 MB of memory costs some 0.3 ms); the partials are the
+  // tiles', the close's scratch and the reductions'.
   const size_t nparts = 3 * (size_t)s->part_cap + 3 * swe::CLOSE_BLOCKS + REDUCTION_BLOCKS;
-  const size_t N = s->N, sizes[11] = {N, N, N, N, N, N, N, (size_t)(SWE_GEOM_NROWS + 5) * s->H, nparts,
-                                      (size_t)std::max(1, s->ny), (sizeof(swe::Control) + 7) / 8};
+  const size_t N = s->N, sizes[12] = {N, N, N, N, N, N, N, (size_t)(SWE_GEOM_NROWS + 5) * s->H, nparts,
+                                      (size_t)std::max(1, s->ny), (sizeof(swe::Control) + 7) / 8,
+                                      s->stage_impl == 1 ? split_doubles(s) : 0};
   double** const ptrs[10] = {&s->d_b, &s->d_A[0], &s->d_A[1], &s->d_A[2], &s->d_B[0], &s->d_B[1], &s->d_B[2],
                              &s->d_geom, &s->d_part, &s->d_rows};
   size_t total = 0;
@@ -748,6 +762,7 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
     else s->d_ctl = reinterpret_cast<swe::Control*>(at);
     at += (sizes[q] + 31) & ~size_t(31);
   }
+  double* const split_mem = at;
   s->d_red = s->d_part + (nparts - REDUCTION_BLOCKS);
   CUB(cudaMemsetAsync(s->d_ctl, 0, sizeof(swe::Control), s->st));
   CUB(cudaMemsetAsync(s->d_part, 0, sizeof(double) * nparts, s->st));
@@ -761,10 +776,7 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
   if (upload_geom(s)) return bail(SWE_ECUDA);
   make_tile_maps(s);
   {
-    const char* env = std::getenv("SWE_B200_STAGE");
-    s->stage_impl = (env && std::strcmp(env, "fused") == 0) ? 0 : (env && std::strcmp(env, "split") == 0) ? 1
-                                                                  : SWE_DEFAULT_STAGE;
-    if (s->stage_impl == 1 && ensure_split(s)) return bail(SWE_ECUDA);
+    if (s->stage_impl == 1 && ensure_split(s, split_mem)) return bail(SWE_ECUDA);
     const char* pe = std::getenv("SWE_B200_PDL");
     s->pdl = (pe && std::strcmp(pe, "0") == 0) ? 0 : 1;
   }
