@@ -184,8 +184,7 @@ __device__ __forceinline__ double lout_of(const Geo& g, const Inter& it, const d
 // Per-cell sums are in FaceIn's left-side order: b, h, normal, transverse,
 // sE, sB, s(normal), s(transverse).
 constexpr int AT_X = 32;           // tile width (one warp)
-constexpr int AT_XROWS = 4;        // rows per x-face block (128 threads)
-constexpr int AT_Y = 8;            // rows per y-face / cell tile (256 threads)
+constexpr int AT_Y = 8;            // rows per face / cell tile (256 threads)
 // The face kernels are latency bound: capped at 64 registers (32 warps per
 // SM; a few hundred bytes of spills) they measured faster than at 80
 // (24 warps) or at their natural 112 (16 warps).
@@ -205,12 +204,10 @@ struct FaceSums {
   int ntx;                         // tiles per row (ceil(W / 32))
 };
 
-__global__ void __launch_bounds__(AT_X * AT_XROWS, SWE_ADJ_FACE_WARPS / AT_XROWS)
-k_adj_xfaces(Geo g, const double* b, const double* h, Inter it, const double* theta, double dt, AdjBuf a,
-             FaceSums S) {
-  pdl_enter();
+__device__ __forceinline__ void adj_xfaces(const Geo& g, const double* b, const double* h, const Inter& it,
+                                           const double* theta, double dt, const AdjBuf& a, const FaceSums& S) {
   const int tx = threadIdx.x, bx = blockIdx.x;
-  const int i = bx * AT_X + tx, j = blockIdx.y * AT_XROWS + threadIdx.y;
+  const int i = bx * AT_X + tx, j = blockIdx.y * AT_Y + threadIdx.y;
   const bool valid = i < g.W && j < g.H;
   const int k = j * g.W + i;
   FaceIn gx = {};
@@ -234,11 +231,9 @@ k_adj_xfaces(Geo g, const double* b, const double* h, Inter it, const double* th
   }
 }
 
-__global__ void __launch_bounds__(AT_X * AT_Y, SWE_ADJ_FACE_WARPS / AT_Y)
-k_adj_yfaces(Geo g, const double* b, const double* h, Inter it, const double* theta, double dt, AdjBuf a,
-             FaceSums S) {
-  pdl_enter();
-  __shared__ double up[AT_Y][8][AT_X];
+__device__ __forceinline__ void adj_yfaces(const Geo& g, const double* b, const double* h, const Inter& it,
+                                           const double* theta, double dt, const AdjBuf& a, const FaceSums& S,
+                                           double (*up)[8][AT_X]) {
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i = blockIdx.x * AT_X + tx, j = blockIdx.y * AT_Y + ty;
   const bool valid = i < g.W && j < g.H;
@@ -264,6 +259,17 @@ k_adj_yfaces(Geo g, const double* b, const double* h, Inter it, const double* th
 #pragma unroll
     for (int q = 0; q < 8; q++) S.ey[q][(size_t)blockIdx.y * g.W + i] = p[8 + q];
   }
+}
+
+// Both directions in one launch (grid z), which neither reads of the other: two
+// launches of a grid that fills the GPU one and a third times left it idle at
+// the end of each.
+__global__ void __launch_bounds__(AT_X * AT_Y, SWE_ADJ_FACE_WARPS / AT_Y)
+k_adj_faces(Geo g, const double* b, const double* h, Inter it, const double* theta, double dt, AdjBuf a, FaceSums S) {
+  __shared__ double up[AT_Y][8][AT_X];
+  pdl_enter();
+  if (blockIdx.z == 0) adj_xfaces(g, b, h, it, theta, dt, a, S);
+  else adj_yfaces(g, b, h, it, theta, dt, a, S, up);
 }
 
 // The face sums of cell (i, j) in direction d (0: x, 1: y), with the half
@@ -864,9 +870,7 @@ int residual_adjoint(swe_adjoint* s, double* const* X, const Inter& it, const do
   const int ntx = (s->W + AT_X - 1) / AT_X;
   const double* b = s->b;
   const double* h = X[0];
-  LAUNCH(k_adj_xfaces, dim3(ntx, (s->H + AT_XROWS - 1) / AT_XROWS), dim3(AT_X, AT_XROWS), g, b, h, it, theta, dt,
-         s->ab, s->fs);
-  LAUNCH(k_adj_yfaces, dim3(ntx, (s->H + AT_Y - 1) / AT_Y), dim3(AT_X, AT_Y), g, b, h, it, theta, dt, s->ab, s->fs);
+  LAUNCH(k_adj_faces, dim3(ntx, (s->H + AT_Y - 1) / AT_Y, 2), dim3(AT_X, AT_Y), g, b, h, it, theta, dt, s->ab, s->fs);
   LAUNCH(k_adj_cells_tiled, dim3(ntx, (s->H + AT_Y - 1) / AT_Y), dim3(AT_X, AT_Y), g, b, h, (const double*)X[1],
          (const double*)X[2], it, theta, dt, s->ab, s->fs, s->lb, lX[0], lX[1], lX[2]);
   return SWE_OK;
