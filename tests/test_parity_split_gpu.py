@@ -149,3 +149,30 @@ def test_face_tile_list_gives_the_same_bits(swe, monkeypatch, nx, ny):
     for x, y in zip(a[:3], b[:3]):
         assert np.array_equal(x, y)
     assert a[3:] == b[3:]
+
+
+@pytest.mark.parametrize("nx,ny", [(2050, 1800), (1801, 2047)])
+def test_looped_tile_lists_give_the_same_bits(swe, monkeypatch, nx, ny):
+    """A grid on which more than 8192 tiles settle and more than 4736 are
+    listed, so that the listed kernels' CTAs take several tiles each: the
+    same bits as without the lists (SWE_B200_FACE_LIST=0).  An odd width has
+    no tensor map of the state."""
+    import numpy as np
+    from water_simulator_b200 import workloads
+
+    X = np.arange(nx + 4)[None, :] / nx + 0 * np.arange(ny + 4)[:, None]
+    b = 40.0 * (X - 0.35) + workloads.uniform_noise(7, X.shape, -0.2, 0.2)
+    eta = np.maximum(b, np.where(X < 0.33, 0.5, 0.0))
+
+    def run(on):
+        monkeypatch.setenv("SWE_B200_FACE_LIST", "1" if on else "0")
+        sim = swe.ShallowWater(nx=nx, ny=ny, dx=2.0, bed=b, eta0=eta, manning=0.03)
+        assert sim.run(150) == 150 and sim.run(20) == 20
+        out = [sim.field(f).view(np.uint64).copy() for f in ("h", "hu", "hv")] + [sim.t, sim.massFloored]
+        sim.close()
+        return out
+
+    a, b_ = run(True), run(False)
+    for x, y in zip(a[:3], b_[:3]):
+        assert np.array_equal(x, y)
+    assert a[3:] == b_[3:]

@@ -123,13 +123,15 @@ struct swe_sim {
   // choice (settle_pref) for shorter runs; grids with little dry land run
   // the plain kernel faster.  The single-step entry points always settle.
   int settle = 1, settle_pref = 1;
-  // device-resident loop graphs, one per value of `settle`
+  // Whether the listed kernels loop (launch_stage_listed), chosen with it.
+  int list_loop = 0;
+  // device-resident loop graphs: without settling, with it, and with the loop
   struct LoopGraph {
     cudaGraphExec_t exec = nullptr;
     int steps = 0, mode = -1;
     double dt = 0, tend = 0;
     unsigned long long version = 0;
-  } graphs[2];
+  } graphs[3];
   unsigned long long version = 1;
 };
 
@@ -417,12 +419,23 @@ swe::TileLists tile_lists(const swe_sim* s, const swe::StageArgs& a) {
   return L;
 }
 
+// The listed kernels loop (k_split_faces_tma_list) where at least LOOP_SETTLED
+// tiles settle, with 8 waves of CTAs.  128 steps of a beach, one CTA per tile of the
+// grid against the loop, with the tiles of the grid and about how many settle:
+//   1300 x 1300  ( 6 724,  4 500)  14.6  15.2 ms   not looped
+//   2048 x 2048  (16 384,  6 400)  72.5  73.8      not looped
+//   1700 x 1700  (11 449,  8 500)  20.2  19.2
+//   3000 x 2400  (28 200, 11 000)  90.2  86.3
+//   2048 x 2048  (16 384, 13 000)  25.8  22.8
+//   3000 x 2400  (28 200, 24 000)  35.9  27.3
+// With 1, 2 and 4 waves the fifth took 27.3, 24.1 and 22.6, the fourth, of 4, 89.2.
+constexpr int LIST_CTAS = 8 * 4 * 148, LOOP_SETTLED = 8192;
 // Stage MODE with the tile lists.  list_done: they were made with the ghost
 // fill (launch_bc_lists).
-template <int MODE>
+template <int MODE, bool LOOP>
 int launch_stage_listed(swe_sim* s, const swe::StageArgs& a, bool pdl, bool list_done) {
   const swe::SplitBufs sb = stage_bufs<MODE>(s);
-  const dim3 blk(swe::SP_THREADS), tiles(tiles_of(s));
+  const dim3 blk(swe::SP_THREADS), tiles(LOOP ? std::min(LIST_CTAS, tiles_of(s)) : tiles_of(s));
   const swe::CellMaps& cm = s->cmaps[MODE - 1];
   if (!list_done)
     CU(launch(pdl, swe::k_face_list, dim3((s->sgrid.x + swe::LX - 1) / swe::LX, (s->sgrid.y + swe::LY - 1) / swe::LY),
@@ -430,11 +443,11 @@ int launch_stage_listed(swe_sim* s, const swe::StageArgs& a, bool pdl, bool list
   const int* list = s->d_flist;
   const int* count = s->d_fcount + (MODE - 1);
   if (s->tma)
-    CU(launch(pdl, swe::k_split_faces_tma_list, tiles, blk, s->st, a, sb, s->d_ctl, s->tmaps[MODE - 1], list, count));
+    CU(launch(pdl, swe::k_split_faces_tma_list<LOOP>, tiles, blk, s->st, a, sb, s->d_ctl, s->tmaps[MODE - 1], list, count));
   else
-    CU(launch(pdl, swe::k_split_faces_list, tiles, blk, s->st, a, sb, s->d_ctl, list, count));
+    CU(launch(pdl, swe::k_split_faces_list<LOOP>, tiles, blk, s->st, a, sb, s->d_ctl, list, count));
   if (cell_listed(s, a))                           // only when tiles may be left out
-    CU(launch(pdl, swe::k_split_cells_tma_list<MODE, true>, tiles, blk, s->st, a, sb, s->d_ctl, cm,
+    CU(launch(pdl, swe::k_split_cells_tma_list<MODE, LOOP>, tiles, blk, s->st, a, sb, s->d_ctl, cm,
               (const int*)s->d_clist, (const int*)(s->d_ccount + (MODE - 1))));
   else
     CU(launch(pdl, swe::k_split_cells_tma<MODE, true>, s->sgrid, blk, s->st, a, sb, s->d_ctl, cm));
@@ -487,8 +500,9 @@ template <int MODE>
 int launch_stage(swe_sim* s, const swe::StageArgs& a, bool pdl = false, bool list_done = false) {
   if (s->stage_impl == 1) {
     const swe::GhostFill none = {};
-    int rc = stage_listed(s) ? launch_stage_listed<MODE>(s, a, pdl, list_done)
-                             : launch_stage_tiles<MODE>(s, a, pdl, none);
+    int rc = !stage_listed(s) ? launch_stage_tiles<MODE>(s, a, pdl, none)
+             : s->list_loop   ? launch_stage_listed<MODE, true>(s, a, pdl, list_done)
+                              : launch_stage_listed<MODE, false>(s, a, pdl, list_done);
     if (rc == SWE_OK && MODE == 2) rc = launch_close(s, a, pdl);
     if (rc) return rc;
   } else {
@@ -1172,9 +1186,9 @@ int swe_run(swe_sim* s, int n, double dt_fixed, double t_end, int* done) {
   // steps launched directly, one of 32 as fast as them.
   const int chunk = 32;
   // The graph of `chunk` steps with the current value of s->settle, built
-  // once per (chunk, mode, dt, tEnd, options) and kept.
+  // once per (settle, list_loop, mode, dt, tEnd, options) and kept.
   auto graph_for = [&](cudaGraphExec_t* out) -> int {
-    swe_sim::LoopGraph& g = s->graphs[s->settle ? 1 : 0];
+    swe_sim::LoopGraph& g = s->graphs[s->settle ? 1 + s->list_loop : 0];
     if (!g.exec || g.steps != chunk || g.mode != mode || g.dt != dtv || g.tend != t_end || g.version != s->version) {
       if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
       cudaGraph_t graph;
@@ -1208,6 +1222,7 @@ int swe_run(swe_sim* s, int n, double dt_fixed, double t_end, int* done) {
       CU(cudaMemcpyAsync(&counted, &s->d_ctl->settled_next, sizeof(int), cudaMemcpyDeviceToHost, s->st));
       CU(cudaStreamSynchronize(s->st));
       s->settle = s->settle_pref = 32 * counted >= (int)(s->sgrid.x * s->sgrid.y) ? 1 : 0;
+      s->list_loop = 8 * counted >= LOOP_SETTLED ? 1 : 0;   // one tile in 16, in each of two stages
     }
   }
   if (left >= chunk) {

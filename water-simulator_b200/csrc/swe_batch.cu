@@ -122,7 +122,7 @@ k_batch_split_faces(BatchBasin* basins, const BatchMaps* maps, const BatchTile* 
         swe::split_faces_tile(A.a, A.sp, tile.strip, tile.y0, sm);
       }
     }
-    __syncthreads();          // the next tile's arguments replace these
+    swe::next_tile();         // whose arguments also replace these
   }
 }
 
@@ -147,7 +147,7 @@ k_batch_split_cells(BatchBasin* basins, const BatchMaps* maps, const BatchTile* 
         swe::split_cells_tile<MODE>(A.a, A.sp, A.ctl, tile.strip, tile.y0, tile.part, A.a.nblocks, sm, false);
       }
     }
-    __syncthreads();          // the next tile reuses the shared memory
+    swe::next_tile();
   }
 }
 

@@ -496,6 +496,9 @@ __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned coun
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 }
+__device__ __forceinline__ void mbar_inval(unsigned long long* bar) {
+  asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_addr(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes)
                : "memory");
@@ -542,6 +545,13 @@ __device__ __forceinline__ bool tile_wait(unsigned long long* bar, unsigned pari
   }
   __syncthreads();
   return false;
+}
+
+// Between two tiles of a CTA: what its threads read and wrote in the shared
+// tiles comes before the copies into them that one thread starts next.
+__device__ __forceinline__ void next_tile() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
 }
 
 // split_faces_tile with the state tile fetched by tensor-map copies, in two
@@ -744,29 +754,51 @@ __global__ void __launch_bounds__(LX * LY) k_bc_face_list(BCArgs b, int respect_
   face_list_region(s, ctl, L, r % nrx, r / nrx);
 }
 
-// The face kernel over the list: CTA b computes the list's entry b, and the
-// CTAs past the list's length exit after reading it.
+// The face kernel over the list.  LOOP false: one CTA per tile of the grid, CTA b
+// computes the list's entry b, and those past its length exit after reading it,
+// of which the chip starts about one in a nanosecond.  LOOP true: LIST_CTAS CTAs
+// each take every gridDim.x-th entry, at about 3% more a tile (swe_api.cu has the
+// rule and what both measured).  What a CTA keeps from tile to tile then stands
+// in shared memory, not in registers that the tile's code would spill around.
+struct ListWalk { volatile int at; volatile unsigned parity; };
+
+template <bool LOOP>
 __global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_MIN_BLOCKS)
 k_split_faces_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ TileMaps maps,
                        const int* list, const int* count) {
   __shared__ FacesSmem sm;
   __shared__ alignas(8) unsigned long long bar;
+  __shared__ ListWalk walk;
   pdl_enter();
   if ((int)blockIdx.x >= min(*count, s.ntx * s.nty) || ctl->stop) return;
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    walk.at = blockIdx.x; walk.parity = 0;
+  }
   __syncthreads();
-  const int tile = list[blockIdx.x];
-  unsigned parity = 0;
-  start_box(sm, tile % s.ntx, tile / s.ntx, maps, &bar);
-  split_faces_started(a, s, tile % s.ntx, tile / s.ntx, sm, &bar, parity, ctl);
+  do {
+    const int tile = list[LOOP ? walk.at : blockIdx.x];
+    unsigned parity = LOOP ? walk.parity : 0;
+    start_box(sm, tile % s.ntx, tile / s.ntx, maps, &bar);
+    split_faces_started(a, s, tile % s.ntx, tile / s.ntx, sm, &bar, parity, ctl);
+    if (!LOOP) return;
+    next_tile();
+    if (threadIdx.x == 0) { walk.at = walk.at + gridDim.x; walk.parity = walk.parity ^ 1u; }
+    __syncthreads();
+  } while (walk.at < min(*count, s.ntx * s.nty));
 }
+template <bool LOOP>
 __global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_FACES_MIN_BLOCKS)
 k_split_faces_list(StageArgs a, SplitBufs s, Control* ctl, const int* list, const int* count) {
   __shared__ FacesSmem sm;
   pdl_enter();
   if ((int)blockIdx.x >= min(*count, s.ntx * s.nty) || ctl->stop) return;
-  const int tile = list[blockIdx.x];
-  split_faces_tile(a, s, tile % s.ntx, tile / s.ntx, sm, false);
+  for (int b = blockIdx.x; b < min(*count, s.ntx * s.nty); b += gridDim.x) {
+    const int tile = list[b];
+    split_faces_tile(a, s, tile % s.ntx, tile / s.ntx, sm, false);
+    if (!LOOP) return;
+    __syncthreads();                              // the next tile reuses the shared memory
+  }
 }
 
 // The cell kernel's inputs from the face kernel, staged for the tile at
@@ -1134,9 +1166,9 @@ __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& 
 // tile is known to be computed; TMA: by tensor-map copies (maps, completing on
 // bar), of which one that does not complete within the bound leaves the tile's
 // output unwritten (tile_wait); parity is bar's phase, which without SETTLE
-// every tile completes once.
+// every tile completes once.  false: given up on (in every thread).
 template <int MODE, bool SETTLE = false, bool TMA = false>
-__device__ __forceinline__ void split_cells_tile(const StageArgs& a, const SplitBufs& s, Control* ctl, int tx,
+__device__ __forceinline__ bool split_cells_tile(const StageArgs& a, const SplitBufs& s, Control* ctl, int tx,
                                                  int ty, int part, int nparts, CellsSmem& sm, bool ticket,
                                                  const CellMaps* maps = nullptr,
                                                  unsigned long long* bar = nullptr, unsigned parity = 0) {
@@ -1188,7 +1220,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
     anyDry = anyDry || f == 1;
   }
   const bool fold = allDry && a.dryfold;          // uniform across the CTA
-  if (EARLY && fold && !tile_wait(bar, parity, ctl)) return;   // nothing of the copies is used, but they must have landed
+  if (EARLY && fold && !tile_wait(bar, parity, ctl)) return false;   // nothing of the copies is used, but they must have landed
   // A folded tile settles without its state.  Its input has h = +-0 on the
   // tile (the flags), and so does U0 in stage 2 (the output record, which
   // describes U0 as this kernel wrote it in the previous step).  Every face
@@ -1216,7 +1248,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
         else { a.part_max[part] = 0; a.part_fl2[part] = 0; }
         if ((part & 15) == 0) atomicAdd(&ctl->settled_next, 1);
       }
-      return;                                     // canSettle excludes the ticket
+      return true;                                // canSettle excludes the ticket
     }
   }
   // the cell's own state, in flight while the limiter is worked out
@@ -1236,7 +1268,7 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
       if (!EARLY) stage_cells_tma(a, sm, i0, j0, *maps, bar);
       if (a.W & 1) stage_depths(a, sm, i0, j0);     // no tensor map of the state
       cp_async_wait_all();
-      if (!tile_wait(bar, parity, ctl)) return;          // uniform: give up on the tile
+      if (!tile_wait(bar, parity, ctl)) return false;          // uniform: give up on the tile
       if (anyDry) { zero_dry_staged(a, s, sm, i0, j0); __syncthreads(); }
     } else {
       stage_cells(a, s, sm, i0, j0);
@@ -1295,11 +1327,12 @@ __device__ __forceinline__ void split_cells_tile(const StageArgs& a, const Split
       sm.last = (tk == (unsigned int)(nparts - 1));
     }
   }
-  if (!ticket) return;
+  if (!ticket) return true;
   __syncthreads();
-  if (!sm.last) return;                         // uniform across the CTA
+  if (!sm.last) return true;                         // uniform across the CTA
   __threadfence();
   split_close_block<MODE>(a, ctl, nparts, sm);
+  return true;
 }
 
 #ifndef SWE_SPLIT_CELLS_MIN_BLOCKS
@@ -1445,20 +1478,35 @@ k_split_cells_tma(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant_
                                        gridDim.x * gridDim.y, sm, false, &maps, &bar);
 }
 
-// The cell kernel over its list: CTA b runs the list's entry b; the CTAs
-// past the list's length exit after reading it.
-template <int MODE, bool SETTLE = false>
+// The cell kernel over its list, as the face kernel over its own.
+template <int MODE, bool LOOP>
 __global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_CELLS_MIN_BLOCKS)
 k_split_cells_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ CellMaps maps,
                        const int* list, const int* count) {
   __shared__ CellsSmem sm;
   __shared__ alignas(8) unsigned long long bar;
+  __shared__ ListWalk walk;
   pdl_enter();
   const int ntiles = s.ntx * s.nty;
   if ((int)blockIdx.x >= min(*count, ntiles) || ctl->stop) return;
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
-  const int tile = list[blockIdx.x];
-  split_cells_tile<MODE, SETTLE, true>(a, s, ctl, tile % s.ntx, tile / s.ntx, tile, ntiles, sm, false, &maps, &bar);
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    walk.at = blockIdx.x; walk.parity = 0;
+  }
+  if (LOOP) __syncthreads();
+  do {
+    const int tile = list[LOOP ? walk.at : blockIdx.x];
+    if (!split_cells_tile<MODE, true, true>(a, s, ctl, tile % s.ntx, tile / s.ntx, tile, ntiles, sm, false, &maps, &bar))
+      return;
+    if (!LOOP) return;
+    next_tile();
+    if (threadIdx.x == 0) {
+      walk.at = walk.at + gridDim.x;
+      mbar_inval(&bar);                           // only tiles that are computed complete its phase
+      mbar_init(&bar, 1);
+    }
+    __syncthreads();
+  } while (walk.at < min(*count, ntiles));
 }
 
 // Closes the stage k_split_cells left open: one block, no atomics (a
