@@ -176,3 +176,35 @@ def test_looped_tile_lists_give_the_same_bits(swe, monkeypatch, nx, ny):
     for x, y in zip(a[:3], b_[:3]):
         assert np.array_equal(x, y)
     assert a[3:] == b_[3:]
+
+
+@pytest.mark.parametrize("side", ["west", "east", "south", "north", "inside"])
+@pytest.mark.parametrize("nx,ny", [(96, 40), (97, 41)])
+def test_a_single_limited_cell_next_to_a_tile(swe, monkeypatch, nx, ny, side):
+    """The cell kernel looks for limited cells in a tile and in the cells
+    beside it, and reads theta only then.  A cell of thin, fast water on each
+    side of the tile of columns 32 to 63 and rows 16 to 23 (padded), and
+    inside it, on dry land: 0.9 s at 26 m/s would take 2.3 times what it
+    holds over one 10 m face.  The same bits as the fused kernel, which forms
+    theta for every cell."""
+    import numpy as np
+
+    j, i = {"west": (18, 31), "east": (19, 64), "south": (15, 40), "north": (24, 50), "inside": (20, 45)}[side]
+
+    def run(impl):
+        monkeypatch.setenv("SWE_B200_STAGE", impl)
+        b = np.zeros((ny + 4, nx + 4))
+        sim = swe.ShallowWater(nx=nx, ny=ny, dx=10.0, bed=b, eta0=b)
+        state = {f: b.copy() for f in ("h", "hu", "hv")}
+        state["h"][17:22, 34:38] = 0.5               # calm, so that the tile has water of its own
+        state["h"][j, i], state["hu"][j, i], state["hv"][j, i] = 0.05, 1.3, -0.9
+        for f, v in state.items():
+            setattr(sim, f, v.reshape(-1))
+        for _ in range(3):
+            sim.step(0.9)
+        out = [sim.field(f).view(np.uint64).copy() for f in ("h", "hu", "hv")]
+        sim.close()
+        return out
+
+    for x, y in zip(run("fused"), run("split")):
+        assert np.array_equal(x, y)

@@ -463,7 +463,7 @@ int launch_stage_tiles(swe_sim* s, const swe::StageArgs& a, bool pdl, const swe:
   const swe::TileMaps& tm = s->tmaps[MODE - 1];
   swe::Control* ctl = s->d_ctl;
   constexpr int WIDE = SWE_SPLIT_FACES_MIN_BLOCKS, ROOMY = WIDE - 1;
-  const bool roomy = tiles_of(s) <= ROOMY * 148;   // see k_split_faces
+  const bool roomy = tiles_of(s) <= ROOMY * 148;   // see k_split_faces, k_split_cells_tma
   if (s->tma) {
     if (!F.on) CU(launch(pdl, swe::k_split_faces_tma<WIDE, false>, grid, blk, s->st, a, sb, ctl, tm, F));
     else if (roomy) CU(launch(pdl, swe::k_split_faces_tma<ROOMY, true>, grid, blk, s->st, a, sb, ctl, tm, F));
@@ -475,6 +475,7 @@ int launch_stage_tiles(swe_sim* s, const swe::StageArgs& a, bool pdl, const swe:
   }
   if (s->cell_tma) {
     if (settles(s)) CU(launch(pdl, swe::k_split_cells_tma<MODE, true>, grid, blk, s->st, a, sb, ctl, cm));
+    else if (roomy) CU(launch(pdl, swe::k_split_cells_tma<MODE, false, ROOMY>, grid, blk, s->st, a, sb, ctl, cm));
     else CU(launch(pdl, swe::k_split_cells_tma<MODE, false>, grid, blk, s->st, a, sb, ctl, cm));
   } else {
     if (settles(s)) CU(launch(pdl, swe::k_split_cells<MODE, true>, grid, blk, s->st, a, sb, ctl));

@@ -122,7 +122,7 @@ k_batch_split_faces(BatchBasin* basins, const BatchMaps* maps, const BatchTile* 
         swe::split_faces_tile(A.a, A.sp, tile.strip, tile.y0, sm);
       }
     }
-    swe::next_tile();         // whose arguments also replace these
+    __syncthreads();          // the next tile's arguments replace these
   }
 }
 
@@ -147,7 +147,7 @@ k_batch_split_cells(BatchBasin* basins, const BatchMaps* maps, const BatchTile* 
         swe::split_cells_tile<MODE>(A.a, A.sp, A.ctl, tile.strip, tile.y0, tile.part, A.a.nblocks, sm, false);
       }
     }
-    swe::next_tile();
+    __syncthreads();          // the next tile reuses the shared memory
   }
 }
 

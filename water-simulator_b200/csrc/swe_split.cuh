@@ -547,13 +547,6 @@ __device__ __forceinline__ bool tile_wait(unsigned long long* bar, unsigned pari
   return false;
 }
 
-// Between two tiles of a CTA: what its threads read and wrote in the shared
-// tiles comes before the copies into them that one thread starts next.
-__device__ __forceinline__ void next_tile() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncthreads();
-}
-
 // split_faces_tile with the state tile fetched by tensor-map copies, in two
 // parts: start_box, in which thread 0 starts them, and the rest.  bar is an
 // initialised mbarrier in shared memory and parity its phase, flipped here for
@@ -782,7 +775,7 @@ k_split_faces_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_cons
     start_box(sm, tile % s.ntx, tile / s.ntx, maps, &bar);
     split_faces_started(a, s, tile % s.ntx, tile / s.ntx, sm, &bar, parity, ctl);
     if (!LOOP) return;
-    next_tile();
+    __syncthreads();                              // the next tile reuses the shared memory
     if (threadIdx.x == 0) { walk.at = walk.at + gridDim.x; walk.parity = walk.parity ^ 1u; }
     __syncthreads();
   } while (walk.at < min(*count, s.ntx * s.nty));
@@ -829,6 +822,7 @@ struct CellsSmem {
   double red[2][SP_THREADS / 32];
   bool zero[SP_THREADS / 32];     // every cell of the warp was left with h == 0
   int dry[3][3];                  // dry flags of the tile's 3 x 3 neighbourhood, 2 outside the grid
+  int flags;                      // bit 0: all nine are set; bit 1: one is 1
   int prev;                       // the output tile's record as this kernel left it last time
   bool last;
 };
@@ -889,22 +883,34 @@ __device__ __forceinline__ void stage_cells(const StageArgs& a, const SplitBufs&
     }
   });
 }
-// Staging by tensor maps: thread 0 starts the copies, bar counts their bytes.
+// Staging by tensor maps: bar counts the copies' bytes.  SPREAD: each warp's first
+// thread starts a share of them (every thread calls it, bar's initialisation behind a
+// barrier), where the CTA has nothing else to do meanwhile: 13 from one thread take
+// their time (100 steps of 256 x 256 3.53 -> 3.49 ms).  Otherwise thread 0 does.
+template <bool SPREAD>
 __device__ __forceinline__ void stage_cells_tma(const StageArgs& a, CellsSmem& sm, int i0, int j0, const CellMaps& maps,
                                                 unsigned long long* bar) {
-  if (threadIdx.x != 0) return;
+  if (SPREAD ? (threadIdx.x & 31) != 0 : threadIdx.x != 0) return;
+  const int w = threadIdx.x >> 5;
+  const auto mine = [w](int of) { return !SPREAD || w == of; };
   // the generic-proxy accesses of the shared memory come before the copies' writes
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  mbar_expect_tx(bar, CELL_TX_BYTES + (a.sph ? CELL_TG_BYTES : 0) + (a.W & 1 ? 0 : CELL_HR_BYTES));
+  if (mine(0)) mbar_expect_tx(bar, CELL_TX_BYTES + (a.sph ? CELL_TG_BYTES : 0) + (a.W & 1 ? 0 : CELL_HR_BYTES));
   const int x = i0 - 2;
   CellFaceTiles& ft = sm.ft;
-  tma_load_tile(&ft.xm[0][0], &maps.m[CM_XM], x, j0 - 1, bar);
-  tma_load_tile(&ft.ym[0][0], &maps.m[CM_YM], x, j0 - 2, bar);
-  if (!(a.W & 1)) tma_load_tile(&ft.hr[0][0], &maps.m[CM_H], x, j0 - 1, bar);
-  for (int q = 0; q < 3; q++) {
+  if (mine(0)) tma_load_tile(&ft.xm[0][0], &maps.m[CM_XM], x, j0 - 1, bar);
+  if (mine(1)) {
+    tma_load_tile(&ft.ym[0][0], &maps.m[CM_YM], x, j0 - 2, bar);
+    if (!(a.W & 1)) tma_load_tile(&ft.hr[0][0], &maps.m[CM_H], x, j0 - 1, bar);
+  }
+  for (int q = SPREAD ? w - 2 : 0; q < 3; q += SPREAD ? 8 : 1) {
+    if (q < 0) break;
     tma_load_tile(&ft.xt[q][0][0], &maps.m[CM_XT + q], x, j0, bar);
-    tma_load_tile(&ft.yt[q][0][0], &maps.m[CM_YT + q], i0, j0 - 1, bar);
     if (q < 2 || a.sph) tma_load_tile(&ft.tb[q][0][0], &maps.m[CM_TB + q], i0, j0, bar);
+  }
+  for (int q = SPREAD ? w - 5 : 0; q < 3; q += SPREAD ? 8 : 1) {
+    if (q < 0) break;
+    tma_load_tile(&ft.yt[q][0][0], &maps.m[CM_YT + q], i0, j0 - 1, bar);
   }
 }
 // After the tensor-map copies: +0 for what dry tiles own (their faces were
@@ -919,8 +925,19 @@ __device__ __forceinline__ void zero_dry_staged(const StageArgs& a, const SplitB
 }
 
 // Positivity limiter of cell (gi, gj), the staged tiles' (ly, lx) from the
-// ring's corner, from its four faces' mass fluxes (src/swe.mjs:511-529), with
-// the same conservative pre-test as stage_tile.
+// ring's corner, from its four faces' mass fluxes (src/swe.mjs:511-529).
+// free_theta says that it is 1 without a division: the sum of all four, of which
+// the outflow is a part, stays below what there is by more than the rounding.
+struct RowMetric { double rdx, rdyS, rdyN; };
+__device__ __forceinline__ RowMetric row_metric(const Metric& m, int gj) {
+  return {m.rdxRow[gj], m.rdyRowS[gj], m.rdyRowN[gj]};
+}
+__device__ __forceinline__ bool free_theta(const CellFaceTiles& ft, const RowMetric& r, double dt, int ly, int lx) {
+  const double fxE = ft.xm[ly][lx + 1], fxW = ft.xm[ly][lx], fyN = ft.ym[ly + 1][lx + 1], fyS = ft.ym[ly][lx + 1];
+  const double x2 = fabs(fxE) + fabs(fxW), avail = ft.hr[ly][lx + 1];
+  const double most = fma(fabs(fyN), fabs(r.rdyN), fma(fabs(fyS), fabs(r.rdyS), x2 * fabs(r.rdx)));
+  return most * dt * (1 + 1e-12) < avail || (avail >= 0 && x2 + fabs(fyN) + fabs(fyS) == 0);   // dry land too
+}
 __device__ __forceinline__ double split_theta(const StageArgs& a, const CellFaceTiles& ft, double dt, int gj, int ly,
                                               int lx) {
   const double fxE = ft.xm[ly][lx + 1], fxW = ft.xm[ly][lx], fyN = ft.ym[ly + 1][lx + 1], fyS = ft.ym[ly][lx + 1];
@@ -1001,9 +1018,11 @@ __device__ __forceinline__ void split_close_block(const StageArgs& a, Control* c
 // added to or taken from a +0 sum, and the bed terms are +0, so the sums
 // are +0 with or without them: DRY leaves them out and gives the same bits.
 // inner: the tile holds no ghost cell, so every cell has its four faces.
+// limited: theta may differ from 1 in a cell of the tile's ring, and sm.th holds it.
 template <int MODE, bool DRY>
 __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& s, const CellsSmem& sm, int t,
-                                           int lx, int ly, int gi, int gj, bool inner, double dt, double& locMax,
+                                           int lx, int ly, int gi, int gj, bool inner, bool limited,
+                                           const RowMetric& row, double dt, double& locMax,
                                            double& locFl, double& hout) {
   const int W = a.W, H = a.H;
   const double dry = a.minDepth, eps4 = a.eps4;
@@ -1022,26 +1041,34 @@ __device__ __forceinline__ void split_cell(const StageArgs& a, const SplitBufs& 
   const double hin = sm.st[0][t], huin = sm.st[1][t], hvin = sm.st[2][t];
   double U0h = 0, U0hu = 0, U0hv = 0;
   if (MODE == 2) { U0h = sm.st[3][t]; U0hu = sm.st[4][t]; U0hv = sm.st[5][t]; }
-  const double thC = DRY ? 1.0 : sm.th[ly + 1][lx + 1];
-  const double rdx = a.m.rdxRow[gj], dxr = a.m.dxRow[gj];
+  const double thC = DRY || !limited ? 1.0 : sm.th[ly + 1][lx + 1];
+  const double rdx = row.rdx, dxr = a.m.dxRow[gj];
   double ah = 0, ahu = 0, ahv = 0;
   if (!DRY) {
     const double wM = ft.xm[ly + 1][lx + 1], eM = ft.xm[ly + 1][lx + 2];
     const double sM = ft.ym[ly + 1][lx + 2], nM = ft.ym[ly + 2][lx + 2];
-    // each face's limiter is its upwind cell's
-    const double tW = wM >= 0 ? sm.th[ly + 1][lx] : thC, tE = eM >= 0 ? thC : sm.th[ly + 1][lx + 2];
-    const double tS = sM >= 0 ? sm.th[ly][lx + 1] : thC, tN = nM >= 0 ? thC : sm.th[ly + 2][lx + 1];
-    double iW = rdx, iE = rdx, iS = a.m.rdyRowS[gj], iN = a.m.rdyRowN[gj];
-    if (!(tW == 1 && tE == 1 && tS == 1 && tN == 1)) {
-      if (tW != 1) iW = tW / dxr;
-      if (tE != 1) iE = tE / dxr;
-      if (tS != 1) iS = tS / a.m.dyRowS[gj];
-      if (tN != 1) iN = tN / a.m.dyRowN[gj];
+    if (inner && !limited) {                      // most tiles: four faces, no limiter to look up
+      const double iS = row.rdyS, iN = row.rdyN;
+      ah += wM * rdx; ahu += ft.xt[2][ly][lx + 1] * rdx; ahv += ft.xt[0][ly][lx + 1] * rdx;
+      ah -= eM * rdx; ahu -= ft.xt[1][ly][lx + 2] * rdx; ahv -= ft.xt[0][ly][lx + 2] * rdx;
+      ah += sM * iS; ahv += ft.yt[2][ly][lx] * iS; ahu += ft.yt[0][ly][lx] * iS;
+      ah -= nM * iN; ahv -= ft.yt[1][ly + 1][lx] * iN; ahu -= ft.yt[0][ly + 1][lx] * iN;
+    } else {
+      // each face's limiter is its upwind cell's
+      const double tW = limited && wM >= 0 ? sm.th[ly + 1][lx] : thC, tE = !limited || eM >= 0 ? thC : sm.th[ly + 1][lx + 2];
+      const double tS = limited && sM >= 0 ? sm.th[ly][lx + 1] : thC, tN = !limited || nM >= 0 ? thC : sm.th[ly + 2][lx + 1];
+      double iW = rdx, iE = rdx, iS = row.rdyS, iN = row.rdyN;
+      if (!(tW == 1 && tE == 1 && tS == 1 && tN == 1)) {
+        if (tW != 1) iW = tW / dxr;
+        if (tE != 1) iE = tE / dxr;
+        if (tS != 1) iS = tS / a.m.dyRowS[gj];
+        if (tN != 1) iN = tN / a.m.dyRowN[gj];
+      }
+      if (hasW) { ah += wM * iW; ahu += ft.xt[2][ly][lx + 1] * iW; ahv += ft.xt[0][ly][lx + 1] * iW; }   // its right side
+      if (hasE) { ah -= eM * iE; ahu -= ft.xt[1][ly][lx + 2] * iE; ahv -= ft.xt[0][ly][lx + 2] * iE; }   // its left side
+      if (hasS) { ah += sM * iS; ahv += ft.yt[2][ly][lx] * iS; ahu += ft.yt[0][ly][lx] * iS; }           // its upper side
+      if (hasN) { ah -= nM * iN; ahv -= ft.yt[1][ly + 1][lx] * iN; ahu -= ft.yt[0][ly + 1][lx] * iN; }   // its lower side
     }
-    if (hasW) { ah += wM * iW; ahu += ft.xt[2][ly][lx + 1] * iW; ahv += ft.xt[0][ly][lx + 1] * iW; }   // its right side
-    if (hasE) { ah -= eM * iE; ahu -= ft.xt[1][ly][lx + 2] * iE; ahv -= ft.xt[0][ly][lx + 2] * iE; }   // its left side
-    if (hasS) { ah += sM * iS; ahv += ft.yt[2][ly][lx] * iS; ahu += ft.yt[0][ly][lx] * iS; }           // its upper side
-    if (hasN) { ah -= nM * iN; ahv -= ft.yt[1][ly + 1][lx] * iN; ahu -= ft.yt[0][ly + 1][lx] * iN; }   // its lower side
   }
   if (interior) {
     if (!DRY && bedOn) {
@@ -1177,7 +1204,7 @@ __device__ __forceinline__ bool split_cells_tile(const StageArgs& a, const Split
   const int i0 = tx * SPX, j0 = ty * SPY;
   const int t = threadIdx.x;
   constexpr bool EARLY = TMA && !SETTLE;          // no tile is left out, few are folded: copy before the flags are known
-  if (EARLY) stage_cells_tma(a, sm, i0, j0, *maps, bar);
+  if (EARLY) stage_cells_tma<true>(a, sm, i0, j0, *maps, bar);
   const double dt = ctl->dt;
   const int lx = t % SPX, ly = t / SPX;
   const int gi = i0 + lx, gj = j0 + ly;
@@ -1203,22 +1230,21 @@ __device__ __forceinline__ bool split_cells_tile(const StageArgs& a, const Split
       cp_async8(&sm.st[5][t], (a.u0[0] ? a.u0[2] : a.ohv) + k);
     }
   }
-  if (t < 9) {
-    const int r = t / 3, c = t - 3 * r, txn = tx - 1 + c, tyn = ty - 1 + r;
-    int f = 0;                                    // no flags: nothing is skipped
-    if (s.dry) {
-      f = 2;                                      // outside the grid: no faces there
-      if (txn >= 0 && txn < s.ntx && tyn >= 0 && tyn < s.nty) f = s.dry[tyn * s.ntx + txn];
+  // the flags by the first warp, which also settles what they say: every thread
+  // testing all nine took a twentieth of stage 1's instructions
+  if (t < 32) {
+    int f = 2;                                    // outside the grid: no faces there
+    if (t < 9) {
+      const int r = t / 3, c = t - 3 * r, txn = tx - 1 + c, tyn = ty - 1 + r;
+      if (!s.dry) f = 0;                          // no flags: nothing is skipped
+      else if (txn >= 0 && txn < s.ntx && tyn >= 0 && tyn < s.nty) f = s.dry[tyn * s.ntx + txn];
+      sm.dry[r][c] = f;
     }
-    sm.dry[r][c] = f;
+    const int allSet = __all_sync(0xffffffffu, f != 0), anySet = __any_sync(0xffffffffu, f == 1);
+    if (t == 0) sm.flags = (allSet ? 1 : 0) | (anySet ? 2 : 0);
   }
   __syncthreads();
-  bool allDry = true, anyDry = false;
-  for (int q = 0; q < 9; q++) {
-    const int f = sm.dry[q / 3][q % 3];
-    allDry = allDry && f != 0;
-    anyDry = anyDry || f == 1;
-  }
+  const bool allDry = sm.flags & 1, anyDry = sm.flags & 2;
   const bool fold = allDry && a.dryfold;          // uniform across the CTA
   if (EARLY && fold && !tile_wait(bar, parity, ctl)) return false;   // nothing of the copies is used, but they must have landed
   // A folded tile settles without its state.  Its input has h = +-0 on the
@@ -1263,9 +1289,27 @@ __device__ __forceinline__ bool split_cells_tile(const StageArgs& a, const Split
       cp_async8(&sm.st[5][t], (a.u0[0] ? a.u0[2] : a.ohv) + k);
     }
   }
+  // Whether a cell of the tile or of those around it may be limited: each thread
+  // tests its own, the last three warps one around it besides.  Only then is theta
+  // worked out, for all of them.  The rows' metric is fetched while the copies are
+  // in flight.  (Theta of all ring cells in every tile, two passes of a loop before a
+  // barrier, made stage 1 of an all-wet 2048 x 2048 grid 132 us and stage 2 173, and
+  // so 116 and 164; without any of it they take 107 and 148.)
+  bool lim = false;
+  RowMetric row = {};
+  const bool own = inner || (gj >= 1 && gj < H - 1 && gi >= 1 && gi < W - 1);
+  if (own) row = row_metric(a.m, gj);
   if (!fold) {
+    // below, above, west, east: whole warps, then parts of one
+    const int e = t - (SP_THREADS - 3 * SPX), eq = e < 2 * SPX ? e % SPX : e % SPY;
+    const int ey = e < SPX ? 0 : (e < 2 * SPX ? SPY + 1 : 1 + eq);
+    const int ex = e < 2 * SPX ? 1 + eq : (e < 2 * SPX + SPY ? 0 : SPX + 1);
+    const int ej = j0 - 1 + ey, ei = i0 - 1 + ex;
+    const bool edge = e >= 0 && e < 2 * (SPX + SPY) && (inner || (ej >= 1 && ej < H - 1 && ei >= 1 && ei < W - 1));
+    RowMetric erow = {};
+    if (edge) erow = row_metric(a.m, ej);
     if (TMA) {
-      if (!EARLY) stage_cells_tma(a, sm, i0, j0, *maps, bar);
+      if (!EARLY) stage_cells_tma<false>(a, sm, i0, j0, *maps, bar);
       if (a.W & 1) stage_depths(a, sm, i0, j0);     // no tensor map of the state
       cp_async_wait_all();
       if (!tile_wait(bar, parity, ctl)) return false;          // uniform: give up on the tile
@@ -1275,6 +1319,11 @@ __device__ __forceinline__ bool split_cells_tile(const StageArgs& a, const Split
       cp_async_wait_all();
       __syncthreads();
     }
+    lim = (own && !free_theta(sm.ft, row, dt, ly + 1, lx + 1)) || (edge && !free_theta(sm.ft, erow, dt, ey, ex));
+  }
+  cp_async_wait_all();
+  const bool limited = __syncthreads_or(lim && dt > 0);
+  if (limited) {
     // the ring's second pass on the last threads, as the velocities'
     constexpr int TREM = (SPX + 2) * (SPY + 2) - SP_THREADS;
     static_assert(TREM > 0 && TREM <= SP_THREADS, "one or two ring cells per thread");
@@ -1284,16 +1333,15 @@ __device__ __forceinline__ bool split_cells_tile(const StageArgs& a, const Split
       const int q = pass == 0 ? t : t + TREM;
       const int ry = q / (SPX + 2), rx = q - ry * (SPX + 2), rj = j0 - 1 + ry, ri = i0 - 1 + rx;
       const bool on = inner || (rj >= 1 && rj < H - 1 && ri >= 1 && ri < W - 1);
-      sm.th[ry][rx] = on && dt > 0 ? split_theta(a, sm.ft, dt, rj, ry, rx) : 1.0;
+      sm.th[ry][rx] = on ? split_theta(a, sm.ft, dt, rj, ry, rx) : 1.0;
     }
+    __syncthreads();
   }
-  cp_async_wait_all();
-  __syncthreads();
 
   double locMax = 0, locFl = 0, hout = 0;
   if (gi < W && gj < H) {
-    if (fold) split_cell<MODE, true>(a, s, sm, t, lx, ly, gi, gj, inner, dt, locMax, locFl, hout);
-    else split_cell<MODE, false>(a, s, sm, t, lx, ly, gi, gj, inner, dt, locMax, locFl, hout);
+    if (fold) split_cell<MODE, true>(a, s, sm, t, lx, ly, gi, gj, inner, false, row, dt, locMax, locFl, hout);
+    else split_cell<MODE, false>(a, s, sm, t, lx, ly, gi, gj, inner, limited, row, dt, locMax, locFl, hout);
   }
   // Per-tile partials: a warp's maximum and sum, then the tile's by one
   // thread.  The maximum is that of non-negative doubles, so it is the
@@ -1462,9 +1510,12 @@ __global__ void __launch_bounds__(32 * CLOSE_BLOCKS) k_split_close_step(StageArg
 }
 
 // The cell kernel with its face and depth inputs staged by tensor-map copies
-// (maps over this simulation's own buffers only, no multicast).
-template <int MODE, bool SETTLE = false>
-__global__ void __launch_bounds__(SP_THREADS, SWE_SPLIT_CELLS_MIN_BLOCKS)
+// (maps over this simulation's own buffers only, no multicast).  On an all-wet
+// 2048 x 2048 grid, where stage 1 moves 540 MB, 3, 4 and 5 CTAs per SM (the last
+// with spills) took 148, 132 and 134 us; grids of at most 3 take the kernel that
+// spills nothing (384 x 256, 100 steps: 3.50 -> 3.32 ms).
+template <int MODE, bool SETTLE = false, int MIN_BLOCKS = SWE_SPLIT_CELLS_MIN_BLOCKS>
+__global__ void __launch_bounds__(SP_THREADS, MIN_BLOCKS)
 k_split_cells_tma(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant__ CellMaps maps) {
   __shared__ CellsSmem sm;
   __shared__ alignas(8) unsigned long long bar;
@@ -1474,6 +1525,7 @@ k_split_cells_tma(StageArgs a, SplitBufs s, Control* ctl, const __grid_constant_
   }
   pdl_enter();
   if (ctl->stop) return;
+  __syncthreads();                                 // bar is ready for the copies' other threads
   split_cells_tile<MODE, SETTLE, true>(a, s, ctl, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x,
                                        gridDim.x * gridDim.y, sm, false, &maps, &bar);
 }
@@ -1499,7 +1551,7 @@ k_split_cells_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_cons
     if (!split_cells_tile<MODE, true, true>(a, s, ctl, tile % s.ntx, tile / s.ntx, tile, ntiles, sm, false, &maps, &bar))
       return;
     if (!LOOP) return;
-    next_tile();
+    __syncthreads();                              // the next tile reuses the shared memory
     if (threadIdx.x == 0) {
       walk.at = walk.at + gridDim.x;
       mbar_inval(&bar);                           // only tiles that are computed complete its phase
