@@ -292,24 +292,16 @@ __device__ __forceinline__ double limiter_mc_tame(double a, double b) {
 // reciprocal is not covered; the caller then uses face_flux.
 struct FaceSums { double M, T, NpL, NpR; };     // N + pL, N + pR
 __device__ __forceinline__ double pos(double x) { return x > 0 ? x : 0; }
-__device__ __forceinline__ FaceSums face_flux_tame(
-    double bL_c, double hL_c, double nL_c, double tL_c, double sEL, double sBL, double sNL, double sTL,
-    double bR_c, double hR_c, double nR_c, double tR_c, double sER, double sBR, double sNR, double sTR, double dry,
-    bool& redo) {
-  const double etaL = fma(0.5, sEL, bL_c + hL_c), etaR = fma(-0.5, sER, bR_c + hR_c);
-  const double bL = fma(0.5, sBL, bL_c), bR = fma(-0.5, sBR, bR_c);
-  const double hLf = pos(etaL - bL), hRf = pos(etaR - bR);
-  const double nL = fma(0.5, sNL, nL_c), nR = fma(-0.5, sNR, nR_c);
-  const double tL = fma(0.5, sTL, tL_c), tR = fma(-0.5, sTR, tR_c);
-  const double bStar = bL > bR ? bL : bR;
-  const double hL = pos(etaL - bStar), hR = pos(etaR - bStar);
+// The solve of two reconstructed states of which one is wet.  BOTH: both are, in
+// every lane of the warp, and the selects of a dry side go (the face kernel of an
+// all-wet 2048 x 2048 grid 239 -> 231 us).
+template <bool BOTH>
+__device__ __forceinline__ FaceSums solve_tame(double hL, double hR, double nL, double nR, double tL, double tR,
+                                               double pL, double pR, bool wetL, bool wetR, bool& redo) {
+  if (BOTH) wetL = wetR = true;
   const double huL = hL * nL, hvL = hL * tL, huR = hR * nR, hvR = hR * tR;
   const double DL = hL * hL, DR = hR * hR;
   FaceSums f;
-  const double pL = 0.5 * SWE_G * (hLf * hLf - DL), pR = 0.5 * SWE_G * (hRf * hRf - DR);
-  const bool wetL = hL > dry, wetR = hR > dry;
-  redo = false;
-  if (!wetL && !wetR) { f.M = 0; f.T = 0; f.NpL = 0 + pL; f.NpR = 0 + pR; return f; }
   // a dry side's quotients are not used (its depth may be 0)
   const double yL = rcp_tame(hL), yR = rcp_tame(hR);
   const double uL = wetL ? div_product(huL, hL, nL, yL) : 0, vL = wetL ? div_product(hvL, hL, tL, yL) : 0;
@@ -341,6 +333,25 @@ __device__ __forceinline__ FaceSums face_flux_tame(
   f.NpL = N + pL;
   f.NpR = N + pR;
   return f;
+}
+__device__ __forceinline__ FaceSums face_flux_tame(
+    double bL_c, double hL_c, double nL_c, double tL_c, double sEL, double sBL, double sNL, double sTL,
+    double bR_c, double hR_c, double nR_c, double tR_c, double sER, double sBR, double sNR, double sTR, double dry,
+    bool& redo) {
+  const double etaL = fma(0.5, sEL, bL_c + hL_c), etaR = fma(-0.5, sER, bR_c + hR_c);
+  const double bL = fma(0.5, sBL, bL_c), bR = fma(-0.5, sBR, bR_c);
+  const double hLf = pos(etaL - bL), hRf = pos(etaR - bR);
+  const double nL = fma(0.5, sNL, nL_c), nR = fma(-0.5, sNR, nR_c);
+  const double tL = fma(0.5, sTL, tL_c), tR = fma(-0.5, sTR, tR_c);
+  const double bStar = bL > bR ? bL : bR;
+  const double hL = pos(etaL - bStar), hR = pos(etaR - bStar);
+  const double pL = 0.5 * SWE_G * (hLf * hLf - hL * hL), pR = 0.5 * SWE_G * (hRf * hRf - hR * hR);
+  const bool wetL = hL > dry, wetR = hR > dry;
+  redo = false;
+  if (__all_sync(__activemask(), wetL && wetR))
+    return solve_tame<true>(hL, hR, nL, nR, tL, tR, pL, pR, true, true, redo);
+  if (!wetL && !wetR) return {0, 0, 0 + pL, 0 + pR};
+  return solve_tame<false>(hL, hR, nL, nR, tL, tR, pL, pR, wetL, wetR, redo);
 }
 
 }  // namespace swe
