@@ -104,7 +104,7 @@ __device__ __forceinline__ FaceAdj xface_adj(const Geo& g, const Inter& it, cons
   if (!xface_on(g, i, j)) return f;
   const int kL = k, kR = k + 1;
   const double M = it.fx[F_M][k], T = it.fx[F_T][k], NpL = it.fx[F_NPL][k], NpR = it.fx[F_NPR][k];
-  const double th = M >= 0 ? theta[kL] : theta[kR];
+  const double tL = theta[kL], tR = theta[kR], th = M >= 0 ? tL : tR;
   const double inv = th / g.dxRow[j];
   f.lM = inv * (a.lR[0][kR] - a.lR[0][kL]);
   f.lN = inv * (a.lR[1][kR] - a.lR[1][kL]);
@@ -123,7 +123,7 @@ __device__ __forceinline__ FaceAdj yface_adj(const Geo& g, const Inter& it, cons
   if (!yface_on(g, i, j)) return f;
   const int kL = k, kR = k + g.W;
   const double M = it.fy[F_M][k], T = it.fy[F_T][k], NpL = it.fy[F_NPL][k], NpR = it.fy[F_NPR][k];
-  const double th = M >= 0 ? theta[kL] : theta[kR];
+  const double tL = theta[kL], tR = theta[kR], th = M >= 0 ? tL : tR;
   const double invL = th / g.dyRowN[j], invR = th / g.dyRowS[j + 1];
   // rh[kL] -= M invL; rhv[kL] -= (N + pL) invL; rhu[kL] -= T invL; rh[kR] += M invR; ...
   f.lM = invR * a.lR[0][kR] - invL * a.lR[0][kL];
@@ -185,11 +185,12 @@ __device__ __forceinline__ double lout_of(const Geo& g, const Inter& it, const d
 // sE, sB, s(normal), s(transverse).
 constexpr int AT_X = 32;           // tile width (one warp)
 constexpr int AT_Y = 8;            // rows per face / cell tile (256 threads)
-// The face kernels are latency bound: capped at 64 registers (32 warps per
-// SM; a few hundred bytes of spills) they measured faster than at 80
-// (24 warps) or at their natural 112 (16 warps).
+// The face kernel waits on memory.  With a face's 32 values loaded at once,
+// before the branches on its flux, 24 warps per SM (80 registers) are enough: a
+// gradient of 60 steps at 512 x 384 takes 14.9 ms, with 32 warps (64 registers,
+// 500 bytes of spills) 15.8, and 15.3 with 32 and the loads where they are used.
 #ifndef SWE_ADJ_FACE_WARPS
-#define SWE_ADJ_FACE_WARPS 32
+#define SWE_ADJ_FACE_WARPS 24
 #endif
 // The cell kernel waits on memory, but it keeps its natural 80 registers
 // (three blocks, 24 warps per SM): capped at 64 (four blocks) or 48 (five)
@@ -213,11 +214,12 @@ __device__ __forceinline__ void adj_xfaces(const Geo& g, const double* b, const 
   FaceIn gx = {};
   if (valid && xface_on(g, i, j)) {
     const FaceAdj f = xface_adj(g, it, theta, a, k, i, j);
+    const FaceIn in = xface_in(g, b, h, it, k);           // in flight while the adjoints are formed
     double lM = f.lM;
     const double M = it.fx[F_M][k];
     if (M > 0) lM += swe::qdiv(lout_of(g, it, theta, h, dt, a, k), g.dxRow[j]);
     if (M < 0) lM -= swe::qdiv(lout_of(g, it, theta, h, dt, a, k + 1), g.dxRow[j]);
-    gx = swe::adj::face_rev(xface_in(g, b, h, it, k), g.minDepth, lM, f.lN, f.lT, f.lpL, f.lpR);
+    gx = swe::adj::face_rev(in, g.minDepth, lM, f.lN, f.lT, f.lpL, f.lpR);
   }
   const double* p = &gx.bL;
 #pragma unroll
@@ -241,11 +243,12 @@ __device__ __forceinline__ void adj_yfaces(const Geo& g, const double* b, const 
   FaceIn gy = {};
   if (valid && yface_on(g, i, j)) {
     const FaceAdj f = yface_adj(g, it, theta, a, k, i, j);
+    const FaceIn in = yface_in(g, b, h, it, k);           // in flight while the adjoints are formed
     double lM = f.lM;
     const double M = it.fy[F_M][k];
     if (M > 0) lM += swe::qdiv(lout_of(g, it, theta, h, dt, a, k), g.dyRowN[j]);
     if (M < 0) lM -= swe::qdiv(lout_of(g, it, theta, h, dt, a, k + g.W), g.dyRowS[j + 1]);
-    gy = swe::adj::face_rev(yface_in(g, b, h, it, k), g.minDepth, lM, f.lN, f.lT, f.lpL, f.lpR);
+    gy = swe::adj::face_rev(in, g.minDepth, lM, f.lN, f.lT, f.lpL, f.lpR);
   }
   const double* p = &gy.bL;
 #pragma unroll
@@ -331,10 +334,13 @@ __device__ __forceinline__ void limiter_adj(const Geo& g, const double* b, const
   for (int q = 0; q < 4; q++) { ga[q] = 0; gc[q] = 0; }
   if (!(g.order >= 2 && i >= 1 && i < g.W - 1 && j >= 1 && j < g.H - 1)) return;
   const int kp = d == 0 ? k + 1 : k + g.W, km = d == 0 ? k - 1 : k - g.W;
-  if (h[k] <= g.minDepth || h[kp] <= g.minDepth || h[km] <= g.minDepth) return;
-  const double eC = b[k] + h[k], eP = b[kp] + h[kp], eM = b[km] + h[km];
-  const double X0[4] = {eC - eM, b[k] - b[km], it.U[k] - it.U[km], it.V[k] - it.V[km]};
-  const double X1[4] = {eP - eC, b[kp] - b[k], it.U[kp] - it.U[k], it.V[kp] - it.V[k]};
+  // all of them in flight at once, before the depths are known
+  const double hC = h[k], hP = h[kp], hM = h[km], bC = b[k], bP = b[kp], bM = b[km];
+  const double uC = it.U[k], uP = it.U[kp], uM = it.U[km], vC = it.V[k], vP = it.V[kp], vM = it.V[km];
+  if (hC <= g.minDepth || hP <= g.minDepth || hM <= g.minDepth) return;
+  const double eC = bC + hC, eP = bP + hP, eM = bM + hM;
+  const double X0[4] = {eC - eM, bC - bM, uC - uM, vC - vM};
+  const double X1[4] = {eP - eC, bP - bC, uP - uC, vP - vC};
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     double da, dc;
@@ -373,6 +379,7 @@ k_adj_cells_tiled(Geo g, const double* b, const double* h, const double* hu, con
   const bool valid = i < g.W && j < g.H;
   const int k = j * g.W + i;
   double db = 0, dh = 0, dU = 0, dV = 0, dhu = 0, dhv = 0;
+  double hk = 0, huk = 0, hvk = 0, ab = 0, ah = 0, ahu = 0, ahv = 0;
   if (valid) {
     double ls[2][4];
     double xb, xh, xU, xV, yb, yh, yU, yV;
@@ -400,6 +407,9 @@ k_adj_cells_tiled(Geo g, const double* b, const double* h, const double* hu, con
 #pragma unroll
       for (int q = 0; q < 4; q++) { sga[d][q][ty + 1][tx + 1] = ga[q]; sgc[d][q][ty + 1][tx + 1] = gc[q]; }
     }
+    // for the end, in flight while the ring and the barrier are waited for
+    hk = h[k]; huk = hu[k]; hvk = hv[k];
+    ab = lb[k]; ah = lh[k]; ahu = lhu[k]; ahv = lhv[k];
   }
   // The ring: what a neighbour outside the tile sends in.  Left column: its
   // x-slope gc; right column: its x-slope ga; bottom row: its y-slope gc;
@@ -442,12 +452,12 @@ k_adj_cells_tiled(Geo g, const double* b, const double* h, const double* hu, con
   }
   const double lU = lX[2] + dU, lV = lX[3] + dV;
   double dqU, dhU, dqV, dhV;
-  swe::adj::vel_grad(hu[k], h[k], g.eps4, dqU, dhU);
-  swe::adj::vel_grad(hv[k], h[k], g.eps4, dqV, dhV);
-  lb[k] += lX[0] + lX[1] + db;
-  lh[k] += lX[0] + dh + lU * dhU + lV * dhV;
-  lhu[k] = (lhu[k] + dhu) + lU * dqU;
-  lhv[k] = (lhv[k] + dhv) + lV * dqV;
+  swe::adj::vel_grad(huk, hk, g.eps4, dqU, dhU);
+  swe::adj::vel_grad(hvk, hk, g.eps4, dqV, dhV);
+  lb[k] = ab + (lX[0] + lX[1] + db);
+  lh[k] = ah + (lX[0] + dh + lU * dhU + lV * dhV);
+  lhu[k] = (ahu + dhu) + lU * dqU;
+  lhv[k] = (ahv + dhv) + lV * dqV;
 }
 
 // ---- the rest of the step backwards ----------------------------------------
@@ -542,7 +552,7 @@ __global__ void k_adj_bc(int nsrc, const int* map, const double* b, const double
 // lB = 0.5 lA, lR = 0.5 dt lA and leaves lA <- 0.5 lA (= lW1).
 __device__ __forceinline__ void friction_rev(double minDepth, double eps4, double n, double dt, double hk,
                                              double qu, double qv, double& a0, double& a1, double& a2,
-                                             double* ln, int k) {
+                                             double* ln, double lnk, int k) {
   if (!(n != 0 && n == n)) return;                  // identity (scalar n == 0 skips entirely)
   if (hk <= minDepth) { a1 = 0; a2 = 0; return; }
   const double den = swe::vel_den(hk, eps4);
@@ -557,7 +567,7 @@ __device__ __forceinline__ void friction_rev(double minDepth, double eps4, doubl
   double gh = 0, gq = swe::qdiv(ghu, denom), gr = swe::qdiv(ghv, denom);
   const double lspeed = lden * K / P;
   const double lP = -lden * K * speed / (P * P);
-  if (ln) ln[k] += lden * dt * SWE_G * 2 * n * speed / P;
+  if (ln) ln[k] = lnk + lden * dt * SWE_G * 2 * n * speed / P;
   gh += lP * (4.0 / 3.0) * P / hk;
   const double lu = lspeed * u / speed, lv = lspeed * v / speed;
   double dqU, dhU, dqV, dhV;
@@ -577,8 +587,8 @@ __global__ void k_adj_tail2(int W, int H, double minDepth, double eps4, double m
     const int i = k % W, j = k / W;
     double a0 = lA0[k], a1 = lA1[k], a2 = lA2[k];
     if (i >= 2 && i < W - 2 && j >= 2 && j < H - 2) {
-      friction_rev(minDepth, eps4, nfield ? nfield[k] : manning, dt, fh[k], fhu[k], fhv[k], a0, a1, a2, ln, k);
-      const double hp = hA[k];
+      const double hp = hA[k], lnk = ln ? ln[k] : 0;         // in flight with the rest
+      friction_rev(minDepth, eps4, nfield ? nfield[k] : manning, dt, fh[k], fhu[k], fhv[k], a0, a1, a2, ln, lnk, k);
       const double hc = hp < 0 ? 0 : hp;
       if (hp < 0) a0 = 0;
       if (hc <= minDepth) { a1 = 0; a2 = 0; }
