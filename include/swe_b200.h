@@ -228,8 +228,9 @@ int swe_synchronize(swe_sim* s);
 /* The handle's CUDA stream (a cudaStream_t), so a caller can record CUDA
  * events on the stream the kernels run on. */
 int swe_get_stream(swe_sim* s, void** stream);
-/* step(dt) with CUDA events between its five launches (prepare, ghost fill,
- * stage 1, ghost fill, stage 2); ms[5] receives each launch's duration. */
+/* step(dt) with CUDA events between its five phases (prepare, ghost fill,
+ * stage 1, ghost fill, stage 2), each launched on its own; ms[5] receives each
+ * phase's duration. */
 int swe_step_timed(swe_sim* s, double dt, double* ms);
 /* Launch shape of the stage kernel: grid x, grid y, threads, output
  * columns per CTA, output rows per CTA. */
@@ -274,7 +275,8 @@ int swe_batch_autotune(swe_batch* s, int trial_steps, int* best4, double* best_m
 /* `steps` ensemble steps: every basin takes `steps` steps of its own maxDt(). */
 int swe_batch_run(swe_batch* s, int steps);
 /* Waits for the ensemble's stream; SWE_ETIMEOUT (once, then cleared) when a
- * work-queue wait of the steps run since the last call ran past its limit. */
+ * work-queue wait or a tile copy of the steps run since the last call ran past
+ * its limit. */
 int swe_batch_synchronize(swe_batch* s);
 /* The launch form of an ensemble step with the tiled pair (rows 0).
  * 0: a launch per phase (prepare, ghost fill, faces, cells, ghost fill,

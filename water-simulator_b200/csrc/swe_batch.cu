@@ -2,15 +2,18 @@
 //
 // Each basin is a complete ShallowWater (its own grid, bed, metric, Manning
 // n, boundaries and Flather tide) with its own dt = maxDt() every step.  One
-// ensemble step is five launches whatever the number of basins:
+// ensemble step is a fixed number of launches whatever the number of basins;
+// with the fused stage kernels five:
 //   k_batch_prepare     dt and Flather values of every basin (one thread each)
 //   k_batch_bc(A)       ghost rings of every basin (grid y = basin)
 //   k_batch_stage<1>    every tile of every basin, from one tile list
 //   k_batch_bc(B)
 //   k_batch_stage<2>    ... the last tile of each basin closes that basin's step
-// and a run of steps is captured as a CUDA graph.  The stage kernel is the
-// same tile function as the single-grid kernel, so each basin's result is
-// bit-identical to advancing it alone.  The tile list's row height, the
+// with the tiled pair k_batch_split_faces and k_batch_split_cells for each stage
+// and k_batch_close (a block per basin) after the second.  A run of steps is
+// captured as a CUDA graph.  The stage kernels run the same tile functions as
+// the single-grid kernels, so each basin's result is bit-identical to advancing
+// it alone.  The tile list's row height, the
 // number of CTAs (one per tile, or a persistent grid looping over the list)
 // and the order of the tiles form the schedule, which swe_batch_autotune
 // chooses by timing candidates on the ensemble itself.

@@ -7,7 +7,8 @@
 //   B = (h, hu, hv)   the stage-1 state U1
 //   metric rows       13 arrays of H doubles (src/geometry.mjs:301-309)
 //
-// One step (src/swe.mjs:754-814) is five launches:
+// One step (src/swe.mjs:754-814) with the fused stage kernels is five launches
+// (swe_split.cuh has the tiled pair that is the default):
 //   k_prepare      dt, t, Flather values for this step (one warp)
 //   k_apply_bc(A)  ghost rings of A (src/swe.mjs:289-303)
 //   k_stage<1>     B = A + dt R(A); dryClean

@@ -6,19 +6,20 @@
 //
 //   k_split_faces   a 32 x 8 tile of cells per CTA: the state of the tile
 //                   and a one-cell halo into shared memory with its
-//                   velocities, the MUSCL slopes of the tile (plus the east
+//                   velocities (on smaller grids it fills the ghosts there
+//                   and prepares the step), the MUSCL slopes (plus the east
 //                   column and north row the faces need), then per cell its
 //                   east x face and north y face (HLLC, src/swe.mjs:415-475)
 //                   and its bed / geometric source terms (src/swe.mjs:570-598),
 //                   written to face and term arrays.  This holds the FP64
 //                   work (two HLLC solves per cell) at 256 threads per CTA.
 //   k_split_cells   per cell: the positivity limiter of the cell and its
-//                   neighbours from the faces (src/swe.mjs:511-529), the
-//                   four faces gathered west, east, south, north
+//                   neighbours from the faces, in tiles where it is not 1
+//                   everywhere (src/swe.mjs:511-529), the four faces gathered west, east, south, north
 //                   (src/swe.mjs:530-555), the source terms, Coriolis, and
 //                   the stage update with its epilogue (dryClean, friction,
-//                   sponge, CFL rate; src/swe.mjs:659-813).  The last block
-//                   to finish closes the step as the fused kernel does.
+//                   sponge, CFL rate; src/swe.mjs:659-813), one partial per
+//                   tile.  After stage 2 a kernel of its own closes the step.
 //
 // Both are written as tile functions (split_faces_tile, split_cells_tile)
 // that a single-grid kernel calls once and the batched ensemble calls for
