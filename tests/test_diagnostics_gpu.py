@@ -96,3 +96,24 @@ def test_a_diagnostic_between_steps_leaves_the_time_step_alone(swe):
     assert np.array_equal(sims[0].field("h"), sims[1].field("h")) and sims[0].t == sims[1].t
     for sim in sims:
         sim.close()
+
+
+@pytest.mark.parametrize("minDepth", [0.0, 1e-3, 1e15, 1e18, 1e19, 1e77, np.float64(1e80), np.inf])
+def test_energy_for_any_min_depth(swe, minDepth):
+    """The velocities' desingularisation is minDepth^4, infinite from about
+    1e77 on: the velocities are 0 then and the energy is the potential one.
+    The same bits as the velocities of the operators at every minDepth."""
+    rng = np.random.default_rng(5)
+    nx, ny = 130, 9
+    b, h = rng.uniform(-1, 0.5, (ny + 4, nx + 4)), rng.uniform(0.5, 3.0, (ny + 4, nx + 4))
+    with np.errstate(over="ignore"):
+        sim = swe.ShallowWater(nx=nx, ny=ny, dx=2.0, bed=b, eta0=0.0, minDepth=minDepth)
+    hu, hv = h * rng.normal(0, 1, h.shape), h * rng.normal(0, 1, h.shape)
+    sim.h, sim.hu, sim.hv = h, hu, hv
+    i = (slice(2, -2), slice(2, -2))
+    B, H = b[i], h[i]
+    u, v = (sim.vel(q[i].reshape(-1), H.reshape(-1)).reshape(ny, nx) for q in (hu, hv))
+    term = 0.5 * H * (u * u + v * v) + 0.5 * swe.G * H * (H + 2 * B)
+    assert np.all(np.isfinite(term))
+    assert sim.energy() == chain([chain(r) for r in term]) * 2.0 * 2.0
+    sim.close()

@@ -747,9 +747,12 @@ __device__ __forceinline__ void for_cells(int j0, int j1, int i0, int i1, F f) {
       for (int i = s + threadIdx.x; i < min(s + RED_SEG, i1); i += BX) f(j, i);
 }
 
-// Both velocities of a cell, branch-free where it is tame.
+// Both velocities of a cell, branch-free where it is tame.  The diagnostics take
+// every minDepth, so eps4 = max(minDepth, 1e-12)^4 may be infinite here, whose
+// root the operators form and the iteration does not; below 2^240 no quotient of
+// a tame cell's momentum leaves the normal range.
 __device__ __forceinline__ void cell_vel(const StageArgs& a, double h, double hu, double hv, double& u, double& v) {
-  if (tame_cell(0, h, hu, hv) && vel_tame(hu, hv, h, a.eps4, u, v)) return;
+  if (a.eps4 < 0x1p240 && tame_cell(0, h, hu, hv) && vel_tame(hu, hv, h, a.eps4, u, v)) return;
   const double den = vel_den(h, a.eps4);
   u = qdiv(vel_num(hu, h), den); v = qdiv(vel_num(hv, h), den);
 }
