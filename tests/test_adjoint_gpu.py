@@ -154,3 +154,107 @@ def test_adjoint_boundary_refusals(swe):
     with pytest.raises(KeyError):
         c.set_boundary("up", "reflect")
     c.close()
+
+
+TIDE_WEST = {"west": ("tide", 2.0, [0.3], [2 * 3.141592653589793 / 250], [40.0], 0.05)}
+
+
+@pytest.mark.parametrize("bad", [0.0, -0.5, np.inf, np.nan])
+@pytest.mark.parametrize("bcs", [None, TIDE_WEST], ids=["walls", "tide"])
+@pytest.mark.parametrize("at", [0, 5, 11])
+def test_a_refused_step_changes_nothing(swe, at, bcs, bad):
+    """A dt that step() refuses leaves the state as it was: the later steps are
+    those of the run without it, and the gradient is that run's, with the
+    misfit of the repeated state counted twice, for any checkpoint interval."""
+    from water_simulator_b200 import workloads
+    c = workloads.adjoint_case(nx=40, ny=30, dx=10.0, n_gauges=6, seed=33, hump=0.4)
+    n = 11
+    rng = np.random.default_rng(8)
+    obs = rng.normal(2.0, 0.05, (n, 6))
+
+    def handle(steps, every):
+        return swe.MisfitAdjoint(40, 30, 10.0, c["b"], c["eta0"], manning_field=c["n"], gauges=c["gauges"],
+                                 steps=steps, checkpoint_every=every, boundaries=bcs)
+
+    plain = handle(n, n)
+    plain.set_observations(obs)
+    _, eta = plain.forward()
+    dts = plain.dt_sequence()
+    if at > 0:                                     # twice the residual of the state that repeats
+        twice = obs.copy()
+        twice[at - 1] = eta[at - 1] - 2 * (eta[at - 1] - obs[at - 1])
+        plain.set_observations(twice)
+    plain.forward()
+    want = plain.backward()
+    plain.close()
+    got = []
+    for every in (1, 5, n + 1):
+        adj = handle(n + 1, every)
+        adj.dt_sequence(fixed=np.insert(dts, at, bad))
+        _, e0 = adj.forward()
+        assert np.array_equal(np.delete(e0, at, axis=0), eta)
+        assert at == 0 or np.array_equal(e0[at], eta[at - 1])
+        adj.set_observations(np.insert(obs, at, obs[at - 1] if at > 0 else e0[0], axis=0))
+        adj.forward()
+        got.append(adj.backward())
+        adj.close()
+    for g in got[1:]:
+        assert np.array_equal(g[0], got[0][0]) and np.array_equal(g[1], got[0][1])
+    for g, w in zip(got[0], want):                 # 2r + 2r against 4r, at most 12 steps of rounding apart
+        assert np.max(np.abs(g - w)) <= 1e-11 * np.max(np.abs(w))
+
+
+@pytest.mark.parametrize("refused", [None, 0, 6])
+@pytest.mark.parametrize("bcs", [None, {"west": ("flather", 2.05, 0.0), "east": "outflow"}], ids=["walls", "flather"])
+def test_gauges_in_ghost_cells(swe, bcs, refused):
+    """Gauges in ghost cells (a corner among them) read what the step left there,
+    after a refused step the filled ghosts: the gradient against central
+    differences with the dt sequence held, the same for any checkpoint interval."""
+    from water_simulator_b200 import workloads
+    nx, ny, steps = 24, 18, 12
+    W = nx + 4
+    c = workloads.adjoint_case(nx=nx, ny=ny, dx=10.0, n_gauges=2, seed=35, hump=0.4)
+    g = np.concatenate([c["gauges"], [9 * W + 1, 9 * W + 2, 1 * W + 1, (ny + 2) * W + 7]]).astype(np.int32)
+    rng = np.random.default_rng(9)
+    obs = rng.normal(2.0, 0.05, (steps, len(g)))
+
+    def handle(b, n, every, dts=None):
+        adj = swe.MisfitAdjoint(nx, ny, 10.0, b, c["eta0"], manning_field=n, gauges=g, steps=steps,
+                                checkpoint_every=every, boundaries=bcs)
+        adj.set_observations(obs)
+        if dts is not None:
+            adj.dt_sequence(fixed=dts)
+        return adj
+
+    first = handle(c["b"], c["n"], steps)
+    first.forward()
+    dts = first.dt_sequence()
+    first.close()
+    if refused is not None:
+        dts[refused] = 0.0
+    got = []
+    for every in (1, 5, steps):
+        adj = handle(c["b"], c["n"], every, dts)
+        _, eta = adj.forward()
+        if refused is not None and bcs is None:    # the wall's ghost is its neighbour's mirror
+            assert np.all(eta[refused, 2] == eta[refused, 3])
+        got.append(adj.backward())
+        adj.close()
+    for q in got[1:]:
+        assert np.array_equal(q[0], got[0][0]) and np.array_equal(q[1], got[0][1])
+
+    def J_at(b, n):
+        f = handle(b, n, steps, dts)
+        v, _ = f.forward()
+        f.close()
+        return v
+
+    for trial in range(4):
+        db = rng.normal(0, 1, c["b"].shape)
+        dn = rng.normal(0, 1e-3, c["n"].shape)
+        want = float(np.dot(got[0][0], db.reshape(-1)) + np.dot(got[0][1], dn.reshape(-1)))
+        errs = []
+        for eps in (1e-4, 1e-5, 1e-6, 1e-7):
+            fd = (J_at(c["b"] + eps * db, c["n"] + eps * dn) - J_at(c["b"] - eps * db, c["n"] - eps * dn)) / (2 * eps)
+            errs.append(abs(fd - want) / abs(want))
+        assert min(errs) <= 1e-5, (trial, errs)

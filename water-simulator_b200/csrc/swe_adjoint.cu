@@ -664,11 +664,18 @@ __global__ void k_adj_misfit(const double* b, const double* h, const int* gcell,
 }
 // The forward's record of a step, before its close: t at its start and the
 // Flather exterior state (rec, STEP_REC doubles), its dt (where dts is given)
-// and the misfit of the state it left.
+// and the misfit of the state it left.  A refused step leaves the state as it
+// was with its ghosts filled, which the face kernel that would have filled them
+// did not do; with `fill` (a gauge lies in a ghost cell) they are filled here.
 __global__ void k_record_step(const Control* ctl, double* rec, double* dts, const double* b, const double* h,
-                              const int* gk, const double* obs, int ng, double* J, double* eta_out) {
+                              const int* gk, const double* obs, int ng, double* J, double* eta_out, BCArgs bc,
+                              int fill) {
   pdl_enter();
   const int t = threadIdx.x;
+  if (fill && ctl->stop) {                        // uniform
+    swe::apply_bc_range(bc, ctl, t, blockDim.x);
+    __syncthreads();
+  }
   if (t < 4) { rec[1 + t] = ctl->fl_eta[t]; rec[5 + t] = ctl->fl_u[t]; }
   if (t == 4) rec[0] = ctl->t;
   if (t == 5 && dts) *dts = ctl->dt;
@@ -862,7 +869,8 @@ int fwd_step(swe_adjoint* s, int k) {
   if (rc) return rc;
   LAUNCH(k_record_step, dim3(1), dim3(MISFIT_THREADS), (const Control*)s->ctl, s->rec + (size_t)STEP_REC * k,
          s->fixed_dt ? (double*)nullptr : s->dts + k, (const double*)s->b, (const double*)s->A[0], (const int*)s->gk,
-         (const double*)(s->obs + (size_t)k * s->ng), s->ng, s->J, s->eta_series + (size_t)k * s->ng);
+         (const double*)(s->obs + (size_t)k * s->ng), s->ng, s->J, s->eta_series + (size_t)k * s->ng,
+         bc_args(s, s->A), s->ghost_gauges ? 1 : 0);
   const int n = (int)(s->sgrid.x * s->sgrid.y);
   if (n <= swe::CLOSE_TILES) LAUNCH(swe::k_split_close_step, dim3(1), dim3(32 * swe::CLOSE_BLOCKS), a2, s->ctl, n);
   else
@@ -941,21 +949,29 @@ swe::SplitBufs tape_bufs(const swe_adjoint* s, const Inter& it) {
 // Step k forward from its tape's W1 into `out` (the next step's W1, or X after
 // the segment's last) and record its tape: the tiled stage kernels write the
 // limiter, the depth before dryClean and friction's input as they go.  Nothing
-// closes the step: its dt and the Flather sides' t are recorded.
+// closes the step: its dt and the Flather sides' t are recorded.  A step that the
+// forward refused (a recorded dt that is not finite and positive) writes no tape:
+// its output is its input with the ghosts filled.
 int tape_step(swe_adjoint* s, double* const* out, int k, const Tape& T) {
   bool tide = false;
   for (int q = 0; q < 4; q++) tide |= s->fl_kind[q] == 1;
   if (tide) LAUNCH(k_set_t, dim3(1), dim3(32), s->ctl, (const double*)(s->rec + (size_t)STEP_REC * k));
   const swe::PrepArgs prep = prep_of(s, false, k);
-  StageArgs a1 = stage_args(s, T.W1, T.Bp);
-  a1.tape_th = T.th1; a1.tape_hpre = T.hB;
-  int rc = stage<1>(s, a1, tape_bufs(s, T.it1), T.W1, &prep, false);
-  if (rc) return rc;
-  StageArgs a2 = stage_args(s, T.Bp, out);
-  a2.tape_th = T.th2; a2.tape_hpre = T.hA;
-  for (int q = 0; q < 3; q++) { a2.tape_pre[q] = T.Bf[q]; a2.u0[q] = T.W1[q]; }
-  rc = stage<2>(s, a2, tape_bufs(s, T.it2), T.Bp, nullptr, false);
-  if (rc) return rc;
+  if (swe::prep_refused(s->dts_host[k])) {
+    LAUNCH(swe::k_prepare, dim3(1), dim3(32), s->ctl, prep);
+    LAUNCH(swe::k_apply_bc, dim3(bcb(s)), dim3(256), bc_args(s, T.W1), (const Control*)s->ctl, 0);
+    if (int rc = copy3(s, out, T.W1)) return rc;
+  } else {
+    StageArgs a1 = stage_args(s, T.W1, T.Bp);
+    a1.tape_th = T.th1; a1.tape_hpre = T.hB;
+    int rc = stage<1>(s, a1, tape_bufs(s, T.it1), T.W1, &prep, false);
+    if (rc) return rc;
+    StageArgs a2 = stage_args(s, T.Bp, out);
+    a2.tape_th = T.th2; a2.tape_hpre = T.hA;
+    for (int q = 0; q < 3; q++) { a2.tape_pre[q] = T.Bf[q]; a2.u0[q] = T.W1[q]; }
+    rc = stage<2>(s, a2, tape_bufs(s, T.it2), T.Bp, nullptr, false);
+    if (rc) return rc;
+  }
   if (s->ghost_gauges)                             // before the next step fills them
     LAUNCH(k_copy, dim3(G1(s)), dim3(256), (size_t)s->N, 1, T.hX, (double*)nullptr, (double*)nullptr,
            (const double*)out[0], (const double*)nullptr, (const double*)nullptr);
@@ -964,12 +980,20 @@ int tape_step(swe_adjoint* s, double* const* out, int k, const Tape& T) {
 
 // Reverse step k: on entry lA holds the adjoint of the step's output
 // (interior), on exit the adjoint of its input (interior); lb and ln
-// accumulate.
+// accumulate.  Of a refused step only the ghost fill is reversed, which matters
+// where a gauge read a ghost.
 int reverse_step(swe_adjoint* s, int k, const Tape& T) {
   const int gb = G1(s);
   const double dt = s->dts_host[k];
   double* lA[3] = {s->lA[0], s->lA[1], s->lA[2]};
   double* lB[3] = {s->lB[0], s->lB[1], s->lB[2]};
+  const auto ghosts = [&](double* const* X, double* const* l) {
+    LAUNCH(k_adj_bc, dim3(adjbc_blocks(s)), dim3(256), s->nsrc, (const int*)s->gmap, (const double*)s->b,
+           (const double*)X[0], (const double*)X[1], (const double*)X[2],
+           (const double*)(s->rec + (size_t)STEP_REC * k + 1), s->o.min_depth, s->eps4, s->lb, l[0], l[1], l[2]);
+    return SWE_OK;
+  };
+  if (swe::prep_refused(dt)) return s->ghost_gauges ? ghosts(T.W1, lA) : SWE_OK;
   // friction, dryClean, A = 0.5 (W1 + Bp + dt R2) backwards in one pass
   LAUNCH(k_adj_tail2, dim3(gb), dim3(256), s->W, s->H, s->o.min_depth, s->eps4, s->o.manning,
          (const double*)s->nfield, dt, (const double*)T.Bf[0], (const double*)T.Bf[1], (const double*)T.Bf[2],
@@ -977,20 +1001,16 @@ int reverse_step(swe_adjoint* s, int k, const Tape& T) {
          s->ab.lR[2]);
   int rc = residual_adjoint(s, T.Bp, T.it2, T.th2, dt, lB);
   if (rc) return rc;
-  LAUNCH(k_adj_bc, dim3(adjbc_blocks(s)), dim3(256), s->nsrc, (const int*)s->gmap, (const double*)s->b,
-         (const double*)T.Bp[0], (const double*)T.Bp[1], (const double*)T.Bp[2],
-         (const double*)(s->rec + (size_t)STEP_REC * k + 1), s->o.min_depth, s->eps4,
-         s->lb, lB[0], lB[1], lB[2]);
+  rc = ghosts(T.Bp, lB);
+  if (rc) return rc;
   // dryClean and B = W1 + dt R1 backwards: lW1 += lB, lR1 = dt lB
   LAUNCH(k_adj_tail1, dim3(gb), dim3(256), s->W, s->H, s->o.min_depth, dt, (const double*)T.hB,
          (const double*)lB[0], (const double*)lB[1], (const double*)lB[2], lA[0], lA[1], lA[2], s->ab.lR[0],
          s->ab.lR[1], s->ab.lR[2]);
   rc = residual_adjoint(s, T.W1, T.it1, T.th1, dt, lA);
   if (rc) return rc;
-  LAUNCH(k_adj_bc, dim3(adjbc_blocks(s)), dim3(256), s->nsrc, (const int*)s->gmap, (const double*)s->b,
-         (const double*)T.W1[0], (const double*)T.W1[1], (const double*)T.W1[2],
-         (const double*)(s->rec + (size_t)STEP_REC * k + 1), s->o.min_depth, s->eps4,
-         s->lb, lA[0], lA[1], lA[2]);
+  rc = ghosts(T.W1, lA);
+  if (rc) return rc;
   CU(cudaGetLastError());
   return SWE_OK;
 }

@@ -133,7 +133,7 @@ __device__ __forceinline__ double prep_dt(const Control* ctl, const PrepArgs& a)
   const double md = inv > 0 ? a.cfl / inv : INFINITY;
   return (a.mode == 3) ? jmin(md, a.t_end - ctl->t) : md;
 }
-__device__ __forceinline__ bool prep_refused(double dt) { return !(dt > 0) || !isfinite(dt); }
+__host__ __device__ __forceinline__ bool prep_refused(double dt) { return !(dt > 0) || !isfinite(dt); }
 // The exterior surface and normal velocity of a Flather side.
 __device__ __forceinline__ void prep_flather(const Control* ctl, const PrepArgs& a, int s, double& eta, double& u) {
   if (a.fl_kind[s] == 1) {
