@@ -314,13 +314,19 @@ int swe_adjoint_create(const swe_options* o, const double* b, const double* eta0
                        int n_gauges, const int* gauge_cells, int steps, int checkpoint_every, swe_adjoint** out);
 int swe_adjoint_destroy(swe_adjoint* s);
 int swe_adjoint_set_observations(swe_adjoint* s, const double* obs);      /* steps x n_gauges */
-/* J, and (optional) eta at the gauges after every step (steps x n_gauges). */
+/* J, and (optional) eta at the gauges after every step (steps x n_gauges).
+ * SWE_ETIMEOUT when a tile copy of the pass did not complete within its time
+ * bound: what was returned is incomplete, and swe_adjoint_backward asks for a
+ * new forward pass. */
 int swe_adjoint_forward(swe_adjoint* s, double* J, double* gauge_eta);
 int swe_adjoint_backward(swe_adjoint* s, double* grad_b, double* grad_n);
 /* The dt of every step (steps doubles): read the sequence of the last
  * forward pass into dts_out, and/or hold the forward to dts_in from now on
  * (a finite-difference check needs the same frozen dts). */
 int swe_adjoint_dt_sequence(swe_adjoint* s, double* dts_out, const double* dts_in);
+/* Test hook: the status bits each forward pass starts with (0: none; 4: as
+ * after a tile copy that did not complete), for checking that it reports them. */
+int swe_adjoint_debug_status(swe_adjoint* s, int bits);
 int swe_adjoint_get_stream(swe_adjoint* s, void** stream);
 /* The boundary of one side (SWE_SIDE_*) for the forward and its reverse:
  * SWE_BC_REFLECT (the default), _OUTFLOW, _PERIODIC, or _FLATHER with the

@@ -258,3 +258,23 @@ def test_gauges_in_ghost_cells(swe, bcs, refused):
             fd = (J_at(c["b"] + eps * db, c["n"] + eps * dn) - J_at(c["b"] - eps * db, c["n"] - eps * dn)) / (2 * eps)
             errs.append(abs(fd - want) / abs(want))
         assert min(errs) <= 1e-5, (trial, errs)
+
+
+def test_an_incomplete_tile_copy_is_reported(swe):
+    """The status bit that a tile copy past its bound sets (put there by the
+    test hook): forward() raises SWE_ETIMEOUT, backward() asks for a new
+    forward pass, and without the bit the handle works as before."""
+    c, obs = case(swe, steps=6)
+    adj, J, gb, gn, _ = gradient(swe, c, obs, 6, 4)
+    adj.debug_status(4)
+    with pytest.raises(swe.SweError) as e:
+        adj.forward()
+    assert e.value.code == -4                      # SWE_ETIMEOUT
+    with pytest.raises(swe.SweError) as e:
+        adj.backward()
+    assert e.value.code == -1                      # SWE_EINVAL: no forward pass
+    adj.debug_status(0)
+    assert adj.forward()[0] == J
+    again = adj.backward()
+    assert np.array_equal(again[0], gb) and np.array_equal(again[1], gn)
+    adj.close()

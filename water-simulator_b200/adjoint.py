@@ -84,7 +84,8 @@ class MisfitAdjoint:
         check(self._lib.swe_adjoint_set_observations(self._h, dptr(o)))
 
     def forward(self):
-        """Returns (J, eta at the gauges after every step)."""
+        """Returns (J, eta at the gauges after every step); raises SweError
+        (SWE_ETIMEOUT) when a tile copy of the pass did not complete in time."""
         J = ctypes.c_double()
         eta = np.zeros((self.steps, len(self.gauges)))
         check(self._lib.swe_adjoint_forward(self._h, ctypes.byref(J), dptr(eta)))
@@ -102,6 +103,10 @@ class MisfitAdjoint:
         inp = None if fixed is None else np.ascontiguousarray(fixed, dtype=np.float64)
         check(self._lib.swe_adjoint_dt_sequence(self._h, dptr(out), dptr(inp) if inp is not None else None))
         return out
+
+    def debug_status(self, bits=0):
+        """Test hook: the status bits each forward starts with (0: none)."""
+        check(self._lib.swe_adjoint_debug_status(self._h, int(bits)))
 
     def stream(self):
         p = ctypes.c_void_p()

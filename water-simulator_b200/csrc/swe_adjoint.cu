@@ -1237,6 +1237,7 @@ int swe_adjoint_set_observations(swe_adjoint* s, const double* obs) {
 
 int swe_adjoint_forward(swe_adjoint* s, double* J, double* gauge_eta) {
   if (!s) return fail(SWE_EINVAL, "null argument");
+  s->forward_done = false;
   const int gb = G1(s);
   k_init_state<<<gb, 256, 0, s->st>>>(s->N, s->b, s->eta0, s->A[0], s->A[1], s->A[2]);
   CU(cudaMemcpyAsync(s->ctl, &s->ctl_init, sizeof(Control), cudaMemcpyHostToDevice, s->st));   // t = 0, tide tables
@@ -1254,10 +1255,16 @@ int swe_adjoint_forward(swe_adjoint* s, double* J, double* gauge_eta) {
     if (int rc = fwd_step(s, k)) return rc;
   }
   CU(cudaGetLastError());
+  int status = 0;
+  CU(cudaMemcpyAsync(&status, &s->ctl->status, sizeof status, cudaMemcpyDeviceToHost, s->st));
   if (J) CU(cudaMemcpyAsync(J, s->J, sizeof(double), cudaMemcpyDeviceToHost, s->st));
   if (gauge_eta)
     CU(cudaMemcpyAsync(gauge_eta, s->eta_series, sizeof(double) * s->steps * s->ng, cudaMemcpyDeviceToHost, s->st));
   CU(cudaStreamSynchronize(s->st));
+  // (swe_split.cuh, tile_wait: the copy's tile was left unwritten)
+  if (status & 4)
+    return fail(SWE_ETIMEOUT, "swe_adjoint_forward: a tile copy did not complete within its time bound; J, the gauges "
+                              "and the checkpoints of this pass are incomplete");
   s->forward_done = true;
   return SWE_OK;
 }
@@ -1360,6 +1367,12 @@ int swe_adjoint_set_flather_tide(swe_adjoint* s, int side, double msl, int n, co
   s->kind[side] = SWE_BC_FLATHER;
   s->forward_done = false;
   return build_ghost_map(s);
+}
+
+int swe_adjoint_debug_status(swe_adjoint* s, int bits) {
+  if (!s) return fail(SWE_EINVAL, "null argument");
+  s->ctl_init.status = bits;
+  return SWE_OK;
 }
 
 int swe_adjoint_get_stream(swe_adjoint* s, void** stream) {
