@@ -294,6 +294,9 @@ int swe_batch_set_wait_limit(swe_batch* s, double seconds);
  * that basin's next phase waits until its limit -- a wait that nothing
  * ends, for checking that it does end, with SWE_ETIMEOUT. */
 int swe_batch_debug_hold(swe_batch* s, int basin);
+/* Test hook: the basin's status bits (4: as after a tile copy that did not
+ * complete), for checking that its next step is not closed and is reported. */
+int swe_batch_debug_status(swe_batch* s, int basin, int bits);
 int swe_batch_get_stream(swe_batch* s, void** stream);
 int swe_batch_get_field(swe_batch* s, int basin, int field, double* out);   /* B, H, HU, HV */
 int swe_batch_get_scalar(swe_batch* s, int basin, int which, double* out);  /* T, STEPS, MASS_FLOORED */

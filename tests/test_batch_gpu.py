@@ -134,3 +134,27 @@ def test_queue_wait_that_nothing_ends_times_out(swe):
     fresh.synchronize()
     assert all(fresh.steps(q) == 3 for q in range(len(bs)))
     fresh.close()
+
+
+def test_an_incomplete_tile_copy_is_reported(swe):
+    """The status bit that a tile copy past its bound sets (put there by the
+    test hook): the basin's step is not closed, synchronize() raises
+    SWE_ETIMEOUT once and says which wait it was, and the other basins go on."""
+    bs = basins(swe)
+    ens = swe.Ensemble(bs)
+    ens.run(3)
+    t = [ens.t(q) for q in range(len(bs))]
+    ens.debug_status(2, 4)
+    ens.run(1)
+    with pytest.raises(swe.SweError) as e:
+        ens.synchronize()
+    assert e.value.code == -4                          # SWE_ETIMEOUT
+    assert "tile copy" in str(e.value) and "work-queue" not in str(e.value)
+    for q in range(len(bs)):
+        assert ens.steps(q) == (3 if q == 2 else 4) and (ens.t(q) == t[q]) == (q == 2)
+    ens.synchronize()                                  # reported once, then cleared
+    ens.set_launch("queue")
+    ens.run(2)
+    ens.synchronize()
+    assert [ens.steps(q) for q in range(3)] == [6, 6, 5]
+    ens.close()

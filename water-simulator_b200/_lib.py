@@ -135,6 +135,7 @@ SIGNATURES = {
     "swe_batch_get_launch": [_P, _IP],
     "swe_batch_set_wait_limit": [_P, _D],
     "swe_batch_debug_hold": [_P, _I],
+    "swe_batch_debug_status": [_P, _I, _I],
     "swe_batch_get_stream": [_P, ctypes.POINTER(_P)],
     "swe_batch_get_field": [_P, _I, _I, _DP],
     "swe_batch_get_scalar": [_P, _I, _I, _DP],

@@ -84,7 +84,7 @@ class Ensemble:
 
     def synchronize(self):
         """Wait for the ensemble; raises SweError (SWE_ETIMEOUT) when a
-        work-queue wait ran past its limit since the last call."""
+        work-queue wait or a tile copy ran past its limit since the last call."""
         check(self._lib.swe_batch_synchronize(self._h))
 
     @property
@@ -104,6 +104,10 @@ class Ensemble:
     def debug_hold(self, basin=-1):
         """Test hook: never mark `basin`'s prepare done (-1: none)."""
         check(self._lib.swe_batch_debug_hold(self._h, int(basin)))
+
+    def debug_status(self, basin, bits):
+        """Test hook: the status bits the basin's next step finds."""
+        check(self._lib.swe_batch_debug_status(self._h, int(basin), int(bits)))
 
     def field(self, basin, name):
         W, H = self.dims[basin]

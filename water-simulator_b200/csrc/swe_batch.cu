@@ -154,18 +154,27 @@ k_batch_split_cells(BatchBasin* basins, const BatchMaps* maps, const BatchTile* 
   }
 }
 
+// What the host reads back of the steps since it last asked.
+enum { BATCH_ERR_WAIT = 1, BATCH_ERR_COPY = 2 };   // a work-queue wait, a tile copy past its bound
+
 // The close of every basin's step after the tiled pair, a block per basin: both
 // stages as their last tile's ticket would have closed them (which made every
 // tile wait for its fence and its place; 24 basins: cell kernel 364 -> 227 us, the
 // staging by tensor maps included).
-// A tile copy that ran past its bound (tile_wait) goes to err, which the host
-// reads, as a work-queue wait's does.
+// A step one of whose tile copies ran past its bound (tile_wait) left a tile
+// unwritten: it goes to err, for the host, and is not closed (t and the number
+// of steps leave it out).
 __global__ void __launch_bounds__(swe::SP_THREADS) k_batch_close(BatchBasin* basins, int* err) {
   __shared__ swe::CellsSmem sm;
   const BatchBasin& B = basins[blockIdx.x];
-  if (threadIdx.x == 0 && (B.ctl->status & 4)) {
-    atomicExch(err, 1);
-    B.ctl->status &= ~4;
+  const bool late = B.ctl->status & 4;
+  __syncthreads();                                 // every thread has read it
+  if (late) {
+    if (threadIdx.x == 0) {
+      atomicOr(err, BATCH_ERR_COPY);
+      B.ctl->status &= ~4;
+    }
+    return;
   }
   if (B.ctl->stop) return;
   swe::split_close_block<1>(B.s1, B.ctl, B.s1.nblocks, sm);
@@ -197,7 +206,7 @@ constexpr int QPHASES = 7;
 struct QueueCtl {
   int* head;                  // next item; reset before every launch
   int* done;                  // [basin * QPHASES + phase]; reset before every launch
-  int* err;                   // 1: a wait ran out of time (sticky until the host reads it)
+  int* err;                   // BATCH_ERR_WAIT: a wait ran out of time (sticky until the host reads it)
   long long limit_ns;         // the time limit of one wait
   int hold;                   // debug: a basin whose prepare is never marked done (-1: none)
 };
@@ -215,9 +224,9 @@ __device__ bool queue_wait(const QueueCtl& q, int slot, int need) {
   if (d[slot] >= need) return true;
   const unsigned long long t0 = global_ns();
   while (d[slot] < need) {
-    if (*e) return false;
+    if (*e & BATCH_ERR_WAIT) return false;
     if ((long long)(global_ns() - t0) > q.limit_ns) {
-      atomicExch(q.err, 1);
+      atomicOr(q.err, BATCH_ERR_WAIT);
       return false;
     }
     __nanosleep(256);
@@ -239,7 +248,7 @@ k_batch_queue_step(BatchBasin* basins, const BatchTile* tiles, int nb, int ntile
   __shared__ int s_item, s_go;
   const int total = 3 * nb + 4 * ntiles;
   for (;;) {
-    if (threadIdx.x == 0) s_item = *(volatile int*)q.err ? total : atomicAdd(q.head, 1);
+    if (threadIdx.x == 0) s_item = *(volatile int*)q.err & BATCH_ERR_WAIT ? total : atomicAdd(q.head, 1);
     __syncthreads();
     const int it = s_item;
     if (it >= total) return;                       // uniform
@@ -717,8 +726,15 @@ int swe_batch_synchronize(swe_batch* s) {
   CU(cudaMemcpy(&e, err, sizeof(int), cudaMemcpyDeviceToHost));
   if (e) {
     CU(cudaMemset(err, 0, sizeof(int)));
-    return fail(SWE_ETIMEOUT, "swe_batch: a work-queue wait ran past its time limit; the steps in flight "
-                              "were dropped and the basins' state is not a completed step");
+    std::string m = "swe_batch: ";
+    if (e & BATCH_ERR_WAIT)
+      m += "a work-queue wait ran past its time limit; the steps in flight were dropped and the basins' state is not "
+           "a completed step";
+    if (e & BATCH_ERR_COPY)
+      m += std::string(e & BATCH_ERR_WAIT ? "; " : "") +
+           "a tile copy did not complete within its time bound; its basin's step was not closed, and the steps since "
+           "the last synchronize ran on with an incomplete tile";
+    return fail(SWE_ETIMEOUT, m);
   }
   return SWE_OK;
 }
@@ -749,6 +765,13 @@ int swe_batch_debug_hold(swe_batch* s, int basin) {
   if (!s || basin < -1 || basin >= s->nb) return fail(SWE_EINVAL, "swe_batch_debug_hold: a basin or -1");
   s->hold = basin;
   s->version++;
+  return SWE_OK;
+}
+
+int swe_batch_debug_status(swe_batch* s, int basin, int bits) {
+  if (!s || basin < 0 || basin >= s->nb) return fail(SWE_EINVAL, "swe_batch_debug_status: bad basin");
+  CU(cudaMemcpyAsync(&s->ctls[basin].status, &bits, sizeof bits, cudaMemcpyHostToDevice, s->st));
+  CU(cudaStreamSynchronize(s->st));
   return SWE_OK;
 }
 
