@@ -239,3 +239,38 @@ def test_globe_refusals(swe):
     with pytest.raises(swe.SweError, match="LUT was baked for"):
         swe.renderGlobe(np.zeros(4 * 32 * 32, np.uint8), bsim, lut)
     lut.close(); a.close(); bsim.close(); flat.close()
+
+
+def test_one_table_serves_several_threads(swe):
+    """Frames of two simulations drawn with one table from two threads: each
+    frame and its statistics are those of its own simulation."""
+    import threading
+    nx, ny, size = 180, 90, 400
+    sims = [swe.ShallowWater(nx=nx, ny=ny, bed=bed, eta0=0.0, sphere={"R": 6371e3, "lat0": -80, "lat1": 80})
+            for bed in (-4000.0, 900.0)]
+    sims[0].h = np.where(np.arange(sims[0].W * sims[0].H) % 7 < 3, 4002.0, 4000.5)
+    lut = swe.buildGlobeLut(swe.globeCamera(size), sims[0])
+
+    def frame(sim):
+        out = np.zeros(4 * size * size, np.uint8)
+        return out, swe.renderGlobe(out, sim, lut, scale=3.0)
+
+    want = [frame(s) for s in sims]
+    assert not np.array_equal(want[0][0], want[1][0]) and want[0][1] != want[1][1]
+    wrong = []
+
+    def draw(q):
+        for _ in range(150):
+            out, stats = frame(sims[q])
+            if not np.array_equal(out, want[q][0]) or stats != want[q][1]:
+                wrong.append(q)
+
+    threads = [threading.Thread(target=draw, args=(q,)) for q in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, f"{len(wrong)} of 300 frames are not their simulation's"
+    lut.close()
+    for s in sims:
+        s.close()

@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 #include <algorithm>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -46,6 +47,9 @@ struct swe_globe_lut {
   double* d_stats = nullptr;     // frame reduction scratch
   unsigned int* d_ticket = nullptr;
   int nblocks = 0;
+  // A table serves every simulation of its grid, from several threads: d_out,
+  // d_stats and d_ticket are one frame's at a time.
+  std::mutex frame;
 };
 
 namespace {
@@ -496,6 +500,7 @@ int swe_render_globe(swe_sim* s, swe_globe_lut* L, double rot_deg, double scale,
   if (rc) return rc;
   const size_t bytes = (size_t)4 * L->size * L->size;
   unsigned char* out = static_cast<unsigned char*>(rgba_device);
+  std::lock_guard<std::mutex> one(L->frame);    // until the frame is complete
   if (!out) out = L->d_out;
   cudaError_t e = cudaMemcpyAsync(out, L->d_bg, bytes, cudaMemcpyDeviceToDevice, st);   // out.set(lut.bg)
   FrameStats* part = reinterpret_cast<FrameStats*>(L->d_stats + 8);
