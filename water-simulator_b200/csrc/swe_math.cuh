@@ -334,10 +334,11 @@ __device__ __forceinline__ FaceSums solve_tame(double hL, double hR, double nL, 
   f.NpR = N + pR;
   return f;
 }
+// lanes: the lanes of the warp that make this call together, for the vote on BOTH.
 __device__ __forceinline__ FaceSums face_flux_tame(
     double bL_c, double hL_c, double nL_c, double tL_c, double sEL, double sBL, double sNL, double sTL,
     double bR_c, double hR_c, double nR_c, double tR_c, double sER, double sBR, double sNR, double sTR, double dry,
-    bool& redo) {
+    bool& redo, unsigned lanes = __activemask()) {
   const double etaL = fma(0.5, sEL, bL_c + hL_c), etaR = fma(-0.5, sER, bR_c + hR_c);
   const double bL = fma(0.5, sBL, bL_c), bR = fma(-0.5, sBR, bR_c);
   const double hLf = pos(etaL - bL), hRf = pos(etaR - bR);
@@ -348,7 +349,7 @@ __device__ __forceinline__ FaceSums face_flux_tame(
   const double pL = 0.5 * SWE_G * (hLf * hLf - hL * hL), pR = 0.5 * SWE_G * (hRf * hRf - hR * hR);
   const bool wetL = hL > dry, wetR = hR > dry;
   redo = false;
-  if (__all_sync(__activemask(), wetL && wetR))
+  if (__all_sync(lanes, wetL && wetR))
     return solve_tame<true>(hL, hR, nL, nR, tL, tR, pL, pR, true, true, redo);
   if (!wetL && !wetR) return {0, 0, 0 + pL, 0 + pR};
   return solve_tame<false>(hL, hR, nL, nR, tL, tR, pL, pR, wetL, wetR, redo);

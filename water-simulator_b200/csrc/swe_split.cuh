@@ -155,10 +155,11 @@ struct FacesSmem {
 
 // One cell of a faces tile: its source terms, its east x face and north y
 // face.  TAME: every cell of the tile's box is tame; returns whether a face
-// must be formed again without.
+// must be formed again without.  lanes: the lanes of the warp that make the call.
 template <bool TAME>
 __device__ __forceinline__ bool split_faces_cell(const StageArgs& a, const SplitBufs& s, const FacesSmem& sm,
-                                                 int lx, int ly, int gi, int gj, bool sph, bool bedOn) {
+                                                 int lx, int ly, int gi, int gj, bool sph, bool bedOn,
+                                                 unsigned lanes) {
   const int W = a.W, H = a.H;
   const double dry = a.minDepth;
   const size_t k = (size_t)gj * s.P + gi;
@@ -225,13 +226,14 @@ __device__ __forceinline__ bool split_faces_cell(const StageArgs& a, const Split
     const int qn = d == 0 ? 2 : 3, qt = 5 - qn;                  // normal and transverse velocity slopes
     const int ry = d == 0 ? cy : cy + 1, rx = d == 0 ? cx + 1 : cx;
     FaceSums f = {0, 0, 0, 0};
+    const unsigned solving = TAME ? __ballot_sync(lanes, on) : 0;
     if (on) {
       const double nl = d == 0 ? Uk : Vk, tl = d == 0 ? Vk : Uk;
       const double nr = d == 0 ? sm.U[ry][rx] : sm.V[ry][rx], tr = d == 0 ? sm.V[ry][rx] : sm.U[ry][rx];
       if (TAME) {
         bool redo;
         f = face_flux_tame(bk, hk, nl, tl, sp[0], sp[fs], sp[qn * fs], sp[qt * fs], sm.b[ry][rx], sm.h[ry][rx], nr,
-                           tr, sp[no], sp[fs + no], sp[qn * fs + no], sp[qt * fs + no], dry, redo);
+                           tr, sp[no], sp[fs + no], sp[qn * fs + no], sp[qt * fs + no], dry, redo, solving);
         again |= redo;
       } else {
         const Face g = face_flux(bk, hk, nl, tl, sp[0], sp[fs], sp[qn * fs], sp[qt * fs], sm.b[ry][rx],
@@ -431,10 +433,12 @@ __device__ __forceinline__ void split_faces_finish(const StageArgs& a, const Spl
 
   const int lx = t % SPX, ly = t / SPX;
   const int gi = i0 + lx, gj = j0 + ly;
+  const bool in = gi < W && gj < H;
+  const unsigned lanes = __ballot_sync(0xffffffffu, in);
   bool again = !tame;
-  if (tame && gi < W && gj < H) again = split_faces_cell<true>(a, s, sm, lx, ly, gi, gj, sph, bedOn);
+  if (tame && in) again = split_faces_cell<true>(a, s, sm, lx, ly, gi, gj, sph, bedOn, lanes);
   if (__syncthreads_or(again)) {
-    if (gi < W && gj < H) split_faces_cell<false>(a, s, sm, lx, ly, gi, gj, sph, bedOn);
+    if (in) split_faces_cell<false>(a, s, sm, lx, ly, gi, gj, sph, bedOn, lanes);
     __syncthreads();
   }
 }
