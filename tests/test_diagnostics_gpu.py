@@ -117,3 +117,34 @@ def test_energy_for_any_min_depth(swe, minDepth):
     assert np.all(np.isfinite(term))
     assert sim.energy() == chain([chain(r) for r in term]) * 2.0 * 2.0
     sim.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (3, 5001), (4, 33), (5, 4), (127, 40), (128, 3), (129, 65), (1025, 2), (5001, 3),
+                                   (1, 300_007), (620_003, 1)])
+def test_reductions_reach_every_cell(swe, nx, ny):
+    """The largest value is found, and one lost cell seen, wherever it lies:
+    narrow and low grids share the blocks' threads out differently."""
+    rng = np.random.default_rng(nx + ny)
+    shape = (ny + 4, nx + 4)
+    h = rng.uniform(1.0, 2.0, shape)
+    sim = swe.ShallowWater(nx=nx, ny=ny, dx=2.0, bed=0.0, eta0=0.0)
+    cells = [(0, 0), (ny - 1, nx - 1), (ny - 1, 0), (0, nx - 1)] + [(rng.integers(ny), rng.integers(nx)) for _ in range(4)]
+    for j, i in cells:
+        x = h.copy()
+        x[j + 2, i + 2] = 9.0
+        sim.h = x
+        assert sim.maxSurfaceDeviation(0.0) == 9.0 and sim.finite()
+        c = np.sqrt(swe.G * 9.0)
+        assert sim.maxDt() == 0.45 / (c / 2.0 + c / 2.0)
+        hu = np.zeros(shape)
+        hu[j + 2, i + 2] = 3.0
+        sim.hu = hu
+        u = sim.vel(3.0, 9.0)
+        assert abs(sim.maxSpeed() - u) <= 4e-16 * u
+        sim.hu = np.zeros(shape)
+    for j, i in [(0, 0), (ny + 3, nx + 3), (ny + 1, 1), (rng.integers(ny + 4), rng.integers(nx + 4))]:   # ghosts too
+        hv = np.zeros(shape)
+        hv[j, i] = np.nan
+        sim.hv = hv
+        assert not sim.finite()
+    sim.close()

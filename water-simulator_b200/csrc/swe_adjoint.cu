@@ -1244,7 +1244,9 @@ int swe_adjoint_forward(swe_adjoint* s, double* J, double* gauge_eta) {
   CU(cudaMemsetAsync(s->J, 0, sizeof(double), s->st));
   {
     StageArgs a = stage_args(s, s->A, nullptr);
-    swe::k_cfl_rate<<<std::min(1024, std::max(1, (s->o.nx * s->o.ny + 255) / 256)), swe::BX, 0, s->st>>>(a, s->ctl, s->part);
+    dim3 grid;                                     // at most REDUCTION_BLOCKS, of 3 * 1024 slots or more
+    const swe::RedWalk w = swe::reduction_walk(s->o.ny, s->o.nx, grid);
+    swe::k_cfl_rate<<<grid, swe::BX, 0, s->st>>>(a, w, s->ctl, s->part);
   }
   for (int k = 0; k < s->steps; k++) {
     if (k % s->every == 0) {

@@ -568,19 +568,12 @@ int enqueue_step(swe_sim* s, int mode, double dt, double t_end, const double* dt
   return rc;
 }
 
-constexpr int REDUCTION_BLOCKS = 16 * 148;
-// The grid of a full-grid reduction (swe_kernels.cuh, for_cells): a block per
-// row and segment, at most 16 per SM of a B200, so that the last block's ticket
-// is shared by a few thousand blocks.
-dim3 reduction_grid(int rows, int cols) {
-  const int segs = std::min(16, (cols + swe::RED_SEG - 1) / swe::RED_SEG);
-  return dim3(std::min(rows, REDUCTION_BLOCKS / segs), segs);
-}
-
 int ensure_cfl(swe_sim* s) {
   if (s->cfl_valid) return SWE_OK;
   swe::StageArgs a = stage_args(s, s->d_A, nullptr);
-  swe::k_cfl_rate<<<reduction_grid(s->ny, s->nx), swe::BX, 0, s->st>>>(a, s->d_ctl, s->d_red);
+  dim3 grid;
+  const swe::RedWalk w = swe::reduction_walk(s->ny, s->nx, grid);
+  swe::k_cfl_rate<<<grid, swe::BX, 0, s->st>>>(a, w, s->d_ctl, s->d_red);
   CU(cudaGetLastError());
   s->cfl_valid = true;
   return SWE_OK;
@@ -762,7 +755,7 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
   // and cudaFree for every one took longer than the rest of a small handle's
   // creation: each new 2 MB of memory costs some 0.3 ms); the partials are the
   // tiles', the close's scratch and the reductions'.
-  const size_t nparts = 3 * (size_t)s->part_cap + 3 * swe::CLOSE_BLOCKS + REDUCTION_BLOCKS;
+  const size_t nparts = 3 * (size_t)s->part_cap + 3 * swe::CLOSE_BLOCKS + swe::REDUCTION_BLOCKS;
   const size_t N = s->N, sizes[12] = {N, N, N, N, N, N, N, (size_t)(SWE_GEOM_NROWS + 5) * s->H, nparts,
                                       (size_t)std::max(1, s->ny), (sizeof(swe::Control) + 7) / 8,
                                       s->stage_impl == 1 ? split_doubles(s) : 0};
@@ -778,7 +771,7 @@ int swe_create(const swe_options* o, const double* b, const double* h, swe_sim**
     at += (sizes[q] + 31) & ~size_t(31);
   }
   double* const split_mem = at;
-  s->d_red = s->d_part + (nparts - REDUCTION_BLOCKS);
+  s->d_red = s->d_part + (nparts - swe::REDUCTION_BLOCKS);
   CUB(cudaMemsetAsync(s->d_ctl, 0, sizeof(swe::Control), s->st));
   CUB(cudaMemsetAsync(s->d_part, 0, sizeof(double) * nparts, s->st));
   for (int q = 0; q < 3; q++) {
@@ -1304,7 +1297,9 @@ int swe_eta_projection(swe_sim* s, const double* coef, double* out) {
 
 static int max_diag(swe_sim* s, int what, double ref, double* out) {
   swe::StageArgs a = stage_args(s, s->d_A, nullptr);
-  swe::k_max_diag<<<what == 2 ? reduction_grid(s->H, s->W) : reduction_grid(s->ny, s->nx), swe::BX, 0, s->st>>>(a, what, ref, s->d_red, s->d_ctl);
+  dim3 grid;
+  const swe::RedWalk w = what == 2 ? swe::reduction_walk(s->H, s->W, grid) : swe::reduction_walk(s->ny, s->nx, grid);
+  swe::k_max_diag<<<grid, swe::BX, 0, s->st>>>(a, w, what, ref, s->d_red, s->d_ctl);
   CU(cudaGetLastError());
   return finish_diag(s, out);
 }

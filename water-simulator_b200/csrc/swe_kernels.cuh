@@ -32,6 +32,7 @@
 // and same-column values ride in registers.  Ring depths (state 3, x slopes
 // 2, x faces 3, theta 2) are what make one barrier per row sufficient.
 #pragma once
+#include <algorithm>
 #include "swe_math.cuh"
 
 namespace swe {
@@ -735,16 +736,48 @@ __device__ __forceinline__ double combine_parts(const double* part, int n, bool 
   return mm;
 }
 
-// The full-grid reductions walk the grid row by row, block (x, y) taking the
-// segments y, y + gridDim.y, ... of RED_SEG columns of the rows x, x +
-// gridDim.x, ... (a division per cell for its row had taken a third of the
-// work of the cheaper ones).
-constexpr int RED_SEG = 8 * BX;
+// The full-grid reductions walk the grid in bands of `per` rows, cut into
+// segments of `seg` columns (a division per cell for its row had taken a third of
+// the work of the cheaper ones): block (x, y) takes the segments y, y +
+// gridDim.y, ... of the bands x, x + gridDim.x, ..., at most 16 blocks per SM of a
+// B200, so that the last block's ticket is shared by a few thousand.  A thread
+// takes 8 columns of a segment: fewer where that leaves less than 4 blocks per SM,
+// more where a few long rows would be unequal shares.  A row narrower than the
+// block takes as many threads as it has columns (a power of two) and the block
+// several rows.  maxSpeed()'s kernel with 1024 columns of one row for every block,
+// whatever the grid, and so: 100 000 x 1 74.0 -> 9.4 us, 1 000 000 x 1 600 -> 18.2,
+// 4 x 20 000 33.0 -> 8.7, 4000 x 4 14.6 -> 6.4; 777 x 501 14.8 -> 13.1,
+// 1536 x 1024 23.7, 2048 x 2048 47.2 -> 47.8.
+struct RedWalk { int lg, per, seg; };              // threads along a row: 1 << lg
+constexpr int REDUCTION_BLOCKS = 16 * 148;
+__host__ inline RedWalk reduction_walk(int rows, int cols, dim3& grid) {
+  constexpr int FEW = 4 * 148;
+  RedWalk w;
+  w.lg = 0;
+  while ((1 << w.lg) < cols && (1 << w.lg) < BX) w.lg++;
+  const int tw = 1 << w.lg;
+  w.per = BX / tw;
+  const int bands = (rows + w.per - 1) / w.per, most = (cols + tw - 1) / tw;   // columns a thread would take of a row
+  int k = 8, segs;
+  const auto few = [&]() { segs = (most + k - 1) / k; return (long long)bands * segs < FEW; };
+  while (few() && k > 1) k /= 2;
+  while (REDUCTION_BLOCKS / segs < std::min(bands, 16) && k < most) { k *= 2; few(); }   // unequal turns of few bands
+  w.seg = k * tw;
+  const int limit = REDUCTION_BLOCKS / segs;
+  int x = std::min(bands, limit);
+  if (most == 1) {                                 // narrow: 2 rows a thread, or equal turns of more
+    const int turns = std::max((bands + limit - 1) / limit, bands >= 2 * FEW ? 2 : 1);
+    x = (bands + turns - 1) / turns;
+  }
+  grid = dim3(x, segs);
+  return w;
+}
 template <class F>
-__device__ __forceinline__ void for_cells(int j0, int j1, int i0, int i1, F f) {
-  for (int j = j0 + blockIdx.x; j < j1; j += gridDim.x)
-    for (int s = i0 + blockIdx.y * RED_SEG; s < i1; s += gridDim.y * RED_SEG)
-      for (int i = s + threadIdx.x; i < min(s + RED_SEG, i1); i += BX) f(j, i);
+__device__ __forceinline__ void for_cells(const RedWalk& w, int j0, int j1, int i0, int i1, F f) {
+  const int tx = threadIdx.x & ((1 << w.lg) - 1), ty = threadIdx.x >> w.lg;
+  for (int j = j0 + blockIdx.x * w.per + ty; j < j1; j += gridDim.x * w.per)
+    for (int s = i0 + blockIdx.y * w.seg; s < i1; s += gridDim.y * w.seg)
+      for (int i = s + tx; i < min(s + w.seg, i1); i += 1 << w.lg) f(j, i);
 }
 
 // Both velocities of a cell, branch-free where it is tame.  The diagnostics take
@@ -758,11 +791,11 @@ __device__ __forceinline__ void cell_vel(const StageArgs& a, double h, double hu
 }
 
 // CFL rate max over wet interior cells (src/swe.mjs:632-647) -> ctl->next_max.
-__global__ void __launch_bounds__(BX) k_cfl_rate(StageArgs a, Control* ctl, double* part) {
+__global__ void __launch_bounds__(BX) k_cfl_rate(StageArgs a, RedWalk w, Control* ctl, double* part) {
   __shared__ double s[BX / 32];
   __shared__ bool s_last;
   double m = 0;
-  for_cells(2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
+  for_cells(w, 2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
     const size_t k = (size_t)j * a.W + i;
     const double hk = a.h[k], huk = a.hu[k], hvk = a.hv[k];
     if (hk <= a.minDepth) return;
@@ -1206,18 +1239,18 @@ __global__ void __launch_bounds__(ROWSUM_THREADS) k_row_sums(StageArgs a, int wh
 
 // what: 0 maxSurfaceDeviation(ref) (src/swe.mjs:880-892), 1 maxSpeed (:895-907),
 // 2 finite count of non-finite cells over all N (:912-917).
-__global__ void __launch_bounds__(BX) k_max_diag(StageArgs a, int what, double ref, double* part, Control* ctl) {
+__global__ void __launch_bounds__(BX) k_max_diag(StageArgs a, RedWalk w, int what, double ref, double* part, Control* ctl) {
   __shared__ double s[BX / 32];
   __shared__ bool s_last;
   double m = 0;
   if (what == 2)
-    for_cells(0, a.H, 0, a.W, [&](int j, int i) {
+    for_cells(w, 0, a.H, 0, a.W, [&](int j, int i) {
       const size_t q = (size_t)j * a.W + i;
       const double hk = a.h[q], huk = a.hu[q], hvk = a.hv[q];
       if (!isfinite(hk) || !isfinite(huk) || !isfinite(hvk)) m += 1;
     });
   else if (what == 0)
-    for_cells(2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
+    for_cells(w, 2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
       const size_t k = (size_t)j * a.W + i;
       const double hk = a.h[k], bk = a.b[k];
       if (hk <= a.minDepth) return;
@@ -1225,7 +1258,7 @@ __global__ void __launch_bounds__(BX) k_max_diag(StageArgs a, int what, double r
       if (d > m) m = d;
     });
   else
-    for_cells(2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
+    for_cells(w, 2, a.H - 2, 2, a.W - 2, [&](int j, int i) {
       const size_t k = (size_t)j * a.W + i;
       const double hk = a.h[k], huk = a.hu[k], hvk = a.hv[k];
       if (hk <= a.minDepth) return;
