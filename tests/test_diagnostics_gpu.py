@@ -148,3 +148,17 @@ def test_reductions_reach_every_cell(swe, nx, ny):
         sim.hv = hv
         assert not sim.finite()
     sim.close()
+
+
+@pytest.mark.parametrize("cells", [1024, 7167, 7168, 7169])
+@pytest.mark.parametrize("kind", ["uniform", "wide", "negative", "lost"])
+def test_volume_where_the_plain_chain_ends(swe, kind, cells):
+    """Up to 7168 cells the sum is the plain chain, from there on cut into runs."""
+    h = depths(kind, cells, np.random.default_rng(cells))
+    sim = swe.ShallowWater(nx=cells, ny=1, dx=2.0, bed=0.0, eta0=0.0)
+    x = np.full((5, cells + 4), 7.0)
+    x[2, 2:-2] = h
+    sim.h = x
+    got, want = sim.volume(), chain(h) * 2.0 * 2.0
+    assert got == want or (np.isnan(got) and np.isnan(want))
+    sim.close()

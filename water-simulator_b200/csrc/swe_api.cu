@@ -1263,12 +1263,13 @@ int swe_volume(swe_sim* s, double* out) {
   if (s->diag_order == SWE_DIAG_ROWS) return row_diag(s, 0, 1, nullptr, out);
   swe::StageArgs a = stage_args(s, s->d_A, nullptr);
   const int chunks = (int)(((long long)s->nx * s->ny + swe::VOL_CELLS - 1) / swe::VOL_CELLS);
-  if (chunks > 2) {                 // a smaller grid's sum is all in its first powers of two
+  const bool runs = chunks > swe::VOL_CHAIN_CHUNKS;
+  if (runs) {
     if (!s->d_vol) CU(cudaMalloc(&s->d_vol, sizeof(swe::VolChunk) * chunks));
     swe::k_volume_sums<<<chunks, swe::CHAIN_THREADS, 0, s->st>>>(a, s->d_vol, chunks, s->d_ctl);
     swe::k_volume_runs<<<chunks, swe::CHAIN_THREADS, 0, s->st>>>(a, s->d_vol);
   }
-  swe::k_volume_walk<<<1, swe::CHAIN_THREADS, 0, s->st>>>(a, chunks > 2 ? s->d_vol : nullptr, chunks, s->dx, s->dy,
+  swe::k_volume_walk<<<1, swe::CHAIN_THREADS, 0, s->st>>>(a, runs ? s->d_vol : nullptr, chunks, s->dx, s->dy,
                                                           s->d_ctl);
   CU(cudaGetLastError());
   return finish_diag(s, out);
