@@ -208,3 +208,117 @@ def test_a_single_limited_cell_next_to_a_tile(swe, monkeypatch, nx, ny, side):
 
     for x, y in zip(run("fused"), run("split")):
         assert np.array_equal(x, y)
+
+
+def _bits(sim):
+    import numpy as np
+    return [sim.field(f).view(np.uint64).copy() for f in ("b", "h", "hu", "hv")], (sim.t, sim.massFloored)
+
+
+def _fused_and_split(monkeypatch, scenario):
+    import numpy as np
+    out = {}
+    for impl in ("fused", "split"):
+        monkeypatch.setenv("SWE_B200_STAGE", impl)
+        out[impl] = scenario()
+    for a, b in zip(out["fused"], out["split"]):
+        for x, y in zip(a[0], b[0]):
+            assert np.array_equal(x, y)
+        assert a[1] == b[1]
+
+
+@pytest.mark.parametrize("sides", ["walls", "mixed"])
+@pytest.mark.parametrize("nx,ny", [(604, 244), (604, 252), (801, 503), (1180, 1020), (1180, 1028)])
+def test_wet_grids_of_several_waves_give_the_fused_kernels_bits(swe, monkeypatch, nx, ny, sides):
+    """589, 608, 1664, 4736 and 4773 tiles: on the second to the fourth the face
+    kernel fills the ghosts and prepares the step, once a run of 128 steps or
+    more has found that few tiles settle; the first never settles, the last is
+    too large.  Then runs with a fixed dt, to a given time, past it (refused
+    steps) and single steps, which settle again."""
+    import numpy as np
+    from water_simulator_b200 import workloads
+
+    X, Y = np.meshgrid(np.arange(nx + 4) / 40.0, np.arange(ny + 4) / 30.0)
+    b = 0.4 * np.sin(X) * np.cos(Y) + workloads.uniform_noise(3, X.shape, -0.1, 0.1)
+    b[ny // 2:ny // 2 + 20, 40:90] = 3.0              # an island
+
+    def scenario():
+        sim = swe.ShallowWater(nx=nx, ny=ny, dx=5.0, bed=b, eta0=np.where(X < 5, 2.4, 2.0))
+        if sides == "mixed":
+            sim.boundaries = {"west": swe.flather(swe.Tide({"M2": [0.4, 30.0]}, msl=2.1).signal()), "east": swe.outflow,
+                              "south": swe.periodic, "north": swe.periodic}
+        assert sim.run(133) == 133
+        out = [_bits(sim)]
+        assert sim.run(5, dt=0.2) == 5
+        done = sim.run(40, tEnd=sim.t + 1.0)
+        assert 0 < done < 40 and sim.run(3, tEnd=sim.t) == 0
+        out.append(_bits(sim))
+        for _ in range(2):
+            sim.step()
+        sim.step(0.1)
+        assert sim.run(9) == 9
+        out.append(_bits(sim))
+        sim.close()
+        return out
+
+    _fused_and_split(monkeypatch, scenario)
+
+
+@pytest.mark.parametrize("case", ["beach", "sphere", "beach_sponge", "host_writes"])
+def test_settling_grids_of_several_waves_give_the_fused_kernels_bits(swe, monkeypatch, case):
+    """Grids of more than 592 tiles, which alone settle: a flooding beach, a
+    sphere with land, a sponge that pours water onto dry tiles, and a state that
+    the host, dryClean, friction and the fused kernels write in between."""
+    import numpy as np
+    from water_simulator_b200 import workloads
+    lib = swe.load_library()
+
+    def beach():
+        b, h = workloads.beach_dam_break(nx=640, ny=320, dx=8.0 * 256 / 640)
+        sim = swe.ShallowWater(nx=640, ny=320, dx=8.0 * 256 / 640, bed=b, eta0=b + h, manning=0.03)
+        sim.boundaries = {"west": swe.flather(swe.Tide({}, msl=0.0).signal())}
+        return sim, b
+
+    def scenario():
+        if case == "sphere":
+            c = workloads.globe_tide(nx=720, ny=360, lat0=-80.0, lat1=80.0, modes=12)
+            sim = swe.ShallowWater(nx=720, ny=360, bed=c["b"], eta0=c["eta0"] + (c["b"] < 0) * 0.5,
+                                   sphere={"R": 6371e3, "lat0": -80.0, "lat1": 80.0, "omega": 7.2921e-5})
+            assert sim.run(150) == 150
+            out = [_bits(sim)]
+            sim.close()
+            return out
+        sim, b = beach()
+        if case == "beach_sponge":
+            sim.forcing = swe.makeSponge(sim, side="east", width=60, strength=0.05, etaRef=float(np.max(b)) + 0.5)
+        assert sim.run(150) == 150
+        out = [_bits(sim)]
+        if case == "host_writes":
+            hh = np.array(sim.field("h")).reshape(sim.H, sim.W)
+            assert (hh[100:220, 400:600] == 0).all()      # dry land, tiles deep inside it
+            hh[140:180, 430:560] += 0.7                   # a pond poured onto it
+            sim.h = hh.reshape(-1)
+            assert sim.run(30) == 30
+            out.append(_bits(sim))
+            sim.dryClean()
+            assert sim.run(10) == 10
+            sim.applyFriction(sim.maxDt())
+            assert sim.run(10) == 10
+            mine = 0 if monkeypatch_impl() == "fused" else 1
+            swe._lib.check(lib.swe_set_stage_kernels(sim._h, 1 - mine))
+            assert sim.run(5) == 5
+            swe._lib.check(lib.swe_set_stage_kernels(sim._h, mine))
+            assert sim.run(25) == 25
+        for _ in range(4):
+            sim.step()
+            sim.maxSurfaceDeviation(1e7)                  # its partials are not the stages'
+        assert sim.run(33) == 33
+        out.append(_bits(sim))
+        sim.close()
+        return out
+
+    def monkeypatch_impl():
+        import os
+        return os.environ["SWE_B200_STAGE"]
+
+    _fused_and_split(monkeypatch, scenario)
