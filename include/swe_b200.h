@@ -280,7 +280,7 @@ int swe_batch_run(swe_batch* s, int steps);
 int swe_batch_synchronize(swe_batch* s);
 /* The launch form of an ensemble step with the tiled pair (rows 0).
  * 0: a launch per phase (prepare, ghost fill, faces, cells, ghost fill,
- * faces, cells).  1: ONE persistent launch per step over a device work
+ * faces, cells, close).  1: ONE persistent launch per step over a device work
  * queue of every (basin, phase, tile) item in phase order; a CTA takes the
  * next item and waits, with a time limit, until the previous phase of that
  * item's basin is complete.  A wait past its limit drops the rest of the

@@ -874,7 +874,7 @@ int fwd_step(swe_adjoint* s, int k) {
   const int n = (int)(s->sgrid.x * s->sgrid.y);
   if (n <= swe::CLOSE_TILES) LAUNCH(swe::k_split_close_step, dim3(1), dim3(32 * swe::CLOSE_BLOCKS), a2, s->ctl, n);
   else
-    LAUNCH(swe::k_split_close_multi<2>, dim3(swe::CLOSE_BLOCKS), dim3(swe::SP_THREADS), a2, s->ctl, n,
+    LAUNCH(swe::k_split_close_multi, dim3(swe::CLOSE_BLOCKS), dim3(swe::SP_THREADS), a2, s->ctl, n,
            s->part + 3 * (size_t)s->pcap);
   return SWE_OK;
 }

@@ -388,7 +388,11 @@ int ensure_split(swe_sim* s, double* mem = nullptr) {
 int tiles_of(const swe_sim* s) { return (int)(s->sgrid.x * s->sgrid.y); }
 // A grid whose tiles all run at once (4 CTAs per SM of 148) is bound by the
 // latency of a step's kernels, not by their work: it keeps no records of dry
-// tiles and makes no lists, whose flags only delay its tiles.
+// tiles and makes no lists, whose flags only delay its tiles, mostly dry or not.  A
+// step of a run of 128 with the records and so, by the wet share of the grid:
+//                        2%          15%         50%         all
+//   256 x 256         45.0 33.0   46.7 32.5   38.1 33.8   37.5 33.0 us
+//   604 x 244         42.8 33.8   46.9 35.3   50.6 38.8   40.3 37.5
 bool one_wave(const swe_sim* s) { return tiles_of(s) <= 4 * 148; }
 bool settles(const swe_sim* s) { return s->settle && !one_wave(s); }
 
@@ -490,7 +494,7 @@ int launch_close(swe_sim* s, const swe::StageArgs& a, bool pdl) {
   if (n <= swe::CLOSE_TILES)
     CU(launch(pdl, swe::k_split_close_step, dim3(1), dim3(32 * swe::CLOSE_BLOCKS), s->st, a, s->d_ctl, n));
   else
-    CU(launch(pdl, swe::k_split_close_multi<2>, dim3(swe::CLOSE_BLOCKS), dim3(swe::SP_THREADS), s->st, a, s->d_ctl, n,
+    CU(launch(pdl, swe::k_split_close_multi, dim3(swe::CLOSE_BLOCKS), dim3(swe::SP_THREADS), s->st, a, s->d_ctl, n,
               s->d_part + 3 * (size_t)s->part_cap));
   return SWE_OK;
 }
@@ -524,10 +528,15 @@ int launch_bc_lists(swe_sim* s, double* const* f, int respect_stop, bool pdl, co
 }
 
 // Most tiles of a grid whose face kernels fill the ghosts and prepare the step
-// (8 waves).  128 steps with the fill in the face kernel against launches of its
-// own: 400 x 330 5.97 -> 5.42 ms, 512 x 512 9.27 -> 9.00, 1020 x 512 15.05 -> 14.85,
-// the sphere 1440 x 720 with its tides 31.0 -> 30.3, 1024 x 1024 30.62 -> 30.76,
-// 2048 x 2048 104.4 -> 106.1 (the fill costs every tile registers).
+// (8 waves).  A step of a run of 128 with launches of their own for both, and so:
+//   604 x 252    (608 tiles)  49.9  47.8 us    two sides with tides  52.4  50.2
+//   1020 x 512   (2 080)     108.8 106.7                            113.1 110.9
+//   900 x 900    (3 277)     173.9 172.5                            178.3 176.7
+//   1024 x 1024  (4 257)     217.2 216.3                            221.2 221.5
+//   1180 x 1020  (4 736)     241.8 240.5                            245.9 245.0
+//   1440 x 720 sphere        212.9 209.8
+// From there on the fill costs every tile registers for a share of the step that
+// shrinks: 2048 x 2048, 128 steps: 104.4 -> 106.1 ms.
 constexpr int FILL_TILES = 8 * 4 * 148;
 
 // One SSP-RK2 step on the device; `mode`/`dt`/`t_end` as k_prepare.  The

@@ -2,16 +2,16 @@
 //
 // Each basin is a complete ShallowWater (its own grid, bed, metric, Manning
 // n, boundaries and Flather tide) with its own dt = maxDt() every step.  One
-// ensemble step is a fixed number of launches whatever the number of basins;
-// with the fused stage kernels five:
-//   k_batch_prepare     dt and Flather values of every basin (one thread each)
-//   k_batch_bc(A)       ghost rings of every basin (grid y = basin)
-//   k_batch_stage<1>    every tile of every basin, from one tile list
-//   k_batch_bc(B)
-//   k_batch_stage<2>    ... the last tile of each basin closes that basin's step
-// with the tiled pair k_batch_split_faces and k_batch_split_cells for each stage
-// and k_batch_close (a block per basin) after the second.  A run of steps is
-// captured as a CUDA graph.  The stage kernels run the same tile functions as
+// ensemble step is eight launches whatever the number of basins:
+//   k_batch_prepare         dt and Flather values of every basin (one thread each)
+//   k_batch_bc(A)           ghost rings of every basin (grid y = basin)
+//   k_batch_split_faces<1>  every tile of every basin, from one tile list,
+//   k_batch_split_cells<1>  and the same again
+//   k_batch_bc(B), k_batch_split_faces<2>, k_batch_split_cells<2>
+//   k_batch_close           a block per basin closes that basin's step
+// With the fused stage kernels (k_batch_stage<1> and <2>, whose last tile of each
+// basin closes its step) it is five, and over the work queue one.  A run of steps
+// is captured as a CUDA graph.  The stage kernels run the same tile functions as
 // the single-grid kernels, so each basin's result is bit-identical to advancing
 // it alone.  The tile list's row height, the
 // number of CTAs (one per tile, or a persistent grid looping over the list)

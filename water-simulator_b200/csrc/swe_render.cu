@@ -143,7 +143,7 @@ void build_tables(Tables* t) {
 bool aligned4(const void* p) { return (reinterpret_cast<size_t>(p) & 3) == 0; }
 
 int ensure_tables() {
-  static int done = -1;                        // per process; the constant banks are per device
+  static int done = -1;                        // per process; the tables are a copy per device
   static int done_dev = -1;
   int dev = 0;
   RCU(cudaGetDevice(&dev));

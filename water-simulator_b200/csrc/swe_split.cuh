@@ -1401,20 +1401,16 @@ k_split_cells(StageArgs a, SplitBufs s, Control* ctl) {
                          gridDim.x * gridDim.y, sm, false);
 }
 
-// The close of a stage over CLOSE_BLOCKS blocks: block b reduces its run of
-// the tiles' partial slots (strided per thread, then a fixed tree) into
-// scratch, and the last block to finish (a ticket among the CLOSE_BLOCKS)
-// combines the blocks' results in block order (a fixed tree in one warp)
-// and closes the stage as split_close_block does.  The maximum is the same
-// in any order; the floored mass is summed in this fixed order.  One block
+// The close of a step over CLOSE_BLOCKS blocks: block b reduces its run of
+// the tiles' partial slots, of both stages (strided per thread, then a fixed
+// tree), into scratch, and the last block to finish (a ticket among the
+// CLOSE_BLOCKS) combines the blocks' results in block order (a fixed tree in one
+// warp) and closes the step as split_close_block does.  The maximum is the same
+// in any order; the floored masses are summed in this fixed order.  One block
 // reading 16 705 slots spent most of its time in dependent rounds of L2
-// loads.  MODE 2 closes the whole step: stage 1's floored mass is needed
-// only there, so it is summed here too (the same order as MODE 1 sums it)
-// and stage 1 needs no close of its own.  scratch holds 3 * CLOSE_BLOCKS
-// doubles.
-template <int MODE>
+// loads.  scratch holds 3 * CLOSE_BLOCKS doubles.
 __global__ void __launch_bounds__(SP_THREADS) k_split_close_multi(StageArgs a, Control* ctl, int nparts,
-                                                                    double* scratch) {
+                                                                  double* scratch) {
   pdl_enter();
   if (ctl->stop) return;
   __shared__ double red[3][SP_THREADS / 32];
@@ -1422,14 +1418,11 @@ __global__ void __launch_bounds__(SP_THREADS) k_split_close_multi(StageArgs a, C
   const int t = threadIdx.x, b = blockIdx.x;
   const int chunk = (nparts + CLOSE_BLOCKS - 1) / CLOSE_BLOCKS;
   const int q0 = b * chunk, q1 = min(nparts, q0 + chunk);
-  const double* pf = MODE == 1 ? a.part_fl1 : a.part_fl2;
   double m = 0, f = 0, f1 = 0;
   for (int q = q0 + t; q < q1; q += SP_THREADS) {
-    if (MODE == 2) {
-      m = fmax(m, __ldcg(a.part_max + q));
-      f1 += __ldcg(a.part_fl1 + q);
-    }
-    f += __ldcg(pf + q);
+    m = fmax(m, __ldcg(a.part_max + q));
+    f1 += __ldcg(a.part_fl1 + q);
+    f += __ldcg(a.part_fl2 + q);
   }
   for (int o = 16; o > 0; o >>= 1) {
     m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
@@ -1460,16 +1453,11 @@ __global__ void __launch_bounds__(SP_THREADS) k_split_close_multi(StageArgs a, C
     f1 += __shfl_down_sync(0xffffffffu, f1, o);
   }
   if (t == 0) {
-    const double dt = ctl->dt;
-    if (MODE == 1) {
-      ctl->floored1 = f;
-    } else {
-      ctl->floored1 = f1;
-      ctl->next_max = m;
-      ctl->mass_floored = f1 + f;
-      ctl->t = ctl->t + dt;
-      ctl->steps = ctl->steps + 1;
-    }
+    ctl->floored1 = f1;
+    ctl->next_max = m;
+    ctl->mass_floored = f1 + f;
+    ctl->t = ctl->t + ctl->dt;
+    ctl->steps = ctl->steps + 1;
     ctl->counter = 0;
   }
 }
@@ -1564,16 +1552,6 @@ k_split_cells_tma_list(StageArgs a, SplitBufs s, Control* ctl, const __grid_cons
     }
     __syncthreads();
   } while (walk.at < min(*count, ntiles));
-}
-
-// Closes the stage k_split_cells left open: one block, no atomics (a
-// ticket shared by every tile of a large grid serialises in L2).
-template <int MODE>
-__global__ void __launch_bounds__(SP_THREADS) k_split_close(StageArgs a, Control* ctl, int nparts) {
-  pdl_enter();
-  if (ctl->stop) return;
-  __shared__ CellsSmem sm;
-  split_close_block<MODE>(a, ctl, nparts, sm);
 }
 
 }  // namespace
