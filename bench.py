@@ -519,7 +519,7 @@ def run_ours(args):
     sim.synchronize()
     res_value = NX * NY * res_steps / (time.perf_counter() - t0)
 
-    n_launches = launches_per_step(swe, lib, sim) * K
+    n_launches = launches(swe, lib, sim, K, settles=True)
     lcfg = launch_cfg(swe, lib, sim)
     sim.close()
     cpu = None
@@ -592,16 +592,24 @@ def fma_build_summary(steps, warmup):
     return out
 
 
-def launches_per_step(swe, lib, sim):
-    """Kernel launches of one step: prepare, two ghost fills and two stages
-    of the stage kernels in use (the tiled pair per stage and one close of
-    the step, or the fused kernel per stage)."""
+def launches(swe, lib, sim, K, settles):
+    """Kernel launches of a run of K steps.  The fused kernels: prepare and,
+    for each stage, a ghost fill and the stage.  The tiled pair: prepare, for
+    each stage a ghost fill (with the tile lists in the same launch), faces and
+    cells, and one close.  On grids of at most 4736 tiles the face kernels fill
+    and prepare, which leaves five: at once on grids of at most 592, and where
+    little settles after the first 32 steps of a run of 128 or more."""
     impl = ctypes.c_int(-1)
     swe._lib.check(lib.swe_get_stage_kernels(sim._h, ctypes.byref(impl)))
-    # the tiled pair per stage and one close; with tile lists each ghost fill
-    # makes the next stage's lists in the same launch.  (Grids of at most 4736
-    # tiles prepare and fill in the face kernels: five launches; none is timed here.)
-    return 3 + (5 if impl.value == 1 else 2)
+    if impl.value != 1:
+        return 5 * K
+    cfg = launch_cfg(swe, lib, sim)
+    tiles = cfg[0] * cfg[1]
+    if tiles <= 592:
+        return 5 * K
+    if tiles > 4736 or settles or K < 128:
+        return 8 * K
+    return 8 * 32 + 5 * (K - 32)
 
 
 def launch_cfg(swe, lib, sim):
@@ -832,7 +840,7 @@ def run_sphere(args):
     value = nx * ny * K / (ms / 1e3)
     dt_last = sim.maxDt()
     finite = sim.finite()
-    per_step = launches_per_step(swe, lib, sim)
+    n_launches = launches(swe, lib, sim, K, settles=False)
     sim.close()
     cpu = None
     if not args.no_cpu_baseline:
@@ -857,7 +865,7 @@ def run_sphere(args):
                                    "the S and N cap edges, Coriolis omega 7.2921e-5, Manning 0.025, dt = maxDt()",
                        "cells": nx * ny, "l2": "state 3 x 8.4 MB per copy: fits L2; steady-state stream"},
             "first_steps_vs_oracle": {"steps": chk, "bit_exact": exact, "max_rel_err": rel}, "finite": finite, "dt_last": dt_last,
-            "gpu_launches": per_step * K, "clocks": clocks, "cpu_baseline": cpu}
+            "gpu_launches": n_launches, "clocks": clocks, "cpu_baseline": cpu}
     print(json.dumps(line))
     return 0
 
